@@ -22,18 +22,9 @@
 #include <cstring>
 #include <vector>
 #include <type_traits>
-#include <cuda_bf16.h>
-#include "ua_amg.h"
+#include "ua_amg_int.h"
 
 namespace ua {
-
-constexpr int kAmgCoarseNodes = 48;   // a system stops coarsening at this many nodes
-constexpr int kAmgMaxRow = 32;        // longest coarse dof row (2 x coarse node degree)
-constexpr int kSaMaxDeg = 256;        // largest coarse node degree of a smoothed hierarchy (shared-memory rows)
-constexpr int kAmgMaxDense = 2 * kAmgCoarseNodes;
-constexpr int kAmgRB = 256;           // rows per row block of a coarse level
-constexpr int kSaRB = 128, kSaLPR = 2;
-constexpr int kAmgNB = 32;            // nodes per node block of the smoothed transfers (one warp's worth)  // smoothed hierarchies (longer coarse rows): rows per block, lanes per row
 
 // Calls f(std::integral_constant<int, LPR>) for the lanes-per-row value lpr (1, 2, 4, 8, 16 or 32).
 template <class F>
@@ -47,122 +38,6 @@ static void dispatch_lpr(int lpr, F&& f) {
     default: f(std::integral_constant<int, 8>());
   }
 }
-
-struct AmgLevel {
-  int nn = 0, ndof = 0;
-  long long nnz = 0;
-  int ap_maxrow = 0;  // longest A P row (coarse columns) of the level
-  int ac_maxdeg = 0;  // largest node degree of the next (coarse) level
-  std::vector<int> node_off, dof_off, knz_off, nnzn;  // per system (0-sized when the system has no such level)
-  // dof-level CSR of a coarse level, same layout rule as the finest level
-  int *rowptr = nullptr, *colind = nullptr;
-  int* dof_sys = nullptr;
-  int* d_dof_off = nullptr;               // per-system dof offsets on the device
-  int* d_knz_off = nullptr;               // per-system non-zero offsets (uvh finest level)
-  int *rb_start = nullptr, *rb_sys = nullptr;
-  int nrb = 0;
-  int* cmap = nullptr;                    // this level's dof -> next level's dof
-  int *mptr = nullptr, *mlist = nullptr;  // per dof of this (coarse) level: member dofs of the finer level
-  void* A = nullptr;                      // coarse values (KT)
-  void* invd = nullptr;                   // l1-Jacobi inverse row sums (VT)
-  void *b = nullptr, *x = nullptr, *x2 = nullptr;  // rhs, pre-smoothed, post-smoothed (VT)
-  int* d_node_off = nullptr;              // per-system node offsets on the device
-  int* node_sys = nullptr;                // node -> system (smoothed hierarchies)
-  std::vector<int> h_sys_rb_off;          // per-system prefix of the row blocks
-  // node blocks (kAmgNB nodes, never straddling two systems) for the smoothed transfers
-  int *nb_start = nullptr, *nb_sys = nullptr;
-  int nnb = 0;
-  std::vector<int> h_sys_nb_off;
-  // smoothed aggregation, transfer from this level to the next (node-level lists, global ids):
-  // pn: fine node -> coarse nodes of its neighbours' aggregates (the prolongator's node pattern);
-  // apn: fine node -> coarse nodes of A P; ptn: coarse node -> (fine node, position in pn)
-  int *sa_agg = nullptr, *pn_ptr = nullptr, *pn_col = nullptr, *apn_ptr = nullptr, *apn_col = nullptr;
-  int *ptn_ptr = nullptr, *ptn_fine = nullptr, *ptn_k = nullptr;
-  int *pbase = nullptr, *pnnz = nullptr, *poff = nullptr, *apbase = nullptr, *apnnz = nullptr, *apoff = nullptr;
-  double *sa_p = nullptr, *sa_ap = nullptr;  // set-up values (FP64 form): 4 per node-level entry
-  float* sa_plo = nullptr;                   // set-up values of P (mixed form)
-  // P in the transfer layout, one quad per node-level entry: pn order (sa_q*) and ptn order
-  // (sa_qt*); BF16 quads for the mixed form, FP64 quads for the FP64 form (allocated on first use)
-  long long np = 0;  // node-level prolongator entries of the level (all systems)
-  void *sa_qh = nullptr, *sa_qth = nullptr, *sa_qd = nullptr, *sa_qtd = nullptr;
-};
-
-// one active-block list to compact: blocks blk_off[s] .. blk_off[s+1] of every system s with
-// sel, !done and depth > lmin, in ascending order
-struct ActSpec {
-  const int* blk_off;
-  int lmin;
-  int* map;
-  int* cnt;
-};
-
-// Finest-level node slices of a uv handle (sliced ELL over nodes).  A slice block is the set of
-// nodes of one u-row block of the handle's Krylov rows (at most kSellNodes nodes of one system);
-// inside it the nodes are ordered by decreasing degree and cut into slices of 32, one warp each.
-// Slice j holds width W_j = its largest degree; its slots are 32 * W_j, entry k of lane t at slot
-// off_j + 32 k + t.  Per slot: the u column (global u dof of the k-th neighbour; v column = u column
-// + the system's node count) and four values (blocks uu, uv, vu, vv at value offsets
-// 4 off_j + b 32 W_j + 32 k + t).  Padding slots hold zeros and the node's own column.  One column
-// index then serves four values, and a warp's loads of one k are contiguous.
-constexpr int kSellNodes = 256;  // nodes per slice block (= rows per row block)
-constexpr int kSellSlices = kSellNodes / 32;
-
-struct Sell {
-  bool ready = false, failed = false;
-  int nsb = 0;
-  long long slots = 0;
-  std::vector<int> h_sys_sb_off;  // per-system prefix of the slice blocks
-  int *sb_sys = nullptr, *sb_n0 = nullptr, *sb_cnt = nullptr, *sb_rbu = nullptr, *sb_rbv = nullptr;
-  int* perm = nullptr;             // [nn_total]: per block, its global node ids in slice order
-  long long* sl_off = nullptr;     // [nsb * kSellSlices + 1] slot offsets of the slices
-  int* cols = nullptr;             // [slots]
-  float* v32 = nullptr;            // [4 slots] FP32 values (mixed-precision PCG operator)
-  double* v64 = nullptr;           // [4 slots] FP64 values
-  __nv_bfloat16* vlo = nullptr;    // [4 slots] BF16 values (mixed-precision V-cycle)
-  double* spart = nullptr;         // [nsb * kSellSlices] per-slice partials (p.q, r.z)
-  int* sys_sl_off = nullptr;       // [nsys + 1] per-system slice prefix
-  ActList act;                     // slice blocks of the systems still iterating
-};
-
-struct Amg {
-  int nsys = 0, nlev = 0, maxdn = 0;
-  Sell sell;
-  // node slices of the coarse levels 1 .. nlev-2 (smoothed hierarchies): BF16 copies of the
-  // coarse operators for the mixed-precision V-cycle's residual and smoothing there
-  std::vector<Sell> csell;
-  // active-block lists: rows[l] (level-l row blocks, depth > l; level 0 = the handle's blocks),
-  // fnodes[l] (level-l node blocks, depth > l), cnodes[l] (level-(l+1) node blocks, depth > l)
-  bool act_ready = false;
-  int nsm = 148;
-  std::vector<ActList> rows, fnodes, cnodes;
-  ActSpec* d_specs = nullptr;
-  int nspecs = 0;
-  bool sa = false;            // smoothed aggregation (else plain)
-  std::vector<AmgLevel> lev;  // lev[0] = the handle's own system
-  std::vector<int> depth;     // per system: its coarsest level (>= 1)
-  std::vector<int> h_dn, h_doff;
-  int *d_depth = nullptr, *d_dn = nullptr, *d_doff = nullptr;
-  double* dense = nullptr;    // per system dn x dn inverse (row-major)
-  void **d_lev_b = nullptr, **d_lev_x2 = nullptr, **d_lev_A = nullptr;
-  int **d_lev_rowptr = nullptr, **d_lev_colind = nullptr, **d_lev_dofoff = nullptr;
-  size_t bytes = 0;
-  __nv_bfloat16* k0lo = nullptr;  // mixed precision: BF16 copy of the finest-level tangent
-  // uvh handles: constraint mask and vectors of the velocity rows (2-dof layout)
-  unsigned char* uvh_mask = nullptr;
-  double *uvh_r = nullptr, *uvh_x0 = nullptr, *uvh_z = nullptr, *uvh_t = nullptr;
-  // per system: numeric set-ups since its solve started (prolongator refresh), and the systems
-  // whose prolongators the current set-up recomputes
-  std::vector<int> p_age, h_prefresh;
-  int* d_prefresh = nullptr;
-  // the numeric set-up of a Newton step captured as one CUDA graph per (precision, selection
-  // kind) and replayed: every argument is a fixed device buffer of the handle
-  cudaGraphExec_t setup_exec[8] = {};
-  long long setup_nodes[8] = {};
-  ~Amg() {
-    for (auto& e : setup_exec)
-      if (e) cudaGraphExecDestroy(e);
-  }
-};
 
 // ---------------------------------------------------------------------------
 // host: aggregation and hierarchy
@@ -198,20 +73,55 @@ static int aggregate(int n, const std::vector<int>& ptr, const std::vector<int>&
   return na;
 }
 
-template <class T>
-static T* upload(ua_mesh* m, Amg* a, const std::vector<T>& v, bool& ok) {
-  T* d = (T*)dev_alloc(m, std::max<size_t>(1, v.size()) * sizeof(T));
-  if (!d) { ok = false; return nullptr; }
-  if (!v.empty() && cudaMemcpy(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) ok = false;
-  a->bytes += v.size() * sizeof(T);
-  return d;
-}
-
-static void* dalloc(ua_mesh* m, Amg* a, size_t bytes, bool& ok) {
-  void* d = dev_alloc(m, std::max<size_t>(bytes, 16));
-  if (!d) ok = false;
-  a->bytes += bytes;
-  return d;
+// Linear interpolation of a six-node system from its corner nodes: per node its corners (ascending
+// corner ids) and weights, 1 at a corner and 1/2 at the two ends of a mid node's edge.  Corner ids
+// follow the node order.  Returns the number of corners, or 0 where the mesh does not allow it (a
+// node that is a corner of one element and a mid node of another, or in no element).
+//
+// A quadratic mesh is coarsened this way once, before the aggregation: the velocity tangent's
+// smooth errors are linear over an element, so the interpolation needs no smoothing, the next
+// operator keeps the sparsity of a linear mesh (about 7 nodes per row, where aggregating the
+// quadratic graph gave 22) and the coarsening ratio is 4 instead of 16.  PCG iterations of one
+// Newton system (relative 1e-6): 101 x 51 vertices 108 -> 39.
+static int linear_corners(const HostSystem& hs, std::vector<int>& ptr, std::vector<int>& col,
+                          std::vector<double>& wgt) {
+  const int n = hs.nn, ne = hs.ne;
+  std::vector<int> c0(n, -1), c1(n, -1);  // a mid node's edge ends; c0 = the node itself at a corner
+  for (int e = 0; e < ne; ++e)
+    for (int k = 0; k < 6; k += 2) {
+      const int a = hs.conn[(size_t)k * ne + e], m = hs.conn[(size_t)(k + 1) * ne + e];
+      const int b = hs.conn[(size_t)((k + 2) % 6) * ne + e];
+      if ((c0[a] >= 0 && c0[a] != a) || a == b || a == m || m == b) return 0;
+      c0[a] = a;
+      const int lo = std::min(a, b), hi = std::max(a, b);
+      if (c0[m] >= 0 && (c0[m] != lo || c1[m] != hi)) return 0;
+      c0[m] = lo;
+      c1[m] = hi;
+    }
+  std::vector<int> id(n, -1);
+  int nc = 0;
+  for (int i = 0; i < n; ++i) {
+    if (c0[i] < 0) return 0;
+    if (c1[i] < 0) id[i] = nc++;
+  }
+  ptr.assign(1, 0);
+  ptr.reserve(n + 1);
+  col.clear();
+  wgt.clear();
+  for (int i = 0; i < n; ++i) {
+    if (c1[i] < 0) {
+      col.push_back(id[i]);
+      wgt.push_back(1.0);
+    } else {
+      if (id[c0[i]] < 0 || id[c1[i]] < 0) return 0;  // an edge end that is a mid node elsewhere
+      col.push_back(id[c0[i]]);
+      col.push_back(id[c1[i]]);
+      wgt.push_back(0.5);
+      wgt.push_back(0.5);
+    }
+    ptr.push_back((int)col.size());
+  }
+  return nc;
 }
 
 // Dof-level CSR of a level from its node graph (global ids of the level):
@@ -261,7 +171,16 @@ static int amg_build(ua_mesh* m, bool smoothed) {
   std::vector<std::vector<int>> g_off{m->h_node_off}, g_ptr{m->h_nodeptr}, g_col{m->h_nodecol}, g_agg;
   // smoothed aggregation lists per transfer (index = fine level)
   std::vector<std::vector<int>> g_pnp, g_pnc, g_apnp, g_apnc, g_ptnp, g_ptnf, g_ptnk;
+  std::vector<double> pn_w;  // weights of the finest level's linear interpolation (else empty)
   a->sa = smoothed;
+  // quadratic meshes: the first transfer interpolates linearly from the corner nodes, for every
+  // system of the handle or for none
+  std::vector<std::vector<int>> lin_ptr(nsys), lin_col(nsys);
+  std::vector<std::vector<double>> lin_w(nsys);
+  std::vector<int> lin_n(nsys, 0);
+  bool linear0 = smoothed && m->nod == 6;
+  for (int s = 0; s < nsys && linear0; ++s)
+    linear0 = (lin_n[s] = linear_corners(m->sys[s], lin_ptr[s], lin_col[s], lin_w[s])) > 0;
   std::vector<char> live(nsys, 1);
   auto fail = [&](const char* why) {
     delete a;
@@ -285,7 +204,15 @@ static int amg_build(ua_mesh* m, bool smoothed) {
         for (int k = fp[no[s] + i]; k < fp[no[s] + i + 1]; ++k) lc.push_back(fc[k] - no[s]);
         lp[i + 1] = (int)lc.size();
       }
-      const int na = aggregate(n, lp, lc, la);
+      const bool lin = linear0 && g_agg.empty();
+      int na;
+      if (lin) {
+        na = lin_n[s];
+        la.resize(n);
+        for (int i = 0; i < n; ++i) la[i] = lin_col[s][lin_ptr[s][i]];
+      } else {
+        na = aggregate(n, lp, lc, la);
+      }
       for (int i = 0; i < n; ++i) agg[no[s] + i] = cno[s] + la[i];
       cno[s + 1] = cno[s] + na;
       std::vector<std::vector<int>> adj(na);
@@ -295,7 +222,12 @@ static int amg_build(ua_mesh* m, bool smoothed) {
       } else {
         // prolongator pattern: node i reaches the aggregates of its neighbours (P = (I - w D^-1 A) P0)
         std::vector<int> lpn(n + 1, 0), lpc, stamp(na, -1);
-        for (int i = 0; i < n; ++i) {
+        if (lin) {
+          lpn = lin_ptr[s];
+          lpc = lin_col[s];
+          pn_w.insert(pn_w.end(), lin_w[s].begin(), lin_w[s].end());
+        }
+        for (int i = 0; i < n && !lin; ++i) {
           const size_t b0 = lpc.size();
           for (int k = lp[i]; k < lp[i + 1]; ++k) {
             const int J = la[lc[k]];
@@ -481,6 +413,7 @@ static int amg_build(ua_mesh* m, bool smoothed) {
       AmgLevel& F = a->lev[l];
       const AmgLevel& C = a->lev[l + 1];
       F.sa_agg = upload(m, a, g_agg[l], ok);
+      if (l == 0 && linear0) F.pn_w = upload(m, a, pn_w, ok);
       F.pn_ptr = upload(m, a, g_pnp[l], ok);
       F.pn_col = upload(m, a, g_pnc[l], ok);
       F.apn_ptr = upload(m, a, g_apnp[l], ok);
@@ -584,7 +517,7 @@ __global__ void k_amg_galerkin(int ncd, const int* mptr, const int* mlist, const
   for (int k = 0; k < len; ++k) cA[c0 + k] = (KT)acc[k];
 }
 
-// l1-Jacobi: invd_i = 1 / sum_j |a_ij| over unmasked columns (0 on masked or empty rows)
+// Damped l1-Jacobi: invd_i = kSmoothOmega / sum_j |a_ij| over unmasked columns (0 on masked or empty rows)
 template <typename KT, typename VT>
 __global__ void k_amg_l1(int n, const int* rowptr, const int* colind, const KT* A, const unsigned char* cmask,
                          VT* invd, const int* dof_sys, const int* sel) {
@@ -595,7 +528,7 @@ __global__ void k_amg_l1(int n, const int* rowptr, const int* colind, const KT* 
   if (!(cmask && cmask[i]))
     for (int q = rowptr[i]; q < rowptr[i + 1]; ++q)
       if (!(cmask && cmask[colind[q]])) s += fabs((double)A[q]);
-  invd[i] = (VT)(s > 0 ? 1.0 / s : 0.0);
+  invd[i] = (VT)(s > 0 ? kSmoothOmega / s : 0.0);
 }
 
 // Inverse of each system's coarsest matrix: Gauss-Jordan on [A | I] in
@@ -708,10 +641,6 @@ __device__ __forceinline__ double row_dot_uv(const int* rowptr, const int* colin
   for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, LPR);
   return acc;
 }
-
-__device__ __forceinline__ double to_d(double v) { return v; }
-__device__ __forceinline__ double to_d(float v) { return (double)v; }
-__device__ __forceinline__ double to_d(__nv_bfloat16 v) { return (double)__bfloat162float(v); }
 
 // Plain CSR row product (every index read); the form that is faster for FP32 and BF16 values.
 template <typename KT, typename XT, int LPR>
@@ -845,30 +774,6 @@ struct SellDev {
   const int *dof_off, *node_off;  // per system, of the slices' level
   unsigned long long* dbg;        // first bounds violation (debug build)
   int lev;                        // the level (residual and smoothing: systems deeper than it)
-};
-
-// The four values of a slot (blocks uu, uv, vu, vv) are adjacent, so a lane reads them with one
-// vector load: 8 bytes (BF16), 16 (FP32) or 32 (FP64, two loads).
-template <typename KT> struct Quad;
-template <> struct Quad<float> {
-  static __device__ __forceinline__ void get(const float* p, double (&e)[4]) {
-    const float4 q = __ldg(reinterpret_cast<const float4*>(p));
-    e[0] = q.x; e[1] = q.y; e[2] = q.z; e[3] = q.w;
-  }
-};
-template <> struct Quad<double> {
-  static __device__ __forceinline__ void get(const double* p, double (&e)[4]) {
-    const double2 q0 = __ldg(reinterpret_cast<const double2*>(p)), q1 = __ldg(reinterpret_cast<const double2*>(p) + 1);
-    e[0] = q0.x; e[1] = q0.y; e[2] = q1.x; e[3] = q1.y;
-  }
-};
-template <> struct Quad<__nv_bfloat16> {
-  static __device__ __forceinline__ void get(const __nv_bfloat16* p, double (&e)[4]) {
-    const uint2 q = __ldg(reinterpret_cast<const uint2*>(p));
-    // a BF16 value is the upper half of the FP32 value with the same bits
-    e[0] = __uint_as_float(q.x << 16); e[1] = __uint_as_float(q.x & 0xffff0000u);
-    e[2] = __uint_as_float(q.y << 16); e[3] = __uint_as_float(q.y & 0xffff0000u);
-  }
 };
 
 // Slice values (and, once per handle, the columns) from the tangent's CSR layout: row (c, g)
@@ -1041,7 +946,6 @@ __global__ void __launch_bounds__(256, sizeof(VT) == 4 ? (MODE == 0 ? 4 : 5) : 0
 // off[s] + c*2*nnz[s] + 2*(ptr[g] - base[s]) + c2*deg(g) + k.  Every output
 // entry is summed in a fixed order (no atomics), so results are reproducible.
 
-constexpr double kSaOmega = 4.0 / 3.0;  // damping of the prolongator smoother (l1 diagonal: rho(D^-1 A) <= 1)
 
 __device__ __forceinline__ int sa_find(const int* list, int n, int key) {  // list sorted ascending
   int lo = 0, hi = n;
@@ -1061,14 +965,15 @@ __device__ __forceinline__ void sa_decode(int i, const int* dof_sys, const int* 
   g = no + (loc - c * nn);
 }
 
-// prolongator rows: P(i,:) = P0(i,:) - w invd_i A(i,:) P0 on unmasked rows and columns
+// prolongator rows: P(i,:) = P0(i,:) - w/l1_i A(i,:) P0 on unmasked rows and columns (invd holds
+// kSmoothOmega / l1), or the linear interpolation pn_w
 // ST: the type the set-up stores and sums P, A P and P' in (FP32 for the mixed-precision form,
 // whose V-cycle transfers read FP32 values, else FP64)
 template <typename KT, typename VT, typename ST>
 __global__ void k_sa_P(int nf, const int* dof_sys, const int* dof_off, const int* node_off, const int* rowptr,
                        const int* colind, const KT* A, const unsigned char* mask, const VT* invd, const int* agg,
-                       const int* pn_ptr, const int* pn_col, const int* pbase, const int* pnnz, const int* poff,
-                       ST* P, const int* sel) {
+                       const int* pn_ptr, const int* pn_col, const double* pn_w, const int* pbase, const int* pnnz,
+                       const int* poff, ST* P, const int* sel) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nf) return;
   int s, c, g;
@@ -1078,9 +983,13 @@ __global__ void k_sa_P(int nf, const int* dof_sys, const int* dof_off, const int
   ST* row = P + poff[s] + (size_t)c * 2 * pnnz[s] + 2 * (size_t)(pr - pbase[s]);
   for (int t = 0; t < 2 * dP; ++t) row[t] = 0;
   if (mask && mask[i]) return;
+  if (pn_w) {  // linear interpolation: the same weights for both components, no smoothing
+    for (int t = 0; t < dP; ++t) row[c * dP + t] = (ST)pn_w[pr + t];
+    return;
+  }
   const int k0 = sa_find(pn_col + pr, dP, agg[g]);
   if (k0 >= 0) row[c * dP + k0] = 1;
-  const ST f = (ST)(kSaOmega * (double)invd[i]);
+  const ST f = (ST)(kSaOmega / kSmoothOmega * (double)invd[i]);
   // the row holds the u block then the v block of the node's deg neighbours (the same nodes in
   // the same order), so one search per neighbour serves both blocks; each target still sums its
   // block's entries in row order
@@ -1093,51 +1002,6 @@ __global__ void k_sa_P(int nf, const int* dof_sys, const int* dof_off, const int
     if (!(mask && mask[ju])) row[kk] -= f * (ST)A[q0 + k];
     if (!(mask && mask[ju + nn])) row[dP + kk] -= f * (ST)A[q0 + deg + k];
   }
-}
-
-// P in the transfer layout: per node-level entry (fine node g, coarse node K) one quad of
-// P((c,g),(c2,K)) in the order (c,c2) = (0,0), (0,1), (1,0), (1,1), read with one load.  The mixed
-// form keeps BF16 quads (its set-up then reads the same rounded values, so the coarse operator is
-// the Galerkin product of the prolongator the V-cycle applies), the FP64 form FP64 quads.
-struct alignas(8) PQuadH {
-  __nv_bfloat162 r0, r1;
-};
-struct alignas(16) PQuadD {
-  double2 r0, r1;
-};
-template <typename VT>
-struct PQuadOf {
-  using T = PQuadD;
-};
-template <>
-struct PQuadOf<float> {
-  using T = PQuadH;
-};
-__device__ __forceinline__ void pq_get(const PQuadH* q, double (&v)[4]) {
-  const uint2 u = __ldg(reinterpret_cast<const uint2*>(q));
-  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
-  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-__device__ __forceinline__ void pq_get(const PQuadH* q, float (&v)[4]) {
-  const uint2 u = __ldg(reinterpret_cast<const uint2*>(q));
-  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
-  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-__device__ __forceinline__ void pq_get(const PQuadD* q, double (&v)[4]) {
-  const double2 a = __ldg(&q->r0), b = __ldg(&q->r1);
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-__device__ __forceinline__ void pq_set(PQuadH* q, double v0, double v1, double v2, double v3) {
-  PQuadH h;
-  h.r0 = __floats2bfloat162_rn((float)v0, (float)v1);
-  h.r1 = __floats2bfloat162_rn((float)v2, (float)v3);
-  *q = h;
-}
-__device__ __forceinline__ void pq_set(PQuadD* q, double v0, double v1, double v2, double v3) {
-  q->r0 = make_double2(v0, v1);
-  q->r1 = make_double2(v2, v3);
 }
 
 // A P rows: AP(i,:) = sum over unmasked columns j of A(i,j) P(j,:), kSaGL lanes per fine node g.
@@ -1552,7 +1416,7 @@ static int numeric_t(ua_mesh* m, const int* rowptr0, const int* colind0, const K
       QT* Qv = (QT*)(sizeof(KT) == 4 ? F.sa_qh : F.sa_qd);
       QT* QTv = (QT*)(sizeof(KT) == 4 ? F.sa_qth : F.sa_qtd);
       k_sa_P<KT, VT, ST><<<nbf, 128, 0, st>>>(F.ndof, F.dof_sys, F.d_dof_off, F.d_node_off, rp, ci, A, mk,
-                                              (const VT*)F.invd, F.sa_agg, F.pn_ptr, F.pn_col, F.pbase, F.pnnz,
+                                              (const VT*)F.invd, F.sa_agg, F.pn_ptr, F.pn_col, F.pn_w, F.pbase, F.pnnz,
                                               F.poff, Pv, psel), ++*launches;
       k_sa_quads<ST, QT><<<(F.nn + 127) / 128, 128, 0, st>>>(F.nn, F.node_sys, F.pn_ptr, F.pbase, F.pnnz, F.poff,
                                                             Pv, Qv, psel), ++*launches;
