@@ -461,6 +461,12 @@ static int amg_build(ua_mesh* m, bool smoothed) {
     delete a;
     return set_error(UA_ERR_OOM, "AMG setup: device allocation failed");
   }
+  if (a->sa) {  // for the structure of the collapsed cycle (cycle_init)
+    a->h_gptr = std::move(g_ptr);
+    a->h_gcol = std::move(g_col);
+    a->h_apnp = std::move(g_apnp);
+    a->h_apnc = std::move(g_apnc);
+  }
   m->amg = a;
   return UA_OK;
 }
@@ -531,21 +537,28 @@ __global__ void k_amg_l1(int n, const int* rowptr, const int* colind, const KT* 
   invd[i] = (VT)(s > 0 ? kSmoothOmega / s : 0.0);
 }
 
-// Inverse of each system's coarsest matrix: Gauss-Jordan on [A | I] in
-// shared memory, one CTA per system, row-major result.  A is the Galerkin
-// product of the SPD tangent (symmetric positive definite on the free dofs),
-// so the diagonal pivots stay positive and no pivoting is needed.  At step k
-// only columns k..n+k of the augmented matrix can be non-zero off the
-// finished part, so the update covers those n+1 columns.  A zero row (an
-// aggregate of constrained dofs only; its column is zero too) is replaced by
-// the identity row.
+// Inverse of each system's coarsest matrix: Gauss-Jordan in place, one CTA per system, row-major
+// result.  A is the Galerkin product of the SPD tangent (symmetric positive definite on the free
+// dofs), so no pivoting is needed; a zero row (an aggregate of constrained dofs only; its column is
+// zero too) is replaced by the identity row.
+//
+// The matrix is scaled to a unit diagonal (pivots in (0, 1]) and lives in registers, kDiT x kDiT
+// entries a thread; the pivot row and column go through shared memory, in two copies so that a step
+// has one barrier.  Step k is one update e_ij -= f_i w_j for every entry, with w_j = row_j / p and
+// f_i = column_i except w_k = 1 + 1/p and f_k = p - 1, which give the pivot row, the pivot column
+// and the pivot their own values without a test in the tile (the additions there are of terms of
+// equal sign as p <= 1).
+constexpr int kDiT = 6, kDiG = kAmgMaxDense / kDiT, kDiThreads = kDiG * kDiG;
+static_assert(kAmgMaxDense % kDiT == 0 && kDiThreads <= 1024, "the threads' tiles cover the largest coarsest matrix");
 template <typename KT>
-__global__ void __launch_bounds__(256) k_amg_dense_inverse(const int* depth, const int* dn_arr, const int* doff,
-                                                           int* const* lev_rowptr, int* const* lev_colind,
-                                                           void* const* lev_A, int* const* lev_dofoff,
-                                                           double* dense, const int* sel) {
-  extern __shared__ double M[];
-  __shared__ double fac[kAmgMaxDense];
+__global__ void __launch_bounds__(kDiThreads) k_amg_dense_inverse(const int* depth, const int* dn_arr,
+                                                                  const int* doff, int* const* lev_rowptr,
+                                                                  int* const* lev_colind, void* const* lev_A,
+                                                                  int* const* lev_dofoff, double* dense,
+                                                                  const int* sel) {
+  constexpr int ND = kAmgMaxDense;
+  extern __shared__ double M[];  // n x n staging of the matrix
+  __shared__ double prow[2][ND], pcol[2][ND], dg[ND];
   const int s = blockIdx.x;
   const int n = dn_arr[s];
   if (n == 0 || (sel && !sel[s])) return;
@@ -554,33 +567,66 @@ __global__ void __launch_bounds__(256) k_amg_dense_inverse(const int* depth, con
   const int* ci = lev_colind[l];
   const KT* A = (const KT*)lev_A[l];
   const int d0 = lev_dofoff[l][s];
-  const int w = 2 * n;
-  for (int t = threadIdx.x; t < n * w; t += blockDim.x) M[t] = ((t % w) - n == t / w) ? 1.0 : 0.0;
+  for (int t = threadIdx.x; t < n * n; t += kDiThreads) M[t] = 0;
   __syncthreads();
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
-    bool zero = true;
-    for (int q = rp[d0 + r]; q < rp[d0 + r + 1]; ++q) {
-      const double v = (double)A[q];
-      M[r * w + (ci[q] - d0)] = v;
-      zero = zero && v == 0.0;
+  for (int r = threadIdx.x >> 3; r < n; r += kDiThreads / 8)  // 8 lanes per row
+    for (int q = rp[d0 + r] + (threadIdx.x & 7); q < rp[d0 + r + 1]; q += 8) M[r * n + (ci[q] - d0)] = (double)A[q];
+  __syncthreads();
+  for (int r = threadIdx.x; r < n; r += kDiThreads) {
+    double d = M[r * n + r];
+    if (!(d > 0)) {
+      bool zero = true;
+      for (int c = 0; c < n; ++c) zero = zero && M[r * n + c] == 0.0;
+      if (zero) M[r * n + r] = 1.0;
+      d = 1.0;
     }
-    if (zero) M[r * w + r] = 1.0;
+    dg[r] = 1.0 / sqrt(d);
   }
   __syncthreads();
-  const int nc = n + 1;  // active columns k..n+k
+  const int r0 = (threadIdx.x / kDiG) * kDiT, c0 = (threadIdx.x % kDiG) * kDiT;
+  const bool mine = r0 < n && c0 < n;
+  double e[kDiT][kDiT];
+#pragma unroll
+  for (int i = 0; i < kDiT; ++i)
+#pragma unroll
+    for (int j = 0; j < kDiT; ++j)
+      e[i][j] = (r0 + i < n && c0 + j < n) ? M[(r0 + i) * n + c0 + j] * dg[r0 + i] * dg[c0 + j] : 0.0;
   for (int k = 0; k < n; ++k) {
-    const double inv = 1.0 / M[k * w + k];
-    for (int r = threadIdx.x; r < n; r += blockDim.x) fac[r] = (r == k) ? 0.0 : M[r * w + k];
-    __syncthreads();
-    for (int c = k + threadIdx.x; c <= n + k; c += blockDim.x) M[k * w + c] *= inv;
-    __syncthreads();
-    for (int t = threadIdx.x; t < n * nc; t += blockDim.x) {
-      const int r = t / nc, c = k + (t - r * nc);
-      if (r != k) M[r * w + c] -= fac[r] * M[k * w + c];
+    double *pr = prow[k & 1], *pc = pcol[k & 1];
+    if (mine && k >= r0 && k < r0 + kDiT) {
+#pragma unroll
+      for (int i = 0; i < kDiT; ++i)
+        if (r0 + i == k)
+#pragma unroll
+          for (int j = 0; j < kDiT; ++j) pr[c0 + j] = e[i][j];
+    }
+    if (mine && k >= c0 && k < c0 + kDiT) {
+#pragma unroll
+      for (int j = 0; j < kDiT; ++j)
+        if (c0 + j == k)
+#pragma unroll
+          for (int i = 0; i < kDiT; ++i) pc[r0 + i] = e[i][j];
     }
     __syncthreads();
+    if (!mine) continue;  // padding only (it still meets the barriers)
+    const double p = pr[k], inv = 1.0 / p;
+    double w[kDiT];
+#pragma unroll
+    for (int j = 0; j < kDiT; ++j) w[j] = (c0 + j == k) ? 1.0 + inv : pr[c0 + j] * inv;
+#pragma unroll
+    for (int i = 0; i < kDiT; ++i) {
+      const double f = (r0 + i == k) ? p - 1.0 : pc[r0 + i];
+#pragma unroll
+      for (int j = 0; j < kDiT; ++j) e[i][j] = fma(-f, w[j], e[i][j]);
+    }
   }
-  for (int t = threadIdx.x; t < n * n; t += blockDim.x) dense[doff[s] + t] = M[(t / n) * w + n + (t % n)];
+  if (!mine) return;
+#pragma unroll
+  for (int i = 0; i < kDiT; ++i)
+#pragma unroll
+    for (int j = 0; j < kDiT; ++j)
+      if (r0 + i < n && c0 + j < n)
+        dense[doff[s] + (r0 + i) * n + c0 + j] = e[i][j] * dg[r0 + i] * dg[c0 + j];
 }
 
 // ---------------------------------------------------------------------------
@@ -1442,8 +1488,8 @@ static int numeric_t(ua_mesh* m, const int* rowptr0, const int* colind0, const K
     }
     for (int l = 0; l < a->nlev; ++l) l1(l);
   }
-  const int sm = (int)(sizeof(double) * (size_t)a->maxdn * 2 * a->maxdn);  // attribute set by the caller
-  k_amg_dense_inverse<KT><<<a->nsys, 256, sm, st>>>(a->d_depth, a->d_dn, a->d_doff, a->d_lev_rowptr,
+  const int sm = (int)(sizeof(double) * (size_t)a->maxdn * a->maxdn);  // attribute set by the caller
+  k_amg_dense_inverse<KT><<<a->nsys, kDiThreads, sm, st>>>(a->d_depth, a->d_dn, a->d_doff, a->d_lev_rowptr,
                                                      a->d_lev_colind, a->d_lev_A, a->d_lev_dofoff, a->dense, sel),
       ++*launches;
   cudaError_t e = cudaGetLastError();
@@ -1569,6 +1615,8 @@ int amg_sell_init(ua_mesh* m, const std::vector<int>& sys_rb_off0) {
   S.sb_rbu = upload(m, a, sb_rbu, ok);
   S.sb_rbv = upload(m, a, sb_rbv, ok);
   S.perm = upload(m, a, perm, ok);
+  S.h_perm = perm;
+  S.h_sl_off = sl_off;
   S.sl_off = upload(m, a, sl_off, ok);
   S.cols = (int*)dalloc(m, a, sizeof(int) * (size_t)S.slots, ok);
   S.spart = (double*)dalloc(m, a, sizeof(double) * kSellSlices * (size_t)std::max(S.nsb, 1), ok);
@@ -1582,7 +1630,6 @@ int amg_sell_init(ua_mesh* m, const std::vector<int>& sys_rb_off0) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { S.failed = true; return set_error(UA_ERR_CUDA, "node slices: %s", cudaGetErrorString(e)); }
   S.ready = true;
-  if (a->sa) csell_init(m);  // the coarse levels keep their CSR passes if this fails
   return UA_OK;
 }
 
@@ -1590,6 +1637,10 @@ int amg_sell_fill(ua_mesh* m, const void* K0, bool fp32, bool lo, long long* lau
   Amg* a = m->amg;
   if (!a || !a->sell.ready) return UA_ERR_INVALID;
   Sell& S = a->sell;
+  if (a->sa && lo && !a->csell_tried) {  // the coarse levels keep their CSR passes if this fails
+    a->csell_tried = true;
+    csell_init(m);
+  }
   bool ok = true;
   const size_t nv = 4 * (size_t)S.slots;
   if (fp32 && !S.v32) S.v32 = (float*)dalloc(m, a, sizeof(float) * nv, ok);
@@ -1668,7 +1719,7 @@ const void* amg_bf16_copy(ua_mesh* m, const float* K0, long long nnz, long long*
 
 int amg_numeric(ua_mesh* m, const int* rowptr0, const int* colind0, const void* K0, bool fp32,
                 const unsigned char* cmask, long long* launches, const int* sel, const std::vector<int>* h_sel,
-                int p_refresh, bool graph) {
+                int p_refresh, bool graph, const CycFillReq* cyc) {
   // prolongators: recomputed for the selected systems on the first set-up of their solve and then
   // every p_refresh-th one (all of them when no host selection is given)
   Amg* a = m->amg;
@@ -1690,7 +1741,7 @@ int amg_numeric(ua_mesh* m, const int* rowptr0, const int* colind0, const void* 
     UA_CUDA_TRY(cudaStreamSynchronize(m->stream));  // h_prefresh is rewritten by the next set-up
     psel = a->d_prefresh;
   }
-  const int sm = (int)(sizeof(double) * (size_t)a->maxdn * 2 * a->maxdn);
+  const int sm = (int)(sizeof(double) * (size_t)a->maxdn * a->maxdn);
   if (fp32)
     UA_CUDA_TRY(cudaFuncSetAttribute(k_amg_dense_inverse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   else
@@ -1721,13 +1772,16 @@ int amg_numeric(ua_mesh* m, const int* rowptr0, const int* colind0, const void* 
     if (!ok) return set_error(UA_ERR_OOM, "AMG: device allocation of the transfer values failed");
   }
   auto run = [&](long long* l) {
-    return fp32 ? numeric_t<float, float>(m, rowptr0, colind0, (const float*)K0, cmask, sel, psel, l)
-                : numeric_t<double, double>(m, rowptr0, colind0, (const double*)K0, cmask, sel, psel, l);
+    int rc = fp32 ? numeric_t<float, float>(m, rowptr0, colind0, (const float*)K0, cmask, sel, psel, l)
+                  : numeric_t<double, double>(m, rowptr0, colind0, (const double*)K0, cmask, sel, psel, l);
+    if (!rc && cyc) cycle_fill(m, rowptr0, colind0, K0, fp32, cyc->lo, cyc->dw, sel, l);
+    return rc;
   };
   if (!graph) return run(launches);
   // one captured graph per kind of call (FP32/FP64 values, prolongator selection, handle's
   // selection), replayed at every later Newton step
-  const int key = (fp32 ? 1 : 0) + (psel == a->d_prefresh && psel ? 2 : 0) + (sel ? 4 : 0);
+  const int key = (fp32 ? 1 : 0) + (psel == a->d_prefresh && psel ? 2 : 0) + (sel ? 4 : 0) + (cyc ? 8 : 0) +
+                  (cyc && cyc->lo ? 16 : 0);
   if (!a->setup_exec[key]) {
     long long n = 0;
     cudaGraph_t gr = nullptr;

@@ -69,9 +69,15 @@ const void* amg_invd0(const ua_mesh* m);
 // and p_refresh > 1: each system's prolongators are recomputed on the first set-up of its solve
 // (amg_restart_P) and then every p_refresh-th set-up, the coarse operators every time.
 // graph: run the set-up's launches as a captured CUDA graph (captured once per kind of call).
+// cyc: also fill the values of the collapsed cycle (cycle_init and cycle_alloc_values done).
+struct CycFillReq {
+  bool lo;   // BF16 copy of the finest level
+  void* dw;  // receives the finest level's damped l1 diagonal per node (value precision)
+};
 int amg_numeric(ua_mesh* m, const int* rowptr0, const int* colind0, const void* K0, bool fp32,
                 const unsigned char* cmask, long long* launches, const int* sel = nullptr,
-                const std::vector<int>* h_sel = nullptr, int p_refresh = 1, bool graph = false);
+                const std::vector<int>* h_sel = nullptr, int p_refresh = 1, bool graph = false,
+                const CycFillReq* cyc = nullptr);
 // the systems of `run` start a solve: their next set-up recomputes the prolongators
 void amg_restart_P(ua_mesh* m, const std::vector<int>& run);
 // uvh handles: extract the velocity block of the 3-dof tangent K3 (and its
@@ -100,5 +106,33 @@ const void* amg_bf16_copy(ua_mesh* m, const float* K0, long long nnz, long long*
 // One V(1,1) cycle.  The finest level runs as row-block kernels (residual,
 // aggregation, correction, smoothing); coarser levels use one thread per aggregate.
 int amg_vcycle(ua_mesh* m, bool fp32, const AmgPcgView& v, long long* launches);
+
+// ---- resident Krylov solves on the collapsed V-cycle (ua_pcg.cu) ----
+bool cycle_supported(const ua_mesh* m);
+int cycle_init(ua_mesh* m);
+int cycle_alloc_values(ua_mesh* m, bool fp32, bool lo);
+void cycle_fill(ua_mesh* m, const int* rowptr0, const int* colind0, const void* K0, bool fp32, bool lo, void* dw,
+                const int* sel, long long* launches);
+struct PcgSolve {
+  bool fp32, lo, prof;
+  const int *rb_start, *rb_sys;
+  int nrb;
+  const int* sel;
+  const int *rowptr, *colind;
+  const void* K;
+  const double* f;        // right-hand side (dofs)
+  double* dX;             // in: the particular solution on the constrained dofs; out: the solution
+  void *r, *z, *p, *q;    // work, one pair per node in the value precision
+  double* x;              // work, one FP64 pair per node
+  const void* dw;
+  double* tol2;           // [nsys]
+  int *done, *its, *status;
+  int maxit;
+};
+// sel: systems to solve; steps: expected iterations (the schedule's weights)
+int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, const std::vector<int>& steps, int nsm,
+                 long long* launches);
+// pass classes of a profiled resident solve: operator, finest restriction, finest up pass, rest
+int pcg_resident_status(ua_mesh* m, bool prof, double* ms, int* cnt);
 
 }  // namespace ua

@@ -88,6 +88,8 @@ struct Sell {
   int nsb = 0;
   long long slots = 0;
   std::vector<int> h_sys_sb_off;  // per-system prefix of the slice blocks
+  std::vector<int> h_perm;
+  std::vector<long long> h_sl_off;
   int *sb_sys = nullptr, *sb_n0 = nullptr, *sb_cnt = nullptr, *sb_rbu = nullptr, *sb_rbv = nullptr;
   int* perm = nullptr;             // [nn_total]: per block, its global node ids in slice order
   long long* sl_off = nullptr;     // [nsb * kSellSlices + 1] slot offsets of the slices
@@ -100,12 +102,91 @@ struct Sell {
   ActList act;                     // slice blocks of the systems still iterating
 };
 
+// Collapsed cycle (ua_cycle.cuh): device pointers of one level.  A quad is the four values of a
+// node pair; the types of the quads are the form's.
+constexpr int kCycMaxLev = 12;
+struct CycLev {
+  const int *aptr, *acol;   // node rows of the level's operator (levels >= 1)
+  void* aval;               // scaled operator, aptr order
+  const int *qptr, *qcol;   // node rows of Q (the A P pattern)
+  void* qval;
+  const int *tptr, *tfine;  // rows of Q' by coarse node
+  void* tval;
+  void *b, *z;              // right-hand side and result, one pair per node (levels >= 1)
+};
+// one system of the handle: first node and node count on every level, slices, dense inverse
+struct CycSys {
+  int depth, dn, doff, sl0, nsl;
+  int n0[kCycMaxLev + 1], nn[kCycMaxLev + 1];
+};
+// node slices of the finest level; columns are slice positions
+struct CycFine {
+  const int* perm;           // position -> node
+  const long long* sl_off;
+  const int* cols;
+};
+struct CycArgs {
+  CycLev lev[kCycMaxLev];
+  CycFine fine;
+  const CycSys* sys;
+  const double* dense;
+  const int4* cta;     // per CTA: queue begin, end, rank in its team, team size
+  const int *team, *queue;
+  unsigned* bar;       // arrival counter of team k at 32 k
+  int* err;
+  unsigned long long* prof;
+  double* part;        // [3][nslices]
+  long long nslices;
+};
+struct CycSchedule {
+  std::vector<int4> cta;
+  std::vector<int> team, queue;
+};
+// Set-up data of the collapsed cycle: structure once per handle, values per tangent.
+struct Cycle {
+  bool ready = false, failed = false;
+  std::vector<CycSys> sys;
+  CycSys* d_sys = nullptr;
+  struct Lev {
+    int *nptr = nullptr, *ncol = nullptr;                      // node graph (levels >= 1)
+    long long nq = 0;                                          // node-level entries of Q
+    int *qptr = nullptr, *qcol = nullptr;                      // rows of Q (level 0: in slice order)
+    int* qrow = nullptr;                                       // node -> first entry of its row of Q
+    int *tptr = nullptr, *tfine = nullptr, *tpos = nullptr;    // Q' lists; tpos: entry of Q -> entry of Q'
+    double2* sc = nullptr;                                     // D^-1/2 per node (u, v)
+    void *a32 = nullptr, *a64 = nullptr;                       // scaled operator quads (levels >= 1)
+    void *qh = nullptr, *qd = nullptr, *th = nullptr, *td = nullptr;  // Q and Q' quads (BF16, FP64)
+  };
+  std::vector<Lev> lev;
+  // resident kernel: schedule (one int4 per CTA: queue begin, end, team rank, team size), queue,
+  // team counters, per-slice partials, profile clocks
+  int last_grid = 0;
+  int4* d_cta = nullptr;
+  int *d_queue = nullptr, *d_team = nullptr;
+  unsigned* d_bar = nullptr;
+  double* d_part = nullptr;   // [3][slices]
+  unsigned long long* d_prof = nullptr;
+  int* d_err = nullptr;
+  int *d_ipos = nullptr, *d_pcol = nullptr;  // node -> slice position; slot columns as positions
+  void* d_r2 = nullptr;       // second residual buffer
+  std::vector<double> h_bytes[2];  // per system: bytes of the matrices a step reads (FP64, mixed)
+  int* h_stage = nullptr;     // pinned staging of the schedule
+  long long nslices = 0;
+  ~Cycle() {
+    if (h_stage) cudaFreeHost(h_stage);
+  }
+};
+
 struct Amg {
   int nsys = 0, nlev = 0, maxdn = 0;
   Sell sell;
+  Cycle cyc;
+  // host node graphs and A P lists of the levels, kept until the cycle's structure is built
+  std::vector<std::vector<int>> h_gptr, h_gcol, h_apnp, h_apnc;
   // node slices of the coarse levels 1 .. nlev-2 (smoothed hierarchies): BF16 copies of the
   // coarse operators for the mixed-precision V-cycle's residual and smoothing there
   std::vector<Sell> csell;
+  bool csell_tried = false;
   // active-block lists: rows[l] (level-l row blocks, depth > l; level 0 = the handle's blocks),
   // fnodes[l] (level-l node blocks, depth > l), cnodes[l] (level-(l+1) node blocks, depth > l)
   bool act_ready = false;
@@ -132,8 +213,8 @@ struct Amg {
   int* d_prefresh = nullptr;
   // the numeric set-up of a Newton step captured as one CUDA graph per (precision, selection
   // kind) and replayed: every argument is a fixed device buffer of the handle
-  cudaGraphExec_t setup_exec[8] = {};
-  long long setup_nodes[8] = {};
+  cudaGraphExec_t setup_exec[32] = {};
+  long long setup_nodes[32] = {};
   ~Amg() {
     for (auto& e : setup_exec)
       if (e) cudaGraphExecDestroy(e);

@@ -1,0 +1,481 @@
+// The V-cycle in collapsed form and the team primitives of the resident Krylov kernels.
+//
+// With one damped l1-Jacobi sweep before and after the coarse correction, a V(1,1) cycle from a
+// zero guess is the sum
+//     z = M b + P~ z_c,   z_c = cycle(P~' b),   M = 2 D^-1 - D^-1 A D^-1,   P~ = (I - D^-1 A) P
+// (D the damped l1 diagonal): the pre-smoothed residual and the post-smoothing of the correction
+// are folded into the transfer P~, whose entries the set-up has at hand (A P is formed for the
+// coarse operator).  Scaled by D^1/2 on every level but a system's coarsest,
+//     A^ = D^-1/2 A D^-1/2,  Q = D^1/2 P~ D_c^-1/2,  b^ = D^-1/2 b,  z^ = D^1/2 z,
+// one level is  b^_c = Q' b^  on the way down and  z^ = 2 b^ - A^ b^ + Q z^_c  on the way up, one
+// pass each, where the uncollapsed cycle makes a residual, a restriction, a prolongation and a
+// smoothing pass in sequence.  The scaled operator has no diagonal, mask or weight to read.
+//
+// Teams.  A resident kernel runs one CTA of kCycThreads threads per SM.  The CTAs are split into
+// teams; a team solves the systems of its queue one after another, its CTAs meeting at a counter
+// in global memory after every pass (a __syncthreads for a team of one).  A system's sums have a
+// fixed order that depends on the system alone (per-slice partials, summed by every CTA of the
+// team), so its result does not depend on its team's size or on the other systems.
+#pragma once
+#include "ua_amg_int.h"
+
+namespace ua {
+
+constexpr int kCycThreads = 512;
+constexpr int kCycWarps = kCycThreads / 32;
+
+template <typename VT> struct Vec2;
+template <> struct Vec2<float> { using T = float2; };
+template <> struct Vec2<double> { using T = double2; };
+
+// a quad as loaded, widened only at its use (registers)
+template <typename KT> struct QuadRaw;
+template <> struct QuadRaw<float> {
+  using T = float4;
+  static __device__ __forceinline__ T load(const char* p) { return *reinterpret_cast<const float4*>(p); }
+  static __device__ __forceinline__ void get(const T& e, double (&q)[4]) { q[0] = e.x; q[1] = e.y; q[2] = e.z; q[3] = e.w; }
+};
+template <> struct QuadRaw<double> {
+  struct T { double2 a, b; };
+  static __device__ __forceinline__ T load(const char* p) {
+    return T{reinterpret_cast<const double2*>(p)[0], reinterpret_cast<const double2*>(p)[1]};
+  }
+  static __device__ __forceinline__ void get(const T& e, double (&q)[4]) { q[0] = e.a.x; q[1] = e.a.y; q[2] = e.b.x; q[3] = e.b.y; }
+};
+template <> struct QuadRaw<__nv_bfloat16> {
+  using T = uint2;
+  static __device__ __forceinline__ T load(const char* p) { return *reinterpret_cast<const uint2*>(p); }
+  static __device__ __forceinline__ void get(const T& e, double (&q)[4]) {
+    q[0] = __uint_as_float(e.x << 16); q[1] = __uint_as_float(e.x & 0xffff0000u);
+    q[2] = __uint_as_float(e.y << 16); q[3] = __uint_as_float(e.y & 0xffff0000u);
+  }
+};
+
+struct TeamCtx {
+  int rank, size;        // this CTA in its team
+  unsigned* bar;         // the team's arrival counter
+  unsigned target;       // arrivals that end the next barrier
+  int* ok;               // shared: the last barrier was met
+};
+
+// Arrive and wait.  The wait is bounded (some seconds): a team that does not meet returns false in
+// every thread and the kernel ends with an error status.
+constexpr unsigned kTeamSpinLimit = 1u << 24;
+__device__ __forceinline__ bool team_sync(TeamCtx& t) {
+  __syncthreads();
+  if (t.size == 1) return true;
+  if (threadIdx.x == 0) {
+    t.target += t.size;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
+    int ok = 0;
+    for (unsigned i = 0; i < kTeamSpinLimit; ++i) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(t.bar) : "memory");
+      if ((int)(v - t.target) >= 0) {
+        ok = 1;
+        break;
+      }
+    }
+    *t.ok = ok;
+  }
+  __syncthreads();
+  return *t.ok != 0;
+}
+
+// Sum of n partials by the whole CTA, the same bits in every thread of every CTA: thread t adds
+// the partials t, t + kCycThreads, ..., then a butterfly.  red: kCycWarps shared doubles that no
+// thread of the CTA still reads.
+__device__ __forceinline__ double team_sum(const double* part, int n, double* red) {
+  double a = 0;
+  for (int i = threadIdx.x; i < n; i += kCycThreads) a += __ldcg(part + i);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
+  __syncthreads();
+  a = (threadIdx.x & 31) < kCycWarps ? red[threadIdx.x & 31] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
+}
+
+__device__ __forceinline__ double lane_sum(double v, int width) {
+  for (int o = width >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// this CTA's share [lo, hi) of n items
+__device__ __forceinline__ void team_share(const TeamCtx& t, int n, int& lo, int& hi) {
+  lo = (int)((long long)n * t.rank / t.size);
+  hi = (int)((long long)n * (t.rank + 1) / t.size);
+}
+
+// Lanes per node: a whole warp (restriction) or eight lanes (coarse up pass) on the small levels,
+// where a pass is a chain of dependent loads, fewer on the large ones, where the lanes are needed
+// for more nodes.  Functions of the level's size alone, as the order of the sums depends on them.
+__device__ __forceinline__ int down_lanes(int nc) { return nc <= 4096 ? 32 : 8; }
+__device__ __forceinline__ int up_lanes(int nn) { return nn <= 4096 ? 8 : (nn <= 32768 ? 4 : 2); }
+
+// What the passes read of one level and of the finest level's operator: global memory, or the
+// copies of this CTA's rows in shared memory (cyc_stage).  Row pointers and entry numbers are the
+// global ones in both, the bases are shifted.  The loads are generic on purpose.
+struct LevS {
+  const int *aptr, *acol;
+  const char* aval;
+  const int *qptr, *qcol;
+  const char* qval;
+  const int *tptr, *tfine;
+  const char* tval;
+};
+struct FineS {
+  const long long* sl_off;
+  const int* cols;
+  const char *kv, *lv;  // operator of the Krylov method and of the cycle
+};
+
+// Shared memory left for copies.
+struct Arena {
+  char* base;
+  int cap, used;
+  __device__ __forceinline__ char* take(long long bytes) {  // uniform over the CTA
+    const long long b = (bytes + 15) & ~15LL;
+    if (used + b > cap) return nullptr;
+    char* p = base + used;
+    used += (int)b;
+    return p;
+  }
+};
+__device__ __forceinline__ void copy8(char* d, const char* s, long long bytes) {
+  for (long long i = threadIdx.x; i < bytes / 8; i += kCycThreads)
+    reinterpret_cast<uint2*>(d)[i] = reinterpret_cast<const uint2*>(s)[i];
+}
+__device__ __forceinline__ void copy4(int* d, const int* s, long long n) {
+  for (long long i = threadIdx.x; i < n; i += kCycThreads) d[i] = s[i];
+}
+// rows [lo, hi) of a node-CSR matrix with quads of qb bytes
+__device__ __forceinline__ void stage_csr(Arena& ar, int lo, int hi, int qb, const int*& ptr, const int*& col,
+                                          const char*& val) {
+  if (lo >= hi) return;
+  const int e0 = ptr[lo], e1 = ptr[hi];
+  char* p = ar.take((long long)(hi - lo + 1) * 4 + 12 + (long long)(e1 - e0) * (4 + qb) + 16);
+  if (!p) return;
+  char* pv = p;  // values first (16-byte aligned), then columns, then row pointers
+  int* pc = reinterpret_cast<int*>(p + (((long long)(e1 - e0) * qb + 15) & ~15LL));
+  int* pp = pc + (e1 - e0);
+  copy8(pv, val + (long long)e0 * qb, (long long)(e1 - e0) * qb);
+  copy4(pc, col + e0, e1 - e0);
+  copy4(pp, ptr + lo, hi - lo + 1);
+  ptr = pp - lo;
+  col = pc - e0;
+  val = pv - (long long)e0 * qb;
+}
+
+// Reads the level tables into shared memory and copies this CTA's rows as far as they fit, the
+// small levels first.  In a team with enough CTAs everything fits: a pass then waits for one
+// gather of the vector instead of three dependent loads.  Every thread keeps the same pointers;
+// thread 0 publishes them.
+template <typename KT, typename LT, typename QT>
+__device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, const void* lv, const CycSys& S,
+                                          const TeamCtx& t, Arena& ar, LevS* lev, FineS* fine, int kslot,
+                                          const double*& dense) {
+  constexpr int qb = 4 * sizeof(QT), ab = 4 * sizeof(KT);
+  int lo, hi;
+  dense = A.dense + S.doff;
+  if (char* p = ar.take(8LL * S.dn * S.dn)) {
+    copy8(p, (const char*)dense, 8LL * S.dn * S.dn);
+    dense = (const double*)p;
+  }
+  for (int l = S.depth - 1; l >= 0; --l) {
+    const CycLev& G = A.lev[l];
+    LevS L{G.aptr, G.acol, (const char*)G.aval, G.qptr, G.qcol, (const char*)G.qval,
+           G.tptr, G.tfine, (const char*)G.tval};
+    team_share(t, S.nn[l + 1], lo, hi);
+    stage_csr(ar, S.n0[l + 1] + lo, S.n0[l + 1] + hi, qb, L.tptr, L.tfine, L.tval);
+    if (l > 0) {
+      team_share(t, S.nn[l], lo, hi);
+      stage_csr(ar, S.n0[l] + lo, S.n0[l] + hi, qb, L.qptr, L.qcol, L.qval);
+      stage_csr(ar, S.n0[l] + lo, S.n0[l] + hi, ab, L.aptr, L.acol, L.aval);
+    } else {
+      team_share(t, S.nsl, lo, hi);
+      stage_csr(ar, S.n0[0] + 32 * lo, S.n0[0] + min(32 * hi, S.nn[0]), qb, L.qptr, L.qcol, L.qval);
+    }
+    if (threadIdx.x == 0) lev[l] = L;
+  }
+  FineS F{A.fine.sl_off, A.fine.cols, (const char*)kv, (const char*)lv};
+  team_share(t, S.nsl, lo, hi);
+  if (lo < hi) {
+    const int s0 = S.sl0 + lo, ns = hi - lo;
+    const long long e0 = F.sl_off[s0], ne = F.sl_off[S.sl0 + hi] - e0;
+    if (char* p = ar.take(ne * 4 + 8LL * (ns + 1))) {
+      long long* po = reinterpret_cast<long long*>(p);
+      int* pc = reinterpret_cast<int*>(po + ns + 1);
+      for (int i = threadIdx.x; i <= ns; i += kCycThreads) po[i] = F.sl_off[s0 + i];
+      copy4(pc, F.cols + e0, ne);
+      F.sl_off = po - s0;
+      F.cols = pc - e0;
+      const int lb = 4 * sizeof(LT);
+      if (char* q = ar.take(ne * lb)) {
+        copy8(q, F.lv + e0 * lb, ne * lb);
+        const bool same = F.kv == F.lv;
+        F.lv = q - e0 * lb;
+        if (same) F.kv = F.lv;
+      }
+      if (kv != lv)
+        if (char* q = ar.take(ne * kslot)) {
+          copy8(q, F.kv + e0 * kslot, ne * kslot);
+          F.kv = q - e0 * kslot;
+        }
+    }
+  }
+  if (threadIdx.x == 0) *fine = F;
+  __syncthreads();
+}
+
+// b_c = Q' b for the coarse nodes of level l + 1; with a second vector, of b - alpha q (rounded as
+// the update of the residual rounds it), scaled by w.
+template <typename VT, typename QT>
+__device__ __forceinline__ void cyc_down(const LevS& L, const CycSys& S, int l, const TeamCtx& t,
+                                         const typename Vec2<VT>::T* b, typename Vec2<VT>::T* bc,
+                                         const typename Vec2<VT>::T* q2 = nullptr, double alpha = 0.0,
+                                         double w = 1.0) {
+  using V2 = typename Vec2<VT>::T;
+  constexpr int CH = sizeof(VT) == 4 ? 4 : 2, qb = 4 * sizeof(QT);
+  int lo, hi;
+  team_share(t, S.nn[l + 1], lo, hi);
+  const int c0 = S.n0[l + 1], lanes = down_lanes(S.nn[l + 1]);
+  const int sub = threadIdx.x / lanes, lane = threadIdx.x & (lanes - 1), nsub = kCycThreads / lanes;
+  for (int j0 = lo; j0 < hi; j0 += nsub) {
+    const int J = c0 + j0 + sub;
+    const bool valid = j0 + sub < hi;
+    double a0 = 0, a1 = 0;
+    if (valid) {
+      const int ue = L.tptr[J + 1];
+      for (int u0 = L.tptr[J] + lane; u0 < ue; u0 += lanes * CH) {
+        int f[CH];
+        typename QuadRaw<QT>::T e[CH];
+#pragma unroll
+        for (int k = 0; k < CH; ++k) {
+          const int u = min(u0 + k * lanes, ue - 1);
+          f[k] = L.tfine[u];
+          e[k] = QuadRaw<QT>::load(L.tval + (long long)u * qb);
+        }
+        V2 x[CH];
+#pragma unroll
+        for (int k = 0; k < CH; ++k) {
+          x[k] = b[f[k]];
+          if (q2) {
+            const V2 y = q2[f[k]];
+            x[k].x = (VT)((double)x[k].x - alpha * (double)y.x);
+            x[k].y = (VT)((double)x[k].y - alpha * (double)y.y);
+          }
+          if (u0 + k * lanes >= ue) x[k].x = x[k].y = 0;
+        }
+#pragma unroll
+        for (int k = 0; k < CH; ++k) {
+          double q[4];
+          QuadRaw<QT>::get(e[k], q);
+          a0 += q[0] * (double)x[k].x + q[2] * (double)x[k].y;
+          a1 += q[1] * (double)x[k].x + q[3] * (double)x[k].y;
+        }
+      }
+    }
+    a0 = lane_sum(a0, lanes);
+    a1 = lane_sum(a1, lanes);
+    if (valid && lane == 0) {
+      V2 o;
+      o.x = (VT)(w * a0);
+      o.y = (VT)(w * a1);
+      bc[J] = o;
+    }
+  }
+}
+
+// a += sign * (row entries [e, ee) in steps of `lanes`) * x, CH entries at a time
+template <int CH, typename QT, typename VT>
+__device__ __forceinline__ void row_product(const int* col, const char* val, int e, int ee, int lanes,
+                                            const typename Vec2<VT>::T* x0, double sign, double& a0, double& a1) {
+  using V2 = typename Vec2<VT>::T;
+  constexpr int qb = 4 * sizeof(QT);
+  for (; e < ee; e += lanes * CH) {
+    int c[CH];
+    typename QuadRaw<QT>::T m[CH];
+#pragma unroll
+    for (int k = 0; k < CH; ++k) {
+      const int u = min(e + k * lanes, ee - 1);
+      c[k] = col[u];
+      m[k] = QuadRaw<QT>::load(val + (long long)u * qb);
+    }
+    V2 x[CH];
+#pragma unroll
+    for (int k = 0; k < CH; ++k) {
+      x[k] = x0[c[k]];
+      if (e + k * lanes >= ee) x[k].x = x[k].y = 0;
+    }
+    double s0 = 0, s1 = 0;
+#pragma unroll
+    for (int k = 0; k < CH; ++k) {
+      double q[4];
+      QuadRaw<QT>::get(m[k], q);
+      s0 += q[0] * (double)x[k].x + q[1] * (double)x[k].y;
+      s1 += q[2] * (double)x[k].x + q[3] * (double)x[k].y;
+    }
+    a0 += sign * s0;
+    a1 += sign * s1;
+  }
+}
+
+// z = 2 b - A b + Q z_c on level l >= 1 (zc: indexed by the coarse level's node numbers).
+template <typename VT, typename AT, typename QT>
+__device__ __forceinline__ void cyc_up(const LevS& L, const CycSys& S, int l, const TeamCtx& t,
+                                       const typename Vec2<VT>::T* b, typename Vec2<VT>::T* z,
+                                       const typename Vec2<VT>::T* zc) {
+  using V2 = typename Vec2<VT>::T;
+  constexpr int CH = sizeof(VT) == 4 ? 4 : 2;
+  int lo, hi;
+  team_share(t, S.nn[l], lo, hi);
+  const int n0 = S.n0[l], lanes = up_lanes(S.nn[l]);
+  const int sub = threadIdx.x / lanes, lane = threadIdx.x & (lanes - 1), nsub = kCycThreads / lanes;
+  for (int j0 = lo; j0 < hi; j0 += nsub) {
+    const int g = n0 + j0 + sub;
+    const bool valid = j0 + sub < hi;
+    double a0 = 0, a1 = 0;
+    if (valid) {
+      if (lane == 0) {
+        const V2 v = b[g];
+        a0 = 2.0 * (double)v.x;
+        a1 = 2.0 * (double)v.y;
+      }
+      row_product<CH, AT, VT>(L.acol, L.aval, L.aptr[g] + lane, L.aptr[g + 1], lanes, b, -1.0, a0, a1);
+      row_product<CH, QT, VT>(L.qcol, L.qval, L.qptr[g] + lane, L.qptr[g + 1], lanes, zc, 1.0, a0, a1);
+    }
+    a0 = lane_sum(a0, lanes);
+    a1 = lane_sum(a1, lanes);
+    if (valid && lane == 0) {
+      V2 o;
+      o.x = (VT)a0;
+      o.y = (VT)a1;
+      z[g] = o;
+    }
+  }
+}
+
+// The coarsest level of the system by every CTA of the team for itself (no team barrier follows):
+// zc = A_L^-1 b_L in shared memory, the dense inverse in the dof order [u; v].  Threads along the
+// rows (the inverse is symmetric, so a row is read as a column: consecutive threads, consecutive
+// words), the columns in as many segments as the CTA has threads for; sums in a fixed order.
+struct DenseSh {
+  double b[kAmgMaxDense];
+  double part[kCycThreads];
+};
+template <typename VT>
+__device__ __forceinline__ void cyc_dense(const CycSys& S, const double* M, const typename Vec2<VT>::T* bL,
+                                          DenseSh& sh, typename Vec2<VT>::T* zc) {
+  using V2 = typename Vec2<VT>::T;
+  const int n = S.dn, nn = n >> 1, c0 = S.n0[S.depth], np = (n + 31) & ~31, seg = kCycThreads / np;
+  for (int i = threadIdx.x; i < nn; i += kCycThreads) {
+    const V2 v = bL[c0 + i];
+    sh.b[i] = (double)v.x;
+    sh.b[nn + i] = (double)v.y;
+  }
+  __syncthreads();
+  const int k = threadIdx.x / np, r = threadIdx.x - k * np;
+  if (k < seg) {
+    double acc = 0;
+    if (r < n) {
+      const int lo = n * k / seg, hi = n * (k + 1) / seg;
+#pragma unroll 8
+      for (int c = lo; c < hi; ++c) acc = fma(M[c * n + r], sh.b[c], acc);
+    }
+    sh.part[threadIdx.x] = acc;
+  }
+  __syncthreads();
+  if (threadIdx.x < n) {
+    double acc = 0;
+    for (int q = 0; q < seg; ++q) acc += sh.part[q * np + threadIdx.x];
+    reinterpret_cast<VT*>(zc)[threadIdx.x < nn ? 2 * threadIdx.x : 2 * (threadIdx.x - nn) + 1] = (VT)acc;
+  }
+  __syncthreads();
+}
+
+// CH slots k0 .. of a slice product: the columns and values load together, then the gathered
+// pairs.  Slots past the width repeat the last one with a zero vector entry, so that nothing
+// branches between the loads.
+template <int CH, typename KT, typename VT>
+__device__ __forceinline__ void slice_chunk(const int* cp, const char* vp, int k0, int W,
+                                            const typename Vec2<VT>::T* v, double& a0, double& a1) {
+  using V2 = typename Vec2<VT>::T;
+  int j[CH];
+  typename QuadRaw<KT>::T e[CH];
+#pragma unroll
+  for (int k = 0; k < CH; ++k) {
+    const int kk = min(k0 + k, W - 1);
+    j[k] = cp[32 * kk];
+    e[k] = QuadRaw<KT>::load(vp + (long long)kk * (128 * sizeof(KT)));
+  }
+  V2 x[CH];
+#pragma unroll
+  for (int k = 0; k < CH; ++k) {
+    x[k] = v[j[k]];
+    if (k0 + k >= W) x[k].x = x[k].y = 0;
+  }
+#pragma unroll
+  for (int k = 0; k < CH; ++k) {
+    double q[4];
+    QuadRaw<KT>::get(e[k], q);
+    a0 = fma(q[0], (double)x[k].x, a0);
+    a0 = fma(q[1], (double)x[k].y, a0);
+    a1 = fma(q[2], (double)x[k].x, a1);
+    a1 = fma(q[3], (double)x[k].y, a1);
+  }
+}
+
+// (A^ v) at slice sl's lane (its node sits at position 32 sl + lane: the vectors of the finest level
+// are kept in slice order), in chunks of ten slots (five for FP64 values and for what is left): a
+// linear mesh's slice is one or two chunks, two dependent loads each, where a plain unrolled loop
+// takes the slots of its remainder one by one.
+template <typename KT, typename VT>
+__device__ __forceinline__ void slice_product(const FineS& F, const char* vals, int sl, int lane,
+                                              const typename Vec2<VT>::T* v, double& a0, double& a1) {
+  const long long off = F.sl_off[sl];
+  const int W = (int)((F.sl_off[sl + 1] - off) >> 5);
+  const int* cp = F.cols + off + lane;
+  const char* vp = vals + (off + lane) * (long long)(4 * sizeof(KT));
+  a0 = 0;
+  a1 = 0;
+  for (int k0 = 0; k0 < W;) {  // the width is the same for the whole warp
+    if (sizeof(KT) < 8 && W - k0 > 5) {
+      slice_chunk<10, KT, VT>(cp, vp, k0, W, v, a0, a1);
+      k0 += 10;
+    } else {
+      slice_chunk<5, KT, VT>(cp, vp, k0, W, v, a0, a1);
+      k0 += 5;
+    }
+  }
+}
+
+// z = w (2 b - A^ b) + Q z_c at the lane of slice sl, finest level (the caller stores it).
+template <typename LT, typename VT, typename QT>
+__device__ __forceinline__ void cyc_up0_node(const FineS& F, const LevS& L, int sl, int lane, int g, bool valid,
+                                             const typename Vec2<VT>::T* b, const typename Vec2<VT>::T* zc, double w,
+                                             typename Vec2<VT>::T& bv, double& z0, double& z1) {
+  constexpr int CH = sizeof(VT) == 4 ? 4 : 2;
+  bv.x = bv.y = 0;
+  z0 = z1 = 0;
+  if (!valid) return;
+  bv = b[g];
+  double a0, a1;
+  slice_product<LT, VT>(F, F.lv, sl, lane, b, a0, a1);
+  z0 = w * (2.0 * (double)bv.x - a0);
+  z1 = w * (2.0 * (double)bv.y - a1);
+  row_product<CH, QT, VT>(L.qcol, L.qval, L.qptr[g], L.qptr[g + 1], 1, zc, 1.0, z0, z1);
+}
+
+// Per-thread phase clock of a profiled solve: the first thread of a team's first CTA adds the time
+// since the last mark, weighted with the team's share of the grid, to the class of the pass.
+enum { CP_SPMV = 0, CP_DOWN0, CP_UP0, CP_OTHER, CP_COUNT };
+__device__ __forceinline__ unsigned long long cyc_now() {
+  unsigned long long v;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v));
+  return v;
+}
+
+}  // namespace ua

@@ -1,0 +1,816 @@
+// Resident PCG of the uv Newton system: one cooperative launch runs the whole preconditioned
+// conjugate-gradient solve of every selected system (ua_cycle.cuh: collapsed V-cycle, teams).
+//
+// What bounds the inner solve of a mesh up to some 100,000 nodes is not memory but the chain of
+// short passes: with one launch per pass a PCG step of the 141x71 mesh took 72 us in 19 launches
+// of about 3.8 us.  Here a step is 1 + 2 L passes for L levels above the dense one (24 us on that
+// mesh), a team barrier costs 1.25 us whatever the team's size, nothing is launched inside the
+// solve, the systems of a batch do not wait for one another and the host neither checks nor
+// over-runs the convergence.  With a launch per pass and with the resident kernel, one B200: uv P1
+// 141x71 FP64 25.8 and 12.9 ms, P2 101x51 mixed 41.6 and 21.6 ms, P2 401x201 FP64 180 and 125 ms,
+// 16 meshes of 2k-200k elements mixed 84 and 58 ms.
+#include <algorithm>
+#include <cstring>
+#include "ua_cycle.cuh"
+
+namespace ua {
+
+// ---------------------------------------------------------------------------
+// set-up: values of the collapsed cycle for a new tangent
+// ---------------------------------------------------------------------------
+
+// D^-1/2 per node of a level (0 on masked and empty rows), and on the finest level D itself in
+// slice order
+template <typename VT>
+__global__ void k_cyc_scale(int nn, const int* node_sys, const int* node_off, const int* dof_off, const VT* invd,
+                            double2* sc, VT* dw, const int* ipos, const int* sel) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= nn) return;
+  const int s = node_sys[g];
+  if (sel && !sel[s]) return;
+  const int no = node_off[s], n = node_off[s + 1] - no, i = dof_off[s] + (g - no);
+  const double du = (double)invd[i], dv = (double)invd[i + n];
+  sc[g] = make_double2(sqrt(du), sqrt(dv));
+  if (dw) {
+    const size_t k = 2 * (size_t)ipos[g];
+    dw[k] = (VT)(du > 0 ? 1.0 / du : 0.0);
+    dw[k + 1] = (VT)(dv > 0 ? 1.0 / dv : 0.0);
+  }
+}
+
+constexpr int kCycArena = 212 * 1024;       // with the kernel's static tables below 227 KB
+constexpr int kCycArenaSmall = 64 * 1024;
+
+template <typename T> struct QuadSet;
+template <> struct QuadSet<double> {
+  static __device__ __forceinline__ void set(void* base, long long e, double a, double b, double c, double d) {
+    double2* p = reinterpret_cast<double2*>(base) + 2 * e;
+    p[0] = make_double2(a, b);
+    p[1] = make_double2(c, d);
+  }
+};
+template <> struct QuadSet<float> {
+  static __device__ __forceinline__ void set(void* base, long long e, double a, double b, double c, double d) {
+    reinterpret_cast<float4*>(base)[e] = make_float4((float)a, (float)b, (float)c, (float)d);
+  }
+};
+template <> struct QuadSet<__nv_bfloat16> {
+  static __device__ __forceinline__ void set(void* base, long long e, double a, double b, double c, double d) {
+    pq_set(reinterpret_cast<PQuadH*>(base) + e, a, b, c, d);
+  }
+};
+
+// Columns of the node slices as slice positions, once per handle (padding slots: the lane's own).
+__global__ void __launch_bounds__(256) k_cyc_cols(CycFine F, const int* sb_n0, const int* sb_cnt, const int* nodeptr,
+                                                  const int* nodecol, const int* ipos, int* cols) {
+  const int sb = blockIdx.x, w = threadIdx.x >> 5, t = threadIdx.x & 31, pos = w * 32 + t, sl = sb * kSellSlices + w;
+  const long long o0 = F.sl_off[sl];
+  const int W = (int)((F.sl_off[sl + 1] - o0) >> 5);
+  const int at = sb_n0[sb] + min(pos, sb_cnt[sb] - 1);
+  const int p0 = nodeptr[F.perm[at]], deg = pos < sb_cnt[sb] ? nodeptr[F.perm[at] + 1] - p0 : 0;
+  for (int k = 0; k < W; ++k) cols[o0 + 32LL * k + t] = k < deg ? ipos[nodecol[p0 + k]] : at;
+}
+
+// Scaled values of the finest level in its node slices (layout of k_sell_fill), from the dof CSR
+// (row (c, g): the u block then the v block of deg(g) entries).  One CTA per slice block.
+template <typename KT>
+__global__ void __launch_bounds__(256) k_cyc_fill0(CycFine F, const int* sb_n0, const int* sb_cnt, const int* sb_sys, const int* node_off,
+                                                   const int* dof_off, const int* rowptr, const int* colind,
+                                                   const KT* K, const double2* sc, KT* vk, __nv_bfloat16* vlo,
+                                                   const int* sel) {
+  const int sb = blockIdx.x, s = sb_sys[sb];
+  if (sel && !sel[s]) return;
+  const int w = threadIdx.x >> 5, t = threadIdx.x & 31, pos = w * 32 + t, sl = sb * kSellSlices + w;
+  const long long o0 = F.sl_off[sl];
+  const int W = (int)((F.sl_off[sl + 1] - o0) >> 5);
+  if (W == 0) return;
+  const int no = node_off[s], nn = node_off[s + 1] - no, d0 = dof_off[s];
+  int r0 = 0, r1 = 0, deg = 0;
+  double2 si = make_double2(0, 0);
+  if (pos < sb_cnt[sb]) {
+    const int g = F.perm[sb_n0[sb] + pos], i = d0 + (g - no);
+    r0 = rowptr[i];
+    r1 = rowptr[i + nn];
+    deg = (rowptr[i + 1] - r0) >> 1;
+    si = sc[g];
+  }
+  for (int k = 0; k < W; ++k) {
+    const long long d = o0 + 32LL * k + t;
+    double e0 = 0, e1 = 0, e2 = 0, e3 = 0;
+    if (k < deg) {
+      const double2 sj = sc[no + (colind[r0 + k] - d0)];
+      e0 = si.x * (double)K[r0 + k] * sj.x;
+      e1 = si.x * (double)K[r0 + deg + k] * sj.y;
+      e2 = si.y * (double)K[r1 + k] * sj.x;
+      e3 = si.y * (double)K[r1 + deg + k] * sj.y;
+    }
+    QuadSet<KT>::set(vk, d, e0, e1, e2, e3);
+    if (vlo) QuadSet<__nv_bfloat16>::set(vlo, d, e0, e1, e2, e3);
+  }
+}
+
+// Scaled quads of a coarse level, node-row order: 4 lanes per node.
+template <typename KT>
+__global__ void k_cyc_a(int nn, const int* node_sys, const int* node_off, const int* dof_off, const int* rowptr,
+                        const KT* A, const int* nptr, const int* ncol, const double2* sc, void* out,
+                        const int* sel) {
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, lane = threadIdx.x & 3;
+  if (g >= nn) return;
+  const int s = node_sys[g];
+  if (sel && !sel[s]) return;
+  const int no = node_off[s], n = node_off[s + 1] - no, i = dof_off[s] + (g - no);
+  const int r0 = rowptr[i], r1 = rowptr[i + n], p0 = nptr[g], deg = nptr[g + 1] - p0;
+  const double2 si = sc[g];
+  for (int k = lane; k < deg; k += 4) {
+    const double2 sj = sc[ncol[p0 + k]];
+    QuadSet<KT>::set(out, p0 + k, si.x * (double)A[r0 + k] * sj.x, si.x * (double)A[r0 + deg + k] * sj.y,
+                     si.y * (double)A[r1 + k] * sj.x, si.y * (double)A[r1 + deg + k] * sj.y);
+  }
+}
+
+// Q = D^1/2 (P - D^-1 A P) D_c^-1/2 in the A P pattern, written in row order and in the order of
+// Q': 4 lanes per fine node.  A P values in the set-up's layout (row c: [c2 = 0 (dA)][c2 = 1 (dA)]);
+// P quads in pn order.  Coarse nodes on the system's coarsest level are not scaled.
+template <typename ST, typename PT, typename QT>
+__global__ void k_cyc_q(int nn, const int* node_sys, const int* depth, int l, const int* pn_ptr, const int* pn_col,
+                        const PT* P, const int* apn_ptr, const int* apn_col, const int* apbase, const int* apnnz,
+                        const int* apoff, const ST* AP, const double2* sc, const double2* scc, const int* qrow,
+                        const int* tpos, void* out, void* outT, const int* sel) {
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, lane = threadIdx.x & 3;
+  if (g >= nn) return;
+  const int s = node_sys[g];
+  if (sel && !sel[s]) return;
+  const int ar = apn_ptr[g], dA = apn_ptr[g + 1] - ar, pr = pn_ptr[g], pe = pn_ptr[g + 1];
+  const size_t ars = (size_t)2 * apnnz[s];
+  const ST* a0 = AP + apoff[s] + 2 * (size_t)(ar - apbase[s]);
+  const double2 si = sc[g];
+  const double iu = si.x > 0 ? 1.0 / si.x : 0.0, iv = si.y > 0 ? 1.0 / si.y : 0.0;
+  const bool scaled = depth[s] > l + 1;
+  for (int t = lane; t < dA; t += 4) {
+    const int J = apn_col[ar + t];
+    double p[4] = {0, 0, 0, 0};
+    for (int k = pr; k < pe; ++k)
+      if (pn_col[k] == J) pq_get(P + k, p);
+    const double2 sj = scaled ? scc[J] : make_double2(1.0, 1.0);
+    const double q0 = (iu * p[0] - si.x * (double)a0[t]) * sj.x, q1 = (iu * p[1] - si.x * (double)a0[dA + t]) * sj.y;
+    const double q2 = (iv * p[2] - si.y * (double)a0[ars + t]) * sj.x,
+                 q3 = (iv * p[3] - si.y * (double)a0[ars + dA + t]) * sj.y;
+    const int e = qrow[g] + t;
+    QuadSet<QT>::set(out, e, q0, q1, q2, q3);
+    QuadSet<QT>::set(outT, tpos[e], q0, q1, q2, q3);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// host: structure
+// ---------------------------------------------------------------------------
+
+bool cycle_supported(const ua_mesh* m) {
+  const Amg* a = m->amg;
+  if (!a || !a->sa || a->nlev > kCycMaxLev || a->cyc.failed) return false;
+  static thread_local int dev = -1, coop = 0;
+  if (dev != m->device) {
+    coop = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->device);
+    dev = m->device;
+  }
+  return coop != 0;
+}
+
+// Lists and buffers of the collapsed cycle, once per handle (the node slices of the finest level
+// must be there).
+int cycle_init(ua_mesh* m) {
+  Amg* a = m->amg;
+  Cycle& C = a->cyc;
+  if (C.ready) return UA_OK;
+  if (!cycle_supported(m) || !a->sell.ready) return UA_ERR_INVALID;
+  const int nsys = a->nsys, nl = a->nlev;
+  bool ok = true;
+  C.lev.resize(nl);
+  const Sell& SL = a->sell;
+  std::vector<int> ipos(std::max(a->lev[0].nn, 1), 0);
+  for (int k = 0; k < a->lev[0].nn; ++k) ipos[SL.h_perm[k]] = k;
+  C.d_ipos = upload(m, a, ipos, ok);
+  C.d_pcol = (int*)dalloc(m, a, sizeof(int) * (size_t)SL.slots, ok);
+  C.d_r2 = dalloc(m, a, 2 * sizeof(double) * (size_t)std::max(a->lev[0].nn, 1), ok);
+  for (int l = 0; l < nl; ++l) {
+    AmgLevel& L = a->lev[l];
+    Cycle::Lev& D = C.lev[l];
+    D.sc = (double2*)dalloc(m, a, sizeof(double2) * (size_t)std::max(L.nn, 1), ok);
+    if (l > 0) {
+      D.nptr = upload(m, a, a->h_gptr[l], ok);
+      D.ncol = upload(m, a, a->h_gcol[l], ok);
+    }
+    if (l + 1 < nl) {
+      // Q: the A P pattern, on the finest level with its rows in slice order; Q': by coarse node,
+      // the fine nodes (positions) ascending
+      const std::vector<int>&ap = a->h_apnp[l], &ac = a->h_apnc[l];
+      const int nc = a->lev[l + 1].nn;
+      D.nq = (long long)ac.size();
+      std::vector<int> qp, qc, qr, tp(nc + 1, 0), tf(ac.size()), tpos(ac.size());
+      const std::vector<int>*pp = &ap, *pc = &ac;
+      if (l == 0) {
+        qp.assign(L.nn + 1, 0);
+        qr.assign(L.nn, 0);
+        qc.resize(ac.size());
+        for (int k = 0; k < L.nn; ++k) {
+          const int g = SL.h_perm[k], b = ap[g], n = ap[g + 1] - b;
+          qr[g] = qp[k];
+          for (int t = 0; t < n; ++t) qc[qp[k] + t] = ac[b + t];
+          qp[k + 1] = qp[k] + n;
+        }
+        pp = &qp;
+        pc = &qc;
+        D.qptr = upload(m, a, qp, ok);
+        D.qcol = upload(m, a, qc, ok);
+        D.qrow = upload(m, a, qr, ok);
+      } else {
+        D.qptr = L.apn_ptr;
+        D.qcol = L.apn_col;
+        D.qrow = L.apn_ptr;
+      }
+      for (int J : *pc) tp[J + 1]++;
+      for (int J = 0; J < nc; ++J) tp[J + 1] += tp[J];
+      std::vector<int> nx(tp.begin(), tp.end() - 1);
+      for (int k = 0; k < L.nn; ++k)
+        for (int t = (*pp)[k]; t < (*pp)[k + 1]; ++t) {
+          const int u = nx[(*pc)[t]]++;
+          tf[u] = k;
+          tpos[t] = u;
+        }
+      D.tptr = upload(m, a, tp, ok);
+      D.tfine = upload(m, a, tf, ok);
+      D.tpos = upload(m, a, tpos, ok);
+      for (int w = 0; w < 2; ++w) {  // bytes a step reads of this level (FP64, mixed form)
+        C.h_bytes[w].resize(nsys, 0.0);
+        for (int s = 0; s < nsys; ++s) {
+          const int g0 = L.node_off[s], g1 = L.node_off[s + 1];
+          if (g1 == g0) continue;
+          double b = 2.0 * (ap[g1] - ap[g0]) * (w ? 12 : 36);
+          if (l == 0)
+            b += (double)(SL.h_sl_off[kSellSlices * SL.h_sys_sb_off[s + 1]] - SL.h_sl_off[kSellSlices * SL.h_sys_sb_off[s]]) *
+                 (w ? 28 : 36);
+          else
+            b += (double)(a->h_gptr[l][g1] - a->h_gptr[l][g0]) * (w ? 20 : 36);
+          C.h_bytes[w][s] += b + 8.0 * (g1 - g0);
+        }
+      }
+    }
+  }
+  C.sys.resize(nsys);
+  for (int s = 0; s < nsys; ++s) {
+    CycSys& S = C.sys[s];
+    std::memset(&S, 0, sizeof(S));
+    S.depth = a->depth[s];
+    S.dn = a->h_dn[s];
+    S.doff = a->h_doff[s];
+    S.sl0 = kSellSlices * a->sell.h_sys_sb_off[s];
+    for (int l = 0; l <= S.depth; ++l) {
+      S.n0[l] = a->lev[l].node_off[s];
+      S.nn[l] = a->lev[l].node_off[s + 1] - S.n0[l];
+    }
+    S.nsl = (S.nn[0] + 31) / 32;
+  }
+  C.d_sys = upload(m, a, C.sys, ok);
+  C.nslices = (long long)kSellSlices * a->sell.nsb;
+  C.d_part = (double*)dalloc(m, a, sizeof(double) * 3 * (size_t)std::max(C.nslices, 1LL), ok);
+  C.d_cta = (int4*)dalloc(m, a, sizeof(int4) * 1024, ok);
+  C.d_team = (int*)dalloc(m, a, sizeof(int) * 1024, ok);
+  C.d_queue = (int*)dalloc(m, a, sizeof(int) * (size_t)nsys, ok);
+  C.d_bar = (unsigned*)dalloc(m, a, sizeof(unsigned) * 32 * 1024, ok);
+  C.d_prof = (unsigned long long*)dalloc(m, a, sizeof(unsigned long long) * 2 * CP_COUNT, ok);
+  C.d_err = (int*)dalloc(m, a, sizeof(int), ok);
+  if (ok && cudaMallocHost(&C.h_stage, sizeof(int) * (5 * 1024 + (size_t)nsys)) != cudaSuccess) ok = false;
+  if (!ok) {
+    C.failed = true;
+    return set_error(UA_ERR_OOM, "collapsed cycle: allocation failed");
+  }
+  if (SL.nsb)
+    k_cyc_cols<<<SL.nsb, 256, 0, m->stream>>>(CycFine{SL.perm, SL.sl_off, nullptr}, SL.sb_n0, SL.sb_cnt,
+                                              m->dm.nodeptr, m->dm.nodecol, C.d_ipos, C.d_pcol);
+  if (cudaGetLastError() != cudaSuccess) {
+    C.failed = true;
+    return set_error(UA_ERR_CUDA, "collapsed cycle: launch failed");
+  }
+  // the host lists served their purpose
+  for (auto* v : {&a->h_gptr, &a->h_gcol, &a->h_apnp, &a->h_apnc}) std::vector<std::vector<int>>().swap(*v);
+  C.ready = true;
+  return UA_OK;
+}
+
+// Buffers of the values in this precision (before any capture).
+int cycle_alloc_values(ua_mesh* m, bool fp32, bool lo) {
+  Amg* a = m->amg;
+  Cycle& C = a->cyc;
+  Sell& S = a->sell;
+  bool ok = true;
+  auto need = [&](void** p, size_t bytes) {
+    if (!*p) *p = dalloc(m, a, std::max<size_t>(bytes, 32), ok);
+  };
+  const size_t nv = 4 * (size_t)S.slots;
+  if (fp32) need((void**)&S.v32, sizeof(float) * nv);
+  else need((void**)&S.v64, sizeof(double) * nv);
+  if (lo) need((void**)&S.vlo, sizeof(__nv_bfloat16) * nv);
+  for (int l = 0; l < a->nlev; ++l) {
+    Cycle::Lev& D = C.lev[l];
+    // levels 1 .. nlev-2 hold an operator; node entries = dof entries / 4
+    if (l > 0 && l + 1 < a->nlev) need(fp32 ? &D.a32 : &D.a64, (fp32 ? 16 : 32) * (size_t)(a->lev[l].nnz / 4));
+    if (l + 1 < a->nlev) {
+      need(fp32 ? &D.qh : &D.qd, (fp32 ? 8 : 32) * (size_t)D.nq);
+      need(fp32 ? &D.th : &D.td, (fp32 ? 8 : 32) * (size_t)D.nq);
+    }
+  }
+  return ok ? UA_OK : set_error(UA_ERR_OOM, "collapsed cycle: device allocation of the values failed");
+}
+
+// Values of the collapsed cycle from the numeric set-up just enqueued (launches only, capturable).
+// dw: the finest level's D per node, for the residual norm.
+template <typename KT, typename VT>
+static void cycle_fill_t(ua_mesh* m, const int* rowptr0, const int* colind0, const KT* K0, bool lo, VT* dw,
+                         const int* sel, long long* launches) {
+  using ST = KT;
+  using PT = typename PQuadOf<KT>::T;
+  using QT = typename std::conditional<sizeof(KT) == 4, __nv_bfloat16, double>::type;
+  Amg* a = m->amg;
+  Cycle& C = a->cyc;
+  Sell& S = a->sell;
+  cudaStream_t st = m->stream;
+  for (int l = 0; l + 1 < a->nlev; ++l) {
+    AmgLevel& L = a->lev[l];
+    if (!L.nn) continue;
+    k_cyc_scale<VT><<<(L.nn + 255) / 256, 256, 0, st>>>(L.nn, L.node_sys, L.d_node_off, L.d_dof_off,
+                                                        (const VT*)L.invd, C.lev[l].sc, l == 0 ? dw : nullptr, C.d_ipos, sel),
+        ++*launches;
+  }
+  const CycFine F{S.perm, S.sl_off, C.d_pcol};
+  KT* vk = sizeof(KT) == 4 ? (KT*)S.v32 : (KT*)S.v64;
+  if (S.nsb)
+    k_cyc_fill0<KT><<<S.nsb, 256, 0, st>>>(F, S.sb_n0, S.sb_cnt, S.sb_sys, a->lev[0].d_node_off, a->lev[0].d_dof_off, rowptr0, colind0,
+                                           K0, C.lev[0].sc, vk, lo ? S.vlo : nullptr, sel), ++*launches;
+  for (int l = 0; l + 1 < a->nlev; ++l) {
+    AmgLevel& L = a->lev[l];
+    Cycle::Lev& D = C.lev[l];
+    if (!L.nn) continue;
+    if (l > 0)
+      k_cyc_a<KT><<<(L.nn + 63) / 64, 256, 0, st>>>(L.nn, L.node_sys, L.d_node_off, L.d_dof_off, L.rowptr,
+                                                    (const KT*)L.A, D.nptr, D.ncol, D.sc,
+                                                    sizeof(KT) == 4 ? D.a32 : D.a64, sel), ++*launches;
+    const PT* P = (const PT*)(sizeof(KT) == 4 ? L.sa_qh : L.sa_qd);
+    void* q = sizeof(KT) == 4 ? D.qh : D.qd;
+    void* qt = sizeof(KT) == 4 ? D.th : D.td;
+    k_cyc_q<ST, PT, QT><<<(L.nn + 63) / 64, 256, 0, st>>>(L.nn, L.node_sys, a->d_depth, l, L.pn_ptr, L.pn_col, P,
+                                                          L.apn_ptr, L.apn_col, L.apbase, L.apnnz, L.apoff,
+                                                          (const ST*)L.sa_ap, D.sc, C.lev[l + 1].sc, D.qrow, D.tpos,
+                                                          q, qt, sel), ++*launches;
+  }
+}
+
+void cycle_fill(ua_mesh* m, const int* rowptr0, const int* colind0, const void* K0, bool fp32, bool lo, void* dw,
+                const int* sel, long long* launches) {
+  if (fp32) cycle_fill_t<float, float>(m, rowptr0, colind0, (const float*)K0, lo, (float*)dw, sel, launches);
+  else cycle_fill_t<double, double>(m, rowptr0, colind0, (const double*)K0, lo, (double*)dw, sel, launches);
+}
+
+// ---------------------------------------------------------------------------
+// schedule: CTAs -> teams, systems -> queues
+// ---------------------------------------------------------------------------
+
+// Up to half as many systems as CTAs: every system gets a team of its own and the CTAs go, one by
+// one, to the team that would finish last.  More systems than that: equal teams, the systems dealt
+// out largest first to the team with the least work.  The time of a system on T CTAs is modelled
+// as steps x (a + nodes / (b T)): a the passes' latency, b the nodes a CTA streams per microsecond.
+void cycle_schedule(const std::vector<CycSys>& sys, const std::vector<int>& sel, const std::vector<int>& steps,
+                    int nsm, CycSchedule& out) {
+  constexpr double kLatency = 16.0, kNodesPerUs = 90.0;
+  constexpr int kSlicesPerCta = 4;  // a team grows while each of its CTAs has at least this many slices
+  std::vector<int> list;
+  for (int s = 0; s < (int)sys.size(); ++s)
+    if (sel[s]) list.push_back(s);
+  const int n = (int)list.size();
+  out.cta.clear();
+  out.team.clear();
+  out.queue.clear();
+  if (!n) return;
+  auto time = [&](int s, int T) {
+    return std::max(1, steps[s]) * (kLatency + sys[s].nn[0] / (kNodesPerUs * T));
+  };
+  auto cap = [&](int s) { return std::max(1, std::min(nsm, (sys[s].nsl + kSlicesPerCta - 1) / kSlicesPerCta)); };
+  if (2 * n <= nsm) {
+    std::vector<int> T(n, 1);
+    for (int left = nsm - n; left > 0; --left) {
+      int best = -1;
+      double tb = -1;
+      for (int i = 0; i < n; ++i) {
+        const double t = time(list[i], T[i]);
+        if (t > tb && T[i] < cap(list[i])) {
+          tb = t;
+          best = i;
+        }
+      }
+      if (best < 0) break;
+      T[best]++;
+    }
+    for (int i = 0; i < n; ++i) {
+      for (int r = 0; r < T[i]; ++r) {
+        out.cta.push_back(make_int4(i, i + 1, r, T[i]));
+        out.team.push_back(i);
+      }
+      out.queue.push_back(list[i]);
+    }
+    return;
+  }
+  const int T = n <= nsm ? 2 : 4, nt = std::max(1, nsm / T);
+  std::sort(list.begin(), list.end(), [&](int p, int q) {
+    const double a = time(p, T), b = time(q, T);
+    return a != b ? a > b : p < q;
+  });
+  std::vector<std::vector<int>> q(nt);
+  std::vector<double> load(nt, 0.0);
+  for (int s : list) {
+    const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    q[k].push_back(s);
+    load[k] += time(s, T);
+  }
+  for (int k = 0; k < nt; ++k) {
+    const int b = (int)out.queue.size();
+    out.queue.insert(out.queue.end(), q[k].begin(), q[k].end());
+    for (int r = 0; r < T; ++r) {
+      out.cta.push_back(make_int4(b, (int)out.queue.size(), r, T));
+      out.team.push_back(k);
+    }
+  }
+}
+
+// Uploads the schedule and clears the team counters (the stream has drained: the pinned staging
+// is free).
+static int upload_schedule(ua_mesh* m, const CycSchedule& s) {
+  Cycle& C = m->amg->cyc;
+  const int nc = (int)s.cta.size(), nq = (int)s.queue.size();
+  if (nc > 1024) return set_error(UA_ERR_INVALID, "resident solve: schedule of %d CTAs", nc);
+  std::memcpy(C.h_stage, s.cta.data(), sizeof(int4) * nc);
+  std::memcpy(C.h_stage + 4 * 1024, s.team.data(), sizeof(int) * nc);
+  std::memcpy(C.h_stage + 5 * 1024, s.queue.data(), sizeof(int) * nq);
+  UA_CUDA_TRY(cudaMemcpyAsync(C.d_cta, C.h_stage, sizeof(int4) * nc, cudaMemcpyHostToDevice, m->stream));
+  UA_CUDA_TRY(cudaMemcpyAsync(C.d_team, C.h_stage + 4 * 1024, sizeof(int) * nc, cudaMemcpyHostToDevice, m->stream));
+  UA_CUDA_TRY(cudaMemcpyAsync(C.d_queue, C.h_stage + 5 * 1024, sizeof(int) * nq, cudaMemcpyHostToDevice, m->stream));
+  UA_CUDA_TRY(cudaMemsetAsync(C.d_bar, 0, sizeof(unsigned) * 32 * (size_t)(s.team.back() + 1), m->stream));
+  UA_CUDA_TRY(cudaMemsetAsync(C.d_err, 0, sizeof(int), m->stream));
+  return UA_OK;
+}
+
+static CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof) {
+  const Amg* a = m->amg;
+  const Cycle& C = a->cyc;
+  CycArgs A{};
+  for (int l = 0; l + 1 < a->nlev; ++l) {
+    const AmgLevel& L = a->lev[l];
+    const Cycle::Lev& D = C.lev[l];
+    A.lev[l] = CycLev{D.nptr, D.ncol, fp32 ? D.a32 : D.a64, D.qptr, D.qcol, fp32 ? D.qh : D.qd,
+                      D.tptr, D.tfine, fp32 ? D.th : D.td, L.b, L.x2};
+  }
+  A.lev[a->nlev - 1].b = a->lev[a->nlev - 1].b;
+  A.fine = CycFine{a->sell.perm, a->sell.sl_off, C.d_pcol};
+  A.sys = C.d_sys;
+  A.dense = a->dense;
+  A.cta = C.d_cta;
+  A.team = C.d_team;
+  A.queue = C.d_queue;
+  A.bar = C.d_bar;
+  A.err = C.d_err;
+  A.prof = prof ? C.d_prof : nullptr;
+  A.part = C.d_part;
+  A.nslices = C.nslices;
+  return A;
+}
+
+// ---------------------------------------------------------------------------
+// device: PCG
+// ---------------------------------------------------------------------------
+
+// First residual in scaled form: r = D^-1/2 mask(f - K x0), LPR lanes per dof row.
+template <typename KT, typename VT, int LPR>
+__global__ void __launch_bounds__(256) k_cyc_r0(const int* rb_start, const int* rb_sys, const int* sel,
+                                                const int* node_off, const int* dof_off, const int* rowptr,
+                                                const int* colind, const KT* K, const double* x0, const double* f,
+                                                const double2* sc, const int* ipos, VT* r) {
+  const int blk = blockIdx.x, s = rb_sys[blk];
+  if (!sel[s]) return;
+  const int rs = rb_start[blk], re = rb_start[blk + 1];
+  const int no = node_off[s], nn = node_off[s + 1] - no, d0 = dof_off[s];
+  const int lane = threadIdx.x % LPR, grp = threadIdx.x / LPR, ngrp = blockDim.x / LPR;
+  for (int row0 = rs; row0 < re; row0 += ngrp) {
+    const int row = row0 + grp;
+    const bool valid = row < re;
+    double acc = 0;
+    if (valid)
+      for (int j = rowptr[row] + lane; j < rowptr[row + 1]; j += LPR) {
+        const double x = x0[colind[j]];
+        if (x != 0) acc += (double)K[j] * x;
+      }
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, LPR);
+    if (valid && lane == 0) {
+      const int i = row - d0, c = i >= nn ? 1 : 0, g = no + i - c * nn;
+      const double2 d = sc[g];
+      const double w = c ? d.y : d.x;
+      r[2 * (size_t)ipos[g] + c] = (VT)(w > 0 ? w * (f[row] - acc) : 0.0);
+    }
+  }
+}
+
+#define UA_TEAM_SYNC(t)                                               \
+  do {                                                                \
+    if (!team_sync(t)) {                                              \
+      if (threadIdx.x == 0) *a.cyc.err = 1;                           \
+      return;                                                         \
+    }                                                                 \
+  } while (0)
+
+struct PcgArgs {
+  CycArgs cyc;
+  const void *kv, *lv;       // finest level: PCG operator, V-cycle operator (scaled, node slices)
+  void *r, *r2, *z, *p, *q;  // pairs per node in slice order (VT)
+  double2* x;                // FP64 pairs
+  const void* dw;            // D per node in slice order (VT pairs): |r|^2 = sum D r^2
+  const double2* sc;
+  double* dX;
+  const int* dof_off;
+  double* sysv_tol2;         // [nsys] squared relative tolerance
+  int *done, *its, *status;
+  int maxit;
+  int arena;                 // dynamic shared memory for copies of the matrices
+};
+
+// The whole PCG of the systems in the team's queue.  The passes of a step, a team barrier after
+// each:  the levels down (but the finest), the dense level (by every CTA for itself, no barrier),
+// the levels up, the finest up pass with the partials of r.z, the operator pass (p and q are
+// updated in it: q = A z + beta q, partials p.q), and the vector update together with the finest
+// restriction, which forms r - alpha q as it gathers (the new residual goes to a second buffer).
+// All scalars are computed by every CTA from the per-slice partials, so nothing but vectors and
+// partials crosses CTAs.
+// 512 threads of up to 128 registers, one CTA per SM: few warps, each with up to ten slots of its
+// slice in flight (1024 threads at 64 registers spilled 800 bytes a thread).
+template <typename KT, typename LT, typename VT, typename QT>
+__global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
+  using V2 = typename Vec2<VT>::T;
+  extern __shared__ __align__(16) char arena_mem[];
+  __shared__ CycSys S;
+  __shared__ LevS lev[kCycMaxLev];
+  __shared__ FineS fine;
+  __shared__ double red[3][32];
+  __shared__ DenseSh dsh;
+  __shared__ V2 zcs[kAmgMaxDense / 2];
+  __shared__ int ok;
+  const int4 c = a.cyc.cta[blockIdx.x];
+  TeamCtx t{c.z, c.w, a.cyc.bar + 32 * a.cyc.team[blockIdx.x], 0u, &ok};
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  V2 *z = (V2*)a.z, *p = (V2*)a.p, *q = (V2*)a.q;
+  const V2* dw = (const V2*)a.dw;
+  double *part_pq = a.cyc.part, *part_rz = part_pq + a.cyc.nslices, *part_rr = part_rz + a.cyc.nslices;
+  const bool clk = a.cyc.prof && t.rank == 0 && threadIdx.x == 0;
+  unsigned long long tick = clk ? cyc_now() : 0;
+  auto mark = [&](int cls) {
+    if (!clk) return;
+    const unsigned long long now = cyc_now();
+    atomicAdd(a.cyc.prof + 2 * cls, (now - tick) * (unsigned long long)t.size);
+    atomicAdd(a.cyc.prof + 2 * cls + 1, 1ULL);
+    tick = now;
+  };
+  for (int qi = c.x; qi < c.y; ++qi) {
+    const int s = a.cyc.queue[qi];
+    __syncthreads();  // the shared tables of the previous system are no longer read
+    if (threadIdx.x < (int)(sizeof(CycSys) / sizeof(int)))
+      reinterpret_cast<int*>(&S)[threadIdx.x] = reinterpret_cast<const int*>(a.cyc.sys + s)[threadIdx.x];
+    __syncthreads();
+    Arena ar{arena_mem, a.arena, 0};
+    const double* dense;
+    cyc_stage<KT, LT, QT>(a.cyc, a.kv, a.lv, S, t, ar, lev, &fine, 4 * sizeof(KT), dense);
+    const int n0 = S.n0[0], nn = S.nn[0], dep = S.depth;
+    const V2* bL = (const V2*)a.cyc.lev[dep].b;
+    V2 *r = (V2*)a.r, *rn = (V2*)a.r2;
+    int lo, hi;
+    team_share(t, S.nsl, lo, hi);
+    for (int i = lo + warp; i < hi; i += kCycWarps) {
+      double v = 0;
+      if (32 * i + lane < nn) {
+        const V2 rv = r[n0 + 32 * i + lane], d = dw[n0 + 32 * i + lane];
+        v = (double)d.x * ((double)rv.x * (double)rv.x) + (double)d.y * ((double)rv.y * (double)rv.y);
+      }
+      v = lane_sum(v, 32);
+      if (lane == 0) part_rr[S.sl0 + i] = v;
+    }
+    cyc_down<VT, QT>(lev[0], S, 0, t, r, (V2*)a.cyc.lev[1].b);
+    UA_TEAM_SYNC(t);
+    const double rr0 = team_sum(part_rr + S.sl0, S.nsl, red[2]);
+    const double stop = a.sysv_tol2[s] * rr0;
+    int its = 0, status = 0;
+    double rz_old = 0;
+    mark(CP_OTHER);
+    while (rr0 != 0.0) {
+      // z = cycle(r), the finest restriction done
+      for (int l = 1; l < dep; ++l) {
+        cyc_down<VT, QT>(lev[l], S, l, t, (const V2*)a.cyc.lev[l].b, (V2*)a.cyc.lev[l + 1].b);
+        UA_TEAM_SYNC(t);
+      }
+      cyc_dense<VT>(S, dense, bL, dsh, zcs);
+      const V2* zc = zcs - S.n0[dep];
+      for (int l = dep - 1; l > 0; --l) {
+        cyc_up<VT, KT, QT>(lev[l], S, l, t, (const V2*)a.cyc.lev[l].b, (V2*)a.cyc.lev[l].z, zc);
+        UA_TEAM_SYNC(t);
+        zc = (const V2*)a.cyc.lev[l].z;
+      }
+      mark(CP_OTHER);
+      for (int i = lo + warp; i < hi; i += kCycWarps) {
+        const int g = n0 + 32 * i + lane;
+        const bool valid = 32 * i + lane < nn;
+        V2 bv, o;
+        double z0, z1;
+        cyc_up0_node<LT, VT, QT>(fine, lev[0], S.sl0 + i, lane, g, valid, r, zc, 1.0, bv, z0, z1);
+        o.x = (VT)z0;
+        o.y = (VT)z1;
+        if (valid) z[g] = o;
+        const double v = lane_sum((double)bv.x * (double)o.x + (double)bv.y * (double)o.y, 32);
+        if (lane == 0) part_rz[S.sl0 + i] = v;
+      }
+      UA_TEAM_SYNC(t);
+      const double rz = team_sum(part_rz + S.sl0, S.nsl, red[0]);
+      mark(CP_UP0);
+      const double beta = its ? rz / rz_old : 0.0;
+      rz_old = rz;
+      // p = z + beta p, q = A z + beta q, partials p.q
+      for (int i = lo + warp; i < hi; i += kCycWarps) {
+        const int g = n0 + 32 * i + lane;
+        double v = 0;
+        if (32 * i + lane < nn) {
+          V2 pn = z[g], po, qo;
+          if (its) {
+            po = p[g];
+            qo = q[g];
+          }
+          double a0, a1;
+          slice_product<KT, VT>(fine, fine.kv, S.sl0 + i, lane, z, a0, a1);
+          if (its) {
+            pn.x = (VT)((double)pn.x + beta * (double)po.x);
+            pn.y = (VT)((double)pn.y + beta * (double)po.y);
+            a0 += beta * (double)qo.x;
+            a1 += beta * (double)qo.y;
+          }
+          V2 qn;
+          qn.x = (VT)a0;
+          qn.y = (VT)a1;
+          p[g] = pn;
+          q[g] = qn;
+          v = (double)pn.x * (double)qn.x + (double)pn.y * (double)qn.y;
+        }
+        v = lane_sum(v, 32);
+        if (lane == 0) part_pq[S.sl0 + i] = v;
+      }
+      UA_TEAM_SYNC(t);
+      const double pq = team_sum(part_pq + S.sl0, S.nsl, red[1]);
+      mark(CP_SPMV);
+      if (!(pq > 0)) {  // not positive definite on the free dofs, or breakdown
+        status = 1;
+        break;
+      }
+      const double alpha = rz / pq;
+      // x += alpha p, r -= alpha q, partials |r|^2, and the restriction of the new residual
+      for (int i = lo + warp; i < hi; i += kCycWarps) {
+        double v = 0;
+        const int g = n0 + 32 * i + lane;
+        if (32 * i + lane < nn) {
+          const V2 pv = p[g], qv = q[g], d = dw[g];
+          V2 rv = r[g];
+          double2 xv = its ? a.x[g] : make_double2(0.0, 0.0);
+          xv.x += alpha * (double)pv.x;
+          xv.y += alpha * (double)pv.y;
+          rv.x = (VT)((double)rv.x - alpha * (double)qv.x);
+          rv.y = (VT)((double)rv.y - alpha * (double)qv.y);
+          a.x[g] = xv;
+          rn[g] = rv;
+          v = (double)d.x * ((double)rv.x * (double)rv.x) + (double)d.y * ((double)rv.y * (double)rv.y);
+        }
+        v = lane_sum(v, 32);
+        if (lane == 0) part_rr[S.sl0 + i] = v;
+      }
+      cyc_down<VT, QT>(lev[0], S, 0, t, r, (V2*)a.cyc.lev[1].b, q, alpha);
+      ++its;
+      UA_TEAM_SYNC(t);
+      const double rr = team_sum(part_rr + S.sl0, S.nsl, red[2]);
+      mark(CP_DOWN0);
+      V2* sw = r;
+      r = rn;
+      rn = sw;
+      if (rr <= stop || its >= a.maxit || !(rr == rr)) break;
+    }
+    // dX += D^-1/2 x on the CTA's nodes (x written by this CTA)
+    if (its)
+      for (int i = 32 * lo + threadIdx.x; i < min(32 * hi, nn); i += kCycThreads) {
+        const int g = a.cyc.fine.perm[n0 + i], j = a.dof_off[s] + (g - n0);
+        const double2 xv = a.x[n0 + i], d = a.sc[g];
+        if (d.x > 0) a.dX[j] += d.x * xv.x;
+        if (d.y > 0) a.dX[j + nn] += d.y * xv.y;
+      }
+    if (t.rank == 0 && threadIdx.x == 0) {
+      a.its[s] = its;
+      a.status[s] = status;
+      a.done[s] = 1;
+    }
+  }
+}
+
+template <typename KT, typename LT, typename VT, typename QT>
+static int launch_pcg(ua_mesh* m, const PcgArgs& a, int nctas) {
+  UA_CUDA_TRY(cudaFuncSetAttribute(k_pcg_team<KT, LT, VT, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   kCycArena));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(nctas);
+  cfg.blockDim = dim3(kCycThreads);
+  cfg.dynamicSmemBytes = a.arena;
+  cfg.stream = m->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  UA_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pcg_team<KT, LT, VT, QT>, a));
+  return UA_OK;
+}
+
+int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, const std::vector<int>& steps, int nsm,
+                 long long* launches) {
+  Amg* a = m->amg;
+  Cycle& C = a->cyc;
+  CycSchedule sch;
+  cycle_schedule(C.sys, sel, steps, std::min(nsm, 1024), sch);
+  if (sch.cta.empty()) return UA_OK;
+  if (int rc = upload_schedule(m, sch)) return rc;
+  if (v.prof) UA_CUDA_TRY(cudaMemsetAsync(C.d_prof, 0, sizeof(unsigned long long) * 2 * CP_COUNT, m->stream));
+  const Sell& S = a->sell;
+  PcgArgs A{};
+  A.cyc = cycle_args(m, v.fp32, v.prof);
+  A.kv = v.fp32 ? (const void*)S.v32 : (const void*)S.v64;
+  A.lv = v.fp32 ? (v.lo ? (const void*)S.vlo : (const void*)S.v32) : (const void*)S.v64;
+  A.r = v.r;
+  A.r2 = C.d_r2;
+  // shared memory for the copies: all of it where the largest share of a CTA fits, else what the
+  // small levels take (the rest serves as L1 for the streamed rows)
+  double need = 0;
+  for (const int4& ct : sch.cta)
+    for (int k = ct.x; k < ct.y; ++k) {
+      const CycSys& y = C.sys[sch.queue[k]];
+      need = std::max(need, C.h_bytes[v.fp32][sch.queue[k]] / ct.w + 8.0 * y.dn * y.dn);
+    }
+  need = 1.15 * need + 8192;
+  A.arena = need <= kCycArena ? std::max(16384, (int)need) & ~15 : kCycArenaSmall;
+  A.z = v.z;
+  A.p = v.p;
+  A.q = v.q;
+  A.x = (double2*)v.x;
+  A.dw = v.dw;
+  A.sc = C.lev[0].sc;
+  A.dX = v.dX;
+  A.dof_off = a->lev[0].d_dof_off;
+  A.sysv_tol2 = v.tol2;
+  A.done = v.done;
+  A.its = v.its;
+  A.status = v.status;
+  A.maxit = v.maxit;
+  const int lpr_grid = v.nrb;
+  if (v.fp32)
+    k_cyc_r0<float, float, 4><<<lpr_grid, 256, 0, m->stream>>>(
+        v.rb_start, v.rb_sys, v.sel, a->lev[0].d_node_off, a->lev[0].d_dof_off, v.rowptr, v.colind,
+        (const float*)v.K, v.dX, v.f, C.lev[0].sc, C.d_ipos, (float*)v.r);
+  else
+    k_cyc_r0<double, double, 4><<<lpr_grid, 256, 0, m->stream>>>(
+        v.rb_start, v.rb_sys, v.sel, a->lev[0].d_node_off, a->lev[0].d_dof_off, v.rowptr, v.colind,
+        (const double*)v.K, v.dX, v.f, C.lev[0].sc, C.d_ipos, (double*)v.r);
+  ++*launches;
+  UA_CUDA_TRY(cudaGetLastError());
+  const int nc = C.last_grid = (int)sch.cta.size();
+  int rc;
+  if (!v.fp32) rc = launch_pcg<double, double, double, double>(m, A, nc);
+  else if (v.lo) rc = launch_pcg<float, __nv_bfloat16, float, __nv_bfloat16>(m, A, nc);
+  else rc = launch_pcg<float, float, float, __nv_bfloat16>(m, A, nc);
+  ++*launches;
+  return rc;
+}
+
+// After the solve's stream has drained: whether every barrier was met, and the pass times (ms of
+// the whole grid) and counts of a profiled solve.
+int pcg_resident_status(ua_mesh* m, bool prof, double* ms, int* cnt) {
+  Cycle& C = m->amg->cyc;
+  int err = 0;
+  UA_CUDA_TRY(cudaMemcpy(&err, C.d_err, sizeof(int), cudaMemcpyDeviceToHost));
+  if (err) return set_error(UA_ERR_TIMEOUT, "resident PCG: a team barrier was not met");
+  if (prof) {
+    unsigned long long h[2 * CP_COUNT];
+    UA_CUDA_TRY(cudaMemcpy(h, C.d_prof, sizeof(h), cudaMemcpyDeviceToHost));
+    for (int k = 0; k < CP_COUNT; ++k) {
+      ms[k] += 1e-6 * (double)h[2 * k] / std::max(C.last_grid, 1);
+      cnt[k] += (int)h[2 * k + 1];
+    }
+  }
+  return UA_OK;
+}
+
+}  // namespace ua

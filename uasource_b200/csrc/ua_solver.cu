@@ -58,7 +58,14 @@ struct Prof {
     }
     return pool[used++];
   }
-  void reset() { used = 0; marks.clear(); }
+  // resident solves: pass times and work by class, measured inside the kernel
+  double xms[7] = {}, xnnz[7] = {}, xrows[7] = {};
+  int xn[7] = {};
+  void reset() {
+    used = 0;
+    marks.clear();
+    for (int k = 0; k < 7; ++k) xms[k] = xnnz[k] = xrows[k] = xn[k] = 0;
+  }
   ~Prof() { for (auto e : pool) cudaEventDestroy(e); }
   // per mark: tangent non-zeros and rows of the systems the timed launch works on
   long long* d_act = nullptr;
@@ -211,6 +218,12 @@ static void prof_collect(Work* w, double* kms, int* kn, double* knnz, double* kr
     kms[mk.first] += t;
     kn[mk.first]++;
     if (2 * i + 1 < (int)act.size()) { knnz[mk.first] += (double)act[2 * i]; krows[mk.first] += (double)act[2 * i + 1]; }
+  }
+  for (int k = 0; k < PK_COUNT; ++k) {
+    kms[k] += w->prof.xms[k];
+    kn[k] += w->prof.xn[k];
+    knnz[k] += w->prof.xnnz[k];
+    krows[k] += w->prof.xrows[k];
   }
 }
 
@@ -1371,6 +1384,65 @@ static int cost_eval(ua_mesh* m, const ua_params* p, bool useDir, bool assembleR
   return UA_OK;
 }
 
+// The solve proper in one resident kernel (tolerances, particular solution and the set-up are on
+// the stream), then the multipliers and the iteration counts.
+static int pcg_resident_solve(ua_mesh* m, const ua_params* p, bool fp32, const void* K, int* its_out) {
+  Work* w = m->work;
+  std::vector<int> sel(w->nsys), steps(w->nsys);
+  for (int s = 0; s < w->nsys; ++s) {
+    sel[s] = its_out[s] != 0;
+    steps[s] = its_out[s];
+  }
+  PcgSolve v{};
+  v.fp32 = fp32;
+  v.lo = fp32 && p->precond_bf16;
+  v.prof = w->prof.on;
+  v.rb_start = w->rb_start; v.rb_sys = w->rb_sys; v.nrb = w->nrb;
+  v.sel = w->sel;
+  v.rowptr = w->rowptr; v.colind = w->colind; v.K = K;
+  v.f = w->frhs; v.dX = w->dX;
+  v.r = w->kr; v.z = w->kz; v.p = w->kp; v.q = w->kq;
+  v.x = (double*)w->kx0;
+  v.dw = w->invd;
+  v.tol2 = w->sysv + SV_TOL2 * w->nsys;
+  v.done = w->done; v.its = w->its; v.status = w->status;
+  v.maxit = p->krylov_maxit;
+  cudaEvent_t kev[2];
+  prof_begin(m, PK_KRYLOV, kev);
+  if (int rc = pcg_resident(m, v, sel, steps, w->nsm, &g_launches)) return rc;
+  prof_end(m, kev);
+  if (w->nc) {
+    if (fp32)
+      k_con_multiplier<float><<<(w->nc + 255) / 256, 256, 0, m->stream>>>(
+          w->nc, w->con_dof, w->con_sys, w->sel, w->rowptr, w->colind, (const float*)K, w->dX, w->frhs, w->dlam,
+          con_pairs(w));
+    else
+      k_con_multiplier<double><<<(w->nc + 255) / 256, 256, 0, m->stream>>>(
+          w->nc, w->con_dof, w->con_sys, w->sel, w->rowptr, w->colind, (const double*)K, w->dX, w->frhs, w->dlam,
+          con_pairs(w));
+    ++g_launches;
+  }
+  UA_CUDA_TRY(cudaGetLastError());
+  UA_CUDA_TRY(cudaMemcpyAsync(w->h_int, w->its, w->nsys * sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+  UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
+  double ms[4] = {};
+  int cnt[4] = {};
+  if (int rc = pcg_resident_status(m, w->prof.on, ms, cnt)) return rc;
+  for (int s = 0; s < w->nsys; ++s) its_out[s] = sel[s] ? w->h_int[s] : 0;
+  if (w->prof.on) {
+    const int cls[3] = {PK_SPMV, PK_AMGR, PK_AMGP};
+    for (int k = 0; k < 3; ++k) {
+      w->prof.xms[cls[k]] += ms[k];
+      w->prof.xn[cls[k]] += cnt[k];
+      for (int s = 0; s < w->nsys; ++s) {
+        w->prof.xnnz[cls[k]] += (double)its_out[s] * (m->h_knz_off[s + 1] - m->h_knz_off[s]);
+        w->prof.xrows[cls[k]] += (double)its_out[s] * (m->h_dof_off[s + 1] - m->h_dof_off[s]);
+      }
+    }
+  }
+  return UA_OK;
+}
+
 template <typename KT, typename VT>
 static int pcg_t(ua_mesh* m, const ua_params* p, const KT* K, int* its_out, const double* eta = nullptr) {
   Work* w = m->work;
@@ -1401,6 +1473,12 @@ static int pcg_t(ua_mesh* m, const ua_params* p, const KT* K, int* its_out, cons
   }
   if (amg && amg_setup(m, p->amg_smoothed != 0) != UA_OK) amg = false;  // shapes the hierarchy cannot take keep point Jacobi
   const bool fp32 = sizeof(KT) == 4;
+  // the whole solve in one resident kernel on the collapsed V-cycle; two-entry constraint rows and
+  // the CSR form (krylov_sell = 0) take the launch-per-pass cycle below
+  const bool res = amg && p->krylov_sell && w->npair == 0 && cycle_supported(m) &&
+                   amg_sell_init(m, w->h_sys_rb_off) == UA_OK && cycle_init(m) == UA_OK &&
+                   cycle_alloc_values(m, fp32, fp32 && p->precond_bf16) == UA_OK;
+  const CycFillReq fill{fp32 && p->precond_bf16, w->invd};
   if (amg) {
     // the systems of this Newton step only (the others' hierarchies are not read)
     // prolongator refresh: every Newton step in FP64 (the Newton trajectory of the reference's
@@ -1409,7 +1487,7 @@ static int pcg_t(ua_mesh* m, const ua_params* p, const KT* K, int* its_out, cons
     cudaEvent_t ev[2];
     prof_begin(m, PK_SETUP, ev);
     int rc = amg_numeric(m, w->rowptr, w->colind, K, fp32, w->cmask, &g_launches, w->sel, &w->h_sel, prefresh,
-                         !w->no_graph && !p->profile);
+                         !w->no_graph && !p->profile, res ? &fill : nullptr);
     prof_end(m, ev);
     if (rc) return rc;
   } else {
@@ -1420,6 +1498,7 @@ static int pcg_t(ua_mesh* m, const ua_params* p, const KT* K, int* its_out, cons
   if (w->nc)
     k_con_particular<<<(w->nc + 255) / 256, 256, 0, m->stream>>>(w->nc, w->con_dof, w->con_sys, w->sel, w->con_rhs,
                                                                  w->X, w->dX, w->grhs, con_pairs(w)), ++g_launches;
+  if (res) return pcg_resident_solve(m, p, fp32, K, its_out);
   VT *r = (VT*)w->kr, *z = (VT*)w->kz, *pp = (VT*)w->kp, *q = (VT*)w->kq;
   // with AMG the Jacobi-type kernels write the l1 pre-smoothed vector x0 and the V-cycle writes z (and r.z)
   const VT* invd = amg ? (const VT*)amg_invd0(m) : (const VT*)w->invd;
@@ -1832,7 +1911,8 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
     double t1 = now_ms();
     t_asm += t1 - t0;
     // linear solve (:242-257)
-    for (int s = 0; s < nsys; ++s) its[s] = sel[s];
+    // (the iterations of the last step weigh the systems in the solve's schedule)
+    for (int s = 0; s < nsys; ++s) its[s] = sel[s] ? std::max(1, st[s].kits) : 0;
     std::vector<double> eta(nsys);
     for (int s = 0; s < nsys; ++s) eta[s] = forcing_term(p, st[s].rForce);
     if ((rc = linear_solve(m, p, its, eta.data()))) return rc;
