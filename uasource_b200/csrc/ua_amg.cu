@@ -814,7 +814,7 @@ __global__ void __launch_bounds__(256) k_amg_smooth(const int* rb_start, const i
 // ---------------------------------------------------------------------------
 
 struct SellDev {
-  const int *sb_sys, *sb_n0, *sb_cnt, *sb_rbu, *sb_rbv, *perm;
+  const int *sb_sys, *sb_n0, *sb_cnt, *perm;
   const long long* sl_off;
   const int* cols;
   const int *dof_off, *node_off;  // per system, of the slices' level
@@ -1498,11 +1498,11 @@ static int numeric_t(ua_mesh* m, const int* rowptr0, const int* colind0, const K
 }
 
 static SellDev sell_dev(const ua_mesh* m, const Sell& S) {
-  return SellDev{S.sb_sys, S.sb_n0, S.sb_cnt, S.sb_rbu, S.sb_rbv, S.perm, S.sl_off, S.cols,
+  return SellDev{S.sb_sys, S.sb_n0, S.sb_cnt, S.perm, S.sl_off, S.cols,
                  m->dm.sys_dof_off, m->dm.sys_node_off, m->dm.dbg, 0};
 }
 static SellDev csell_dev(const ua_mesh* m, const Sell& S, const AmgLevel& L, int l) {
-  return SellDev{S.sb_sys, S.sb_n0, S.sb_cnt, nullptr, nullptr, S.perm, S.sl_off, S.cols,
+  return SellDev{S.sb_sys, S.sb_n0, S.sb_cnt, S.perm, S.sl_off, S.cols,
                  L.d_dof_off, L.d_node_off, m->dm.dbg, l};
 }
 
@@ -1569,13 +1569,13 @@ static void csell_init(ua_mesh* m) {
 
 int amg_sell_init(ua_mesh* m, const std::vector<int>& sys_rb_off0) {
   Amg* a = m->amg;
-  if (!a || m->ndof != 2 || m->h_nodeptr.empty()) return UA_ERR_INVALID;
+  if (!a || m->h_nodeptr.empty()) return UA_ERR_INVALID;
   Sell& S = a->sell;
   if (S.ready) return UA_OK;
   if (S.failed) return UA_ERR_INVALID;
   const int nsys = a->nsys;
   if ((int)sys_rb_off0.size() != nsys + 1) { S.failed = true; return UA_ERR_INVALID; }
-  std::vector<int> sb_sys, sb_n0, sb_cnt, sb_rbu, sb_rbv, perm(m->nn_total), idx;
+  std::vector<int> sb_sys, sb_n0, sb_cnt, perm(m->nn_total), idx;
   std::vector<long long> sl_off(1, 0);
   S.h_sys_sb_off.assign(nsys + 1, 0);
   auto deg = [&](int g) { return m->h_nodeptr[g + 1] - m->h_nodeptr[g]; };
@@ -1583,7 +1583,7 @@ int amg_sell_init(ua_mesh* m, const std::vector<int>& sys_rb_off0) {
     const int no = m->h_node_off[s], nn = m->h_node_off[s + 1] - no;
     const int nbc = (nn + kSellNodes - 1) / kSellNodes;
     // the handle's row blocks must be the u blocks then the v blocks of kSellNodes rows each
-    if (sys_rb_off0[s + 1] - sys_rb_off0[s] != 2 * nbc || 2 * nn != m->h_dof_off[s + 1] - m->h_dof_off[s]) {
+    if (m->ndof == 2 && (sys_rb_off0[s + 1] - sys_rb_off0[s] != 2 * nbc || 2 * nn != m->h_dof_off[s + 1] - m->h_dof_off[s])) {
       S.failed = true;
       return set_error(UA_ERR_INVALID, "node slices: row blocks of system %d do not split at the u/v boundary", s);
     }
@@ -1601,8 +1601,6 @@ int amg_sell_init(ua_mesh* m, const std::vector<int>& sys_rb_off0) {
       sb_sys.push_back(s);
       sb_n0.push_back(n0);
       sb_cnt.push_back(cnt);
-      sb_rbu.push_back(sys_rb_off0[s] + i);
-      sb_rbv.push_back(sys_rb_off0[s] + nbc + i);
     }
     S.h_sys_sb_off[s + 1] = (int)sb_sys.size();
   }
@@ -1612,19 +1610,17 @@ int amg_sell_init(ua_mesh* m, const std::vector<int>& sys_rb_off0) {
   S.sb_sys = upload(m, a, sb_sys, ok);
   S.sb_n0 = upload(m, a, sb_n0, ok);
   S.sb_cnt = upload(m, a, sb_cnt, ok);
-  S.sb_rbu = upload(m, a, sb_rbu, ok);
-  S.sb_rbv = upload(m, a, sb_rbv, ok);
   S.perm = upload(m, a, perm, ok);
   S.h_perm = perm;
   S.h_sl_off = sl_off;
   S.sl_off = upload(m, a, sl_off, ok);
-  S.cols = (int*)dalloc(m, a, sizeof(int) * (size_t)S.slots, ok);
+  if (m->ndof == 2) S.cols = (int*)dalloc(m, a, sizeof(int) * (size_t)S.slots, ok);
   S.spart = (double*)dalloc(m, a, sizeof(double) * kSellSlices * (size_t)std::max(S.nsb, 1), ok);
   std::vector<int> sl_pre(nsys + 1);
   for (int s = 0; s <= nsys; ++s) sl_pre[s] = kSellSlices * S.h_sys_sb_off[s];
   S.sys_sl_off = upload(m, a, sl_pre, ok);
   if (!ok) { S.failed = true; return set_error(UA_ERR_OOM, "node slices: device allocation failed"); }
-  if (S.nsb)
+  if (S.nsb && m->ndof == 2)
     k_sell_fill<double><<<S.nsb, 256, 0, m->stream>>>(sell_dev(m, S), m->dm, nullptr, nullptr, nullptr, S.cols,
                                                        nullptr);
   cudaError_t e = cudaGetLastError();
@@ -1986,13 +1982,14 @@ __global__ void k_uvh_scatter(const DevMesh dm, int n2, const int* dof_sys2, con
   out3[dm.sys_dof_off[s] + (i2 - dof2_off[s])] = z2[i2];
 }
 
-int amg_numeric_uvh(ua_mesh* m, const double* K3, const unsigned char* cmask3, long long* launches) {
+int amg_numeric_uvh(ua_mesh* m, const double* K3, const unsigned char* cmask3, long long* launches,
+                    const CycFillReq* cyc, bool graph) {
   Amg* a = m->amg;
   if (!a || m->ndof != 3) return set_error(UA_ERR_INVALID, "no uvh AMG hierarchy");
   AmgLevel& F = a->lev[0];
   k_uvh_extract<<<(F.ndof + 255) / 256, 256, 0, m->stream>>>(m->dm, F.ndof, F.dof_sys, F.d_dof_off, F.d_knz_off,
                                                              K3, cmask3, (double*)F.A, a->uvh_mask), ++*launches;
-  return amg_numeric(m, F.rowptr, F.colind, F.A, false, a->uvh_mask, launches);
+  return amg_numeric(m, F.rowptr, F.colind, F.A, false, a->uvh_mask, launches, nullptr, nullptr, 1, graph, cyc);
 }
 
 int amg_apply_uvh(ua_mesh* m, const double* p3, double* out3, const int* sel, const int* done, int lpr,

@@ -6,6 +6,12 @@ namespace ua {
 
 struct Amg;
 
+// Values of the collapsed cycle to fill after a numeric set-up.
+struct CycFillReq {
+  bool lo;   // BF16 copy of the finest level
+  void* dw;  // receives the finest level's damped l1 diagonal per node (value precision)
+};
+
 // Fine-level view of one preconditioner application z = M^-1 r inside PCG.
 // x0 holds the pre-smoothed fine vector (l1-Jacobi of r, written by the
 // caller with amg_invd0); z receives the result (and pcopy, if set, a copy);
@@ -70,10 +76,6 @@ const void* amg_invd0(const ua_mesh* m);
 // (amg_restart_P) and then every p_refresh-th set-up, the coarse operators every time.
 // graph: run the set-up's launches as a captured CUDA graph (captured once per kind of call).
 // cyc: also fill the values of the collapsed cycle (cycle_init and cycle_alloc_values done).
-struct CycFillReq {
-  bool lo;   // BF16 copy of the finest level
-  void* dw;  // receives the finest level's damped l1 diagonal per node (value precision)
-};
 int amg_numeric(ua_mesh* m, const int* rowptr0, const int* colind0, const void* K0, bool fp32,
                 const unsigned char* cmask, long long* launches, const int* sel = nullptr,
                 const std::vector<int>* h_sel = nullptr, int p_refresh = 1, bool graph = false,
@@ -83,7 +85,8 @@ void amg_restart_P(ua_mesh* m, const std::vector<int>& run);
 // uvh handles: extract the velocity block of the 3-dof tangent K3 (and its
 // constraint mask) into the hierarchy's own finest level, then the numeric
 // phase (FP64).
-int amg_numeric_uvh(ua_mesh* m, const double* K3, const unsigned char* cmask3, long long* launches);
+int amg_numeric_uvh(ua_mesh* m, const double* K3, const unsigned char* cmask3, long long* launches,
+                    const CycFillReq* cyc = nullptr, bool graph = false);
 // out3 = V-cycle(p3) on the velocity rows of 3-dof vectors (other rows untouched).
 int amg_apply_uvh(ua_mesh* m, const double* p3, double* out3, const int* sel, const int* done, int lpr,
                   long long* launches);
@@ -132,6 +135,21 @@ struct PcgSolve {
 // sel: systems to solve; steps: expected iterations (the schedule's weights)
 int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, const std::vector<int>& steps, int nsm,
                  long long* launches);
+struct GmSolve {
+  const int* rowptr;      // 3-dof CSR
+  const double* K;
+  const unsigned char* cmask;
+  const int* sel;
+  const double* f;
+  double* dX;             // in: the particular solution on the constrained dofs; out: the solution
+  const double* tol;      // [nsys] relative tolerances
+  int *done, *its;
+  int mr, hsw, maxit, max_cycles;
+};
+// restarted GMRES of the uvh system (ua_gmres.cu), restart up to gmres_resident_max_restart()
+int gmres_resident_max_restart();
+int gmres_resident(ua_mesh* m, const GmSolve& v, const std::vector<int>& sel, const std::vector<int>& steps, int nsm,
+                   long long* launches);
 // pass classes of a profiled resident solve: operator, finest restriction, finest up pass, rest
 int pcg_resident_status(ua_mesh* m, bool prof, double* ms, int* cnt);
 

@@ -90,7 +90,7 @@ struct Sell {
   std::vector<int> h_sys_sb_off;  // per-system prefix of the slice blocks
   std::vector<int> h_perm;
   std::vector<long long> h_sl_off;
-  int *sb_sys = nullptr, *sb_n0 = nullptr, *sb_cnt = nullptr, *sb_rbu = nullptr, *sb_rbv = nullptr;
+  int *sb_sys = nullptr, *sb_n0 = nullptr, *sb_cnt = nullptr;
   int* perm = nullptr;             // [nn_total]: per block, its global node ids in slice order
   long long* sl_off = nullptr;     // [nsb * kSellSlices + 1] slot offsets of the slices
   int* cols = nullptr;             // [slots]
@@ -138,10 +138,6 @@ struct CycArgs {
   double* part;        // [3][nslices]
   long long nslices;
 };
-struct CycSchedule {
-  std::vector<int4> cta;
-  std::vector<int> team, queue;
-};
 // Set-up data of the collapsed cycle: structure once per handle, values per tangent.
 struct Cycle {
   bool ready = false, failed = false;
@@ -168,6 +164,9 @@ struct Cycle {
   unsigned long long* d_prof = nullptr;
   int* d_err = nullptr;
   int *d_ipos = nullptr, *d_pcol = nullptr;  // node -> slice position; slot columns as positions
+  // uvh: basis and work vectors, partials, 3-dof tangent and inverse thickness l1 sums (slice order)
+  double *gm_buf = nullptr, *gm_part = nullptr, *gm_v3 = nullptr, *gm_hinv = nullptr;
+  int gm_mr = 0;
   void* d_r2 = nullptr;       // second residual buffer
   std::vector<double> h_bytes[2];  // per system: bytes of the matrices a step reads (FP64, mixed)
   int* h_stage = nullptr;     // pinned staging of the schedule

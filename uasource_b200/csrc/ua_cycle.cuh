@@ -171,11 +171,12 @@ __device__ __forceinline__ void stage_csr(Arena& ar, int lo, int hi, int qb, con
 
 // Reads the level tables into shared memory and copies this CTA's rows as far as they fit, the
 // small levels first.  In a team with enough CTAs everything fits: a pass then waits for one
-// gather of the vector instead of three dependent loads.  Every thread keeps the same pointers;
+// gather of the vector instead of three dependent loads.  [slo, shi): the CTA's slices of the finest
+// level (the passes of that level visit no others).  Every thread keeps the same pointers;
 // thread 0 publishes them.
 template <typename KT, typename LT, typename QT>
 __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, const void* lv, const CycSys& S,
-                                          const TeamCtx& t, Arena& ar, LevS* lev, FineS* fine, int kslot,
+                                          const TeamCtx& t, int slo, int shi, Arena& ar, LevS* lev, FineS* fine, int kslot,
                                           const double*& dense) {
   constexpr int qb = 4 * sizeof(QT), ab = 4 * sizeof(KT);
   int lo, hi;
@@ -195,13 +196,13 @@ __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, cons
       stage_csr(ar, S.n0[l] + lo, S.n0[l] + hi, qb, L.qptr, L.qcol, L.qval);
       stage_csr(ar, S.n0[l] + lo, S.n0[l] + hi, ab, L.aptr, L.acol, L.aval);
     } else {
-      team_share(t, S.nsl, lo, hi);
-      stage_csr(ar, S.n0[0] + 32 * lo, S.n0[0] + min(32 * hi, S.nn[0]), qb, L.qptr, L.qcol, L.qval);
+      stage_csr(ar, S.n0[0] + 32 * slo, S.n0[0] + min(32 * shi, S.nn[0]), qb, L.qptr, L.qcol, L.qval);
     }
     if (threadIdx.x == 0) lev[l] = L;
   }
   FineS F{A.fine.sl_off, A.fine.cols, (const char*)kv, (const char*)lv};
-  team_share(t, S.nsl, lo, hi);
+  lo = slo;
+  hi = shi;
   if (lo < hi) {
     const int s0 = S.sl0 + lo, ns = hi - lo;
     const long long e0 = F.sl_off[s0], ne = F.sl_off[S.sl0 + hi] - e0;
@@ -467,6 +468,32 @@ __device__ __forceinline__ void cyc_up0_node(const FineS& F, const LevS& L, int 
   z0 = w * (2.0 * (double)bv.x - a0);
   z1 = w * (2.0 * (double)bv.y - a1);
   row_product<CH, QT, VT>(L.qcol, L.qval, L.qptr[g], L.qptr[g + 1], 1, zc, 1.0, z0, z1);
+}
+
+// ---- host side of a resident launch (ua_pcg.cu) ----
+struct CycSchedule {
+  std::vector<int4> cta;
+  std::vector<int> team, queue;
+};
+void cycle_schedule(const std::vector<CycSys>& sys, const std::vector<int>& sel, const std::vector<int>& steps,
+                    int nsm, CycSchedule& out);
+int upload_schedule(ua_mesh* m, const CycSchedule& s);
+CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof);
+// cooperative launch of a team kernel, one CTA per SM
+template <typename A>
+inline int launch_team(ua_mesh* m, void (*k)(const A), const A& a, int nctas, int smem) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(nctas);
+  cfg.blockDim = dim3(kCycThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = m->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  UA_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, a));
+  return UA_OK;
 }
 
 // Per-thread phase clock of a profiled solve: the first thread of a team's first CTA adds the time

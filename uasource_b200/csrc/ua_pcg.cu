@@ -443,7 +443,7 @@ void cycle_schedule(const std::vector<CycSys>& sys, const std::vector<int>& sel,
 
 // Uploads the schedule and clears the team counters (the stream has drained: the pinned staging
 // is free).
-static int upload_schedule(ua_mesh* m, const CycSchedule& s) {
+int upload_schedule(ua_mesh* m, const CycSchedule& s) {
   Cycle& C = m->amg->cyc;
   const int nc = (int)s.cta.size(), nq = (int)s.queue.size();
   if (nc > 1024) return set_error(UA_ERR_INVALID, "resident solve: schedule of %d CTAs", nc);
@@ -458,7 +458,7 @@ static int upload_schedule(ua_mesh* m, const CycSchedule& s) {
   return UA_OK;
 }
 
-static CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof) {
+CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof) {
   const Amg* a = m->amg;
   const Cycle& C = a->cyc;
   CycArgs A{};
@@ -584,12 +584,12 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
     __syncthreads();
     Arena ar{arena_mem, a.arena, 0};
     const double* dense;
-    cyc_stage<KT, LT, QT>(a.cyc, a.kv, a.lv, S, t, ar, lev, &fine, 4 * sizeof(KT), dense);
+    int lo, hi;
+    team_share(t, S.nsl, lo, hi);
+    cyc_stage<KT, LT, QT>(a.cyc, a.kv, a.lv, S, t, lo, hi, ar, lev, &fine, 4 * sizeof(KT), dense);
     const int n0 = S.n0[0], nn = S.nn[0], dep = S.depth;
     const V2* bL = (const V2*)a.cyc.lev[dep].b;
     V2 *r = (V2*)a.r, *rn = (V2*)a.r2;
-    int lo, hi;
-    team_share(t, S.nsl, lo, hi);
     for (int i = lo + warp; i < hi; i += kCycWarps) {
       double v = 0;
       if (32 * i + lane < nn) {
@@ -722,18 +722,7 @@ template <typename KT, typename LT, typename VT, typename QT>
 static int launch_pcg(ua_mesh* m, const PcgArgs& a, int nctas) {
   UA_CUDA_TRY(cudaFuncSetAttribute(k_pcg_team<KT, LT, VT, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    kCycArena));
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(nctas);
-  cfg.blockDim = dim3(kCycThreads);
-  cfg.dynamicSmemBytes = a.arena;
-  cfg.stream = m->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeCooperative;
-  at[0].val.cooperative = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  UA_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_pcg_team<KT, LT, VT, QT>, a));
-  return UA_OK;
+  return launch_team(m, k_pcg_team<KT, LT, VT, QT>, a, nctas, a.arena);
 }
 
 int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, const std::vector<int>& steps, int nsm,
@@ -801,7 +790,7 @@ int pcg_resident_status(ua_mesh* m, bool prof, double* ms, int* cnt) {
   Cycle& C = m->amg->cyc;
   int err = 0;
   UA_CUDA_TRY(cudaMemcpy(&err, C.d_err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (err) return set_error(UA_ERR_TIMEOUT, "resident PCG: a team barrier was not met");
+  if (err) return set_error(UA_ERR_TIMEOUT, "resident solve: a team barrier was not met");
   if (prof) {
     unsigned long long h[2 * CP_COUNT];
     UA_CUDA_TRY(cudaMemcpy(h, C.d_prof, sizeof(h), cudaMemcpyDeviceToHost));

@@ -2524,11 +2524,64 @@ struct GmSys {
   bool active = false, cycle_done = false;
 };
 
+static int gmres_resident_solve(ua_mesh* m, const ua_params* p, const double* K, int mr, int* its_out,
+                                const double* eta) {
+  Work* w = m->work;
+  const int nsys = w->nsys;
+  std::vector<int> sel(nsys), steps(nsys);
+  for (int s = 0; s < nsys; ++s) {
+    sel[s] = its_out[s] != 0;
+    steps[s] = its_out[s];
+    w->h_sysv[s] = eta ? eta[s] : p->krylov_rtol;
+  }
+  UA_CUDA_TRY(cudaMemcpyAsync(w->sysv + SV_TOL2 * nsys, w->h_sysv, nsys * sizeof(double), cudaMemcpyHostToDevice,
+                              m->stream));
+  const CycFillReq fill{false, nullptr};
+  cudaEvent_t ev[2];
+  prof_begin(m, PK_SETUP, ev);
+  if (int rc = amg_numeric_uvh(m, K, w->cmask, &g_launches, &fill, !w->no_graph && !p->profile)) return rc;
+  prof_end(m, ev);
+  k_zero_sel<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->dX), ++g_launches;
+  if (w->nc)
+    k_con_particular<<<(w->nc + 255) / 256, 256, 0, m->stream>>>(w->nc, w->con_dof, w->con_sys, w->sel, w->con_rhs,
+                                                                 w->X, w->dX, w->grhs, con_pairs(w)), ++g_launches;
+  GmSolve v{};
+  v.rowptr = w->rowptr; v.K = K; v.cmask = w->cmask; v.sel = w->sel;
+  v.f = w->frhs; v.dX = w->dX;
+  v.tol = w->sysv + SV_TOL2 * nsys;
+  v.done = w->done; v.its = w->its;
+  v.mr = mr;
+  v.hsw = p->uvh_h_sweeps > 0 ? p->uvh_h_sweeps : 8;
+  v.maxit = p->krylov_maxit;
+  v.max_cycles = std::max(1, p->krylov_maxit / mr + 1);
+  cudaEvent_t kev[2];
+  prof_begin(m, PK_KRYLOV, kev);
+  if (int rc = gmres_resident(m, v, sel, steps, w->nsm, &g_launches)) return rc;
+  prof_end(m, kev);
+  if (w->nc)
+    k_con_multiplier<double><<<(w->nc + 255) / 256, 256, 0, m->stream>>>(w->nc, w->con_dof, w->con_sys, w->sel,
+                                                                         w->rowptr, w->colind, K, w->dX, w->frhs,
+                                                                         w->dlam, con_pairs(w)), ++g_launches;
+  UA_CUDA_TRY(cudaGetLastError());
+  UA_CUDA_TRY(cudaMemcpyAsync(w->h_int, w->its, nsys * sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+  UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
+  if (int rc = pcg_resident_status(m, false, nullptr, nullptr)) return rc;
+  for (int s = 0; s < nsys; ++s) its_out[s] = sel[s] ? w->h_int[s] : 0;
+  return UA_OK;
+}
+
 template <typename KT>
 static int gmres_t(ua_mesh* m, const ua_params* p, const KT* K, int* its_out, const double* eta) {
   Work* w = m->work;
   const int nsys = w->nsys, N = m->ndof_total;
   const int mr = std::max(4, std::min(200, p->krylov_restart > 0 ? p->krylov_restart : 40));
+  // the whole solve in one resident kernel: AMG on the velocity block, one-entry constraint rows, a
+  // restart whose triangular factor fits shared memory
+  if (p->krylov_precond == UA_PC_AMG && m->ndof == 3 && !m->h_nodeptr.empty() && sizeof(KT) == 8 &&
+      p->krylov_sell && w->npair == 0 && mr <= gmres_resident_max_restart() &&
+      amg_setup(m, p->amg_smoothed != 0) == UA_OK && cycle_supported(m) && amg_sell_init(m, w->h_sys_rb_off) == UA_OK &&
+      cycle_init(m) == UA_OK && cycle_alloc_values(m, false, false) == UA_OK)
+    return gmres_resident_solve(m, p, (const double*)K, mr, its_out, eta);
   const size_t ldv = (size_t)N;
   const int ld = mr + 1;
   // work space: basis V (mr+1 vectors), w, z, u; per-system coefficient arrays
@@ -2930,7 +2983,7 @@ static int newton_run_uvh(ua_mesh* m, const ua_params* p, std::vector<ua_newton_
     UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
     double t1 = now_ms();
     t_asm += t1 - t0;
-    for (int s = 0; s < nsys; ++s) its[s] = sel[s];
+    for (int s = 0; s < nsys; ++s) its[s] = sel[s] ? std::max(1, st[s].kits) : 0;
     std::vector<double> eta(nsys);
     for (int s = 0; s < nsys; ++s) eta[s] = forcing_term_uvh(p, st[s].rForce == INFINITY ? 1.0 : st[s].rForce);
     if (p->uvh_krylov == UA_KRYLOV_BICGSTAB) {
