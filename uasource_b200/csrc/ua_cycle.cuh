@@ -51,6 +51,19 @@ template <> struct QuadRaw<__nv_bfloat16> {
   }
 };
 
+// The quad of a lane in a slice's slot block (32 quads): FP64 quads are kept as two blocks of 32
+// pairs, so that a warp's 16-byte loads are contiguous.
+template <typename KT> struct SliceQuad {
+  static __device__ __forceinline__ typename QuadRaw<KT>::T load(const char* blk, int lane) {
+    return QuadRaw<KT>::load(blk + lane * (4 * sizeof(KT)));
+  }
+};
+template <> struct SliceQuad<double> {
+  static __device__ __forceinline__ QuadRaw<double>::T load(const char* blk, int lane) {
+    return QuadRaw<double>::T{reinterpret_cast<const double2*>(blk)[lane], reinterpret_cast<const double2*>(blk + 512)[lane]};
+  }
+};
+
 struct TeamCtx {
   int rank, size;        // this CTA in its team
   unsigned* bar;         // the team's arrival counter
@@ -397,26 +410,26 @@ __device__ __forceinline__ void cyc_dense(const CycSys& S, const double* M, cons
   __syncthreads();
 }
 
-// CH slots k0 .. of a slice product: the columns and values load together, then the gathered
-// pairs.  Slots past the width repeat the last one with a zero vector entry, so that nothing
-// branches between the loads.
+// CH slots k0 .. of a slice product of width k1: the columns and values load
+// together, then the gathered pairs.  Slots past the end repeat the last one with a zero vector
+// entry, so that nothing branches between the loads.
 template <int CH, typename KT, typename VT>
-__device__ __forceinline__ void slice_chunk(const int* cp, const char* vp, int k0, int W,
+__device__ __forceinline__ void slice_chunk(const int* cp, const char* vp, int lane, int k0, int k1,
                                             const typename Vec2<VT>::T* v, double& a0, double& a1) {
   using V2 = typename Vec2<VT>::T;
   int j[CH];
   typename QuadRaw<KT>::T e[CH];
 #pragma unroll
   for (int k = 0; k < CH; ++k) {
-    const int kk = min(k0 + k, W - 1);
-    j[k] = cp[32 * kk];
-    e[k] = QuadRaw<KT>::load(vp + (long long)kk * (128 * sizeof(KT)));
+    const int kk = min(k0 + k, k1 - 1);
+    j[k] = cp[32 * kk + lane];
+    e[k] = SliceQuad<KT>::load(vp + (long long)kk * (128 * sizeof(KT)), lane);
   }
   V2 x[CH];
 #pragma unroll
   for (int k = 0; k < CH; ++k) {
     x[k] = v[j[k]];
-    if (k0 + k >= W) x[k].x = x[k].y = 0;
+    if (k0 + k >= k1) x[k].x = x[k].y = 0;
   }
 #pragma unroll
   for (int k = 0; k < CH; ++k) {
@@ -429,45 +442,70 @@ __device__ __forceinline__ void slice_chunk(const int* cp, const char* vp, int k
   }
 }
 
-// (A^ v) at slice sl's lane (its node sits at position 32 sl + lane: the vectors of the finest level
-// are kept in slice order), in chunks of ten slots (five for FP64 values and for what is left): a
-// linear mesh's slice is one or two chunks, two dependent loads each, where a plain unrolled loop
-// takes the slots of its remainder one by one.
+// (A^ v) at slice sl's lane (its node sits at position 32 sl + lane: the vectors of
+// the finest level are kept in slice order), in chunks of ten slots (five for FP64 values and for
+// what is left): a linear mesh's slice is one or two chunks, two dependent loads each, where a plain
+// unrolled loop takes the slots of its remainder one by one.
 template <typename KT, typename VT>
 __device__ __forceinline__ void slice_product(const FineS& F, const char* vals, int sl, int lane,
                                               const typename Vec2<VT>::T* v, double& a0, double& a1) {
   const long long off = F.sl_off[sl];
-  const int W = (int)((F.sl_off[sl + 1] - off) >> 5);
-  const int* cp = F.cols + off + lane;
-  const char* vp = vals + (off + lane) * (long long)(4 * sizeof(KT));
-  a0 = 0;
-  a1 = 0;
-  for (int k0 = 0; k0 < W;) {  // the width is the same for the whole warp
-    if (sizeof(KT) < 8 && W - k0 > 5) {
-      slice_chunk<10, KT, VT>(cp, vp, k0, W, v, a0, a1);
+  const int k1 = (int)((F.sl_off[sl + 1] - off) >> 5);
+  const int* cp = F.cols + off;
+  const char* vp = vals + off * (long long)(4 * sizeof(KT));
+  a0 = a1 = 0;
+  for (int k0 = 0; k0 < k1;) {  // the width is the same for the whole warp
+    if (sizeof(KT) < 8 && k1 - k0 > 5) {
+      slice_chunk<10, KT, VT>(cp, vp, lane, k0, k1, v, a0, a1);
       k0 += 10;
-    } else {
-      slice_chunk<5, KT, VT>(cp, vp, k0, W, v, a0, a1);
+    } else if (k1 - k0 > 3) {
+      slice_chunk<5, KT, VT>(cp, vp, lane, k0, k1, v, a0, a1);
       k0 += 5;
+    } else {
+      slice_chunk<3, KT, VT>(cp, vp, lane, k0, k1, v, a0, a1);
+      k0 += 3;
     }
   }
 }
 
-// z = w (2 b - A^ b) + Q z_c at the lane of slice sl, finest level (the caller stores it).
+// The slices' columns and values into L2 ahead of their use (one lane; sizes and addresses are
+// multiples of 128 bytes): the demand loads then wait for L2 instead of DRAM.
+__device__ __forceinline__ void prefetch_l2(const void* p, long long bytes) {
+  if (bytes >= 16)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"((unsigned)bytes) : "memory");
+}
+template <typename KT>
+__device__ __forceinline__ void slice_prefetch(const CycFine& G, const void* vals, int sl) {
+  const long long off = G.sl_off[sl], n = G.sl_off[sl + 1] - off;
+  prefetch_l2(G.cols + off, 4 * n);
+  prefetch_l2((const char*)vals + off * (4 * sizeof(KT)), n * (4 * sizeof(KT)));
+}
+
+// Runs the slices [lo, hi) over the CTA's warps: f(i, lane's node, node is there).  The slices of a
+// block of eight are ordered by width (25 down to 9 slots on a quadratic mesh), so the warps rotate
+// from round to round: with a plain stride of 16 a warp met the same place of a block every time,
+// and a pass waited for the warps of the widest one (401x201 P2: CTAs of 52k and 110k cycles side
+// by side).  (Splitting a slice's slots over two or four warps of a CTA that has few was slower
+// at every size: the exchange through shared memory costs what the shorter chains save.)
+template <typename F>
+__device__ __forceinline__ void for_slices(int lo, int hi, int n0, int nn, F f) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int b = lo, r = 0; b < hi; b += kCycWarps, r += 5) {
+    const int i = b + ((warp + r) & (kCycWarps - 1));
+    if (i < hi) f(i, n0 + 32 * i + lane, 32 * i + lane < nn);
+  }
+}
+
+// - w A^ b + Q z_c at the lane of slice sl, finest level (the caller adds 2 w b).
 template <typename LT, typename VT, typename QT>
-__device__ __forceinline__ void cyc_up0_node(const FineS& F, const LevS& L, int sl, int lane, int g, bool valid,
+__device__ __forceinline__ void cyc_up0_node(const FineS& F, const LevS& L, int sl, int lane, int g,
                                              const typename Vec2<VT>::T* b, const typename Vec2<VT>::T* zc, double w,
-                                             typename Vec2<VT>::T& bv, double& z0, double& z1) {
-  constexpr int CH = sizeof(VT) == 4 ? 4 : 2;
-  bv.x = bv.y = 0;
-  z0 = z1 = 0;
-  if (!valid) return;
-  bv = b[g];
+                                             double& z0, double& z1) {
   double a0, a1;
   slice_product<LT, VT>(F, F.lv, sl, lane, b, a0, a1);
-  z0 = w * (2.0 * (double)bv.x - a0);
-  z1 = w * (2.0 * (double)bv.y - a1);
-  row_product<CH, QT, VT>(L.qcol, L.qval, L.qptr[g], L.qptr[g + 1], 1, zc, 1.0, z0, z1);
+  z0 = -w * a0;
+  z1 = -w * a1;
+  row_product<sizeof(VT) == 4 ? 8 : 6, QT, VT>(L.qcol, L.qval, L.qptr[g], L.qptr[g + 1], 1, zc, 1.0, z0, z1);
 }
 
 // ---- host side of a resident launch (ua_pcg.cu) ----

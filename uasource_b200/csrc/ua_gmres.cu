@@ -97,27 +97,27 @@ __device__ __forceinline__ GmVec gm_basis(const GmArgs& a, int i) {
 }
 
 // (K v) at the lane of slice sl
-__device__ __forceinline__ void gm_product(const CycFine& F, const double* v3, int sl, int lane, const GmVec& v,
-                                           double (&r)[3]) {
+__device__ __forceinline__ void gm_product(const CycFine& F, const double* v3, int sl, int lane,
+                                           const GmVec& v, double (&r)[3]) {
   const long long off = F.sl_off[sl];
-  const int W = (int)((F.sl_off[sl + 1] - off) >> 5);
+  const int k1 = (int)((F.sl_off[sl + 1] - off) >> 5);
   const int* cp = F.cols + off + lane;
   const double* vp = v3 + 9 * off + lane;
   r[0] = r[1] = r[2] = 0;
-  constexpr int CH = 4;
-  for (int k0 = 0; k0 < W; k0 += CH) {
+  constexpr int CH = 5;
+  for (int k0 = 0; k0 < k1; k0 += CH) {
     double2 xu[CH];
     double xh[CH];
 #pragma unroll
     for (int k = 0; k < CH; ++k) {
-      const int j = __ldg(cp + 32 * min(k0 + k, W - 1));
+      const int j = __ldg(cp + 32 * min(k0 + k, k1 - 1));
       xu[k] = v.uv[j];
       xh[k] = v.h[j];
     }
 #pragma unroll
     for (int k = 0; k < CH; ++k) {
-      if (k0 + k >= W) xu[k].x = xu[k].y = xh[k] = 0;
-      const double* e = vp + 288 * min(k0 + k, W - 1);
+      if (k0 + k >= k1) xu[k].x = xu[k].y = xh[k] = 0;
+      const double* e = vp + 288 * min(k0 + k, k1 - 1);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         r[c] = fma(__ldg(e + 96 * c), xu[k].x, r[c]);
@@ -129,27 +129,27 @@ __device__ __forceinline__ void gm_product(const CycFine& F, const double* v3, i
 }
 // thickness row: B = 0: (K_hu v_u + K_hv v_v), B = 1: K_hh v_h
 template <int B>
-__device__ __forceinline__ double gm_hrow(const CycFine& F, const double* v3, int sl, int lane, const double2* uv,
-                                          const double* h) {
+__device__ __forceinline__ double gm_hrow(const CycFine& F, const double* v3, int sl, int lane,
+                                          const double2* uv, const double* h) {
   const long long off = F.sl_off[sl];
-  const int W = (int)((F.sl_off[sl + 1] - off) >> 5);
+  const int k1 = (int)((F.sl_off[sl + 1] - off) >> 5);
   const int* cp = F.cols + off + lane;
   const double* vp = v3 + 9 * off + lane + (B ? 256 : 192);
   double acc = 0;
   constexpr int CH = 5;
-  for (int k0 = 0; k0 < W; k0 += CH) {
+  for (int k0 = 0; k0 < k1; k0 += CH) {
     int j[CH];
     double e0[CH], e1[CH];
 #pragma unroll
     for (int k = 0; k < CH; ++k) {
-      const int kk = min(k0 + k, W - 1);
+      const int kk = min(k0 + k, k1 - 1);
       j[k] = __ldg(cp + 32 * kk);
       e0[k] = __ldg(vp + 288 * kk);
       if (!B) e1[k] = __ldg(vp + 288 * kk + 32);
     }
 #pragma unroll
     for (int k = 0; k < CH; ++k) {
-      const bool in = k0 + k < W;
+      const bool in = k0 + k < k1;
       if (B) {
         const double x = h[j[k]];
         acc = fma(e0[k], in ? x : 0.0, acc);
@@ -191,8 +191,9 @@ struct GmShared {
 };
 
 // Dot products of w with the basis vectors 0 .. nv-1 (nv = 0: with itself) over the slices of the
-// CTA's units; one partial per vector and unit.  A thread reads the entries of w that it wrote (the
-// slices of a slab go to the warps like those of the passes: kGmSlab is a multiple of the warps).
+// CTA's units; one partial per vector and unit.  Within a Gram-Schmidt pass a
+// thread reads the entries of w that it wrote (the slices of a slab go to the warps like those of
+// the update: kGmSlab is a multiple of the warps); after a product the CTA has to meet first.
 static_assert(kGmSlab % kCycWarps == 0, "");
 __device__ __forceinline__ void gm_dots(const GmArgs& a, GmShared& sh, const CycSys& S, int U, int u0, int u1, int nv,
                                         double* part) {
@@ -310,19 +311,18 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
     const double tol = a.tol[s];
     while (true) {
       // residual
-      for (int i = lo + warp; i < hi; i += kCycWarps) {
-        const int k = n0 + 32 * i + lane;
-        if (32 * i + lane < nn) {
-          double kx[3];
-          gm_product(a.cyc.fine, a.v3, S.sl0 + i, lane, a.x, kx);
-          const double2 f = a.fs.uv[k], d = a.scp[k];
-          const double2 r = make_double2(f.x - kx[0], f.y - kx[1]);
-          // constrained rows: f and the product are zero
-          a.w.uv[k] = r;
-          a.w.h[k] = a.fs.h[k] - kx[2];
-          a.ws[k] = make_double2(d.x * r.x, d.y * r.y);
-        }
-      }
+      for_slices(lo, hi, n0, nn, [&](int i, int k, bool in) {
+        if (!in) return;
+        double kx[3];
+        gm_product(a.cyc.fine, a.v3, S.sl0 + i, lane, a.x, kx);
+        const double2 f = a.fs.uv[k], d = a.scp[k];
+        const double2 r = make_double2(f.x - kx[0], f.y - kx[1]);
+        // constrained rows: f and the product are zero
+        a.w.uv[k] = r;
+        a.w.h[k] = a.fs.h[k] - kx[2];
+        a.ws[k] = make_double2(d.x * r.x, d.y * r.y);
+      });
+      __syncthreads();
       gm_dots(a, sh, S, U, u0, u1, 0, part3);
       UA_TEAM_SYNC(t);
       gm_totals(a, part3, units, 1, sh.scal);
@@ -361,53 +361,45 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
           UA_TEAM_SYNC(t);
           zc = (const double2*)a.cyc.lev[l].z;
         }
-        for (int i = lo + warp; i < hi; i += kCycWarps) {
-          const int k = n0 + 32 * i + lane;
-          const bool valid = 32 * i + lane < nn;
-          double2 bv;
+        for_slices(lo, hi, n0, nn, [&](int i, int k, bool in) {
+          if (!in) return;
           double z0, z1;
-          cyc_up0_node<double, double, double>(fine, lev[0], S.sl0 + i, lane, k, valid, a.ws, zc, inv, bv, z0, z1);
-          if (valid) {
-            const double2 d = a.scp[k];
-            a.z.uv[k] = make_double2(d.x * z0, d.y * z1);
-          }
-        }
+          cyc_up0_node<double, double, double>(fine, lev[0], S.sl0 + i, lane, k, a.ws, zc, inv, z0, z1);
+          const double2 d = a.scp[k], b = a.ws[k];
+          a.z.uv[k] = make_double2(d.x * (2.0 * inv * b.x + z0), d.y * (2.0 * inv * b.y + z1));
+        });
         UA_TEAM_SYNC(t);
         // thickness rows; the sweeps ping-pong so that the last one writes z.h
         double* bufs[2] = {a.z.h, a.ht};
         int cur = (a.hsw - 1) % 2 == 0 ? 0 : 1;
-        for (int i = lo + warp; i < hi; i += kCycWarps) {
-          const int k = n0 + 32 * i + lane;
-          if (32 * i + lane < nn) {
-            const double b = vj.h[k] - gm_hrow<0>(a.cyc.fine, a.v3, S.sl0 + i, lane, a.z.uv, nullptr);
-            const double hi1 = a.hinv[k];
-            a.bh[k] = hi1 > 0 ? b : 0.0;
-            bufs[cur][k] = b * hi1;
-          }
-        }
+        for_slices(lo, hi, n0, nn, [&](int i, int k, bool in) {
+          if (!in) return;
+          const double b = vj.h[k] - gm_hrow<0>(a.cyc.fine, a.v3, S.sl0 + i, lane, a.z.uv, nullptr);
+          const double hi1 = a.hinv[k];
+          a.bh[k] = hi1 > 0 ? b : 0.0;
+          bufs[cur][k] = b * hi1;
+        });
         UA_TEAM_SYNC(t);
         for (int q = 1; q < a.hsw; ++q) {
           const double* zi = bufs[cur];
           double* zo = bufs[1 - cur];
-          for (int i = lo + warp; i < hi; i += kCycWarps) {
-            const int k = n0 + 32 * i + lane;
-            if (32 * i + lane < nn)
+          for_slices(lo, hi, n0, nn, [&](int i, int k, bool in) {
+            if (in)
               zo[k] = zi[k] + (a.bh[k] - gm_hrow<1>(a.cyc.fine, a.v3, S.sl0 + i, lane, nullptr, zi)) * a.hinv[k];
-          }
+          });
           UA_TEAM_SYNC(t);
           cur = 1 - cur;
         }
         if (combine) break;
         // w = K z and its dot products
-        for (int i = lo + warp; i < hi; i += kCycWarps) {
-          const int k = n0 + 32 * i + lane;
-          if (32 * i + lane < nn) {
-            double kx[3];
-            gm_product(a.cyc.fine, a.v3, S.sl0 + i, lane, a.z, kx);
-            a.w.uv[k] = make_double2(kx[0], kx[1]);
-            a.w.h[k] = kx[2];
-          }
-        }
+        for_slices(lo, hi, n0, nn, [&](int i, int k, bool in) {
+          if (!in) return;
+          double kx[3];
+          gm_product(a.cyc.fine, a.v3, S.sl0 + i, lane, a.z, kx);
+          a.w.uv[k] = make_double2(kx[0], kx[1]);
+          a.w.h[k] = kx[2];
+        });
+        __syncthreads();
         gm_dots(a, sh, S, U, u0, u1, j + 1, part1);
         UA_TEAM_SYNC(t);
         for (int pass = 0; pass < 2; ++pass) {

@@ -104,7 +104,13 @@ __global__ void __launch_bounds__(256) k_cyc_fill0(CycFine F, const int* sb_n0, 
       e2 = si.y * (double)K[r1 + k] * sj.x;
       e3 = si.y * (double)K[r1 + deg + k] * sj.y;
     }
-    QuadSet<KT>::set(vk, d, e0, e1, e2, e3);
+    if (sizeof(KT) == 8) {  // two blocks of 32 pairs (SliceQuad)
+      double2* q = reinterpret_cast<double2*>(vk) + 2 * (d - t);
+      q[t] = make_double2(e0, e1);
+      q[32 + t] = make_double2(e2, e3);
+    } else {
+      QuadSet<KT>::set(vk, d, e0, e1, e2, e3);
+    }
     if (vlo) QuadSet<__nv_bfloat16>::set(vlo, d, e0, e1, e2, e3);
   }
 }
@@ -588,6 +594,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
     team_share(t, S.nsl, lo, hi);
     cyc_stage<KT, LT, QT>(a.cyc, a.kv, a.lv, S, t, lo, hi, ar, lev, &fine, 4 * sizeof(KT), dense);
     const int n0 = S.n0[0], nn = S.nn[0], dep = S.depth;
+    const bool stream = fine.cols == a.cyc.fine.cols;  // rows read from global memory
     const V2* bL = (const V2*)a.cyc.lev[dep].b;
     V2 *r = (V2*)a.r, *rn = (V2*)a.r2;
     for (int i = lo + warp; i < hi; i += kCycWarps) {
@@ -620,28 +627,32 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
         zc = (const V2*)a.cyc.lev[l].z;
       }
       mark(CP_OTHER);
-      for (int i = lo + warp; i < hi; i += kCycWarps) {
-        const int g = n0 + 32 * i + lane;
-        const bool valid = 32 * i + lane < nn;
-        V2 bv, o;
-        double z0, z1;
-        cyc_up0_node<LT, VT, QT>(fine, lev[0], S.sl0 + i, lane, g, valid, r, zc, 1.0, bv, z0, z1);
-        o.x = (VT)z0;
-        o.y = (VT)z1;
-        if (valid) z[g] = o;
-        const double v = lane_sum((double)bv.x * (double)o.x + (double)bv.y * (double)o.y, 32);
+      for_slices(lo, hi, n0, nn, [&](int i, int g, bool in) {
+        if (stream && lane == 0 && i + kCycWarps < hi) slice_prefetch<LT>(a.cyc.fine, a.lv, S.sl0 + i + kCycWarps);
+        double v = 0;
+        if (in) {
+          const V2 bv = r[g];
+          double z0, z1;
+          cyc_up0_node<LT, VT, QT>(fine, lev[0], S.sl0 + i, lane, g, r, zc, 1.0, z0, z1);
+          V2 o;
+          o.x = (VT)(2.0 * (double)bv.x + z0);
+          o.y = (VT)(2.0 * (double)bv.y + z1);
+          z[g] = o;
+          v = (double)bv.x * (double)o.x + (double)bv.y * (double)o.y;
+        }
+        v = lane_sum(v, 32);
         if (lane == 0) part_rz[S.sl0 + i] = v;
-      }
+      });
       UA_TEAM_SYNC(t);
       const double rz = team_sum(part_rz + S.sl0, S.nsl, red[0]);
       mark(CP_UP0);
       const double beta = its ? rz / rz_old : 0.0;
       rz_old = rz;
       // p = z + beta p, q = A z + beta q, partials p.q
-      for (int i = lo + warp; i < hi; i += kCycWarps) {
-        const int g = n0 + 32 * i + lane;
+      for_slices(lo, hi, n0, nn, [&](int i, int g, bool in) {
+        if (stream && lane == 0 && i + kCycWarps < hi) slice_prefetch<KT>(a.cyc.fine, a.kv, S.sl0 + i + kCycWarps);
         double v = 0;
-        if (32 * i + lane < nn) {
+        if (in) {
           V2 pn = z[g], po, qo;
           if (its) {
             po = p[g];
@@ -664,7 +675,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
         }
         v = lane_sum(v, 32);
         if (lane == 0) part_pq[S.sl0 + i] = v;
-      }
+      });
       UA_TEAM_SYNC(t);
       const double pq = team_sum(part_pq + S.sl0, S.nsl, red[1]);
       mark(CP_SPMV);
