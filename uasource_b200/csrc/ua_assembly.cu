@@ -1,14 +1,13 @@
 // uv residual/tangent assembly: uvMatrixAssemblySSTREAM.m:6-553 on the device.
 //
-// One CTA per node patch.  Phase 1: one thread per element of the patch
-// gathers its nodal fields, loops over the integration points and writes the
-// element tangent (uu and vv blocks symmetric, uv block full) and the four
-// residual parts Tx, Fx, Ty, Fy into shared memory (element-fastest layout,
-// so the writes are bank-conflict free).  Phase 2: one thread per node-level
+// One CTA per node patch.  Phase 1 computes the element tangents of the patch
+// (uu and vv blocks symmetric, uv block full) and the four residual parts Tx,
+// Fx, Ty, Fy into shared memory (element-fastest layout).  Phase 2: one thread per node-level
 // non-zero of the patch's rows sums the element contributions listed for it
 // (increasing global element order) and writes the four dof-level values;
 // the same for the residual on the diagonal entries.  No atomics: every
 // matrix entry is produced by exactly one thread, in a fixed order.
+#include <algorithm>
 #include "ua_internal.h"
 #include "ua_physics.cuh"
 #include "ua_kernels.h"
@@ -24,210 +23,6 @@ struct ElemIdx {
     return a <= b ? a * NOD - a * (a - 1) / 2 + (b - a) : b * NOD - b * (b - 1) / 2 + (a - b);
   }
 };
-
-// derivVector.m:96-109 at integration point ip
-template <int NOD>
-__device__ __forceinline__ void uv_deriv(const QuadTable& Q, int ip, const double (&xe)[NOD], const double (&ye)[NOD],
-                                         double (&Dx)[NOD], double (&Dy)[NOD], double& detJ) {
-  double J11 = 0, J12 = 0, J21 = 0, J22 = 0;
-#pragma unroll
-  for (int a = 0; a < NOD; ++a) {
-    J11 += xe[a] * Q.der[ip][0][a];
-    J12 += ye[a] * Q.der[ip][0][a];
-    J21 += xe[a] * Q.der[ip][1][a];
-    J22 += ye[a] * Q.der[ip][1][a];
-  }
-  detJ = J11 * J22 - J12 * J21;
-#pragma unroll
-  for (int a = 0; a < NOD; ++a) {
-    Dx[a] = (J22 * Q.der[ip][0][a] - J12 * Q.der[ip][1][a]) / detJ;
-    Dy[a] = (-J21 * Q.der[ip][0][a] + J11 * Q.der[ip][1][a]) / detJ;
-  }
-}
-
-// Contribution of integration point ip to the element tangent and residual
-// parts (accumulated into the outputs).
-template <int NOD, bool WITHK, typename KT, bool GEN>
-__device__ __forceinline__ void uv_ip(const QuadTable& Q, const UvPhys& P, const SysScal& S, int ip,
-                                      const int (&gn)[NOD], const DragFields& DF,
-                                      const double (&Dx)[NOD], const double (&Dy)[NOD], double detJ,
-                                      const double (&hn)[NOD], const double (&sn)[NOD], const double (&un)[NOD],
-                                      const double (&vn)[NOD], const double (&Cn)[NOD], const double (&mn)[NOD],
-                                      const double (&An)[NOD], const double (&nn)[NOD], const double (&Sn)[NOD],
-                                      const double (&Bn)[NOD], const double (&rn)[NOD], KT* Kuu, KT* Kvv, KT* Kuv,
-                                      double* Tx, double* Fx, double* Ty, double* Fy) {
-  using I = ElemIdx<NOD>;
-  const double rhow = S.rhow, g = S.g, ca = S.ca, sa = S.sa;
-  {
-    double N[NOD];
-#pragma unroll
-    for (int a = 0; a < NOD; ++a) N[a] = Q.fun[ip][a];
-    double hint = 0, sint = 0, uint = 0, vint = 0, Cint = 0, mint = 0, Aint = 0, nint = 0, Bint = 0, Sint = 0,
-           rhoint = 0;
-#pragma unroll
-    for (int a = 0; a < NOD; ++a) {
-      hint += hn[a] * N[a]; sint += sn[a] * N[a];
-      uint += un[a] * N[a]; vint += vn[a] * N[a];
-      Cint += Cn[a] * N[a]; mint += mn[a] * N[a];
-      Aint += An[a] * N[a]; nint += nn[a] * N[a];
-      Bint += Bn[a] * N[a]; Sint += Sn[a] * N[a];
-      rhoint += rn[a] * N[a];
-    }
-    if (Cint < P.Cmin) Cint = P.Cmin;        // :205
-    if (Aint < P.AGlenmin) Aint = P.AGlenmin;  // :243
-    const double Hint = Sint - Bint;
-    const double hfint = rhow * Hint / rhoint;  // :300
-    // flotation steps (:300-310): one expm1 per argument
-    const StepPulse fl = step_pulse(P.kH, hint - hfint, P.Hh0);
-    const double Heint = 0.5 + 0.5 * fl.t;
-    const double HEint = P.Hh0 == 0.0 ? 0.5 - 0.5 * fl.t : heaviside_approx(P.kH, hfint - hint, P.Hh0);
-    const double deltaint = fl.delta;
-    const double Hposint = (0.5 + 0.5 * step_pulse(P.kH, Hint, P.Hh0).t) * Hint;
-    const bool cube = S.cube != 0.0;  // n = m = 3 at every node of the system
-    const double dint = HEint * rhoint * hint / rhow + Heint * Hposint;  // :310
-    double dsdx = 0, dhdx = 0, dsdy = 0, dhdy = 0, exx = 0, eyy = 0, exy = 0;
-#pragma unroll
-    for (int a = 0; a < NOD; ++a) {  // :332-347
-      dsdx += Dx[a] * sn[a]; dhdx += Dx[a] * hn[a];
-      dsdy += Dy[a] * sn[a]; dhdy += Dy[a] * hn[a];
-      exx += Dx[a] * un[a]; eyy += Dy[a] * vn[a];
-      exy += 0.5 * (Dx[a] * vn[a] + Dy[a] * un[a]);
-    }
-    // GEN: any sliding law and the melange terms; else Weertman (the general code stays out of
-    // the Weertman build, whose registers it would crowd)
-    const Drag d = !GEN ? basal_drag_weertman(P, Heint, deltaint, uint, vint, Cint, mint, cube)
-                        : basal_drag_general(P, Heint, deltaint, hint, Hint, rhoint, rhow, g, uint, vint, Cint, mint,
-                                             drag_interp<NOD>(DF, gn, N));
-    double eta, E;
-    effective_viscosity(P, Aint, nint, exx, eyy, exy, eta, E, cube);
-    const double dbdx = dsdx - dhdx, dbdy = dsdy - dhdy;
-    const double detJw = detJ * Q.w[ip];
-    if (WITHK) {
-      const KT cxu = (KT)(d.dxu * detJw), cyv = (KT)(d.dyv * detJw), cxv = (KT)(d.dxv * detJw);
-      KT Nk[NOD];
-#pragma unroll
-      for (int a = 0; a < NOD; ++a) Nk[a] = (KT)N[a];
-      if constexpr (sizeof(KT) == 8) {
-        const KT he = hint * eta * detJw;
-        const KT hE2 = P.Dvisk * 2.0 * hint * E * detJw;
-        KT Pu[NOD], Pv[NOD];
-#pragma unroll
-        for (int a = 0; a < NOD; ++a) {
-          Pu[a] = (2 * exx + eyy) * Dx[a] + exy * Dy[a];
-          Pv[a] = (2 * eyy + exx) * Dy[a] + exy * Dx[a];
-        }
-#pragma unroll
-        for (int a = 0; a < NOD; ++a) {
-#pragma unroll
-          for (int b = a; b < NOD; ++b) {
-            const int i = I::sym(a, b);
-            const KT NN = Nk[a] * Nk[b];
-            Kuu[i] += he * (4 * Dx[a] * Dx[b] + Dy[a] * Dy[b]) + cxu * NN + hE2 * Pu[a] * Pu[b];
-            Kvv[i] += he * (4 * Dy[a] * Dy[b] + Dx[a] * Dx[b]) + cyv * NN + hE2 * Pv[a] * Pv[b];
-          }
-#pragma unroll
-          for (int b = 0; b < NOD; ++b)
-            Kuv[a * NOD + b] += he * (2 * Dx[a] * Dy[b] + Dy[a] * Dx[b]) + cxv * Nk[a] * Nk[b] + hE2 * Pu[a] * Pv[b];
-        }
-      } else {
-        // FP32 tangent: h*eta*detJw and 2*h*E*detJw span far beyond the float
-        // range (E grows as e^((1-3n)/n) when the strain rate e -> EpsZero), so
-        // their square roots are folded into the per-node vectors in FP64 and
-        // only the bounded products are rounded to float.
-        const double he = hint * eta * detJw;
-        const double hE2 = P.Dvisk * 2.0 * hint * E * detJw;
-        const double sh = sqrt(he), sE = sqrt(fabs(hE2));
-        const KT sgn = hE2 < 0 ? KT(-1) : KT(1);
-        KT dx[NOD], dy[NOD], Pu[NOD], Pv[NOD];
-#pragma unroll
-        for (int a = 0; a < NOD; ++a) {
-          dx[a] = (KT)(sh * Dx[a]); dy[a] = (KT)(sh * Dy[a]);
-          Pu[a] = (KT)(sE * ((2 * exx + eyy) * Dx[a] + exy * Dy[a]));
-          Pv[a] = (KT)(sE * ((2 * eyy + exx) * Dy[a] + exy * Dx[a]));
-        }
-#pragma unroll
-        for (int a = 0; a < NOD; ++a) {
-#pragma unroll
-          for (int b = a; b < NOD; ++b) {
-            const int i = I::sym(a, b);
-            const KT NN = Nk[a] * Nk[b];
-            Kuu[i] += (4 * dx[a] * dx[b] + dy[a] * dy[b]) + cxu * NN + sgn * Pu[a] * Pu[b];
-            Kvv[i] += (4 * dy[a] * dy[b] + dx[a] * dx[b]) + cyv * NN + sgn * Pv[a] * Pv[b];
-          }
-#pragma unroll
-          for (int b = 0; b < NOD; ++b)
-            Kuv[a * NOD + b] += (2 * dx[a] * dy[b] + dy[a] * dx[b]) + cxv * Nk[a] * Nk[b] + sgn * Pu[a] * Pv[b];
-        }
-      }
-    }
-    const double rr = rhoint * hint - rhow * dint;
-    const double pp = 0.5 * g * ca * (rhoint * hint * hint - rhow * dint * dint);
-#pragma unroll
-    for (int a = 0; a < NOD; ++a) {  // :431-449
-      double t1 = -g * rr * dbdx * N[a] * ca + rhoint * g * hint * sa * N[a];
-      double t2 = pp * Dx[a];
-      double t3 = hint * eta * (4 * exx + 2 * eyy) * Dx[a];
-      double t4 = hint * eta * 2 * exy * Dy[a];
-      double t5 = d.taux * N[a];
-      Tx[a] += (t3 + t4 + t5) * detJw;
-      Fx[a] += (t1 + t2) * detJw;
-      t1 = -g * rr * dbdy * N[a] * ca;
-      t2 = pp * Dy[a];
-      t3 = hint * eta * (4 * eyy + 2 * exx) * Dy[a];
-      t4 = hint * eta * 2 * exy * Dx[a];
-      t5 = d.tauy * N[a];
-      Ty[a] += (t3 + t4 + t5) * detJw;
-      Fy[a] += (t1 + t2) * detJw;
-    }
-  }
-}
-
-template <int NOD, bool WITHK, typename KT>
-__device__ __forceinline__ void uv_zero(KT* Kuu, KT* Kvv, KT* Kuv, double* Tx, double* Fx, double* Ty, double* Fy) {
-  using I = ElemIdx<NOD>;
-#pragma unroll
-  for (int a = 0; a < NOD; ++a) { Tx[a] = 0; Fx[a] = 0; Ty[a] = 0; Fy[a] = 0; }
-  if (WITHK) {
-#pragma unroll
-    for (int i = 0; i < I::NS; ++i) { Kuu[i] = 0; Kvv[i] = 0; }
-#pragma unroll
-    for (int i = 0; i < NOD * NOD; ++i) Kuv[i] = 0;
-  }
-}
-
-// Element computation.  Follows uvMatrixAssemblySSTREAM.m :168-455 for one
-// element: interpolation and clamps (:186-254), post-2025 flotation at the
-// integration points (:300-310), nodal-derivative sums (:332-347), drag and
-// viscosity (:351-353), tangent blocks including the Newton viscosity terms
-// (:362-425) and residual terms (:431-449).
-//
-// The Newton viscosity terms E11..E22 are written as the rank-one product
-// 2 h E P_I P_J with P_u = (2exx+eyy) dN/dx + exy dN/dy and
-// P_v = (2eyy+exx) dN/dy + exy dN/dx, which is the same expression as
-// :398-417 regrouped (E11 = h(4exx+2eyy) Deu dNI/dx + 2h exy Deu dNI/dy with
-// Deu = E P_u(J)).  The tangent is produced symmetric, which is what
-// (K+K.')/2 at :530-531 yields.
-template <int NOD, bool WITHK, typename KT, bool GEN>
-__device__ __forceinline__ void uv_element(const QuadTable& Q, const UvPhys& P, const SysScal& S,
-                                           const int (&gn)[NOD], const DragFields& DF,
-                                           const double (&xe)[NOD], const double (&ye)[NOD],
-                                           const double (&hn)[NOD], const double (&sn)[NOD],
-                                           const double (&un)[NOD], const double (&vn)[NOD],
-                                           const double (&Cn)[NOD], const double (&mn)[NOD],
-                                           const double (&An)[NOD], const double (&nn)[NOD],
-                                           const double (&Sn)[NOD], const double (&Bn)[NOD],
-                                           const double (&rn)[NOD], KT* Kuu, KT* Kvv, KT* Kuv,
-                                           double* Tx, double* Fx, double* Ty, double* Fy) {
-  uv_zero<NOD, WITHK, KT>(Kuu, Kvv, Kuv, Tx, Fx, Ty, Fy);
-  double Dx[NOD], Dy[NOD], detJ = 0;
-  if (NOD == 3) uv_deriv<NOD>(Q, 0, xe, ye, Dx, Dy, detJ);  // P1: constant over the element
-#pragma unroll 1
-  for (int ip = 0; ip < Q.nip; ++ip) {
-    if (NOD != 3) uv_deriv<NOD>(Q, ip, xe, ye, Dx, Dy, detJ);
-    uv_ip<NOD, WITHK, KT, GEN>(Q, P, S, ip, gn, DF, Dx, Dy, detJ, hn, sn, un, vn, Cn, mn, An, nn, Sn, Bn, rn, Kuu, Kvv,
-                          Kuv, Tx, Fx, Ty, Fy);
-  }
-}
 
 // Phase 2 of the patch kernels: one thread per node-level non-zero of the
 // patch's rows sums the element contributions listed for it (increasing global
@@ -603,83 +398,254 @@ size_t uv_p1_smem(bool withK, bool fp32, int E, int threads, int MH) {
          (size_t)p1::ND_COUNT * MH * 8;
 }
 
-// P2 (6-node elements): one element per thread in 128-thread blocks, the
-// integration points in a loop (the derivatives vary over the element).
-template <int NOD, bool WITHK, typename KT, bool GEN>
-__global__ void __launch_bounds__(128, 1) uv_patch_kernel(DevMesh M, QuadTable Q, UvPhys P, UvIn in, UvOut out) {
-  using I = ElemIdx<NOD>;
+// ---------------------------------------------------------------------------
+// P2 (6-node elements): integration points first, then rows.
+//
+// Per integration point the tangent is a sum of products of the nodes' reference derivatives
+// d_a = (dN_a/dxi, dN_a/deta) and values N_a,
+//   Kuu_ab = d_a' Muu d_b + cxu N_a N_b, likewise Kvv and Kuv,
+// with 2x2 matrices of the point: the ones in x and y (the Newton viscosity term is the rank-one
+// product of P_u = p1 Dx + q2 Dy and P_v = q1 Dy + q2 Dx) between the point's inverse Jacobian and
+// its transpose.  d_a and N_a are the same for every element, so what an element adds is 25
+// coefficients a point.  A patch's elements go in groups: (a) a thread per element and point
+// interpolates, evaluates the physics once and leaves the coefficients in shared memory, kIpc points
+// at a time; (b) a thread per element and node a accumulates its rows of the three blocks and its
+// residual parts over those points in registers.  Then the patch's segmented sum (patch_scatter).
+//
+// One thread per element held 78 + 24 accumulators and 78 nodal values, spilled most of them and ran
+// four warps per SM: 1.55 ms (tangent) and 0.52 ms (residual) for 160,000 elements in FP64, where
+// this split takes 0.76 and 0.34 ms (mixed, 10,000 elements: 0.36 and 0.15 before, 0.070 and 0.046
+// now).  At 128 registers two CTAs share an SM and hide each other's
+// staging and barriers (residual 0.34 ms against 0.52 with one CTA of 168 registers); the FP64
+// tangent needs the whole SM's shared memory and runs one.  The residual-only pass runs the same
+// code with the tangent's part switched off, so its R is the same bit for bit.  All of it in FP64;
+// the mixed form rounds the finished element entries.
+namespace p2 {
+constexpr int kMaxG = 64, kMaxG2 = 42, kIpc = 6, kIps = 16;
+// staged node fields
+enum { ND_X = 0, ND_Y, ND_H, ND_BL, ND_U, ND_V, ND_C, ND_A, ND_HB, ND_RHO, ND_M, ND_N, ND_COUNT };
+// pairs of coefficients of a point
+enum { PR_UU = 0, PR_UUC, PR_VV, PR_VVC, PR_UV1, PR_UV2, PR_XV, PR_TX, PR_TY, PR_PX, PR_PY, PR_TN, PR_FN, kPairs };
+}  // namespace p2
+
+template <typename KT, bool GEN, int CTAS>
+__global__ void __launch_bounds__(CTAS == 2 ? 256 : 6 * p2::kMaxG, CTAS) uv_p2_kernel(DevMesh M, QuadTable Q, UvPhys P, UvIn in, UvOut out,
+                                                                 int G) {
+  using namespace p2;
+  using p1::tanh_step;
+  using I = ElemIdx<6>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int p = blockIdx.x;
   const int s = M.patch_sys[p];
   if (in.active && !in.active[s]) return;
-  const int E = M.max_patch_elems;
-  KT* sK = reinterpret_cast<KT*>(smem);
-  size_t koff = WITHK ? (((size_t)I::NKE * E * sizeof(KT) + 15) & ~(size_t)15) : 0;
-  double* sR = reinterpret_cast<double*>(smem + koff);
+  const bool kw = out.K != nullptr;
+  const int E = M.max_patch_elems, MH = M.max_patch_hnodes;
+  double2* pts = reinterpret_cast<double2*>(smem);  // [G][kIpc][kPairs]
+  double2* sD = pts + (size_t)G * kIpc * kPairs;              // reference derivatives [ip][6]
+  double* sN = reinterpret_cast<double*>(sD + kIps * 6);      // N [ip][6], then the weights
+  double* nd = sN + kIps * 7;
+  double* sR = nd + (size_t)ND_COUNT * MH;
+  KT* sK = reinterpret_cast<KT*>(sR + (size_t)24 * E);
   const int e0 = M.patch_elem_ptr[p], ne = M.patch_elem_ptr[p + 1] - e0;
   const int uoff = M.sys_dof_off[s] - M.sys_node_off[s];
-  const int nn_s = M.sys_node_off[s + 1] - M.sys_node_off[s];
-  const int voff = uoff + nn_s;
+  const int voff = uoff + (M.sys_node_off[s + 1] - M.sys_node_off[s]);
   const double gam = in.gamma ? in.gamma[s] : 0.0;
   const SysScal S = in.scal[s];
-  // nodal values of element e (u, v at X + gamma dX)
-  auto gather = [&](int e, int (&gn)[NOD], double (&xe)[NOD], double (&ye)[NOD], double (&hn)[NOD],
-                    double (&sn)[NOD], double (&un)[NOD], double (&vn)[NOD], double (&Cn)[NOD], double (&mn)[NOD],
-                    double (&An)[NOD], double (&nn)[NOD], double (&Sn)[NOD], double (&Bn)[NOD], double (&rn)[NOD]) {
-#pragma unroll
-    for (int a = 0; a < NOD; ++a) {
-      int gnode = __ldg(M.conn + (size_t)a * M.ne + e);
-      bool okn = true;
-      UA_CHECK_INDEX(M.dbg, gnode, 0, M.nn, BS_ELEM_NODE, okn);
-      (void)okn;
-      gn[a] = gnode;
-      xe[a] = __ldg(M.x + gnode); ye[a] = __ldg(M.y + gnode);
-      hn[a] = __ldg(in.h + gnode); sn[a] = __ldg(in.s + gnode);
-      double u = __ldg(in.X + uoff + gnode), v = __ldg(in.X + voff + gnode);
-      if (in.dX) { u += gam * __ldg(in.dX + uoff + gnode); v += gam * __ldg(in.dX + voff + gnode); }
-      un[a] = u; vn[a] = v;
-      Cn[a] = __ldg(in.C + gnode); mn[a] = __ldg(in.m + gnode);
-      An[a] = __ldg(in.A + gnode); nn[a] = __ldg(in.n + gnode);
-      Sn[a] = __ldg(in.S + gnode); Bn[a] = __ldg(in.B + gnode);
-      rn[a] = __ldg(in.rho + gnode);
-    }
-  };
-  auto store = [&](int t, const KT* Kuu, const KT* Kvv, const KT* Kuv, const double* Tx, const double* Fx,
-                   const double* Ty, const double* Fy) {
-    if (WITHK) {
-#pragma unroll
-      for (int i = 0; i < I::NS; ++i) { sK[i * E + t] = Kuu[i]; sK[(I::NS + i) * E + t] = Kvv[i]; }
-#pragma unroll
-      for (int i = 0; i < NOD * NOD; ++i) sK[(2 * I::NS + i) * E + t] = Kuv[i];
-    }
-#pragma unroll
-    for (int a = 0; a < NOD; ++a) {
-      sR[(0 * NOD + a) * E + t] = Tx[a];
-      sR[(1 * NOD + a) * E + t] = Fx[a];
-      sR[(2 * NOD + a) * E + t] = Ty[a];
-      sR[(3 * NOD + a) * E + t] = Fy[a];
-    }
-  };
-  for (int t = threadIdx.x; t < ne; t += blockDim.x) {
-    int gn[NOD];
-    double xe[NOD], ye[NOD], hn[NOD], sn[NOD], un[NOD], vn[NOD], Cn[NOD], mn[NOD], An[NOD], nn[NOD], Sn[NOD],
-        Bn[NOD], rn[NOD];
-    gather(__ldg(M.patch_elems + e0 + t), gn, xe, ye, hn, sn, un, vn, Cn, mn, An, nn, Sn, Bn, rn);
-    KT Kuu[I::NS], Kvv[I::NS], Kuv[NOD * NOD];
-    double Tx[NOD], Fx[NOD], Ty[NOD], Fy[NOD];
-    uv_element<NOD, WITHK, KT, GEN>(Q, P, S, gn, in.drag, xe, ye, hn, sn, un, vn, Cn, mn, An, nn, Sn, Bn, rn, Kuu, Kvv,
-                               Kuv, Tx, Fx, Ty, Fy);
-    store(t, Kuu, Kvv, Kuv, Tx, Fx, Ty, Fy);
+  const bool cube = S.cube != 0.0;  // n = m = 3 at every node of the system
+  // the rule's tables (lanes of a warp work on different points)
+  for (int t = threadIdx.x; t < kIps * 6; t += blockDim.x) {
+    sN[t] = Q.fun[t / 6][t % 6];
+    sD[t] = make_double2(Q.der[t / 6][0][t % 6], Q.der[t / 6][1][t % 6]);
+  }
+  for (int t = threadIdx.x; t < kIps; t += blockDim.x) sN[kIps * 6 + t] = Q.w[t];
+  const int hb0 = M.patch_hnode_ptr[p], nh = M.patch_hnode_ptr[p + 1] - hb0;
+  for (int t = threadIdx.x; t < nh; t += blockDim.x) {
+    int gn = __ldg(M.patch_hnodes + hb0 + t);
+    bool okn = true;
+    UA_CHECK_INDEX(M.dbg, gn, M.sys_node_off[s], M.sys_node_off[s + 1], BS_ELEM_NODE, okn);
+    (void)okn;
+    double u = __ldg(in.X + uoff + gn), v = __ldg(in.X + voff + gn);  // at X + gamma dX (CalcCostFunctionNR.m:14-16)
+    if (in.dX) { u += gam * __ldg(in.dX + uoff + gn); v += gam * __ldg(in.dX + voff + gn); }
+    const double h = __ldg(in.h + gn);
+    nd[ND_X * MH + t] = __ldg(M.x + gn); nd[ND_Y * MH + t] = __ldg(M.y + gn);
+    nd[ND_U * MH + t] = u; nd[ND_V * MH + t] = v;
+    nd[ND_H * MH + t] = h; nd[ND_BL * MH + t] = __ldg(in.s + gn) - h;
+    nd[ND_C * MH + t] = __ldg(in.C + gn); nd[ND_A * MH + t] = __ldg(in.A + gn);
+    nd[ND_HB * MH + t] = __ldg(in.S + gn) - __ldg(in.B + gn);
+    nd[ND_RHO * MH + t] = __ldg(in.rho + gn);
+    nd[ND_M * MH + t] = cube ? 3.0 : __ldg(in.m + gn);
+    nd[ND_N * MH + t] = cube ? 3.0 : __ldg(in.n + gn);
   }
   __syncthreads();
-  patch_scatter<NOD, WITHK, KT>(M, out, p, s, uoff, voff, sK, sR, E);
+  const double rhow = S.rhow, g = S.g, ca = S.ca, sa = S.sa;
+  const int ngr = (ne + G - 1) / G, gs = (ne + ngr - 1) / ngr;  // groups of equal size
+  for (int gb = 0; gb < ne; gb += gs) {
+    const int gn_ = min(gs, ne - gb);
+    // rows of this thread: element el of the group, node a
+    const int el = threadIdx.x / 6, a = threadIdx.x - 6 * el;
+    double kuu[6] = {}, kvv[6] = {}, kuv[6] = {}, Tx = 0, Fx = 0, Ty = 0, Fy = 0;
+    for (int ip0 = 0; ip0 < kIps; ip0 += kIpc) {
+      const int nip = min(kIpc, kIps - ip0);
+      // (a) points
+      for (int t = threadIdx.x; t < gn_ * nip; t += blockDim.x) {
+        const int pe = t / nip, pi = t - pe * nip, ip = ip0 + pi;
+        const uint16_t* ln = M.patch_elnodes + (size_t)(e0 + gb + pe) * 6;
+        int l[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+          l[k] = __ldg(ln + k);
+          bool okn = true;
+          UA_CHECK_INDEX(M.dbg, l[k], 0, nh, BS_ELEM_NODE, okn);
+          (void)okn;
+        }
+        const double* N = sN + ip * 6;
+        // derivVector.m:96-109, gradients by the chain rule
+        double J11 = 0, J12 = 0, J21 = 0, J22 = 0, u1 = 0, u2 = 0, v1 = 0, v2 = 0, b1 = 0, b2 = 0;
+        double hint = 0, uint = 0, vint = 0, Cint = 0, Aint = 0, Hint = 0, rhoint = 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+          const double2 dr = sD[ip * 6 + k];
+          const double Nk = N[k], x = nd[ND_X * MH + l[k]], y = nd[ND_Y * MH + l[k]];
+          const double u = nd[ND_U * MH + l[k]], v = nd[ND_V * MH + l[k]], b = nd[ND_BL * MH + l[k]];
+          J11 += x * dr.x; J12 += y * dr.x;
+          J21 += x * dr.y; J22 += y * dr.y;
+          u1 += u * dr.x; u2 += u * dr.y;
+          v1 += v * dr.x; v2 += v * dr.y;
+          b1 += b * dr.x; b2 += b * dr.y;
+          uint += u * Nk; vint += v * Nk;
+          hint += nd[ND_H * MH + l[k]] * Nk;
+          Cint += nd[ND_C * MH + l[k]] * Nk; Aint += nd[ND_A * MH + l[k]] * Nk;
+          Hint += nd[ND_HB * MH + l[k]] * Nk; rhoint += nd[ND_RHO * MH + l[k]] * Nk;
+        }
+        const double detJ = J11 * J22 - J12 * J21, rd = 1.0 / detJ;
+        // d/dx = ix d/dxi + jx d/deta, d/dy = iy d/dxi + jy d/deta
+        const double ix = J22 * rd, jx = -J12 * rd, iy = -J21 * rd, jy = J11 * rd;
+        const double exx = ix * u1 + jx * u2, eyy = iy * v1 + jy * v2;
+        const double exy = 0.5 * ((ix * v1 + jx * v2) + (iy * u1 + jy * u2));
+        const double dbdx = ix * b1 + jx * b2, dbdy = iy * b1 + jy * b2;
+        double2* o = pts + ((size_t)pe * kIpc + pi) * kPairs;
+        if (Cint < P.Cmin) Cint = P.Cmin;          // :205
+        if (Aint < P.AGlenmin) Aint = P.AGlenmin;  // :243
+        double mint = 3.0, nint = 3.0;
+        if (!cube) {
+          mint = nint = 0;
+#pragma unroll
+          for (int k = 0; k < 6; ++k) { mint += nd[ND_M * MH + l[k]] * N[k]; nint += nd[ND_N * MH + l[k]] * N[k]; }
+        }
+        const double hfint = rhow * Hint / rhoint;  // :300-310
+        const double tf = tanh_step(P.kH, hint - hfint, P.Hh0);
+        const double Heint = 0.5 + 0.5 * tf;
+        const double HEint = P.Hh0 == 0.0 ? 0.5 - 0.5 * tf : 0.5 + 0.5 * tanh_step(P.kH, hfint - hint, P.Hh0);
+        const double Hposint = (0.5 + 0.5 * tanh_step(P.kH, Hint, P.Hh0)) * Hint;
+        const double dint = HEint * rhoint * hint / rhow + Heint * Hposint;
+        Drag d{};  // :351-352; Weertman drag is identically zero on floating ice (He = 0)
+        if (GEN) {
+          int gn[6];
+          double Nw[6];
+#pragma unroll
+          for (int k = 0; k < 6; ++k) { gn[k] = __ldg(M.patch_hnodes + hb0 + l[k]); Nw[k] = N[k]; }
+          d = basal_drag_general(P, Heint, 0.0, hint, Hint, rhoint, rhow, g, uint, vint, Cint, mint,
+                                 drag_interp<6>(in.drag, gn, Nw));
+        } else if (Heint > 0) {
+          d = basal_drag_weertman(P, Heint, 0.0, uint, vint, Cint, mint, cube);
+        }
+        double eta, Ev;
+        effective_viscosity(P, Aint, nint, exx, eyy, exy, eta, Ev, cube);  // :353
+        const double w = detJ * Q.w[ip], he = hint * eta * w;
+        if (kw) {
+          const double hE = P.Dvisk * 2.0 * hint * Ev * w;
+          const double p1 = 2 * exx + eyy, q1 = 2 * eyy + exx, q2 = exy;  // P_u = p1 Dx + q2 Dy, P_v = q1 Dy + q2 Dx
+          // the rows of a 2x2 matrix between the inverse Jacobian's columns (ix, jx) and (iy, jy)
+          auto ref = [&](double axx, double axy, double ayx, double ayy, double2& r1, double2& r2) {
+            const double x1 = axx * ix + axy * iy, x2 = axx * jx + axy * jy;
+            const double y1 = ayx * ix + ayy * iy, y2 = ayx * jx + ayy * jy;
+            r1 = make_double2(ix * x1 + iy * y1, ix * x2 + iy * y2);
+            r2 = make_double2(jx * x1 + jy * y1, jx * x2 + jy * y2);
+          };
+          double2 r1, r2;
+          ref(4 * he + hE * p1 * p1, hE * p1 * q2, hE * p1 * q2, he + hE * q2 * q2, r1, r2);
+          o[PR_UU] = r1;
+          o[PR_UUC] = make_double2(r2.y, d.dxu * w);
+          ref(he + hE * q2 * q2, hE * q1 * q2, hE * q1 * q2, 4 * he + hE * q1 * q1, r1, r2);
+          o[PR_VV] = r1;
+          o[PR_VVC] = make_double2(r2.y, d.dyv * w);
+          ref(hE * p1 * q2, 2 * he + hE * p1 * q1, he + hE * q2 * q2, hE * q2 * q1, r1, r2);
+          o[PR_UV1] = r1;
+          o[PR_UV2] = r2;
+        }
+        const double rr = rhoint * hint - rhow * dint;  // :431-449
+        const double pp = 0.5 * g * ca * (rhoint * hint * hint - rhow * dint * dint) * w;
+        const double sx = he * (4 * exx + 2 * eyy), sy = he * (4 * eyy + 2 * exx), sq = he * 2 * exy;
+        o[PR_TX] = make_double2(sx * ix + sq * iy, sx * jx + sq * jy);
+        o[PR_TY] = make_double2(sq * ix + sy * iy, sq * jx + sy * jy);
+        // pressure term: pp d/dx and pp d/dy from the transformed pairs (pp ix, pp jx), (pp iy, pp jy)
+        o[PR_PX] = make_double2(pp * ix, pp * jx);
+        o[PR_PY] = make_double2(pp * iy, pp * jy);
+        o[PR_XV] = make_double2(d.dxv * w, 0.0);
+        o[PR_TN] = make_double2(d.taux * w, d.tauy * w);
+        o[PR_FN] = make_double2((-g * rr * dbdx * ca + rhoint * g * hint * sa) * w, -g * rr * dbdy * ca * w);
+      }
+      __syncthreads();
+      // (b) rows
+      if (el < gn_) {
+        const double2* q = pts + (size_t)el * kIpc * kPairs;
+        for (int pi = 0; pi < nip; ++pi, q += kPairs) {
+          const double* N = sN + (ip0 + pi) * 6;
+          const double2* dr = sD + (ip0 + pi) * 6;
+          const double2 da = dr[a], tx = q[PR_TX], ty = q[PR_TY], px = q[PR_PX], py = q[PR_PY],
+                        tn = q[PR_TN], fn = q[PR_FN];
+          const double Na = N[a];
+          Tx += tx.x * da.x + tx.y * da.y + tn.x * Na;
+          Fx += px.x * da.x + px.y * da.y + fn.x * Na;
+          Ty += ty.x * da.x + ty.y * da.y + tn.y * Na;
+          Fy += py.x * da.x + py.y * da.y + fn.y * Na;
+          if (kw) {
+            const double2 uu = q[PR_UU], uc = q[PR_UUC], vv = q[PR_VV], vc = q[PR_VVC], c1 = q[PR_UV1], c2 = q[PR_UV2];
+            const double ux = uu.x * da.x + uu.y * da.y, uy = uu.y * da.x + uc.x * da.y, un = uc.y * Na;
+            const double vx = vv.x * da.x + vv.y * da.y, vy = vv.y * da.x + vc.x * da.y, vn = vc.y * Na;
+            const double wx = c1.x * da.x + c2.x * da.y, wy = c1.y * da.x + c2.y * da.y, wn = q[PR_XV].x * Na;
+#pragma unroll
+            for (int b = 0; b < 6; ++b) {
+              const double2 db = dr[b];
+              const double Nb = N[b];
+              kuu[b] += ux * db.x + uy * db.y + un * Nb;
+              kvv[b] += vx * db.x + vy * db.y + vn * Nb;
+              kuv[b] += wx * db.x + wy * db.y + wn * Nb;
+            }
+          }
+        }
+      }
+      __syncthreads();  // the points are rewritten
+    }
+    if (el < gn_) {
+      const int t = gb + el;
+      sR[(0 * 6 + a) * E + t] = Tx;
+      sR[(1 * 6 + a) * E + t] = Fx;
+      sR[(2 * 6 + a) * E + t] = Ty;
+      sR[(3 * 6 + a) * E + t] = Fy;
+      if (kw) {
+#pragma unroll
+        for (int b = 0; b < 6; ++b) {
+          if (b >= a) {  // the symmetric blocks keep their upper triangle
+            const int y = I::sym(a, b);
+            sK[y * E + t] = (KT)kuu[b];
+            sK[(I::NS + y) * E + t] = (KT)kvv[b];
+          }
+          sK[(2 * I::NS + a * 6 + b) * E + t] = (KT)kuv[b];
+        }
+      }
+    }
+  }
+  __syncthreads();
+  patch_scatter<6, true, KT>(M, out, p, s, uoff, voff, sK, sR, E);
 }
 
-size_t uv_patch_smem(int nod, bool withK, bool fp32, int E) {
-  int NS = nod * (nod + 1) / 2, NKE = 2 * NS + nod * nod;
-  size_t k = withK ? (((size_t)NKE * E * (fp32 ? 4 : 8) + 15) & ~(size_t)15) : 0;
-  return k + (size_t)4 * nod * E * 8;
+// shared memory of the P2 kernel without its points, and of one element's points
+static size_t uv_p2_smem_base(bool withK, bool fp32, int E, int MH) {
+  return (size_t)p2::kIps * 19 * 8 + (size_t)p2::ND_COUNT * MH * 8 + (size_t)24 * E * 8 +
+         (withK ? (size_t)ElemIdx<6>::NKE * E * (fp32 ? 4 : 8) : 0);
 }
+constexpr size_t kP2Point = (size_t)p2::kIpc * p2::kPairs * sizeof(double2);
 
 template <bool WITHK, typename KT, bool GEN>
 static auto p1_kernel(int rv) {
@@ -705,17 +671,30 @@ static cudaError_t launch_p1(const ua_mesh* m, const UvPhys& P, const UvIn& in, 
   return cudaGetLastError();
 }
 
-template <int NOD, bool WITHK, typename KT>
-static cudaError_t launch_t(const ua_mesh* m, const UvPhys& P, const UvIn& in, const UvOut& out, int threads) {
-  size_t sm = uv_patch_smem(NOD, WITHK, sizeof(KT) == 4, m->dm.max_patch_elems);
+template <typename KT>
+static cudaError_t launch_p2(const ua_mesh* m, const UvPhys& P, const UvIn& in, const UvOut& out) {
+  if (quad_table(6).nip != p2::kIps) return cudaErrorInvalidConfiguration;
+  constexpr size_t kLimit = 227 * 1024, kHalf = 113 * 1024;
+  const int E = m->dm.max_patch_elems;
+  const size_t base = uv_p2_smem_base(out.K != nullptr, sizeof(KT) == 4, E, m->dm.max_patch_hnodes);
+  if (base + kP2Point > kLimit) return cudaErrorInvalidConfiguration;
+  // elements of a group: what the shared memory of half an SM takes if that is 12 or more (two CTAs
+  // of 128 registers hide each other's staging and barriers), else of the whole one (one CTA of 168)
+  int G = base < kHalf ? (int)((kHalf - base) / kP2Point) : 0;
+  const bool two = G >= std::min(12, E);
+  if (two) G = std::min(G, p2::kMaxG2);
+  else G = std::min((int)((kLimit - base) / kP2Point), p2::kMaxG);
+  G = std::max(1, std::min(G, E));
+  const size_t sm = base + (size_t)G * kP2Point;
   const bool gen = P.law != UA_SLIDING_WEERTMAN || P.melange;
-  auto kern = gen ? uv_patch_kernel<NOD, WITHK, KT, true> : uv_patch_kernel<NOD, WITHK, KT, false>;
+  auto kern = two ? (gen ? uv_p2_kernel<KT, true, 2> : uv_p2_kernel<KT, false, 2>)
+                  : (gen ? uv_p2_kernel<KT, true, 1> : uv_p2_kernel<KT, false, 1>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  // all of the unified L1/shared storage as shared memory: several patch blocks per SM
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
-  kern<<<m->dm.npatch, NOD == 3 ? threads : 128, sm, m->stream>>>(m->dm, quad_table(NOD), P, in, out);
+  const int threads = std::max(128, (6 * G + 31) & ~31);
+  kern<<<m->dm.npatch, threads, sm, m->stream>>>(m->dm, quad_table(6), P, in, out, G);
   return cudaGetLastError();
 }
 
@@ -728,8 +707,9 @@ cudaError_t launch_uv_assembly(const ua_mesh* m, const UvPhys& P, const UvIn& in
     const int t = threads > 0 ? threads : p1::kThreads;
     return fp32K ? launch_p1<true, float>(m, P, in, o, t, regs) : launch_p1<true, double>(m, P, in, o, t, regs);
   }
-  if (!withK) return launch_t<6, false, double>(m, P, in, out, 128);
-  return fp32K ? launch_t<6, true, float>(m, P, in, out, 128) : launch_t<6, true, double>(m, P, in, out, 128);
+  UvOut o = out;
+  if (!withK) o.K = nullptr;
+  return fp32K ? launch_p2<float>(m, P, in, o) : launch_p2<double>(m, P, in, o);
 }
 
 }  // namespace ua
