@@ -1732,9 +1732,13 @@ int amg_numeric(ua_mesh* m, const int* rowptr0, const int* colind0, const void* 
     bool ok = true;
     if (!a->d_prefresh) a->d_prefresh = (int*)dalloc(m, a, sizeof(int) * ns, ok);
     if (!ok) return set_error(UA_ERR_OOM, "AMG: device allocation failed");
-    UA_CUDA_TRY(cudaMemcpyAsync(a->d_prefresh, a->h_prefresh.data(), sizeof(int) * ns, cudaMemcpyHostToDevice,
-                                m->stream));
-    UA_CUDA_TRY(cudaStreamSynchronize(m->stream));  // h_prefresh is rewritten by the next set-up
+    // the pinned copies alternate, so that one is rewritten two set-ups later (a Newton step drains
+    // the stream in between)
+    if (!a->h_pin && cudaMallocHost(&a->h_pin, 2 * sizeof(int) * ns) != cudaSuccess)
+      return set_error(UA_ERR_OOM, "AMG: pinned host allocation failed");
+    int* hp = a->h_pin + (a->pin_at ^= 1) * ns;
+    std::copy(a->h_prefresh.begin(), a->h_prefresh.end(), hp);
+    UA_CUDA_TRY(cudaMemcpyAsync(a->d_prefresh, hp, sizeof(int) * ns, cudaMemcpyHostToDevice, m->stream));
     psel = a->d_prefresh;
   }
   const int sm = (int)(sizeof(double) * (size_t)a->maxdn * a->maxdn);

@@ -150,6 +150,8 @@ struct GmSolve {
 int gmres_resident_max_restart();
 int gmres_resident(ua_mesh* m, const GmSolve& v, const std::vector<int>& sel, const std::vector<int>& steps, int nsm,
                    long long* launches);
+// device flag set by a resident solve whose team did not meet
+const int* resident_error_flag(const ua_mesh* m);
 // pass classes of a profiled resident solve: operator, finest restriction, finest up pass, rest
 int pcg_resident_status(ua_mesh* m, bool prof, double* ms, int* cnt);
 

@@ -210,11 +210,14 @@ struct Amg {
   // whose prolongators the current set-up recomputes
   std::vector<int> p_age, h_prefresh;
   int* d_prefresh = nullptr;
+  int* h_pin = nullptr;  // pinned, two alternating copies of the refresh selection
+  int pin_at = 0;
   // the numeric set-up of a Newton step captured as one CUDA graph per (precision, selection
   // kind) and replayed: every argument is a fixed device buffer of the handle
   cudaGraphExec_t setup_exec[32] = {};
   long long setup_nodes[32] = {};
   ~Amg() {
+    if (h_pin) cudaFreeHost(h_pin);
     for (auto& e : setup_exec)
       if (e) cudaGraphExecDestroy(e);
   }

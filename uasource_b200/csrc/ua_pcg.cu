@@ -795,6 +795,8 @@ int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, con
   return rc;
 }
 
+const int* resident_error_flag(const ua_mesh* m) { return m->amg->cyc.d_err; }
+
 // After the solve's stream has drained: whether every barrier was met, and the pass times (ms of
 // the whole grid) and counts of a profiled solve.
 int pcg_resident_status(ua_mesh* m, bool prof, double* ms, int* cnt) {

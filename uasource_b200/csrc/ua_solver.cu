@@ -138,6 +138,13 @@ struct Work {
   // pinned host staging
   double* h_sysv = nullptr;
   int* h_int = nullptr;
+  // pinned staging ring of the small per-iteration uploads (selections, step lengths): a slot is
+  // rewritten only after the stream has drained once since its use
+  char* h_ring = nullptr;
+  size_t ring_at = 0, ring_cap = 0;
+  double* h_sysv0 = nullptr;  // cost at gamma = 0, read with the one at gamma = 1
+  int* h_res = nullptr;       // iteration counts and error flag of a deferred resident solve
+  bool defer = false, deferred = false;
   int* nan_first = nullptr;  // device NaN scan result (9 ints) and its pinned host copy
   int* h_nan = nullptr;
   double* h_gamma = nullptr;
@@ -866,6 +873,9 @@ static int ensure_work(ua_mesh* m, const ua_params* p) {
   if (cudaMallocHost(&w->h_sysv, SV_COUNT * sizeof(double) * nsys) != cudaSuccess ||
       cudaMallocHost(&w->h_int, 4 * sizeof(int) * (nsys + 1)) != cudaSuccess ||
       cudaMallocHost(&w->h_nan, 16 * sizeof(int)) != cudaSuccess ||
+      cudaMallocHost(&w->h_sysv0, SV_COUNT * sizeof(double) * nsys) != cudaSuccess ||
+      cudaMallocHost(&w->h_res, sizeof(int) * (nsys + 1)) != cudaSuccess ||
+      cudaMallocHost(&w->h_ring, w->ring_cap = 65536 + 256 * (size_t)nsys) != cudaSuccess ||
       cudaMallocHost(&w->h_gamma, sizeof(double) * nsys) != cudaSuccess) {
     delete w;
     return set_error(UA_ERR_OOM, "pinned host allocation failed");
@@ -1323,22 +1333,54 @@ static int build_constraints(ua_mesh* m, const ua_bcs* bcs, int nB) {
   return UA_OK;
 }
 
-// The host staging buffers (pinned) are rewritten only after the stream has drained, so an
-// earlier asynchronous copy from them cannot pick up the new values.
+// A slot of the pinned ring for an asynchronous upload; the ring starts over after a drain.
+static void* ring_slot(ua_mesh* m, size_t bytes) {
+  Work* w = m->work;
+  bytes = (bytes + 15) & ~(size_t)15;
+  if (w->ring_at + bytes > w->ring_cap) {
+    if (cudaStreamSynchronize(m->stream) != cudaSuccess) return nullptr;
+    w->ring_at = 0;
+  }
+  void* p = w->h_ring + w->ring_at;
+  w->ring_at += bytes;
+  return p;
+}
+
 static int set_sel(ua_mesh* m, const std::vector<int>& sel) {
   Work* w = m->work;
-  UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
+  int* h = (int*)ring_slot(m, w->nsys * sizeof(int));
+  if (!h) return set_error(UA_ERR_CUDA, "selection upload: the stream failed");
   w->h_sel.assign(sel.begin(), sel.begin() + w->nsys);
-  for (int s = 0; s < w->nsys; ++s) w->h_int[s] = sel[s];
-  UA_CUDA_TRY(cudaMemcpyAsync(w->sel, w->h_int, w->nsys * sizeof(int), cudaMemcpyHostToDevice, m->stream));
+  for (int s = 0; s < w->nsys; ++s) h[s] = sel[s];
+  UA_CUDA_TRY(cudaMemcpyAsync(w->sel, h, w->nsys * sizeof(int), cudaMemcpyHostToDevice, m->stream));
   return UA_OK;
 }
 
 static int set_gamma(ua_mesh* m, const std::vector<double>& g) {
   Work* w = m->work;
-  UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
-  for (int s = 0; s < w->nsys; ++s) w->h_gamma[s] = g[s];
-  UA_CUDA_TRY(cudaMemcpyAsync(w->gamma, w->h_gamma, w->nsys * sizeof(double), cudaMemcpyHostToDevice, m->stream));
+  double* h = (double*)ring_slot(m, w->nsys * sizeof(double));
+  if (!h) return set_error(UA_ERR_CUDA, "step length upload: the stream failed");
+  for (int s = 0; s < w->nsys; ++s) h[s] = g[s];
+  UA_CUDA_TRY(cudaMemcpyAsync(w->gamma, h, w->nsys * sizeof(double), cudaMemcpyHostToDevice, m->stream));
+  return UA_OK;
+}
+
+// Ends a deferred resident solve once the stream has drained: its iteration counts.
+static int finish_deferred(ua_mesh* m, std::vector<int>& its) {
+  Work* w = m->work;
+  if (!w->deferred) return UA_OK;
+  w->deferred = false;
+  if (w->h_res[w->nsys]) return set_error(UA_ERR_TIMEOUT, "resident solve: a team barrier was not met");
+  for (int s = 0; s < w->nsys; ++s) its[s] = its[s] ? w->h_res[s] : 0;
+  return UA_OK;
+}
+// Enqueues the counts of a resident solve for finish_deferred.
+static int defer_result(ua_mesh* m) {
+  Work* w = m->work;
+  UA_CUDA_TRY(cudaMemcpyAsync(w->h_res, w->its, w->nsys * sizeof(int), cudaMemcpyDeviceToHost, m->stream));
+  UA_CUDA_TRY(cudaMemcpyAsync(w->h_res + w->nsys, resident_error_flag(m), sizeof(int), cudaMemcpyDeviceToHost,
+                              m->stream));
+  w->deferred = true;
   return UA_OK;
 }
 
@@ -1365,22 +1407,26 @@ static int assemble(ua_mesh* m, const ua_params* p, bool withK, bool useDir, con
 // Cost function at X + gamma dX.  assembleR = false takes w->R as it stands:
 // the residual just assembled at X, which is the R-only assembly at gamma = 0.
 // withK: assemble the tangent too (the next Newton system's, if this point is accepted).
-static int cost_eval(ua_mesh* m, const ua_params* p, bool useDir, bool assembleR = true, bool withK = false) {
+// host: the pinned array that receives sysv; wait: drain the stream (else the caller does).
+// atX: gamma = 0 whatever w->gamma holds.
+static int cost_eval(ua_mesh* m, const ua_params* p, bool useDir, bool assembleR = true, bool withK = false,
+                     bool atX = false, double* host = nullptr, bool wait = true) {
   Work* w = m->work;
   if (assembleR) {
     int rc = assemble(m, p, withK, useDir, w->X, false);
     if (rc) return rc;
   }
+  const double* gamma = useDir && !atX ? w->gamma : nullptr;
   k_cost_rows<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->nrb, w->sel, w->R, w->dof_con, w->lam,
-                                             w->dlam, useDir ? w->gamma : nullptr, w->dX, w->part, w->con_dof, con_pairs(w)), ++g_launches;
+                                             w->dlam, gamma, w->dX, w->part, w->con_dof, con_pairs(w)), ++g_launches;
   k_cost_reduce<<<w->nsys, kRedThreads, 0, m->stream>>>(w->sys_rb_off, w->nrb, w->sel, w->part, w->nsys, w->sysv,
                                                          w->sys_con_off, w->con_dof, w->con_rhs, w->X,
-                                                         useDir ? w->dX : nullptr, w->dlam,
-                                                         useDir ? w->gamma : nullptr, 0, con_pairs(w)), ++g_launches;
+                                                         useDir ? w->dX : nullptr, w->dlam, gamma, 0, con_pairs(w)),
+      ++g_launches;
   UA_CUDA_TRY(cudaGetLastError());
-  UA_CUDA_TRY(cudaMemcpyAsync(w->h_sysv, w->sysv, SV_COUNT * w->nsys * sizeof(double), cudaMemcpyDeviceToHost,
-                              m->stream));
-  UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
+  UA_CUDA_TRY(cudaMemcpyAsync(host ? host : w->h_sysv, w->sysv, SV_COUNT * w->nsys * sizeof(double),
+                              cudaMemcpyDeviceToHost, m->stream));
+  if (wait) UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
   return UA_OK;
 }
 
@@ -1423,6 +1469,7 @@ static int pcg_resident_solve(ua_mesh* m, const ua_params* p, bool fp32, const v
     ++g_launches;
   }
   UA_CUDA_TRY(cudaGetLastError());
+  if (w->defer && !w->prof.on) return defer_result(m);
   UA_CUDA_TRY(cudaMemcpyAsync(w->h_int, w->its, w->nsys * sizeof(int), cudaMemcpyDeviceToHost, m->stream));
   UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
   double ms[4] = {};
@@ -1907,37 +1954,47 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
       if ((rc = set_sel(m, sel))) return rc;
     }
     k_frhs<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->R, w->dof_con, w->lam, w->frhs, w->con_dof, con_pairs(w)), ++g_launches;
-    UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
     double t1 = now_ms();
     t_asm += t1 - t0;
-    // linear solve (:242-257)
+    // linear solve (:242-257); a resident solve is not waited for: its counts come with the costs
     // (the iterations of the last step weigh the systems in the solve's schedule)
     for (int s = 0; s < nsys; ++s) its[s] = sel[s] ? std::max(1, st[s].kits) : 0;
     std::vector<double> eta(nsys);
     for (int s = 0; s < nsys; ++s) eta[s] = forcing_term(p, st[s].rForce);
-    if ((rc = linear_solve(m, p, its, eta.data()))) return rc;
-    double t2 = now_ms();
-    t_sol += t2 - t1;
-    for (int s = 0; s < nsys; ++s) if (sel[s]) st[s].kits = its[s];
-    // gamma=0 (:260-283): R at X is the residual assembled with K above
-    for (int s = 0; s < nsys; ++s) gam[s] = 0.0;
-    if ((rc = set_gamma(m, gam))) return rc;
-    if ((rc = cost_eval(m, p, true, false))) return rc;
-    for (int s = 0; s < nsys; ++s) {
-      if (!sel[s]) continue;
-      SysState& S = st[s];
-      S.r0 = S.rForce0 = w->h_sysv[SV_FF * nsys + s];
-      double D2 = w->h_sysv[SV_FD * nsys + s];
-      S.rWork0 = D2 * D2;
-      if (S.iteration == 1 && residual_criteria(p, S.rForce0, S.rWork0, S.iteration, 1.0)) {
-        S.iteration -= 1; S.converged = true; S.active = false; sel[s] = 0;
+    const std::vector<int> solved = sel;
+    w->defer = true;
+    rc = linear_solve(m, p, its, eta.data());
+    w->defer = false;
+    if (rc) return rc;
+    // gamma=0 (:260-283): R at X is the residual assembled with K above.  Only the first iteration
+    // decides on it before gamma = 1 is evaluated; else the two costs come back together.
+    bool first = false;
+    for (int s = 0; s < nsys; ++s) first = first || (sel[s] && st[s].iteration == 1);
+    auto cost0 = [&]() {
+      for (int s = 0; s < nsys; ++s) {
+        if (!sel[s]) continue;
+        SysState& S = st[s];
+        S.r0 = S.rForce0 = w->h_sysv0[SV_FF * nsys + s];
+        double D2 = w->h_sysv0[SV_FD * nsys + s];
+        S.rWork0 = D2 * D2;
+        if (S.iteration == 1 && residual_criteria(p, S.rForce0, S.rWork0, S.iteration, 1.0)) {
+          S.iteration -= 1; S.converged = true; S.active = false; sel[s] = 0;
+        }
       }
+    };
+    if ((rc = cost_eval(m, p, true, false, false, true, w->h_sysv0, first))) return rc;
+    if (first) {
+      cost0();
+      if ((rc = set_sel(m, sel))) return rc;
     }
     // gamma=1 (:288), with the tangent there when it is assembled ahead
     for (int s = 0; s < nsys; ++s) gam[s] = 1.0;
-    if ((rc = set_sel(m, sel))) return rc;
     if ((rc = set_gamma(m, gam))) return rc;
     if ((rc = cost_eval(m, p, true, true, ahead))) return rc;
+    if (!first) cost0();
+    if ((rc = finish_deferred(m, its))) return rc;
+    t_sol += now_ms() - t1;
+    for (int s = 0; s < nsys; ++s) if (solved[s]) st[s].kits = its[s];
     for (int s = 0; s < nsys; ++s) {
       if (!sel[s]) continue;
       SysState& S = st[s];
@@ -2563,6 +2620,7 @@ static int gmres_resident_solve(ua_mesh* m, const ua_params* p, const double* K,
                                                                          w->rowptr, w->colind, K, w->dX, w->frhs,
                                                                          w->dlam, con_pairs(w)), ++g_launches;
   UA_CUDA_TRY(cudaGetLastError());
+  if (w->defer && !w->prof.on) return defer_result(m);
   UA_CUDA_TRY(cudaMemcpyAsync(w->h_int, w->its, nsys * sizeof(int), cudaMemcpyDeviceToHost, m->stream));
   UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
   if (int rc = pcg_resident_status(m, false, nullptr, nullptr)) return rc;
@@ -2899,7 +2957,8 @@ static int assemble_uvh(ua_mesh* m, const ua_params* p, bool withK, bool useDir,
 // CalcCostFunctionNRuvh.m:12-105 for the selected systems
 // uvh cost function at X + gamma dX; assembleR = false takes w->R as it stands
 // (the residual just assembled at X, i.e. gamma = 0).
-static int cost_eval_uvh(ua_mesh* m, const ua_params* p, bool assembleR = true) {
+static int cost_eval_uvh(ua_mesh* m, const ua_params* p, bool assembleR = true, double* host = nullptr,
+                         bool wait = true) {
   Work* w = m->work;
   if (assembleR) {
     int rc = assemble_uvh(m, p, false, true, false, false);
@@ -2911,9 +2970,9 @@ static int cost_eval_uvh(ua_mesh* m, const ua_params* p, bool assembleR = true) 
                                                          w->sys_con_off, w->con_dof, w->con_rhs, w->X, w->dX, w->dlam,
                                                          w->gamma, 0, con_pairs(w)), ++g_launches;
   UA_CUDA_TRY(cudaGetLastError());
-  UA_CUDA_TRY(cudaMemcpyAsync(w->h_sysv, w->sysv, SV_COUNT * w->nsys * sizeof(double), cudaMemcpyDeviceToHost,
+  UA_CUDA_TRY(cudaMemcpyAsync(host ? host : w->h_sysv, w->sysv, SV_COUNT * w->nsys * sizeof(double), cudaMemcpyDeviceToHost,
                               m->stream));
-  UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
+  if (wait) UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
   return UA_OK;
 }
 
@@ -2980,7 +3039,6 @@ static int newton_run_uvh(ua_mesh* m, const ua_params* p, std::vector<ua_newton_
     double t0 = now_ms();
     if ((rc = assemble_uvh(m, p, true, false, false, false))) return rc;  // :127
     k_frhs<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->R, w->dof_con, w->lam, w->frhs, w->con_dof, con_pairs(w)), ++g_launches;
-    UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
     double t1 = now_ms();
     t_asm += t1 - t0;
     for (int s = 0; s < nsys; ++s) its[s] = sel[s] ? std::max(1, st[s].kits) : 0;
@@ -2989,22 +3047,28 @@ static int newton_run_uvh(ua_mesh* m, const ua_params* p, std::vector<ua_newton_
     if (p->uvh_krylov == UA_KRYLOV_BICGSTAB) {
       if ((rc = bicgstab_t<double>(m, p, w->Kd, its.data(), eta.data()))) return rc;  // :136
     } else {
-      if ((rc = gmres_t<double>(m, p, w->Kd, its.data(), eta.data()))) return rc;
+      w->defer = true;
+      rc = gmres_t<double>(m, p, w->Kd, its.data(), eta.data());
+      w->defer = false;
+      if (rc) return rc;
     }
-    t_sol += now_ms() - t1;
-    for (int s = 0; s < nsys; ++s) if (sel[s]) st[s].kits = its[s];
-    // r0 = func(0), r1 = func(1) (:155-156)
+    // r0 = func(0), r1 = func(1) (:155-156); the two come back together, with the iteration counts
     for (int g1 = 0; g1 < 2; ++g1) {
       for (int s = 0; s < nsys; ++s) gam[s] = (double)g1;
       if ((rc = set_gamma(m, gam))) return rc;
-      if ((rc = cost_eval_uvh(m, p, g1 != 0))) return rc;  // R at gamma = 0 was assembled with K
-      for (int s = 0; s < nsys; ++s) {
-        if (!sel[s]) continue;
-        const double rf = w->h_sysv[SV_FF * nsys + s], d2 = w->h_sysv[SV_FD * nsys + s];
-        UvhSys& S = st[s];
-        if (g1 == 0) { S.r0 = rf; S.ls_g.assign({0.0}); S.ls_D2.assign({d2}); }
-        else { S.r1 = rf; S.ls_g.push_back(1.0); S.ls_D2.push_back(d2); }
-      }
+      // R at gamma = 0 was assembled with K
+      if ((rc = cost_eval_uvh(m, p, g1 != 0, g1 ? nullptr : w->h_sysv0, g1 != 0))) return rc;
+    }
+    if ((rc = finish_deferred(m, its))) return rc;
+    t_sol += now_ms() - t1;
+    for (int s = 0; s < nsys; ++s) {
+      if (!sel[s]) continue;
+      UvhSys& S = st[s];
+      S.kits = its[s];
+      S.r0 = w->h_sysv0[SV_FF * nsys + s];
+      S.r1 = w->h_sysv[SV_FF * nsys + s];
+      S.ls_g.assign({0.0, 1.0});
+      S.ls_D2.assign({w->h_sysv0[SV_FD * nsys + s], w->h_sysv[SV_FD * nsys + s]});
     }
     // rLineminUa (:157): Newton-direction backtracking, BackTracking accepts
     // gamma=1 at once when r1 is below its target
@@ -3420,6 +3484,9 @@ extern "C" void ua_mesh_destroy(ua_mesh* m) {
       if (e) cudaGraphExecDestroy(e);
     if (w->h_sysv) cudaFreeHost(w->h_sysv);
     if (w->h_int) cudaFreeHost(w->h_int);
+    if (w->h_sysv0) cudaFreeHost(w->h_sysv0);
+    if (w->h_res) cudaFreeHost(w->h_res);
+    if (w->h_ring) cudaFreeHost(w->h_ring);
     if (w->h_nan) cudaFreeHost(w->h_nan);
     if (w->h_gamma) cudaFreeHost(w->h_gamma);
     delete w;
