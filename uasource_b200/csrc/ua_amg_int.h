@@ -16,7 +16,11 @@ constexpr int kAmgRB = 256;           // rows per row block of a coarse level
 constexpr int kSaRB = 128, kSaLPR = 2;
 constexpr int kAmgNB = 32;            // nodes per node block of the smoothed transfers (one warp's worth)  // smoothed hierarchies (longer coarse rows): rows per block, lanes per row
 
-constexpr double kSaOmega = 4.0 / 3.0;  // damping of the prolongator smoother (l1 diagonal: rho(D^-1 A) <= 1)
+// Damping of the prolongator smoother (l1 diagonal: rho(D^-1 A) <= 1).  4/3 is the textbook value for
+// a diagonal with rho = 1; the l1 diagonal overestimates rho, and the iteration counts fall until
+// about 1.7 (B200, summed Krylov iterations of a Newton solve, 4/3 -> 1.7: P1 229x113 mixed 187 ->
+// 169, P2 401x201 FP64 353 -> 324, uvh P1 141x71 329 -> 309, C adjoint 75 -> 68).
+constexpr double kSaOmega = 1.7;
 // Damping of the smoother, folded into its inverse diagonal.  With the l1 row sums the spectrum of
 // D^-1 A lies in (0, 1], so any factor below 2 keeps the sweep convergent and the cycle positive
 // definite (0.5% of room covers the BF16 values of the mixed form), and the plain sweep (factor 1)
