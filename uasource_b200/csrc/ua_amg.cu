@@ -421,27 +421,11 @@ static int amg_build(ua_mesh* m, bool smoothed) {
       F.ptn_ptr = upload(m, a, g_ptnp[l], ok);
       F.ptn_fine = upload(m, a, g_ptnf[l], ok);
       F.ptn_k = upload(m, a, g_ptnk[l], ok);
-      std::vector<int> pbase(nsys), pnnz(nsys), poff(nsys + 1, 0), apbase(nsys), apnnz(nsys), apoff(nsys + 1, 0);
-      for (int s = 0; s < nsys; ++s) {
-        pbase[s] = g_pnp[l][F.node_off[s]];
-        pnnz[s] = g_pnp[l][F.node_off[s + 1]] - pbase[s];
-        poff[s + 1] = poff[s] + 4 * pnnz[s];
-        apbase[s] = g_apnp[l][F.node_off[s]];
-        apnnz[s] = g_apnp[l][F.node_off[s + 1]] - apbase[s];
-        apoff[s + 1] = apoff[s] + 4 * apnnz[s];
-      }
-      F.pbase = upload(m, a, pbase, ok); F.pnnz = upload(m, a, pnnz, ok); F.poff = upload(m, a, poff, ok);
-      F.apbase = upload(m, a, apbase, ok); F.apnnz = upload(m, a, apnnz, ok); F.apoff = upload(m, a, apoff, ok);
-      F.ap_maxrow = 0;
-      for (size_t i = 0; i + 1 < g_apnp[l].size(); ++i)
-        F.ap_maxrow = std::max(F.ap_maxrow, g_apnp[l][i + 1] - g_apnp[l][i]);
-      F.ac_maxdeg = 0;
-      for (size_t I = 0; I + 1 < g_ptr[l + 1].size(); ++I)
-        F.ac_maxdeg = std::max(F.ac_maxdeg, g_ptr[l + 1][I + 1] - g_ptr[l + 1][I]);
-      F.sa_p = (double*)dalloc(m, a, sizeof(double) * (size_t)poff[nsys], ok);
       F.np = g_pnp[l].back();
-      F.sa_ap = (double*)dalloc(m, a, sizeof(double) * (size_t)apoff[nsys], ok);
-      F.sa_plo = (float*)dalloc(m, a, sizeof(float) * (size_t)poff[nsys], ok);
+      F.nap = g_apnp[l].back();
+      F.sa_ap = dalloc(m, a, 4 * sizeof(double) * (size_t)std::max(F.nap, 1LL), ok);
+      a->lev[l + 1].gptr = upload(m, a, g_ptr[l + 1], ok);
+      a->lev[l + 1].ng = g_ptr[l + 1].back();
     }
     pb[l] = a->lev[l].b;
     px2[l] = a->lev[l].x2;
@@ -547,7 +531,9 @@ __global__ void k_amg_l1(int n, const int* rowptr, const int* colind, const KT* 
 // has one barrier.  Step k is one update e_ij -= f_i w_j for every entry, with w_j = row_j / p and
 // f_i = column_i except w_k = 1 + 1/p and f_k = p - 1, which give the pivot row, the pivot column
 // and the pivot their own values without a test in the tile (the additions there are of terms of
-// equal sign as p <= 1).
+// equal sign as p <= 1).  The steps are unrolled over a tile's pivots, so that a pivot's place in the
+// tile is a compile-time index, and the pivot's owner takes the reciprocal: n = 94 in 44 us (every
+// thread selecting and dividing, 265 instructions a step: 102 us).
 constexpr int kDiT = 6, kDiG = kAmgMaxDense / kDiT, kDiThreads = kDiG * kDiG;
 static_assert(kAmgMaxDense % kDiT == 0 && kDiThreads <= 1024, "the threads' tiles cover the largest coarsest matrix");
 template <typename KT>
@@ -559,6 +545,7 @@ __global__ void __launch_bounds__(kDiThreads) k_amg_dense_inverse(const int* dep
   constexpr int ND = kAmgMaxDense;
   extern __shared__ double M[];  // n x n staging of the matrix
   __shared__ double prow[2][ND], pcol[2][ND], dg[ND];
+  __shared__ double2 piv[2];  // the pivot and its reciprocal
   const int s = blockIdx.x;
   const int n = dn_arr[s];
   if (n == 0 || (sel && !sel[s])) return;
@@ -591,33 +578,36 @@ __global__ void __launch_bounds__(kDiThreads) k_amg_dense_inverse(const int* dep
 #pragma unroll
     for (int j = 0; j < kDiT; ++j)
       e[i][j] = (r0 + i < n && c0 + j < n) ? M[(r0 + i) * n + c0 + j] * dg[r0 + i] * dg[c0 + j] : 0.0;
-  for (int k = 0; k < n; ++k) {
-    double *pr = prow[k & 1], *pc = pcol[k & 1];
-    if (mine && k >= r0 && k < r0 + kDiT) {
+  const int ty = threadIdx.x / kDiG, tx = threadIdx.x % kDiG;
+  for (int kb = 0; kb * kDiT < n; ++kb) {
+#pragma unroll
+    for (int kk = 0; kk < kDiT; ++kk) {  // pivot kb kDiT + kk: entry kk of tile row and column kb
+      const int k = kb * kDiT + kk;
+      if (k >= n) break;
+      double *pr = prow[kk & 1], *pc = pcol[kk & 1];
+      if (ty == kb) {
+        if (tx == kb) piv[kk & 1] = make_double2(e[kk][kk], 1.0 / e[kk][kk]);
+#pragma unroll
+        for (int j = 0; j < kDiT; ++j) pr[c0 + j] = e[kk][j];
+      }
+      if (tx == kb) {
+#pragma unroll
+        for (int i = 0; i < kDiT; ++i) pc[r0 + i] = e[i][kk];
+      }
+      __syncthreads();
+      if (!mine) continue;  // padding only (it still meets the barriers)
+      const double p = piv[kk & 1].x, inv = piv[kk & 1].y;
+      double w[kDiT], f[kDiT];
+#pragma unroll
+      for (int j = 0; j < kDiT; ++j) w[j] = pr[c0 + j] * inv;
+      if (tx == kb) w[kk] = 1.0 + inv;
+#pragma unroll
+      for (int i = 0; i < kDiT; ++i) f[i] = pc[r0 + i];
+      if (ty == kb) f[kk] = p - 1.0;
 #pragma unroll
       for (int i = 0; i < kDiT; ++i)
-        if (r0 + i == k)
 #pragma unroll
-          for (int j = 0; j < kDiT; ++j) pr[c0 + j] = e[i][j];
-    }
-    if (mine && k >= c0 && k < c0 + kDiT) {
-#pragma unroll
-      for (int j = 0; j < kDiT; ++j)
-        if (c0 + j == k)
-#pragma unroll
-          for (int i = 0; i < kDiT; ++i) pc[r0 + i] = e[i][j];
-    }
-    __syncthreads();
-    if (!mine) continue;  // padding only (it still meets the barriers)
-    const double p = pr[k], inv = 1.0 / p;
-    double w[kDiT];
-#pragma unroll
-    for (int j = 0; j < kDiT; ++j) w[j] = (c0 + j == k) ? 1.0 + inv : pr[c0 + j] * inv;
-#pragma unroll
-    for (int i = 0; i < kDiT; ++i) {
-      const double f = (r0 + i == k) ? p - 1.0 : pc[r0 + i];
-#pragma unroll
-      for (int j = 0; j < kDiT; ++j) e[i][j] = fma(-f, w[j], e[i][j]);
+        for (int j = 0; j < kDiT; ++j) e[i][j] = fma(-f[i], w[j], e[i][j]);
     }
   }
   if (!mine) return;
@@ -987,11 +977,11 @@ __global__ void __launch_bounds__(256, sizeof(VT) == 4 ? (MODE == 0 ? 4 : 5) : 0
 // device: smoothed aggregation (P = (I - w D^-1 A) P0, coarse operator P' A P)
 // ---------------------------------------------------------------------------
 //
-// Values live on node-level lists with the tangent's layout rule: the entry of
-// dof row (c, g), column component c2 and list position k of system s sits at
-// off[s] + c*2*nnz[s] + 2*(ptr[g] - base[s]) + c2*deg(g) + k.  Every output
-// entry is summed in a fixed order (no atomics), so results are reproducible.
-
+// Values are quads (the four entries of a node pair) on node-level lists.  The products that make an
+// entry of A P or of the coarse operator are listed once per handle (sa_lists), so a set-up has no
+// searches: a lane owns an entry, reads its products and writes it, in a fixed order and without
+// atomics.  (Scattering the products of a row into shared memory, with a search per product, issued
+// 456 warp instructions per node of P2 401x201; the lists issue about 30.)
 
 __device__ __forceinline__ int sa_find(const int* list, int n, int key) {  // list sorted ascending
   int lo = 0, hi = n;
@@ -1002,178 +992,253 @@ __device__ __forceinline__ int sa_find(const int* list, int n, int key) {  // li
   return lo < n && list[lo] == key ? lo : -1;
 }
 
-// dof row -> system, component, node (global) of a level
-__device__ __forceinline__ void sa_decode(int i, const int* dof_sys, const int* dof_off, const int* node_off, int& s,
-                                          int& c, int& g) {
-  s = dof_sys[i];
-  const int no = node_off[s], nn = node_off[s + 1] - no, loc = i - dof_off[s];
-  c = loc / nn;
-  g = no + (loc - c * nn);
+// ---- lists (once per handle) ----
+
+__global__ void k_sa_nrow(int nn, const int* node_sys, const int* node_off, const int* dof_off, const int* rowptr,
+                          int4* nrow) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= nn) return;
+  const int s = node_sys[g], no = node_off[s], n = node_off[s + 1] - no, i = dof_off[s] + (g - no);
+  nrow[g] = make_int4(rowptr[i], rowptr[i + n], (rowptr[i + 1] - rowptr[i]) >> 1, s);
+}
+__global__ void k_sa_ids(int nn, const int* ptr, int* node) {
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, lane = threadIdx.x & 3;
+  if (g >= nn) return;
+  for (int e = ptr[g] + lane; e < ptr[g + 1]; e += 4) node[e] = g;
+}
+// products of A P entry e = (g, J): neighbours h of g with J in P(h); lst = null: counts only
+__global__ void k_sa_ap_list(long long n, const int* node, const int* col, const int4* nrow, const int* node_off,
+                             const int* dof_off, const int* colind, const int* pn_ptr, const int* pn_col,
+                             unsigned* ptr, int2* lst, int* own) {
+  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const int g = node[e], J = col[e];
+  const int4 r = nrow[g];
+  const int sh = node_off[r.w] - dof_off[r.w];
+  unsigned at = lst ? ptr[e] : 0;
+  int p = -1;
+  for (int k = 0; k < r.z; ++k) {
+    const int h = colind[r.x + k] + sh;
+    for (int t = pn_ptr[h]; t < pn_ptr[h + 1]; ++t)
+      if (pn_col[t] == J) {
+        if (h == g) p = t;
+        if (lst) lst[at] = make_int2(k, t);
+        ++at;
+      }
+  }
+  if (!lst) ptr[e] = at;
+  else own[e] = p;
+}
+// products of coarse entry o = (J, K): fine nodes g of P'(J) with K in A P(g)
+__global__ void k_sa_ac_list(long long n, const int* node, const int* gptr, const int4* nrow_c, const int* node_off,
+                             const int* dof_off, const int* colind, const int* ptn_ptr, const int* ptn_fine,
+                             const int* ptn_k, const int* pn_ptr, const int* apn_ptr, const int* apn_col,
+                             unsigned* ptr, int2* lst) {
+  const long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (o >= n) return;
+  const int J = node[o];
+  const int4 r = nrow_c[J];
+  const int K = colind[r.x + (int)(o - gptr[J])] + node_off[r.w] - dof_off[r.w];
+  unsigned at = lst ? ptr[o] : 0;
+  for (int u = ptn_ptr[J]; u < ptn_ptr[J + 1]; ++u) {
+    const int g = ptn_fine[u], a0 = apn_ptr[g];
+    const int t = sa_find(apn_col + a0, apn_ptr[g + 1] - a0, K);
+    if (t < 0) continue;
+    if (lst) lst[at] = make_int2(pn_ptr[g] + ptn_k[u], a0 + t);
+    ++at;
+  }
+  if (!lst) ptr[o] = at;
+}
+// exclusive scan of v[0..n) in place, the sum in v[n] and total (one CTA of 1024 threads)
+__device__ int block_excl_scan(int v, int* sh, int& total);
+__global__ void __launch_bounds__(1024) k_sa_scan(long long n, unsigned* v, unsigned long long* total) {
+  __shared__ int sh[32];
+  constexpr int IT = 8;
+  unsigned long long base = 0;
+  for (long long b = 0; b < n; b += 1024 * IT) {
+    const long long i0 = b + (long long)threadIdx.x * IT;
+    int c[IT], sum = 0;
+#pragma unroll
+    for (int t = 0; t < IT; ++t) {
+      c[t] = i0 + t < n ? (int)v[i0 + t] : 0;
+      sum += c[t];
+    }
+    int tot;
+    const int ex = block_excl_scan(sum, sh, tot);
+    unsigned at = (unsigned)(base + (unsigned)ex);
+#pragma unroll
+    for (int t = 0; t < IT; ++t)
+      if (i0 + t < n) {
+        v[i0 + t] = at;
+        at += c[t];
+      }
+    base += (unsigned)tot;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    v[n] = (unsigned)base;
+    *total = base;
+  }
 }
 
-// prolongator rows: P(i,:) = P0(i,:) - w/l1_i A(i,:) P0 on unmasked rows and columns (invd holds
-// kSmoothOmega / l1), or the linear interpolation pn_w
-// ST: the type the set-up stores and sums P, A P and P' in (FP32 for the mixed-precision form,
-// whose V-cycle transfers read FP32 values, else FP64)
-template <typename KT, typename VT, typename ST>
-__global__ void k_sa_P(int nf, const int* dof_sys, const int* dof_off, const int* node_off, const int* rowptr,
-                       const int* colind, const KT* A, const unsigned char* mask, const VT* invd, const int* agg,
-                       const int* pn_ptr, const int* pn_col, const double* pn_w, const int* pbase, const int* pnnz,
-                       const int* poff, ST* P, const int* sel) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nf) return;
-  int s, c, g;
-  sa_decode(i, dof_sys, dof_off, node_off, s, c, g);
-  if (sel && !sel[s]) return;
-  const int pr = pn_ptr[g], dP = pn_ptr[g + 1] - pr;
-  ST* row = P + poff[s] + (size_t)c * 2 * pnnz[s] + 2 * (size_t)(pr - pbase[s]);
-  for (int t = 0; t < 2 * dP; ++t) row[t] = 0;
-  if (mask && mask[i]) return;
-  if (pn_w) {  // linear interpolation: the same weights for both components, no smoothing
-    for (int t = 0; t < dP; ++t) row[c * dP + t] = (ST)pn_w[pr + t];
-    return;
-  }
-  const int k0 = sa_find(pn_col + pr, dP, agg[g]);
-  if (k0 >= 0) row[c * dP + k0] = 1;
-  const ST f = (ST)(kSaOmega / kSmoothOmega * (double)invd[i]);
-  // the row holds the u block then the v block of the node's deg neighbours (the same nodes in
-  // the same order), so one search per neighbour serves both blocks; each target still sums its
-  // block's entries in row order
-  const int q0 = rowptr[i], deg = (rowptr[i + 1] - q0) >> 1;
-  const int d0 = dof_off[s], no = node_off[s], nn = node_off[s + 1] - no;
-  for (int k = 0; k < deg; ++k) {
-    const int ju = colind[q0 + k];
-    const int kk = sa_find(pn_col + pr, dP, agg[no + (ju - d0)]);
-    if (kk < 0) continue;
-    if (!(mask && mask[ju])) row[kk] -= f * (ST)A[q0 + k];
-    if (!(mask && mask[ju + nn])) row[dP + kk] -= f * (ST)A[q0 + deg + k];
-  }
-}
+// ---- values ----
 
-// A P rows: AP(i,:) = sum over unmasked columns j of A(i,j) P(j,:), kSaGL lanes per fine node g.
-// Both rows (c = 0, 1) of the node share its neighbour list, so each neighbour h contributes
-// A((c,g),(c2,h)) P((c2,h),:) to four output blocks (c, c3) at once.  The lanes first load the
-// data of up to kSaGL neighbours (column, the four A entries, the row of P(h,:)); the neighbours
-// then go in order.  A row of at most kSaApSm coarse columns is summed in shared memory (its
-// column list there too, for the searches): the lanes split into kSaApG groups of kSaGL / kSaApG,
-// group q takes the neighbours q, q + kSaApG, ... into its own copy of the row, its lanes the
-// entries of P(h,:), whose targets in the AP row are distinct, and the copies are added in group
-// order at the one write.  Longer rows are summed in place in global memory by all kSaGL lanes,
-// neighbour after neighbour.  Either way a fixed summation order without atomics.  FP32 values:
-// at most 48 registers, ten CTAs (40 warps) per SM for the gathers in flight.
+// Smoother diagonal and prolongator rows of fine node g, kSaGL lanes per node: the damped l1 diagonal
+// invd = kSmoothOmega / sum |a| over unmasked columns (0 on masked or empty rows) with its square root
+// sc and, in slice order, its inverse dw for the collapsed cycle; and P(g,:) = P0 - w/l1 A P0 on
+// unmasked rows and columns, or the linear interpolation pn_w.  The row's entries are staged in shared
+// memory with their neighbours' aggregates; a lane owns an entry of P and takes the neighbours of its
+// aggregate in row order.  ST: the type of the sums (FP32 in the mixed-precision form, else FP64).
+// One pass over the row instead of an l1 kernel, a scattered P, a repacking and the scaling: latency on
+// the coarse levels (P1 141x71, three levels: 113 -> 23 us cold), the row's bytes on large ones (P2
+// 401x201, four levels: 276 -> 133 us).
 constexpr int kSaGL = 8;
-constexpr int kSaApG = 2;
-constexpr int kSaApSm = 64;  // longest row summed in shared memory
-// dynamic shared memory: per fine node kSaApG copies of 4 * ms sums and ms columns (ms = 0: none)
-template <typename ST>
-size_t sa_ap_smem(int ms) { return (size_t)(128 / kSaGL) * ms * (kSaApG * 4 * sizeof(ST) + sizeof(int)); }
-template <typename KT, typename ST>
-__global__ void __launch_bounds__(128, sizeof(ST) == 4 ? 10 : 0) k_sa_AP(int nfn, const int* node_sys, const int* dof_off, const int* node_off,
-                                               const int* rowptr, const int* colind, const KT* A,
-                                               const unsigned char* mask, const int* pn_ptr, const int* pn_col,
-                                               const typename PQuadOf<KT>::T* Q, const int* apn_ptr,
-                                               const int* apn_col, const int* apbase, const int* apnnz,
-                                               const int* apoff, ST* AP, const int* sel, int ms) {
-  extern __shared__ __align__(16) unsigned char sa_smem[];
-  const int gi = threadIdx.x / kSaGL;
-  ST* g_acc = reinterpret_cast<ST*>(sa_smem) + (size_t)gi * kSaApG * 4 * ms;
-  int* g_col = reinterpret_cast<int*>(reinterpret_cast<ST*>(sa_smem) + (size_t)(128 / kSaGL) * kSaApG * 4 * ms) +
-               gi * ms;
-  const int g = (blockIdx.x * blockDim.x + threadIdx.x) / kSaGL, lane = threadIdx.x % kSaGL;
-  if (g >= nfn) return;  // whole groups leave together
+constexpr int kSaStage = 32;  // neighbours staged at a time
+template <typename KT, typename VT, typename QT>
+__global__ void __launch_bounds__(128) k_sa_P(int nf, const int4* nrow, const int* dof_off, const int* node_off,
+                                              const int* colind, const KT* A, const unsigned char* mask,
+                                              const int* agg, const int* pn_ptr, const int* pn_col,
+                                              const double* pn_w, QT* Q, VT* invd, double2* sc, VT* dw,
+                                              const int* ipos, const int* sel, const int* psel) {
+  using ST = KT;
+  __shared__ ST sv[128 / kSaGL][4][kSaStage];
+  __shared__ int sj[128 / kSaGL][kSaStage];
+  const int gi = threadIdx.x / kSaGL, lane = threadIdx.x % kSaGL;
+  const int g = blockIdx.x * (128 / kSaGL) + gi;
+  if (g >= nf) return;  // whole groups leave together
   const unsigned gmask = ((1u << kSaGL) - 1u) << ((threadIdx.x & 31) & ~(kSaGL - 1));
-  const int s = node_sys[g];
-  if (sel && !sel[s]) return;  // whole groups
+  const int4 r = nrow[g];
+  const int s = r.w, deg = r.z;
+  if (sel && !sel[s]) return;
   const int no = node_off[s], nn = node_off[s + 1] - no, d0 = dof_off[s];
   const int i0 = d0 + (g - no), i1 = i0 + nn;
-  const int ar = apn_ptr[g], dA = apn_ptr[g + 1] - ar;
-  const size_t ars = (size_t)2 * apnnz[s];  // AP row stride between c = 0 and c = 1
-  ST* r0 = AP + apoff[s] + 2 * (size_t)(ar - apbase[s]);
-  const bool sm = ms > 0;  // every row of the launch fits (ms is the level's longest row)
-  const int ng = sm ? kSaApG : 1, gw = kSaGL / ng;  // lane groups, lanes per group
-  const int q = lane / gw, ql = lane % gw;
-  ST* o0 = sm ? g_acc + (size_t)q * 4 * dA : r0;  // this group's copy
-  const size_t o1 = sm ? (size_t)2 * dA : ars;   // offset of row c = 1
-  const int* acol = apn_col + ar;
-  if (sm) {
-    for (int t = lane; t < dA; t += kSaGL) g_col[t] = acol[t];
-    acol = g_col;
-  }
-  for (int t = lane; t < (sm ? kSaApG * 4 * dA : 2 * dA); t += kSaGL) {
-    if (sm) g_acc[t] = 0;
-    else { r0[t] = 0; r0[ars + t] = 0; }
-  }
   const bool m0 = mask && mask[i0], m1 = mask && mask[i1];
-  if (!(m0 && m1)) {
-    const int q0 = rowptr[i0], q1 = rowptr[i1], deg = (rowptr[i0 + 1] - q0) >> 1;
-    for (int k0 = 0; k0 < deg; k0 += kSaGL) {
-      // lane k loads neighbour k0 + k
-      ST b00 = 0, b01 = 0, b10 = 0, b11 = 0;
-      int bpj = 0, bdP = 0;
-      if (k0 + lane < deg) {
-        const int k = k0 + lane;
-        const int ju = colind[q0 + k], jv = ju + nn;  // u and v dofs of neighbour node h
-        const bool cu = mask && mask[ju], cv = mask && mask[jv];
-        b00 = (m0 || cu) ? ST(0) : (ST)A[q0 + k];
-        b01 = (m0 || cv) ? ST(0) : (ST)A[q0 + deg + k];
-        b10 = (m1 || cu) ? ST(0) : (ST)A[q1 + k];
-        b11 = (m1 || cv) ? ST(0) : (ST)A[q1 + deg + k];
-        const int h = no + (ju - d0);
-        bpj = pn_ptr[h];
-        bdP = pn_ptr[h + 1] - bpj;
+  const int pr = pn_ptr[g], dP = pn_ptr[g + 1] - pr, ag = agg[g];
+  double l0 = 0, l1 = 0;
+  const bool smooth = !pn_w;
+  auto stage = [&](int k0) {  // two neighbours a lane at a time, all their loads ahead of the uses
+    for (int b = 0; b < kSaStage && k0 + b < deg; b += 2 * kSaGL) {
+      int ju[2];
+      KT a[2][4];
+      bool in[2], cu[2], cv[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int k = k0 + b + q * kSaGL + lane;
+        in[q] = k < deg;
+        const int kc = min(k, deg - 1);
+        ju[q] = colind[r.x + kc];
+        a[q][0] = A[r.x + kc];
+        a[q][1] = A[r.x + deg + kc];
+        a[q][2] = A[r.y + kc];
+        a[q][3] = A[r.y + deg + kc];
       }
-      const int nk = min(kSaGL, deg - k0);
-      for (int e0 = 0; e0 < nk; e0 += ng) {
-        const int e = e0 + q;  // this group's neighbour (lanes past nk read zeros)
-        const ST a00 = __shfl_sync(gmask, b00, e, kSaGL), a01 = __shfl_sync(gmask, b01, e, kSaGL);
-        const ST a10 = __shfl_sync(gmask, b10, e, kSaGL), a11 = __shfl_sync(gmask, b11, e, kSaGL);
-        const int pj = __shfl_sync(gmask, bpj, e, kSaGL), dPj = __shfl_sync(gmask, bdP, e, kSaGL);
-        __syncwarp(gmask);  // the previous neighbours' updates (and the zeroed rows) are visible
-        if (e >= nk || (a00 == ST(0) && a01 == ST(0) && a10 == ST(0) && a11 == ST(0))) continue;
-        for (int t = ql; t < dPj; t += gw) {
-          // the P entries load beside the column, ahead of the search
-          const int colp = pn_col[pj + t];
-          double pq[4];
-          pq_get(Q + pj + t, pq);
-          const ST p00 = (ST)pq[0], p01 = (ST)pq[1], p10 = (ST)pq[2], p11 = (ST)pq[3];
-          const int kk = sa_find(acol, dA, colp);
-          if (kk < 0) continue;
-          o0[kk] += a00 * p00 + a01 * p10;
-          o0[dA + kk] += a00 * p01 + a01 * p11;
-          o0[o1 + kk] += a10 * p00 + a11 * p10;
-          o0[o1 + dA + kk] += a10 * p01 + a11 * p11;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        cu[q] = mask && mask[ju[q]];
+        cv[q] = mask && mask[ju[q] + nn];
+        const int c = b + q * kSaGL + lane;
+        if (smooth && in[q]) sj[gi][c] = agg[no + (ju[q] - d0)];
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        if (!in[q]) continue;
+        const int c = b + q * kSaGL + lane;
+        const ST a00 = (m0 || cu[q]) ? ST(0) : a[q][0], a01 = (m0 || cv[q]) ? ST(0) : a[q][1];
+        const ST a10 = (m1 || cu[q]) ? ST(0) : a[q][2], a11 = (m1 || cv[q]) ? ST(0) : a[q][3];
+        if (smooth) {
+          sv[gi][0][c] = a00; sv[gi][1][c] = a01; sv[gi][2][c] = a10; sv[gi][3][c] = a11;
         }
+        l0 += fabs((double)a00) + fabs((double)a01);
+        l1 += fabs((double)a10) + fabs((double)a11);
       }
+    }
+  };
+  for (int k0 = 0; k0 < deg; k0 += kSaStage) {
+    __syncwarp(gmask);
+    stage(k0);
+  }
+#pragma unroll
+  for (int o = kSaGL / 2; o > 0; o >>= 1) {
+    l0 += __shfl_xor_sync(gmask, l0, o, kSaGL);
+    l1 += __shfl_xor_sync(gmask, l1, o, kSaGL);
+  }
+  const VT v0 = (VT)(l0 > 0 ? kSmoothOmega / l0 : 0.0), v1 = (VT)(l1 > 0 ? kSmoothOmega / l1 : 0.0);
+  if (lane == 0) {
+    invd[i0] = v0;
+    invd[i1] = v1;
+    if (sc) sc[g] = make_double2(sqrt((double)v0), sqrt((double)v1));
+    if (dw) {
+      const size_t k = 2 * (size_t)ipos[g];
+      dw[k] = (VT)(v0 > 0 ? 1.0 / (double)v0 : 0.0);
+      dw[k + 1] = (VT)(v1 > 0 ? 1.0 / (double)v1 : 0.0);
     }
   }
-  if (sm) {  // one write of the two rows, the group copies added in order
-    __syncwarp(gmask);
-    for (int t = lane; t < 2 * dA; t += kSaGL) {
-      ST v0 = g_acc[t], v1 = g_acc[2 * dA + t];
-#pragma unroll
-      for (int c = 1; c < kSaApG; ++c) {
-        v0 += g_acc[(size_t)c * 4 * dA + t];
-        v1 += g_acc[(size_t)c * 4 * dA + 2 * dA + t];
-      }
-      r0[t] = v0;
-      r0[ars + t] = v1;
+  if (psel && !psel[s]) return;
+  const ST f0 = (ST)(kSaOmega / kSmoothOmega * (double)v0), f1 = (ST)(kSaOmega / kSmoothOmega * (double)v1);
+  __syncwarp(gmask);
+  for (int t0 = 0; t0 < dP; t0 += kSaGL) {
+    const int t = t0 + lane;
+    if (pn_w) {  // the same weights for both components, no smoothing
+      if (t < dP) pq_set(Q + pr + t, m0 ? 0.0 : pn_w[pr + t], 0.0, 0.0, m1 ? 0.0 : pn_w[pr + t]);
+      continue;
     }
+    const int J = t < dP ? pn_col[pr + t] : -1;
+    ST p00 = (J == ag && !m0) ? ST(1) : ST(0), p11 = (J == ag && !m1) ? ST(1) : ST(0), p01 = 0, p10 = 0;
+    for (int k0 = 0; k0 < deg; k0 += kSaStage) {
+      if (deg > kSaStage) {
+        __syncwarp(gmask);
+        stage(k0);
+        __syncwarp(gmask);
+      }
+      const int nk = min(kSaStage, deg - k0);
+      for (int c = 0; c < nk; ++c)
+        if (sj[gi][c] == J) {
+          p00 -= f0 * sv[gi][0][c];
+          p01 -= f0 * sv[gi][1][c];
+          p10 -= f1 * sv[gi][2][c];
+          p11 -= f1 * sv[gi][3][c];
+        }
+    }
+    if (t < dP) pq_set(Q + pr + t, (double)p00, (double)p01, (double)p10, (double)p11);
   }
 }
 
-// quads of the prolongator rows of fine node g (pn order): thread per fine node
-template <typename ST, typename QT>
-__global__ void k_sa_quads(int nfn, const int* node_sys, const int* pn_ptr, const int* pbase, const int* pnnz,
-                           const int* poff, const ST* P, QT* Q, const int* sel) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= nfn) return;
-  const int s = node_sys[g];
-  if (sel && !sel[s]) return;
-  const int pr = pn_ptr[g], dP = pn_ptr[g + 1] - pr;
-  const size_t prs = (size_t)2 * pnnz[s];  // row c = 1 after row c = 0
-  const ST* p0 = P + poff[s] + 2 * (size_t)(pr - pbase[s]);  // row c: [c2 = 0 (dP)][c2 = 1 (dP)]
-  for (int k = 0; k < dP; ++k)
-    pq_set(Q + pr + k, (double)p0[k], (double)p0[dP + k], (double)p0[prs + k], (double)p0[prs + dP + k]);
+// A P, one lane per entry (g, J).  Masked columns are zero rows of P.  Bound by the gathers of A and
+// the product list (8 bytes a product) on large levels: P2 401x201, four levels, 330 -> 137 us; P1
+// 141x71, three levels, 37 -> 29 us.
+template <typename KT>
+__global__ void __launch_bounds__(256) k_sa_AP(long long n, const int* node, const int4* nrow, const int* dof_off,
+                                               const int* node_off, const KT* A, const unsigned char* mask,
+                                               const typename PQuadOf<KT>::T* Q, const unsigned* lptr,
+                                               const int2* lst, KT* AP, const int* sel) {
+  using ST = KT;
+  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const int g = node[e];
+  const unsigned u0 = lptr[e], u1 = lptr[e + 1];
+  const int4 r = nrow[g];
+  if (sel && !sel[r.w]) return;
+  bool m0 = false, m1 = false;
+  if (mask) {
+    const int no = node_off[r.w], i0 = dof_off[r.w] + (g - no);
+    m0 = mask[i0];
+    m1 = mask[i0 + node_off[r.w + 1] - no];
+  }
+  ST b00 = 0, b01 = 0, b10 = 0, b11 = 0;
+#pragma unroll 4
+  for (unsigned u = u0; u < u1; ++u) {
+    const int2 c = lst[u];
+    double pq[4];
+    pq_get(Q + c.y, pq);
+    const ST p00 = (ST)pq[0], p01 = (ST)pq[1], p10 = (ST)pq[2], p11 = (ST)pq[3];
+    const ST a00 = (ST)A[r.x + c.x], a01 = (ST)A[r.x + r.z + c.x], a10 = (ST)A[r.y + c.x],
+             a11 = (ST)A[r.y + r.z + c.x];
+    b00 += a00 * p00 + a01 * p10;
+    b01 += a00 * p01 + a01 * p11;
+    b10 += a10 * p00 + a11 * p10;
+    b11 += a10 * p01 + a11 * p11;
+  }
+  quad_put(AP, e, m0 ? ST(0) : b00, m0 ? ST(0) : b01, m1 ? ST(0) : b10, m1 ? ST(0) : b11);
 }
 
 // the same quads in ptn order (coarse node J, its fine nodes u): thread per ptn entry (its
@@ -1188,97 +1253,45 @@ __global__ void k_sa_qt(long long np, const int* fnode_sys, const int* ptn_fine,
   QTr[u] = Q[pn_ptr[g] + ptn_k[u]];
 }
 
-// coarse operator rows: Ac((c2,J),:) = sum over P'((c2,J), (c,g)) AP((c,g),:), into the coarse
-// level's CSR.  One warp per coarse node J: its two rows share the column list (sorted, in
-// shared memory) and the fine nodes g of P'(J,:).  The lanes first load the fine-node data of 32
-// list entries.  The warp is split into kSaAcG groups of kSaAcW lanes: group q takes the entries
-// q, q + kSaAcG, ... in order, its lanes the entries of AP(g,:), whose columns are distinct, and
-// sums into the group's own copy of the four FP64 blocks; the copies are added in group order at
-// the end.  A fixed summation order without atomics.
-constexpr int kSaAcWarps = 4;
-constexpr int kSaAcG = 4, kSaAcW = 32 / kSaAcG;
-// dynamic shared memory of a CTA for coarse rows of at most md nodes
-inline size_t sa_ac_smem(int md) { return (size_t)kSaAcWarps * md * (kSaAcG * 4 * sizeof(double) + sizeof(int)); }
-template <typename KT, typename ST>
-__global__ void __launch_bounds__(32 * kSaAcWarps, sizeof(ST) == 4 ? 10 : 0) k_sa_Ac(int ncn, const int* cnode_sys, const int* cdof_off,
-                                                           const int* cnode_off, const int* crowptr,
-                                                           const int* ccolind, const int* ptn_ptr,
-                                                           const int* ptn_fine, const typename PQuadOf<KT>::T* QTr,
-                                                           const int* apn_ptr,
-                                                           const int* apn_col, const int* apbase, const int* apnnz,
-                                                           const int* apoff, const ST* AP, KT* Ac, const int* sel,
-                                                           int md) {
-  extern __shared__ __align__(16) unsigned char sa_smem[];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int J = blockIdx.x * kSaAcWarps + wid;
-  if (J >= ncn) return;  // whole warps leave together
-  const int s = cnode_sys[J];
-  if (sel && !sel[s]) return;  // whole warps
-  const int cno = cnode_off[s], cnn = cnode_off[s + 1] - cno;
-  const int R0 = cdof_off[s] + (J - cno), R1 = R0 + cnn;
-  const int cr0 = crowptr[R0], cr1 = crowptr[R1], degc = min((crowptr[R0 + 1] - cr0) >> 1, md);
-  const int cbase = cdof_off[s] - cno;  // u-column dof of coarse node K: cbase + K
-  double* acc = reinterpret_cast<double*>(sa_smem) + (size_t)wid * kSaAcG * 4 * md;
-  int* col = reinterpret_cast<int*>(reinterpret_cast<double*>(sa_smem) + (size_t)kSaAcWarps * kSaAcG * 4 * md) +
-             wid * md;
-  // copy q, block (c2, c3) at acc[(4 q + 2 c2 + c3) degc + pos]
-  for (int t = lane; t < kSaAcG * 4 * degc; t += 32) acc[t] = 0;
-  for (int t = lane; t < degc; t += 32) col[t] = ccolind[cr0 + t] - cbase;
-  const int q = lane / kSaAcW, ql = lane % kSaAcW;
-  double* ga = acc + (size_t)q * 4 * degc;
-  const int tr = ptn_ptr[J], dT = ptn_ptr[J + 1] - tr;
-  const size_t ars = (size_t)2 * apnnz[s];
-  const ST* apb = AP + apoff[s];
-  const int apb0 = apbase[s];
-  for (int u0 = 0; u0 < dT; u0 += 32) {
-    const int my = u0 + lane;
-    int g_ar = 0, g_dA = 0;
-    double w00 = 0, w01 = 0, w10 = 0, w11 = 0;
-    if (my < dT) {
-      const int g = ptn_fine[tr + my];
-      g_ar = apn_ptr[g];
-      g_dA = apn_ptr[g + 1] - g_ar;
-      // w(c2, c) = P'((c2,J),(c,g)) = P((c,g),(c2,J)), quad entry 2 c + c2
-      double pq[4];
-      pq_get(QTr + tr + my, pq);
-      w00 = pq[0];
-      w01 = pq[2];
-      w10 = pq[1];
-      w11 = pq[3];
-    }
-    const int nstep = min(32, dT - u0);
-    for (int e0 = 0; e0 < nstep; e0 += kSaAcG) {
-      const int e = e0 + q;  // this group's entry (lanes past nstep hold dA = 0)
-      const int ar = __shfl_sync(0xffffffffu, g_ar, e), dA = __shfl_sync(0xffffffffu, g_dA, e);
-      const double v00 = __shfl_sync(0xffffffffu, w00, e), v01 = __shfl_sync(0xffffffffu, w01, e);
-      const double v10 = __shfl_sync(0xffffffffu, w10, e), v11 = __shfl_sync(0xffffffffu, w11, e);
-      const ST* a0 = apb + 2 * (size_t)(ar - apb0);  // AP((c,g),(c3,kk)) = a0[c ars + c3 dA + kk]
-      __syncwarp();  // the previous entries' sums (and the zeroed copies) are visible to the warp
-      for (int kk = ql; kk < dA; kk += kSaAcW) {
-        // the AP entries load beside the column, ahead of the search
-        const int cK = apn_col[ar + kk];
-        const double x00 = (double)a0[kk], x01 = (double)a0[dA + kk], x10 = (double)a0[ars + kk],
-                     x11 = (double)a0[ars + dA + kk];
-        const int pos = sa_find(col, degc, cK);
-        if (pos < 0) continue;
-        ga[pos] += v00 * x00 + v01 * x10;
-        ga[degc + pos] += v00 * x01 + v01 * x11;
-        ga[2 * degc + pos] += v10 * x00 + v11 * x10;
-        ga[3 * degc + pos] += v10 * x01 + v11 * x11;
-      }
-    }
+// Coarse operator, kSaAcL lanes per entry (J, K): Ac = sum of P(g, J)' A P(g, K) in FP64, a lane sum in
+// a fixed order; the diagonal entries have several times the products of the others.  P2 401x201, four
+// levels: 205 -> 121 us; P1 141x71, three levels: 57 -> 31 us.
+constexpr int kSaAcL = 4;
+template <typename KT>
+__global__ void __launch_bounds__(256) k_sa_Ac(long long n, const int* node, const int* gptr, const int4* nrow_c,
+                                               const typename PQuadOf<KT>::T* Q, const KT* AP,
+                                               const unsigned* lptr, const int2* lst, KT* Ac, const int* sel) {
+  const long long o = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / kSaAcL;
+  const int lane = threadIdx.x % kSaAcL;
+  if (o >= n) return;  // whole groups leave together
+  const int J = node[o];
+  const unsigned u0 = lptr[o], u1 = lptr[o + 1];
+  const int4 r = nrow_c[J];
+  if (sel && !sel[r.w]) return;
+  const int k = (int)(o - gptr[J]);
+  double b00 = 0, b01 = 0, b10 = 0, b11 = 0;
+#pragma unroll 4
+  for (unsigned u = u0 + lane; u < u1; u += kSaAcL) {
+    const int2 c = lst[u];
+    double p[4], x[4];
+    pq_get(Q + c.x, p);  // P((c,g),(c2,J)) at 2 c + c2
+    quad_at(AP, c.y, x);
+    b00 += p[0] * x[0] + p[2] * x[2];
+    b01 += p[0] * x[1] + p[2] * x[3];
+    b10 += p[1] * x[0] + p[3] * x[2];
+    b11 += p[1] * x[1] + p[3] * x[3];
   }
-  __syncwarp();
-  for (int t = lane; t < 2 * degc; t += 32) {
-    double a0 = acc[t], a1 = acc[2 * degc + t];
+  const unsigned gmask = ((1u << kSaAcL) - 1u) << ((threadIdx.x & 31) & ~(kSaAcL - 1));
 #pragma unroll
-    for (int c = 1; c < kSaAcG; ++c) {
-      a0 += acc[(size_t)c * 4 * degc + t];
-      a1 += acc[(size_t)c * 4 * degc + 2 * degc + t];
-    }
-    Ac[cr0 + t] = (KT)a0;
-    Ac[cr1 + t] = (KT)a1;
+  for (int d = kSaAcL / 2; d > 0; d >>= 1) {
+    b00 += __shfl_xor_sync(gmask, b00, d, kSaAcL);
+    b01 += __shfl_xor_sync(gmask, b01, d, kSaAcL);
+    b10 += __shfl_xor_sync(gmask, b10, d, kSaAcL);
+    b11 += __shfl_xor_sync(gmask, b11, d, kSaAcL);
   }
+  static_assert(kSaAcL == 4, "a lane writes one of the four values");
+  const double v = lane == 0 ? b00 : lane == 1 ? b01 : lane == 2 ? b10 : b11;
+  Ac[(lane < 2 ? r.x : r.y) + (lane & 1 ? r.z : 0) + k] = (KT)v;
 }
 
 // The transfers are gather chains (list entry -> node block -> P list -> vector entries).  They
@@ -1431,11 +1444,70 @@ __global__ void __launch_bounds__(32 * kSaPW, 4) k_sa_prolong(int nnb, const int
 // host drivers
 // ---------------------------------------------------------------------------
 
-template <typename KT, typename VT>
-static int numeric_t(ua_mesh* m, const int* rowptr0, const int* colind0, const KT* K0, const unsigned char* cmask,
-                     const int* sel, const int* psel, long long* launches) {
+// The lists of a smoothed hierarchy's set-up, once per handle.
+static int sa_lists(ua_mesh* m, const int* rowptr0, const int* colind0) {
   Amg* a = m->amg;
   cudaStream_t st = m->stream;
+  bool ok = true;
+  auto grid = [](long long n, int t) { return (unsigned)std::max<long long>(1, (n + t - 1) / t); };
+  unsigned long long* d_tot = (unsigned long long*)dalloc(m, a, sizeof(unsigned long long), ok);
+  for (int l = 0; ok && l < a->nlev; ++l) {
+    AmgLevel& L = a->lev[l];
+    L.nrow = (int4*)dalloc(m, a, sizeof(int4) * (size_t)std::max(L.nn, 1), ok);
+    if (ok && L.nn)
+      k_sa_nrow<<<grid(L.nn, 256), 256, 0, st>>>(L.nn, L.node_sys, L.d_node_off, L.d_dof_off,
+                                                 l == 0 ? rowptr0 : L.rowptr, L.nrow);
+  }
+  // counts, offsets, products: fill(lst) launches the list kernel
+  auto build = [&](long long n, unsigned*& ptr, int2*& lst, auto fill) -> int {
+    ptr = (unsigned*)dalloc(m, a, sizeof(unsigned) * (size_t)(n + 1), ok);
+    if (!ok) return UA_ERR_OOM;
+    fill((int2*)nullptr);
+    k_sa_scan<<<1, 1024, 0, st>>>(n, ptr, d_tot);
+    unsigned long long tot = 0;
+    UA_CUDA_TRY(cudaMemcpyAsync(&tot, d_tot, sizeof(tot), cudaMemcpyDeviceToHost, st));
+    UA_CUDA_TRY(cudaStreamSynchronize(st));
+    if (tot > 0xffffffffull) return UA_ERR_OOM;  // 34 GB of products
+    lst = (int2*)dalloc(m, a, sizeof(int2) * (size_t)std::max<unsigned long long>(tot, 1), ok);
+    if (!ok) return UA_ERR_OOM;
+    fill(lst);
+    return UA_OK;
+  };
+  for (int l = 0; ok && l + 1 < a->nlev; ++l) {
+    AmgLevel& F = a->lev[l];
+    const AmgLevel& C = a->lev[l + 1];
+    F.ap_node = (int*)dalloc(m, a, sizeof(int) * (size_t)std::max(F.nap, 1LL), ok);
+    F.ap_p = (int*)dalloc(m, a, sizeof(int) * (size_t)std::max(F.nap, 1LL), ok);
+    F.ac_node = (int*)dalloc(m, a, sizeof(int) * (size_t)std::max(C.ng, 1LL), ok);
+    if (!ok) break;
+    k_sa_ids<<<grid(4LL * F.nn, 256), 256, 0, st>>>(F.nn, F.apn_ptr, F.ap_node);
+    k_sa_ids<<<grid(4LL * C.nn, 256), 256, 0, st>>>(C.nn, C.gptr, F.ac_node);
+    int rc = build(F.nap, F.ap_lptr, F.ap_l, [&](int2* lst) {
+      k_sa_ap_list<<<grid(F.nap, 256), 256, 0, st>>>(F.nap, F.ap_node, F.apn_col, F.nrow, F.d_node_off, F.d_dof_off,
+                                                     l == 0 ? colind0 : F.colind, F.pn_ptr, F.pn_col, F.ap_lptr,
+                                                     lst, F.ap_p);
+    });
+    if (!rc)
+      rc = build(C.ng, F.ac_lptr, F.ac_l, [&](int2* lst) {
+        k_sa_ac_list<<<grid(C.ng, 256), 256, 0, st>>>(C.ng, F.ac_node, C.gptr, C.nrow, C.d_node_off, C.d_dof_off,
+                                                      C.colind, F.ptn_ptr, F.ptn_fine, F.ptn_k, F.pn_ptr, F.apn_ptr,
+                                                      F.apn_col, F.ac_lptr, lst);
+      });
+    if (rc == UA_ERR_OOM) ok = false;
+    else if (rc) return rc;
+  }
+  if (!ok) return set_error(UA_ERR_OOM, "AMG: device allocation of the set-up lists failed");
+  UA_CUDA_TRY(cudaGetLastError());
+  a->lists = true;
+  return UA_OK;
+}
+
+// cyc: also the values of the collapsed cycle; branch: run them beside the coarse levels (a capture)
+template <typename KT, typename VT>
+static int numeric_t(ua_mesh* m, const int* rowptr0, const int* colind0, const KT* K0, const unsigned char* cmask,
+                     const int* sel, const int* psel, const CycFillReq* cyc, bool branch, long long* launches) {
+  Amg* a = m->amg;
+  cudaStream_t st = m->stream, sd = branch ? a->side : st;
   auto l1 = [&](int l) {
     const AmgLevel& L = a->lev[l];
     k_amg_l1<KT, VT><<<(L.ndof + 255) / 256, 256, 0, st>>>(
@@ -1443,41 +1515,44 @@ static int numeric_t(ua_mesh* m, const int* rowptr0, const int* colind0, const K
         l == 0 ? cmask : nullptr, (VT*)L.invd, L.dof_sys, sel), ++*launches;
   };
   if (a->sa) {
-    // per level: smoother diagonal, smoothed prolongator, A P, P' values, coarse operator
+    auto grid = [](long long n, int t) { return (unsigned)std::max<long long>(1, (n + t - 1) / t); };
+    // the mixed form sums in FP32, the FP64 form in FP64 (the coarse operators in FP64 in both)
+    using QT = typename PQuadOf<KT>::T;
+    // per level: smoother diagonal and smoothed prolongator, A P, coarse operator
     for (int l = 0; l + 1 < a->nlev; ++l) {
       AmgLevel& F = a->lev[l];
       AmgLevel& C = a->lev[l + 1];
-      const int* rp = l == 0 ? rowptr0 : F.rowptr;
       const int* ci = l == 0 ? colind0 : F.colind;
       const KT* A = l == 0 ? K0 : (const KT*)F.A;
       const unsigned char* mk = l == 0 ? cmask : nullptr;
-      l1(l);
-      const int nbf = (F.ndof + 127) / 128;
-      // the mixed form sets up in FP32, the FP64 form in FP64; P then goes into the transfer
-      // layout (quads, pn and ptn order), which A P, the coarse operator and the V-cycle read
-      using ST = typename std::conditional<sizeof(KT) == 4, float, double>::type;
-      using QT = typename PQuadOf<KT>::T;
-      ST* Pv = sizeof(KT) == 4 ? (ST*)F.sa_plo : (ST*)F.sa_p;
-      ST* APv = (ST*)F.sa_ap;
+      KT* APv = (KT*)F.sa_ap;
       QT* Qv = (QT*)(sizeof(KT) == 4 ? F.sa_qh : F.sa_qd);
-      QT* QTv = (QT*)(sizeof(KT) == 4 ? F.sa_qth : F.sa_qtd);
-      k_sa_P<KT, VT, ST><<<nbf, 128, 0, st>>>(F.ndof, F.dof_sys, F.d_dof_off, F.d_node_off, rp, ci, A, mk,
-                                              (const VT*)F.invd, F.sa_agg, F.pn_ptr, F.pn_col, F.pn_w, F.pbase, F.pnnz,
-                                              F.poff, Pv, psel), ++*launches;
-      k_sa_quads<ST, QT><<<(F.nn + 127) / 128, 128, 0, st>>>(F.nn, F.node_sys, F.pn_ptr, F.pbase, F.pnnz, F.poff,
-                                                            Pv, Qv, psel), ++*launches;
-      k_sa_qt<QT><<<(int)((F.np + 255) / 256), 256, 0, st>>>(F.np, F.node_sys, F.ptn_fine, F.ptn_k, F.pn_ptr, Qv,
-                                                               QTv, psel), ++*launches;
-      const int ms = F.ap_maxrow <= kSaApSm ? F.ap_maxrow : 0;  // rows summed in shared memory
-      k_sa_AP<KT, ST><<<(int)(((long long)F.nn * kSaGL + 127) / 128), 128, sa_ap_smem<ST>(ms), st>>>(
-          F.nn, F.node_sys, F.d_dof_off, F.d_node_off, rp, ci, A, mk, F.pn_ptr, F.pn_col, Qv, F.apn_ptr, F.apn_col,
-          F.apbase, F.apnnz, F.apoff, APv, sel, ms), ++*launches;
-      k_sa_Ac<KT, ST><<<(C.nn + kSaAcWarps - 1) / kSaAcWarps, 32 * kSaAcWarps, sa_ac_smem(F.ac_maxdeg), st>>>(
-          C.nn, C.node_sys, C.d_dof_off, C.d_node_off, C.rowptr, C.colind, F.ptn_ptr, F.ptn_fine, QTv, F.apn_ptr,
-          F.apn_col, F.apbase, F.apnnz, F.apoff, APv, (KT*)C.A, sel, F.ac_maxdeg),
+      k_sa_P<KT, VT, QT><<<grid((long long)F.nn * kSaGL, 128), 128, 0, st>>>(
+          F.nn, F.nrow, F.d_dof_off, F.d_node_off, ci, A, mk, F.sa_agg, F.pn_ptr, F.pn_col, F.pn_w, Qv, (VT*)F.invd,
+          cyc ? a->cyc.lev[l].sc : nullptr, cyc && l == 0 ? (VT*)cyc->dw : nullptr, a->cyc.d_ipos, sel, psel),
           ++*launches;
+      if (cyc && l == 0) {  // the finest level's slice values need its diagonal only
+        if (branch) {
+          UA_CUDA_TRY(cudaEventRecord(a->fork, st));
+          UA_CUDA_TRY(cudaStreamWaitEvent(sd, a->fork, 0));
+        }
+        cycle_fill_fine(m, colind0, K0, sizeof(KT) == 4, cyc->lo, sel, sd, launches);
+      }
+      if (!cyc)
+        k_sa_qt<QT><<<grid(F.np, 256), 256, 0, st>>>(F.np, F.node_sys, F.ptn_fine, F.ptn_k, F.pn_ptr, Qv,
+                                                     (QT*)(sizeof(KT) == 4 ? F.sa_qth : F.sa_qtd), sel), ++*launches;
+      k_sa_AP<KT><<<grid(F.nap, 256), 256, 0, st>>>(F.nap, F.ap_node, F.nrow, F.d_dof_off, F.d_node_off, A, mk, Qv,
+                                                    F.ap_lptr, F.ap_l, APv, sel), ++*launches;
+      if (cyc && l + 2 == a->nlev) {  // every diagonal and A P is there
+        if (branch) {
+          UA_CUDA_TRY(cudaEventRecord(a->fork, st));
+          UA_CUDA_TRY(cudaStreamWaitEvent(sd, a->fork, 0));
+        }
+        cycle_fill_levels(m, sizeof(KT) == 4, sel, sd, launches);
+      }
+      k_sa_Ac<KT><<<grid(C.ng * kSaAcL, 256), 256, 0, st>>>(C.ng, F.ac_node, C.gptr, C.nrow, Qv, APv, F.ac_lptr,
+                                                            F.ac_l, (KT*)C.A, sel), ++*launches;
     }
-    l1(a->nlev - 1);
   } else {
     for (int l = 0; l + 1 < a->nlev; ++l) {
       const AmgLevel& F = a->lev[l];
@@ -1492,6 +1567,10 @@ static int numeric_t(ua_mesh* m, const int* rowptr0, const int* colind0, const K
   k_amg_dense_inverse<KT><<<a->nsys, kDiThreads, sm, st>>>(a->d_depth, a->d_dn, a->d_doff, a->d_lev_rowptr,
                                                      a->d_lev_colind, a->d_lev_A, a->d_lev_dofoff, a->dense, sel),
       ++*launches;
+  if (cyc && branch) {
+    UA_CUDA_TRY(cudaEventRecord(a->join, sd));
+    UA_CUDA_TRY(cudaStreamWaitEvent(st, a->join, 0));
+  }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(UA_ERR_CUDA, "AMG numeric phase: %s", cudaGetErrorString(e));
   return UA_OK;
@@ -1746,19 +1825,8 @@ int amg_numeric(ua_mesh* m, const int* rowptr0, const int* colind0, const void* 
     UA_CUDA_TRY(cudaFuncSetAttribute(k_amg_dense_inverse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   else
     UA_CUDA_TRY(cudaFuncSetAttribute(k_amg_dense_inverse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-  if (a->sa) {  // the set-up's shared-memory rows, sized by the hierarchy's longest ones
-    int smd = 0;
-    for (int l = 0; l + 1 < a->nlev; ++l) smd = std::max(smd, a->lev[l].ac_maxdeg);
-    const int sac = (int)sa_ac_smem(smd);
-    const int sap = fp32 ? (int)sa_ap_smem<float>(kSaApSm) : (int)sa_ap_smem<double>(kSaApSm);
-    if (fp32) {
-      UA_CUDA_TRY(cudaFuncSetAttribute(k_sa_Ac<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sac));
-      UA_CUDA_TRY(cudaFuncSetAttribute(k_sa_AP<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sap));
-    } else {
-      UA_CUDA_TRY(cudaFuncSetAttribute(k_sa_Ac<double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, sac));
-      UA_CUDA_TRY(cudaFuncSetAttribute(k_sa_AP<double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, sap));
-    }
-  }
+  if (a->sa && !a->lists)
+    if (int rc = sa_lists(m, rowptr0, colind0)) return rc;
   if (a->sa) {  // the transfer quads of this precision, allocated before any capture
     bool ok = true;
     for (int l = 0; l + 1 < a->nlev; ++l) {
@@ -1767,15 +1835,18 @@ int amg_numeric(ua_mesh* m, const int* rowptr0, const int* colind0, const void* 
       void*& qt = fp32 ? F.sa_qth : F.sa_qtd;
       const size_t qb = fp32 ? sizeof(PQuadH) : sizeof(PQuadD);
       if (!q) q = dalloc(m, a, qb * (size_t)std::max(F.np, 1LL), ok);
-      if (!qt) qt = dalloc(m, a, qb * (size_t)std::max(F.np, 1LL), ok);
+      if (!qt && !cyc) qt = dalloc(m, a, qb * (size_t)std::max(F.np, 1LL), ok);
     }
     if (!ok) return set_error(UA_ERR_OOM, "AMG: device allocation of the transfer values failed");
   }
+  if (a->sa && cyc && graph && !a->side) {
+    UA_CUDA_TRY(cudaStreamCreateWithFlags(&a->side, cudaStreamNonBlocking));
+    UA_CUDA_TRY(cudaEventCreateWithFlags(&a->fork, cudaEventDisableTiming));
+    UA_CUDA_TRY(cudaEventCreateWithFlags(&a->join, cudaEventDisableTiming));
+  }
   auto run = [&](long long* l) {
-    int rc = fp32 ? numeric_t<float, float>(m, rowptr0, colind0, (const float*)K0, cmask, sel, psel, l)
-                  : numeric_t<double, double>(m, rowptr0, colind0, (const double*)K0, cmask, sel, psel, l);
-    if (!rc && cyc) cycle_fill(m, rowptr0, colind0, K0, fp32, cyc->lo, cyc->dw, sel, l);
-    return rc;
+    return fp32 ? numeric_t<float, float>(m, rowptr0, colind0, (const float*)K0, cmask, sel, psel, cyc, graph, l)
+                : numeric_t<double, double>(m, rowptr0, colind0, (const double*)K0, cmask, sel, psel, cyc, graph, l);
   };
   if (!graph) return run(launches);
   // one captured graph per kind of call (FP32/FP64 values, prolongator selection, handle's

@@ -114,8 +114,11 @@ int amg_vcycle(ua_mesh* m, bool fp32, const AmgPcgView& v, long long* launches);
 bool cycle_supported(const ua_mesh* m);
 int cycle_init(ua_mesh* m);
 int cycle_alloc_values(ua_mesh* m, bool fp32, bool lo);
-void cycle_fill(ua_mesh* m, const int* rowptr0, const int* colind0, const void* K0, bool fp32, bool lo, void* dw,
-                const int* sel, long long* launches);
+// values of the collapsed cycle: the finest level's slices (after its diagonal), and the coarse levels'
+// operators and every Q (after the last A P)
+void cycle_fill_fine(ua_mesh* m, const int* colind0, const void* K0, bool fp32, bool lo, const int* sel,
+                     cudaStream_t st, long long* launches);
+void cycle_fill_levels(ua_mesh* m, bool fp32, const int* sel, cudaStream_t st, long long* launches);
 struct PcgSolve {
   bool fp32, lo, prof;
   const int *rb_start, *rb_sys;

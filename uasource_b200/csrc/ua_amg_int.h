@@ -30,8 +30,6 @@ constexpr double kSmoothOmega = 1.8;
 struct AmgLevel {
   int nn = 0, ndof = 0;
   long long nnz = 0;
-  int ap_maxrow = 0;  // longest A P row (coarse columns) of the level
-  int ac_maxdeg = 0;  // largest node degree of the next (coarse) level
   std::vector<int> node_off, dof_off, knz_off, nnzn;  // per system (0-sized when the system has no such level)
   // dof-level CSR of a coarse level, same layout rule as the finest level
   int *rowptr = nullptr, *colind = nullptr;
@@ -58,9 +56,17 @@ struct AmgLevel {
   double* pn_w = nullptr;  // interpolation weights in pn order (the finest level of a quadratic mesh), else null
   int *sa_agg = nullptr, *pn_ptr = nullptr, *pn_col = nullptr, *apn_ptr = nullptr, *apn_col = nullptr;
   int *ptn_ptr = nullptr, *ptn_fine = nullptr, *ptn_k = nullptr;
-  int *pbase = nullptr, *pnnz = nullptr, *poff = nullptr, *apbase = nullptr, *apnnz = nullptr, *apoff = nullptr;
-  double *sa_p = nullptr, *sa_ap = nullptr;  // set-up values (FP64 form): 4 per node-level entry
-  float* sa_plo = nullptr;                   // set-up values of P (mixed form)
+  // lists of the set-up (sa_lists): per node {first entry of its u row, of its v row, degree, system};
+  // per entry of A P its fine node, its entry of P (-1: none) and its products (neighbour position,
+  // entry of P); per entry of the next level's operator its node and its products (entry of P, entry
+  // of A P)
+  int4* nrow = nullptr;
+  int *ap_node = nullptr, *ap_p = nullptr, *ac_node = nullptr;
+  unsigned *ap_lptr = nullptr, *ac_lptr = nullptr;
+  int2 *ap_l = nullptr, *ac_l = nullptr;
+  int* gptr = nullptr;       // node graph of a coarse level
+  long long nap = 0, ng = 0;  // entries of A P, of the node graph (coarse levels)
+  void* sa_ap = nullptr;      // A P, one quad per entry (value type of the form)
   // P in the transfer layout, one quad per node-level entry: pn order (sa_q*) and ptn order
   // (sa_qt*); BF16 quads for the mixed form, FP64 quads for the FP64 form (allocated on first use)
   long long np = 0;  // node-level prolongator entries of the level (all systems)
@@ -148,7 +154,7 @@ struct Cycle {
   std::vector<CycSys> sys;
   CycSys* d_sys = nullptr;
   struct Lev {
-    int *nptr = nullptr, *ncol = nullptr;                      // node graph (levels >= 1)
+    int* ncol = nullptr;                                       // node graph (levels >= 1)
     long long nq = 0;                                          // node-level entries of Q
     int *qptr = nullptr, *qcol = nullptr;                      // rows of Q (level 0: in slice order)
     int* qrow = nullptr;                                       // node -> first entry of its row of Q
@@ -216,12 +222,19 @@ struct Amg {
   int* d_prefresh = nullptr;
   int* h_pin = nullptr;  // pinned, two alternating copies of the refresh selection
   int pin_at = 0;
+  bool lists = false;  // the levels' set-up lists are built
+  // side branch of the captured set-up: the finest level's slice values beside the coarse levels
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   // the numeric set-up of a Newton step captured as one CUDA graph per (precision, selection
   // kind) and replayed: every argument is a fixed device buffer of the handle
   cudaGraphExec_t setup_exec[32] = {};
   long long setup_nodes[32] = {};
   ~Amg() {
     if (h_pin) cudaFreeHost(h_pin);
+    if (side) cudaStreamDestroy(side);
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
     for (auto& e : setup_exec)
       if (e) cudaGraphExecDestroy(e);
   }
@@ -241,6 +254,25 @@ inline void* dalloc(ua_mesh* m, Amg* a, size_t bytes, bool& ok) {
   if (!d) ok = false;
   a->bytes += bytes;
   return d;
+}
+
+// quads of the set-up (A P): four values of a node pair
+__device__ __forceinline__ void quad_put(double* base, long long e, double a, double b, double c, double d) {
+  double2* p = reinterpret_cast<double2*>(base) + 2 * e;
+  p[0] = make_double2(a, b);
+  p[1] = make_double2(c, d);
+}
+__device__ __forceinline__ void quad_put(float* base, long long e, float a, float b, float c, float d) {
+  reinterpret_cast<float4*>(base)[e] = make_float4(a, b, c, d);
+}
+__device__ __forceinline__ void quad_at(const double* base, long long e, double* v) {
+  const double2* p = reinterpret_cast<const double2*>(base) + 2 * e;
+  const double2 a = p[0], b = p[1];
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void quad_at(const float* base, long long e, double* v) {
+  const float4 a = reinterpret_cast<const float4*>(base)[e];
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
 }
 
 __device__ __forceinline__ double to_d(double v) { return v; }

@@ -19,25 +19,6 @@ namespace ua {
 // set-up: values of the collapsed cycle for a new tangent
 // ---------------------------------------------------------------------------
 
-// D^-1/2 per node of a level (0 on masked and empty rows), and on the finest level D itself in
-// slice order
-template <typename VT>
-__global__ void k_cyc_scale(int nn, const int* node_sys, const int* node_off, const int* dof_off, const VT* invd,
-                            double2* sc, VT* dw, const int* ipos, const int* sel) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= nn) return;
-  const int s = node_sys[g];
-  if (sel && !sel[s]) return;
-  const int no = node_off[s], n = node_off[s + 1] - no, i = dof_off[s] + (g - no);
-  const double du = (double)invd[i], dv = (double)invd[i + n];
-  sc[g] = make_double2(sqrt(du), sqrt(dv));
-  if (dw) {
-    const size_t k = 2 * (size_t)ipos[g];
-    dw[k] = (VT)(du > 0 ? 1.0 / du : 0.0);
-    dw[k + 1] = (VT)(dv > 0 ? 1.0 / dv : 0.0);
-  }
-}
-
 constexpr int kCycArena = 212 * 1024;       // with the kernel's static tables below 227 KB
 constexpr int kCycArenaSmall = 64 * 1024;
 
@@ -71,100 +52,132 @@ __global__ void __launch_bounds__(256) k_cyc_cols(CycFine F, const int* sb_n0, c
   for (int k = 0; k < W; ++k) cols[o0 + 32LL * k + t] = k < deg ? ipos[nodecol[p0 + k]] : at;
 }
 
-// Scaled values of the finest level in its node slices (layout of k_sell_fill), from the dof CSR
-// (row (c, g): the u block then the v block of deg(g) entries).  One CTA per slice block.
+// Scaled values of the finest level in its node slices (SliceQuad layouts), from the dof CSR (row
+// (c, g): the u block then the v block of deg(g) entries).  One warp per kFillN nodes of a slice: 8
+// neighbours at a time, a load covering both rows and both blocks of one node in 64-byte segments;
+// turned in shared memory and written as kFillN nodes of the slice row (whole sectors).  Bound by
+// memory: P2 401x201 moves 0.26 GB in 81 us (a lane per row, each with four streams: 116 us).
+constexpr int kFillWarps = 4, kFillN = 8;
 template <typename KT>
-__global__ void __launch_bounds__(256) k_cyc_fill0(CycFine F, const int* sb_n0, const int* sb_cnt, const int* sb_sys, const int* node_off,
-                                                   const int* dof_off, const int* rowptr, const int* colind,
-                                                   const KT* K, const double2* sc, KT* vk, __nv_bfloat16* vlo,
-                                                   const int* sel) {
-  const int sb = blockIdx.x, s = sb_sys[sb];
+__global__ void __launch_bounds__(32 * kFillWarps) k_cyc_fill0(
+    CycFine F, int nsl, const int* sb_n0, const int* sb_cnt, const int* sb_sys, const int* node_off,
+    const int* dof_off, const int4* nrow, const int* colind, const KT* K, const double2* sc, KT* vk,
+    __nv_bfloat16* vlo, const int* sel) {
+  static_assert(kFillN == 8, "lane = 16 row + 8 block + neighbour");
+  __shared__ KT sv[kFillWarps][4][8][kFillN + 1];
+  __shared__ int4 hr[kFillWarps][kFillN];
+  __shared__ double hs[kFillWarps][kFillN][2];
+  const int wid = threadIdx.x >> 5, t = threadIdx.x & 31;
+  const int sub = blockIdx.x * kFillWarps + wid, sl = sub / (32 / kFillN), n0 = (sub % (32 / kFillN)) * kFillN;
+  if (sl >= nsl) return;  // whole warps
+  const int sb = sl / kSellSlices, s = sb_sys[sb];
   if (sel && !sel[s]) return;
-  const int w = threadIdx.x >> 5, t = threadIdx.x & 31, pos = w * 32 + t, sl = sb * kSellSlices + w;
   const long long o0 = F.sl_off[sl];
   const int W = (int)((F.sl_off[sl + 1] - o0) >> 5);
   if (W == 0) return;
-  const int no = node_off[s], nn = node_off[s + 1] - no, d0 = dof_off[s];
-  int r0 = 0, r1 = 0, deg = 0;
-  double2 si = make_double2(0, 0);
-  if (pos < sb_cnt[sb]) {
-    const int g = F.perm[sb_n0[sb] + pos], i = d0 + (g - no);
-    r0 = rowptr[i];
-    r1 = rowptr[i + nn];
-    deg = (rowptr[i + 1] - r0) >> 1;
-    si = sc[g];
-  }
-  for (int k = 0; k < W; ++k) {
-    const long long d = o0 + 32LL * k + t;
-    double e0 = 0, e1 = 0, e2 = 0, e3 = 0;
-    if (k < deg) {
-      const double2 sj = sc[no + (colind[r0 + k] - d0)];
-      e0 = si.x * (double)K[r0 + k] * sj.x;
-      e1 = si.x * (double)K[r0 + deg + k] * sj.y;
-      e2 = si.y * (double)K[r1 + k] * sj.x;
-      e3 = si.y * (double)K[r1 + deg + k] * sj.y;
+  const int no = node_off[s], shift = no - dof_off[s];
+  if (t < kFillN) {
+    const int pos = (sl % kSellSlices) * 32 + n0 + t;
+    int4 r = make_int4(0, 0, 0, 0);
+    double2 si = make_double2(0, 0);
+    if (pos < sb_cnt[sb]) {
+      const int g = F.perm[sb_n0[sb] + pos];
+      r = nrow[g];
+      si = sc[g];
     }
+    hr[wid][t] = r;
+    hs[wid][t][0] = si.x;
+    hs[wid][t][1] = si.y;
+  }
+  const int row = t >> 4, blk = (t >> 3) & 1, kl = t & 7;
+  for (int k0 = 0; k0 < W; k0 += 8) {
+    __syncwarp();
+    const int k = k0 + kl;
+    int c[kFillN];
+    double v[kFillN];
+#pragma unroll
+    for (int n = 0; n < kFillN; ++n) {
+      const int4 r = hr[wid][n];
+      c[n] = k < r.z ? colind[r.x + k] + shift : -1;
+      v[n] = k < r.z ? (double)K[(row ? r.y : r.x) + (blk ? r.z : 0) + k] : 0.0;
+    }
+#pragma unroll
+    for (int n = 0; n < kFillN; ++n) {
+      const double sj = c[n] >= 0 ? reinterpret_cast<const double*>(sc)[2 * (size_t)c[n] + blk] : 0.0;
+      sv[wid][2 * row + blk][kl][n] = (KT)(hs[wid][n][row] * v[n] * sj);
+    }
+    __syncwarp();
     if (sizeof(KT) == 8) {  // two blocks of 32 pairs (SliceQuad)
-      double2* q = reinterpret_cast<double2*>(vk) + 2 * (d - t);
-      q[t] = make_double2(e0, e1);
-      q[32 + t] = make_double2(e2, e3);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int u = q * 32 + t, n = u & 7, half = (u >> 3) & 1, kk = u >> 4;
+        if (k0 + kk < W)
+          reinterpret_cast<double2*>(vk)[2 * (o0 + 32LL * (k0 + kk)) + 32 * half + n0 + n] =
+              make_double2((double)sv[wid][2 * half][kk][n], (double)sv[wid][2 * half + 1][kk][n]);
+      }
     } else {
-      QuadSet<KT>::set(vk, d, e0, e1, e2, e3);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int u = q * 32 + t, n = u & 7, kk = u >> 3;
+        if (k0 + kk >= W) break;
+        const long long d = o0 + 32LL * (k0 + kk) + n0 + n;
+        const KT e0 = sv[wid][0][kk][n], e1 = sv[wid][1][kk][n], e2 = sv[wid][2][kk][n], e3 = sv[wid][3][kk][n];
+        QuadSet<KT>::set(vk, d, e0, e1, e2, e3);
+        if (vlo) QuadSet<__nv_bfloat16>::set(vlo, d, e0, e1, e2, e3);
+      }
     }
-    if (vlo) QuadSet<__nv_bfloat16>::set(vlo, d, e0, e1, e2, e3);
   }
 }
 
-// Scaled quads of a coarse level, node-row order: 4 lanes per node.
-template <typename KT>
-__global__ void k_cyc_a(int nn, const int* node_sys, const int* node_off, const int* dof_off, const int* rowptr,
-                        const KT* A, const int* nptr, const int* ncol, const double2* sc, void* out,
-                        const int* sel) {
-  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, lane = threadIdx.x & 3;
-  if (g >= nn) return;
-  const int s = node_sys[g];
-  if (sel && !sel[s]) return;
-  const int no = node_off[s], n = node_off[s + 1] - no, i = dof_off[s] + (g - no);
-  const int r0 = rowptr[i], r1 = rowptr[i + n], p0 = nptr[g], deg = nptr[g + 1] - p0;
-  const double2 si = sc[g];
-  for (int k = lane; k < deg; k += 4) {
-    const double2 sj = sc[ncol[p0 + k]];
-    QuadSet<KT>::set(out, p0 + k, si.x * (double)A[r0 + k] * sj.x, si.x * (double)A[r0 + deg + k] * sj.y,
-                     si.y * (double)A[r1 + k] * sj.x, si.y * (double)A[r1 + deg + k] * sj.y);
+// Scaled values of the coarse levels' operators (node-row order) and of Q = D^1/2 (P - D^-1 A P)
+// D_c^-1/2 (A P pattern, in row order and in the order of Q'; coarse nodes on a system's coarsest level
+// are not scaled), every level in one launch: a lane per entry, the blocks dealt out by segment.
+struct CycSeg {
+  int b0;          // first block
+  int lev;         // level of Q, or -1: an operator
+  long long n;     // entries
+  const int *node, *col, *ptr;  // entry -> node, its column, node -> first entry
+  const int4* nrow;
+  const double2 *sc, *scc;
+  const void* val;  // A P quads, or the operator's dof CSR values
+  const void* P;
+  const int *own, *qrow, *tpos;
+  void *out, *outT;
+};
+struct CycSegs {
+  int n;
+  CycSeg s[2 * kCycMaxLev];
+};
+template <typename KT, typename PT, typename QT>
+__global__ void __launch_bounds__(256) k_cyc_levels(const CycSegs S, const int* depth, const int* sel) {
+  int k = 0;
+  while (k + 1 < S.n && blockIdx.x >= S.s[k + 1].b0) ++k;
+  const CycSeg& G = S.s[k];
+  const long long e = (blockIdx.x - G.b0) * 256LL + threadIdx.x;
+  if (e >= G.n) return;
+  const int g = G.node[e];
+  const int4 r = G.nrow[g];
+  if (sel && !sel[r.w]) return;
+  const double2 si = G.sc[g];
+  const int t = (int)(e - G.ptr[g]);
+  if (G.lev < 0) {
+    const KT* A = (const KT*)G.val;
+    const double2 sj = G.sc[G.col[e]];
+    QuadSet<KT>::set(G.out, e, si.x * (double)A[r.x + t] * sj.x, si.x * (double)A[r.x + r.z + t] * sj.y,
+                     si.y * (double)A[r.y + t] * sj.x, si.y * (double)A[r.y + r.z + t] * sj.y);
+    return;
   }
-}
-
-// Q = D^1/2 (P - D^-1 A P) D_c^-1/2 in the A P pattern, written in row order and in the order of
-// Q': 4 lanes per fine node.  A P values in the set-up's layout (row c: [c2 = 0 (dA)][c2 = 1 (dA)]);
-// P quads in pn order.  Coarse nodes on the system's coarsest level are not scaled.
-template <typename ST, typename PT, typename QT>
-__global__ void k_cyc_q(int nn, const int* node_sys, const int* depth, int l, const int* pn_ptr, const int* pn_col,
-                        const PT* P, const int* apn_ptr, const int* apn_col, const int* apbase, const int* apnnz,
-                        const int* apoff, const ST* AP, const double2* sc, const double2* scc, const int* qrow,
-                        const int* tpos, void* out, void* outT, const int* sel) {
-  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, lane = threadIdx.x & 3;
-  if (g >= nn) return;
-  const int s = node_sys[g];
-  if (sel && !sel[s]) return;
-  const int ar = apn_ptr[g], dA = apn_ptr[g + 1] - ar, pr = pn_ptr[g], pe = pn_ptr[g + 1];
-  const size_t ars = (size_t)2 * apnnz[s];
-  const ST* a0 = AP + apoff[s] + 2 * (size_t)(ar - apbase[s]);
-  const double2 si = sc[g];
+  const int J = G.col[e], own = G.own[e];
+  double a[4], p[4] = {0, 0, 0, 0};
+  quad_at((const KT*)G.val, e, a);
+  if (own >= 0) pq_get((const PT*)G.P + own, p);
   const double iu = si.x > 0 ? 1.0 / si.x : 0.0, iv = si.y > 0 ? 1.0 / si.y : 0.0;
-  const bool scaled = depth[s] > l + 1;
-  for (int t = lane; t < dA; t += 4) {
-    const int J = apn_col[ar + t];
-    double p[4] = {0, 0, 0, 0};
-    for (int k = pr; k < pe; ++k)
-      if (pn_col[k] == J) pq_get(P + k, p);
-    const double2 sj = scaled ? scc[J] : make_double2(1.0, 1.0);
-    const double q0 = (iu * p[0] - si.x * (double)a0[t]) * sj.x, q1 = (iu * p[1] - si.x * (double)a0[dA + t]) * sj.y;
-    const double q2 = (iv * p[2] - si.y * (double)a0[ars + t]) * sj.x,
-                 q3 = (iv * p[3] - si.y * (double)a0[ars + dA + t]) * sj.y;
-    const int e = qrow[g] + t;
-    QuadSet<QT>::set(out, e, q0, q1, q2, q3);
-    QuadSet<QT>::set(outT, tpos[e], q0, q1, q2, q3);
-  }
+  const double2 sj = depth[r.w] > G.lev + 1 ? G.scc[J] : make_double2(1.0, 1.0);
+  const double q0 = (iu * p[0] - si.x * a[0]) * sj.x, q1 = (iu * p[1] - si.x * a[1]) * sj.y;
+  const double q2 = (iv * p[2] - si.y * a[2]) * sj.x, q3 = (iv * p[3] - si.y * a[3]) * sj.y;
+  const int o = G.qrow[g] + t;
+  QuadSet<QT>::set(G.out, o, q0, q1, q2, q3);
+  QuadSet<QT>::set(G.outT, G.tpos[o], q0, q1, q2, q3);
 }
 
 // ---------------------------------------------------------------------------
@@ -204,7 +217,6 @@ int cycle_init(ua_mesh* m) {
     Cycle::Lev& D = C.lev[l];
     D.sc = (double2*)dalloc(m, a, sizeof(double2) * (size_t)std::max(L.nn, 1), ok);
     if (l > 0) {
-      D.nptr = upload(m, a, a->h_gptr[l], ok);
       D.ncol = upload(m, a, a->h_gcol[l], ok);
     }
     if (l + 1 < nl) {
@@ -331,50 +343,56 @@ int cycle_alloc_values(ua_mesh* m, bool fp32, bool lo) {
 
 // Values of the collapsed cycle from the numeric set-up just enqueued (launches only, capturable).
 // dw: the finest level's D per node, for the residual norm.
-template <typename KT, typename VT>
-static void cycle_fill_t(ua_mesh* m, const int* rowptr0, const int* colind0, const KT* K0, bool lo, VT* dw,
-                         const int* sel, long long* launches) {
-  using ST = KT;
-  using PT = typename PQuadOf<KT>::T;
-  using QT = typename std::conditional<sizeof(KT) == 4, __nv_bfloat16, double>::type;
+template <typename KT>
+static void fill_fine_t(ua_mesh* m, const int* colind0, const KT* K0, bool lo, const int* sel,
+                        cudaStream_t st, long long* launches) {
   Amg* a = m->amg;
   Cycle& C = a->cyc;
   Sell& S = a->sell;
-  cudaStream_t st = m->stream;
-  for (int l = 0; l + 1 < a->nlev; ++l) {
-    AmgLevel& L = a->lev[l];
-    if (!L.nn) continue;
-    k_cyc_scale<VT><<<(L.nn + 255) / 256, 256, 0, st>>>(L.nn, L.node_sys, L.d_node_off, L.d_dof_off,
-                                                        (const VT*)L.invd, C.lev[l].sc, l == 0 ? dw : nullptr, C.d_ipos, sel),
-        ++*launches;
-  }
+  if (!S.nsb) return;
   const CycFine F{S.perm, S.sl_off, C.d_pcol};
   KT* vk = sizeof(KT) == 4 ? (KT*)S.v32 : (KT*)S.v64;
-  if (S.nsb)
-    k_cyc_fill0<KT><<<S.nsb, 256, 0, st>>>(F, S.sb_n0, S.sb_cnt, S.sb_sys, a->lev[0].d_node_off, a->lev[0].d_dof_off, rowptr0, colind0,
-                                           K0, C.lev[0].sc, vk, lo ? S.vlo : nullptr, sel), ++*launches;
+  const int nsl = S.nsb * kSellSlices;
+  const int nsub = nsl * (32 / kFillN);
+  k_cyc_fill0<KT><<<(nsub + kFillWarps - 1) / kFillWarps, 32 * kFillWarps, 0, st>>>(
+      F, nsl, S.sb_n0, S.sb_cnt, S.sb_sys, a->lev[0].d_node_off, a->lev[0].d_dof_off, a->lev[0].nrow, colind0, K0,
+      C.lev[0].sc, vk, lo ? S.vlo : nullptr, sel), ++*launches;
+}
+void cycle_fill_fine(ua_mesh* m, const int* colind0, const void* K0, bool fp32, bool lo,
+                     const int* sel, cudaStream_t st, long long* launches) {
+  if (fp32) fill_fine_t<float>(m, colind0, (const float*)K0, lo, sel, st, launches);
+  else fill_fine_t<double>(m, colind0, (const double*)K0, lo, sel, st, launches);
+}
+
+template <typename KT>
+static void fill_levels_t(ua_mesh* m, const int* sel, cudaStream_t st, long long* launches) {
+  using PT = typename PQuadOf<KT>::T;
+  using QT = typename std::conditional<sizeof(KT) == 4, __nv_bfloat16, double>::type;
+  constexpr bool f = sizeof(KT) == 4;
+  Amg* a = m->amg;
+  Cycle& C = a->cyc;
+  CycSegs S{};
+  long long nb = 0;
+  auto add = [&](CycSeg g) {
+    if (!g.n) return;
+    g.b0 = (int)nb;
+    S.s[S.n++] = g;
+    nb += (g.n + 255) / 256;
+  };
   for (int l = 0; l + 1 < a->nlev; ++l) {
     AmgLevel& L = a->lev[l];
     Cycle::Lev& D = C.lev[l];
-    if (!L.nn) continue;
+    add(CycSeg{0, l, L.nap, L.ap_node, L.apn_col, L.apn_ptr, L.nrow, D.sc, C.lev[l + 1].sc, L.sa_ap,
+               f ? L.sa_qh : L.sa_qd, L.ap_p, D.qrow, D.tpos, f ? D.qh : D.qd, f ? D.th : D.td});
     if (l > 0)
-      k_cyc_a<KT><<<(L.nn + 63) / 64, 256, 0, st>>>(L.nn, L.node_sys, L.d_node_off, L.d_dof_off, L.rowptr,
-                                                    (const KT*)L.A, D.nptr, D.ncol, D.sc,
-                                                    sizeof(KT) == 4 ? D.a32 : D.a64, sel), ++*launches;
-    const PT* P = (const PT*)(sizeof(KT) == 4 ? L.sa_qh : L.sa_qd);
-    void* q = sizeof(KT) == 4 ? D.qh : D.qd;
-    void* qt = sizeof(KT) == 4 ? D.th : D.td;
-    k_cyc_q<ST, PT, QT><<<(L.nn + 63) / 64, 256, 0, st>>>(L.nn, L.node_sys, a->d_depth, l, L.pn_ptr, L.pn_col, P,
-                                                          L.apn_ptr, L.apn_col, L.apbase, L.apnnz, L.apoff,
-                                                          (const ST*)L.sa_ap, D.sc, C.lev[l + 1].sc, D.qrow, D.tpos,
-                                                          q, qt, sel), ++*launches;
+      add(CycSeg{0, -1, L.ng, a->lev[l - 1].ac_node, D.ncol, L.gptr, L.nrow, D.sc, nullptr, L.A, nullptr, nullptr,
+                 nullptr, nullptr, f ? D.a32 : D.a64, nullptr});
   }
+  if (nb) k_cyc_levels<KT, PT, QT><<<(unsigned)nb, 256, 0, st>>>(S, a->d_depth, sel), ++*launches;
 }
-
-void cycle_fill(ua_mesh* m, const int* rowptr0, const int* colind0, const void* K0, bool fp32, bool lo, void* dw,
-                const int* sel, long long* launches) {
-  if (fp32) cycle_fill_t<float, float>(m, rowptr0, colind0, (const float*)K0, lo, (float*)dw, sel, launches);
-  else cycle_fill_t<double, double>(m, rowptr0, colind0, (const double*)K0, lo, (double*)dw, sel, launches);
+void cycle_fill_levels(ua_mesh* m, bool fp32, const int* sel, cudaStream_t st, long long* launches) {
+  if (fp32) fill_levels_t<float>(m, sel, st, launches);
+  else fill_levels_t<double>(m, sel, st, launches);
 }
 
 // ---------------------------------------------------------------------------
@@ -471,7 +489,7 @@ CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof) {
   for (int l = 0; l + 1 < a->nlev; ++l) {
     const AmgLevel& L = a->lev[l];
     const Cycle::Lev& D = C.lev[l];
-    A.lev[l] = CycLev{D.nptr, D.ncol, fp32 ? D.a32 : D.a64, D.qptr, D.qcol, fp32 ? D.qh : D.qd,
+    A.lev[l] = CycLev{L.gptr, D.ncol, fp32 ? D.a32 : D.a64, D.qptr, D.qcol, fp32 ? D.qh : D.qd,
                       D.tptr, D.tfine, fp32 ? D.th : D.td, L.b, L.x2};
   }
   A.lev[a->nlev - 1].b = a->lev[a->nlev - 1].b;
