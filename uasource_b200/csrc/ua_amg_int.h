@@ -118,7 +118,9 @@ constexpr int kCycMaxLev = 12;
 struct CycLev {
   const int *aptr, *acol;   // node rows of the level's operator (levels >= 1)
   void* aval;               // scaled operator, aptr order
-  const int *qptr, *qcol;   // node rows of Q (the A P pattern)
+  const int* qptr;          // node rows of Q (the A P pattern), levels >= 1
+  const long long* qoff;    // slices of Q, finest level
+  const int* qcol;
   void* qval;
   const int *tptr, *tfine;  // rows of Q' by coarse node
   void* tval;
@@ -156,9 +158,11 @@ struct Cycle {
   struct Lev {
     int* ncol = nullptr;                                       // node graph (levels >= 1)
     long long nq = 0;                                          // node-level entries of Q
-    int *qptr = nullptr, *qcol = nullptr;                      // rows of Q (level 0: in slice order)
-    int* qrow = nullptr;                                       // node -> first entry of its row of Q
-    int *tptr = nullptr, *tfine = nullptr, *tpos = nullptr;    // Q' lists; tpos: entry of Q -> entry of Q'
+    // Q: the A P lists on levels >= 1; on the finest level node slices (qoff, padding slots zero),
+    // qslot the slot of an A P entry
+    long long* qoff = nullptr;
+    int *qcol = nullptr, *qslot = nullptr;
+    int *tptr = nullptr, *tfine = nullptr, *tpos = nullptr;    // Q' lists; tpos: A P entry -> entry of Q'
     double2* sc = nullptr;                                     // D^-1/2 per node (u, v)
     void *a32 = nullptr, *a64 = nullptr;                       // scaled operator quads (levels >= 1)
     void *qh = nullptr, *qd = nullptr, *th = nullptr, *td = nullptr;  // Q and Q' quads (BF16, FP64)

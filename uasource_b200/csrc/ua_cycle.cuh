@@ -122,11 +122,13 @@ __device__ __forceinline__ void team_share(const TeamCtx& t, int n, int& lo, int
   hi = (int)((long long)n * (t.rank + 1) / t.size);
 }
 
-// Lanes per node: a whole warp (restriction) or eight lanes (coarse up pass) on the small levels,
-// where a pass is a chain of dependent loads, fewer on the large ones, where the lanes are needed
-// for more nodes.  Functions of the level's size alone, as the order of the sums depends on them.
-__device__ __forceinline__ int down_lanes(int nc) { return nc <= 4096 ? 32 : 8; }
-__device__ __forceinline__ int up_lanes(int nn) { return nn <= 4096 ? 8 : (nn <= 32768 ? 4 : 2); }
+// Lanes per node.  A row's entries are dealt to kDownW (restriction) or kUpW (coarse up pass) virtual
+// lanes, each summed in order, the lanes' sums added by a butterfly: an order that does not depend on
+// how many physical lanes work on it.  A CTA with few nodes takes one lane per virtual lane (a pass is
+// then one round of dependent loads); one with more nodes than that fills gives every lane four of
+// them, which keeps four times the nodes in flight (a warp per coarse node: 33 rounds of 1900 cycles
+// for the 528 coarse nodes of a 4,753-node mesh on one CTA).
+constexpr int kDownW = 32, kUpW = 8;
 
 // What the passes read of one level and of the finest level's operator: global memory, or the
 // copies of this CTA's rows in shared memory (cyc_stage).  Row pointers and entry numbers are the
@@ -134,7 +136,9 @@ __device__ __forceinline__ int up_lanes(int nn) { return nn <= 4096 ? 8 : (nn <=
 struct LevS {
   const int *aptr, *acol;
   const char* aval;
-  const int *qptr, *qcol;
+  const int* qptr;        // rows of Q (levels >= 1)
+  const long long* qoff;  // slices of Q (finest level)
+  const int* qcol;
   const char* qval;
   const int *tptr, *tfine;
   const char* tval;
@@ -182,6 +186,24 @@ __device__ __forceinline__ void stage_csr(Arena& ar, int lo, int hi, int qb, con
   val = pv - (long long)e0 * qb;
 }
 
+// slices [lo, hi) of a sliced matrix with quads of qb bytes
+__device__ __forceinline__ void stage_slices(Arena& ar, int lo, int hi, int qb, const long long*& off,
+                                             const int*& col, const char*& val) {
+  if (lo >= hi) return;
+  const long long e0 = off[lo], ne = off[hi] - e0;
+  char* p = ar.take(8LL * (hi - lo + 2) + ne * (4 + qb));
+  if (!p) return;
+  long long* po = reinterpret_cast<long long*>(p);
+  char* pv = p + ((8LL * (hi - lo + 1) + 15) & ~15LL);  // slots come in blocks of 32: 16-byte aligned
+  int* pc = reinterpret_cast<int*>(pv + ne * qb);
+  for (int i = threadIdx.x; i <= hi - lo; i += kCycThreads) po[i] = off[lo + i];
+  copy8(pv, val + e0 * qb, ne * qb);
+  copy4(pc, col + e0, ne);
+  off = po - lo;
+  col = pc - e0;
+  val = pv - e0 * qb;
+}
+
 // Reads the level tables into shared memory and copies this CTA's rows as far as they fit, the
 // small levels first.  In a team with enough CTAs everything fits: a pass then waits for one
 // gather of the vector instead of three dependent loads.  [slo, shi): the CTA's slices of the finest
@@ -200,7 +222,7 @@ __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, cons
   }
   for (int l = S.depth - 1; l >= 0; --l) {
     const CycLev& G = A.lev[l];
-    LevS L{G.aptr, G.acol, (const char*)G.aval, G.qptr, G.qcol, (const char*)G.qval,
+    LevS L{G.aptr, G.acol, (const char*)G.aval, G.qptr, G.qoff, G.qcol, (const char*)G.qval,
            G.tptr, G.tfine, (const char*)G.tval};
     team_share(t, S.nn[l + 1], lo, hi);
     stage_csr(ar, S.n0[l + 1] + lo, S.n0[l + 1] + hi, qb, L.tptr, L.tfine, L.tval);
@@ -209,7 +231,7 @@ __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, cons
       stage_csr(ar, S.n0[l] + lo, S.n0[l] + hi, qb, L.qptr, L.qcol, L.qval);
       stage_csr(ar, S.n0[l] + lo, S.n0[l] + hi, ab, L.aptr, L.acol, L.aval);
     } else {
-      stage_csr(ar, S.n0[0] + 32 * slo, S.n0[0] + min(32 * shi, S.nn[0]), qb, L.qptr, L.qcol, L.qval);
+      stage_slices(ar, S.sl0 + slo, S.sl0 + shi, qb, L.qoff, L.qcol, L.qval);
     }
     if (threadIdx.x == 0) lev[l] = L;
   }
@@ -244,132 +266,144 @@ __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, cons
   __syncthreads();
 }
 
+// KC entries of each of a lane's NV virtual lanes from entry e on: their columns and values load
+// together, then the vector's pairs get(column).  Entries past the row's end repeat its last one with a
+// zero vector pair.
+template <int W, int NV, int KC, bool TR, typename QT, typename G>
+__device__ __forceinline__ void row_chunk(const int* col, const char* val, int e, int ee, int lane, double sign, G get,
+                                          double (&a0)[NV], double (&a1)[NV]) {
+  using V2 = decltype(get(0));
+  constexpr int qb = 4 * sizeof(QT), CH = NV * KC;
+  int c[CH];
+  typename QuadRaw<QT>::T m[CH];
+#pragma unroll
+  for (int k = 0; k < CH; ++k) {
+    const int u = min(e + W * (k / NV) + (W / NV) * (k % NV) + lane, ee - 1);
+    c[k] = col[u];
+    m[k] = QuadRaw<QT>::load(val + (long long)u * qb);
+  }
+  V2 x[CH];
+#pragma unroll
+  for (int k = 0; k < CH; ++k) {
+    x[k] = get(c[k]);
+    if (e + W * (k / NV) + (W / NV) * (k % NV) + lane >= ee) x[k].x = x[k].y = 0;
+  }
+#pragma unroll
+  for (int k = 0; k < CH; ++k) {
+    double q[4];
+    QuadRaw<QT>::get(m[k], q);
+    const double xu = sign * (double)x[k].x, xv = sign * (double)x[k].y;
+    a0[k % NV] = fma(q[TR ? 2 : 1], xv, fma(q[0], xu, a0[k % NV]));
+    a1[k % NV] = fma(q[3], xv, fma(q[TR ? 1 : 2], xu, a1[k % NV]));
+  }
+}
+// Entries [e, ee) of a row over W virtual lanes, NV of them per physical lane, in chunks of KC entries
+// each (of one for a rest that W entries hold: a short row does not pay for a long chunk).  TR: the quad
+// transposed (restriction).  a0, a1: the virtual lanes' sums.
+template <int W, int NV, int KC, bool TR, typename QT, typename G>
+__device__ __forceinline__ void row_sums(const int* col, const char* val, int e, int ee, int lane, double sign, G get,
+                                         double (&a0)[NV], double (&a1)[NV]) {
+  while (e < ee) {
+    if (KC == 1 || ee - e <= W) {
+      row_chunk<W, NV, 1, TR, QT>(col, val, e, ee, lane, sign, get, a0, a1);
+      e += W;
+    } else {
+      row_chunk<W, NV, KC, TR, QT>(col, val, e, ee, lane, sign, get, a0, a1);
+      e += W * KC;
+    }
+  }
+}
+// the butterfly of W virtual lanes, its first stages inside the physical lane
+template <int W, int NV>
+__device__ __forceinline__ double lanes_total(const double (&a)[NV]) {
+  static_assert(NV == 1 || NV == 4, "one or four virtual lanes a lane");
+  return lane_sum(NV == 1 ? a[0] : (a[0] + a[NV / 2]) + (a[NV / 4] + a[NV / 2 + NV / 4]), W / NV);
+}
+
 // b_c = Q' b for the coarse nodes of level l + 1; with a second vector, of b - alpha q (rounded as
 // the update of the residual rounds it), scaled by w.
-template <typename VT, typename QT>
-__device__ __forceinline__ void cyc_down(const LevS& L, const CycSys& S, int l, const TeamCtx& t,
-                                         const typename Vec2<VT>::T* b, typename Vec2<VT>::T* bc,
-                                         const typename Vec2<VT>::T* q2 = nullptr, double alpha = 0.0,
-                                         double w = 1.0) {
+template <int NV, typename VT, typename QT>
+__device__ __forceinline__ void cyc_down_nv(const LevS& L, int c0, int lo, int hi, const typename Vec2<VT>::T* b,
+                                            typename Vec2<VT>::T* bc, const typename Vec2<VT>::T* q2, double alpha,
+                                            double w, bool rev) {
   using V2 = typename Vec2<VT>::T;
-  constexpr int CH = sizeof(VT) == 4 ? 4 : 2, qb = 4 * sizeof(QT);
-  int lo, hi;
-  team_share(t, S.nn[l + 1], lo, hi);
-  const int c0 = S.n0[l + 1], lanes = down_lanes(S.nn[l + 1]);
-  const int sub = threadIdx.x / lanes, lane = threadIdx.x & (lanes - 1), nsub = kCycThreads / lanes;
+  constexpr int lanes = kDownW / NV, nsub = kCycThreads / lanes, KC = sizeof(VT) == 4 ? (NV == 1 ? 4 : 2) : (NV == 1 ? 2 : 1);
+  const int sub = threadIdx.x / lanes, lane = threadIdx.x & (lanes - 1);
   for (int j0 = lo; j0 < hi; j0 += nsub) {
-    const int J = c0 + j0 + sub;
+    const int J = c0 + (rev ? lo + hi - 1 - (j0 + sub) : j0 + sub);
     const bool valid = j0 + sub < hi;
-    double a0 = 0, a1 = 0;
-    if (valid) {
-      const int ue = L.tptr[J + 1];
-      for (int u0 = L.tptr[J] + lane; u0 < ue; u0 += lanes * CH) {
-        int f[CH];
-        typename QuadRaw<QT>::T e[CH];
-#pragma unroll
-        for (int k = 0; k < CH; ++k) {
-          const int u = min(u0 + k * lanes, ue - 1);
-          f[k] = L.tfine[u];
-          e[k] = QuadRaw<QT>::load(L.tval + (long long)u * qb);
+    double a0[NV] = {}, a1[NV] = {};
+    if (valid)
+      row_sums<kDownW, NV, KC, true, QT>(L.tfine, L.tval, L.tptr[J], L.tptr[J + 1], lane, 1.0, [&](int f) {
+        V2 x = b[f];
+        if (q2) {
+          const V2 y = q2[f];
+          x.x = (VT)((double)x.x - alpha * (double)y.x);
+          x.y = (VT)((double)x.y - alpha * (double)y.y);
         }
-        V2 x[CH];
-#pragma unroll
-        for (int k = 0; k < CH; ++k) {
-          x[k] = b[f[k]];
-          if (q2) {
-            const V2 y = q2[f[k]];
-            x[k].x = (VT)((double)x[k].x - alpha * (double)y.x);
-            x[k].y = (VT)((double)x[k].y - alpha * (double)y.y);
-          }
-          if (u0 + k * lanes >= ue) x[k].x = x[k].y = 0;
-        }
-#pragma unroll
-        for (int k = 0; k < CH; ++k) {
-          double q[4];
-          QuadRaw<QT>::get(e[k], q);
-          a0 += q[0] * (double)x[k].x + q[2] * (double)x[k].y;
-          a1 += q[1] * (double)x[k].x + q[3] * (double)x[k].y;
-        }
-      }
-    }
-    a0 = lane_sum(a0, lanes);
-    a1 = lane_sum(a1, lanes);
+        return x;
+      }, a0, a1);
+    const double s0 = lanes_total<kDownW, NV>(a0), s1 = lanes_total<kDownW, NV>(a1);
     if (valid && lane == 0) {
       V2 o;
-      o.x = (VT)(w * a0);
-      o.y = (VT)(w * a1);
+      o.x = (VT)(w * s0);
+      o.y = (VT)(w * s1);
       bc[J] = o;
     }
   }
 }
-
-// a += sign * (row entries [e, ee) in steps of `lanes`) * x, CH entries at a time
-template <int CH, typename QT, typename VT>
-__device__ __forceinline__ void row_product(const int* col, const char* val, int e, int ee, int lanes,
-                                            const typename Vec2<VT>::T* x0, double sign, double& a0, double& a1) {
-  using V2 = typename Vec2<VT>::T;
-  constexpr int qb = 4 * sizeof(QT);
-  for (; e < ee; e += lanes * CH) {
-    int c[CH];
-    typename QuadRaw<QT>::T m[CH];
-#pragma unroll
-    for (int k = 0; k < CH; ++k) {
-      const int u = min(e + k * lanes, ee - 1);
-      c[k] = col[u];
-      m[k] = QuadRaw<QT>::load(val + (long long)u * qb);
-    }
-    V2 x[CH];
-#pragma unroll
-    for (int k = 0; k < CH; ++k) {
-      x[k] = x0[c[k]];
-      if (e + k * lanes >= ee) x[k].x = x[k].y = 0;
-    }
-    double s0 = 0, s1 = 0;
-#pragma unroll
-    for (int k = 0; k < CH; ++k) {
-      double q[4];
-      QuadRaw<QT>::get(m[k], q);
-      s0 += q[0] * (double)x[k].x + q[1] * (double)x[k].y;
-      s1 += q[2] * (double)x[k].x + q[3] * (double)x[k].y;
-    }
-    a0 += sign * s0;
-    a1 += sign * s1;
-  }
+template <typename VT, typename QT>
+__device__ __forceinline__ void cyc_down(const LevS& L, const CycSys& S, int l, const TeamCtx& t,
+                                         const typename Vec2<VT>::T* b, typename Vec2<VT>::T* bc,
+                                         const typename Vec2<VT>::T* q2 = nullptr, double alpha = 0.0,
+                                         double w = 1.0, bool rev = false) {
+  int lo, hi;
+  team_share(t, S.nn[l + 1], lo, hi);
+  if (hi - lo <= kCycThreads / kDownW)
+    cyc_down_nv<1, VT, QT>(L, S.n0[l + 1], lo, hi, b, bc, q2, alpha, w, rev);
+  else
+    cyc_down_nv<4, VT, QT>(L, S.n0[l + 1], lo, hi, b, bc, q2, alpha, w, rev);
 }
 
 // z = 2 b - A b + Q z_c on level l >= 1 (zc: indexed by the coarse level's node numbers).
+template <int NV, typename VT, typename AT, typename QT>
+__device__ __forceinline__ void cyc_up_nv(const LevS& L, int n0, int lo, int hi, const typename Vec2<VT>::T* b,
+                                          typename Vec2<VT>::T* z, const typename Vec2<VT>::T* zc) {
+  using V2 = typename Vec2<VT>::T;
+  constexpr int lanes = kUpW / NV, nsub = kCycThreads / lanes, KC = sizeof(VT) == 4 ? (NV == 1 ? 4 : 2) : (NV == 1 ? 2 : 1);
+  const int sub = threadIdx.x / lanes, lane = threadIdx.x & (lanes - 1);
+  for (int j0 = lo; j0 < hi; j0 += nsub) {
+    const int g = n0 + j0 + sub;
+    const bool valid = j0 + sub < hi;
+    double a0[NV] = {}, a1[NV] = {};
+    V2 bv;
+    bv.x = bv.y = 0;
+    if (valid) {
+      bv = b[g];
+      row_sums<kUpW, NV, KC, false, AT>(L.acol, L.aval, L.aptr[g], L.aptr[g + 1], lane, -1.0,
+                                        [&](int c) { return b[c]; }, a0, a1);
+      row_sums<kUpW, NV, KC, false, QT>(L.qcol, L.qval, L.qptr[g], L.qptr[g + 1], lane, 1.0,
+                                        [&](int c) { return zc[c]; }, a0, a1);
+    }
+    const double s0 = lanes_total<kUpW, NV>(a0), s1 = lanes_total<kUpW, NV>(a1);
+    if (valid && lane == 0) {
+      V2 o;
+      o.x = (VT)(2.0 * (double)bv.x + s0);
+      o.y = (VT)(2.0 * (double)bv.y + s1);
+      z[g] = o;
+    }
+  }
+}
 template <typename VT, typename AT, typename QT>
 __device__ __forceinline__ void cyc_up(const LevS& L, const CycSys& S, int l, const TeamCtx& t,
                                        const typename Vec2<VT>::T* b, typename Vec2<VT>::T* z,
                                        const typename Vec2<VT>::T* zc) {
-  using V2 = typename Vec2<VT>::T;
-  constexpr int CH = sizeof(VT) == 4 ? 4 : 2;
   int lo, hi;
   team_share(t, S.nn[l], lo, hi);
-  const int n0 = S.n0[l], lanes = up_lanes(S.nn[l]);
-  const int sub = threadIdx.x / lanes, lane = threadIdx.x & (lanes - 1), nsub = kCycThreads / lanes;
-  for (int j0 = lo; j0 < hi; j0 += nsub) {
-    const int g = n0 + j0 + sub;
-    const bool valid = j0 + sub < hi;
-    double a0 = 0, a1 = 0;
-    if (valid) {
-      if (lane == 0) {
-        const V2 v = b[g];
-        a0 = 2.0 * (double)v.x;
-        a1 = 2.0 * (double)v.y;
-      }
-      row_product<CH, AT, VT>(L.acol, L.aval, L.aptr[g] + lane, L.aptr[g + 1], lanes, b, -1.0, a0, a1);
-      row_product<CH, QT, VT>(L.qcol, L.qval, L.qptr[g] + lane, L.qptr[g + 1], lanes, zc, 1.0, a0, a1);
-    }
-    a0 = lane_sum(a0, lanes);
-    a1 = lane_sum(a1, lanes);
-    if (valid && lane == 0) {
-      V2 o;
-      o.x = (VT)a0;
-      o.y = (VT)a1;
-      z[g] = o;
-    }
-  }
+  if (hi - lo <= kCycThreads / kUpW)
+    cyc_up_nv<1, VT, AT, QT>(L, S.n0[l], lo, hi, b, z, zc);
+  else
+    cyc_up_nv<4, VT, AT, QT>(L, S.n0[l], lo, hi, b, z, zc);
 }
 
 // The coarsest level of the system by every CTA of the team for itself (no team barrier follows):
@@ -447,11 +481,11 @@ __device__ __forceinline__ void slice_chunk(const int* cp, const char* vp, int l
 // what is left): a linear mesh's slice is one or two chunks, two dependent loads each, where a plain
 // unrolled loop takes the slots of its remainder one by one.
 template <typename KT, typename VT>
-__device__ __forceinline__ void slice_product(const FineS& F, const char* vals, int sl, int lane,
-                                              const typename Vec2<VT>::T* v, double& a0, double& a1) {
-  const long long off = F.sl_off[sl];
-  const int k1 = (int)((F.sl_off[sl + 1] - off) >> 5);
-  const int* cp = F.cols + off;
+__device__ __forceinline__ void slice_product(const long long* sl_off, const int* cols, const char* vals, int sl,
+                                              int lane, const typename Vec2<VT>::T* v, double& a0, double& a1) {
+  const long long off = sl_off[sl];
+  const int k1 = (int)((sl_off[sl + 1] - off) >> 5);
+  const int* cp = cols + off;
   const char* vp = vals + off * (long long)(4 * sizeof(KT));
   a0 = a1 = 0;
   for (int k0 = 0; k0 < k1;) {  // the width is the same for the whole warp
@@ -475,37 +509,41 @@ __device__ __forceinline__ void prefetch_l2(const void* p, long long bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"((unsigned)bytes) : "memory");
 }
 template <typename KT>
-__device__ __forceinline__ void slice_prefetch(const CycFine& G, const void* vals, int sl) {
-  const long long off = G.sl_off[sl], n = G.sl_off[sl + 1] - off;
-  prefetch_l2(G.cols + off, 4 * n);
+__device__ __forceinline__ void slice_prefetch(const long long* sl_off, const int* cols, const void* vals, int sl) {
+  const long long off = sl_off[sl], n = sl_off[sl + 1] - off;
+  prefetch_l2(cols + off, 4 * n);
   prefetch_l2((const char*)vals + off * (4 * sizeof(KT)), n * (4 * sizeof(KT)));
 }
 
-// Runs the slices [lo, hi) over the CTA's warps: f(i, lane's node, node is there).  The slices of a
+// Runs the slices [lo, hi) over the CTA's warps: f(i, lane's node, node is there, a slice of the next
+// round, which may lie outside).  The slices of a
 // block of eight are ordered by width (25 down to 9 slots on a quadratic mesh), so the warps rotate
 // from round to round: with a plain stride of 16 a warp met the same place of a block every time,
 // and a pass waited for the warps of the widest one (401x201 P2: CTAs of 52k and 110k cycles side
 // by side).  (Splitting a slice's slots over two or four warps of a CTA that has few was slower
 // at every size: the exchange through shared memory costs what the shorter chains save.)
+//
+// rev: from the last slice to the first.  A pass that reads what the pass before it (or the same pass of
+// the step before) has read goes the other way, so that it meets in L2 what was read last.
 template <typename F>
-__device__ __forceinline__ void for_slices(int lo, int hi, int n0, int nn, F f) {
+__device__ __forceinline__ void for_slices(int lo, int hi, int n0, int nn, bool rev, F f) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int b = lo, r = 0; b < hi; b += kCycWarps, r += 5) {
-    const int i = b + ((warp + r) & (kCycWarps - 1));
-    if (i < hi) f(i, n0 + 32 * i + lane, 32 * i + lane < nn);
+    const int k = b + ((warp + r) & (kCycWarps - 1)), i = rev ? hi - 1 - (k - lo) : k;
+    if (k < hi) f(i, n0 + 32 * i + lane, 32 * i + lane < nn, rev ? i - kCycWarps : i + kCycWarps);
   }
 }
 
 // - w A^ b + Q z_c at the lane of slice sl, finest level (the caller adds 2 w b).
 template <typename LT, typename VT, typename QT>
-__device__ __forceinline__ void cyc_up0_node(const FineS& F, const LevS& L, int sl, int lane, int g,
+__device__ __forceinline__ void cyc_up0_node(const FineS& F, const LevS& L, int sl, int lane,
                                              const typename Vec2<VT>::T* b, const typename Vec2<VT>::T* zc, double w,
                                              double& z0, double& z1) {
-  double a0, a1;
-  slice_product<LT, VT>(F, F.lv, sl, lane, b, a0, a1);
-  z0 = -w * a0;
-  z1 = -w * a1;
-  row_product<sizeof(VT) == 4 ? 8 : 6, QT, VT>(L.qcol, L.qval, L.qptr[g], L.qptr[g + 1], 1, zc, 1.0, z0, z1);
+  double a0, a1, q0, q1;
+  slice_product<LT, VT>(F.sl_off, F.cols, F.lv, sl, lane, b, a0, a1);
+  slice_product<QT, VT>(L.qoff, L.qcol, L.qval, sl, lane, zc, q0, q1);
+  z0 = q0 - w * a0;
+  z1 = q1 - w * a1;
 }
 
 // ---- host side of a resident launch (ua_pcg.cu) ----

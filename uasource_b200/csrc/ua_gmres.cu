@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
     const double tol = a.tol[s];
     while (true) {
       // residual
-      for_slices(lo, hi, n0, nn, [&](int i, int k, bool in) {
+      for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
         if (!in) return;
         double kx[3];
         gm_product(a.cyc.fine, a.v3, S.sl0 + i, lane, a.x, kx);
@@ -361,10 +361,10 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
           UA_TEAM_SYNC(t);
           zc = (const double2*)a.cyc.lev[l].z;
         }
-        for_slices(lo, hi, n0, nn, [&](int i, int k, bool in) {
+        for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
           if (!in) return;
           double z0, z1;
-          cyc_up0_node<double, double, double>(fine, lev[0], S.sl0 + i, lane, k, a.ws, zc, inv, z0, z1);
+          cyc_up0_node<double, double, double>(fine, lev[0], S.sl0 + i, lane, a.ws, zc, inv, z0, z1);
           const double2 d = a.scp[k], b = a.ws[k];
           a.z.uv[k] = make_double2(d.x * (2.0 * inv * b.x + z0), d.y * (2.0 * inv * b.y + z1));
         });
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
         // thickness rows; the sweeps ping-pong so that the last one writes z.h
         double* bufs[2] = {a.z.h, a.ht};
         int cur = (a.hsw - 1) % 2 == 0 ? 0 : 1;
-        for_slices(lo, hi, n0, nn, [&](int i, int k, bool in) {
+        for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
           if (!in) return;
           const double b = vj.h[k] - gm_hrow<0>(a.cyc.fine, a.v3, S.sl0 + i, lane, a.z.uv, nullptr);
           const double hi1 = a.hinv[k];
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
         for (int q = 1; q < a.hsw; ++q) {
           const double* zi = bufs[cur];
           double* zo = bufs[1 - cur];
-          for_slices(lo, hi, n0, nn, [&](int i, int k, bool in) {
+          for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
             if (in)
               zo[k] = zi[k] + (a.bh[k] - gm_hrow<1>(a.cyc.fine, a.v3, S.sl0 + i, lane, nullptr, zi)) * a.hinv[k];
           });
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
         }
         if (combine) break;
         // w = K z and its dot products
-        for_slices(lo, hi, n0, nn, [&](int i, int k, bool in) {
+        for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
           if (!in) return;
           double kx[3];
           gm_product(a.cyc.fine, a.v3, S.sl0 + i, lane, a.z, kx);

@@ -21,6 +21,7 @@ namespace ua {
 
 constexpr int kCycArena = 212 * 1024;       // with the kernel's static tables below 227 KB
 constexpr int kCycArenaSmall = 64 * 1024;
+constexpr int kSplitSlices = 12;
 
 template <typename T> struct QuadSet;
 template <> struct QuadSet<double> {
@@ -141,7 +142,7 @@ struct CycSeg {
   const double2 *sc, *scc;
   const void* val;  // A P quads, or the operator's dof CSR values
   const void* P;
-  const int *own, *qrow, *tpos;
+  const int *own, *qslot, *tpos;
   void *out, *outT;
 };
 struct CycSegs {
@@ -159,8 +160,8 @@ __global__ void __launch_bounds__(256) k_cyc_levels(const CycSegs S, const int* 
   const int4 r = G.nrow[g];
   if (sel && !sel[r.w]) return;
   const double2 si = G.sc[g];
-  const int t = (int)(e - G.ptr[g]);
   if (G.lev < 0) {
+    const int t = (int)(e - G.ptr[g]);
     const KT* A = (const KT*)G.val;
     const double2 sj = G.sc[G.col[e]];
     QuadSet<KT>::set(G.out, e, si.x * (double)A[r.x + t] * sj.x, si.x * (double)A[r.x + r.z + t] * sj.y,
@@ -175,9 +176,15 @@ __global__ void __launch_bounds__(256) k_cyc_levels(const CycSegs S, const int* 
   const double2 sj = depth[r.w] > G.lev + 1 ? G.scc[J] : make_double2(1.0, 1.0);
   const double q0 = (iu * p[0] - si.x * a[0]) * sj.x, q1 = (iu * p[1] - si.x * a[1]) * sj.y;
   const double q2 = (iv * p[2] - si.y * a[2]) * sj.x, q3 = (iv * p[3] - si.y * a[3]) * sj.y;
-  const int o = G.qrow[g] + t;
-  QuadSet<QT>::set(G.out, o, q0, q1, q2, q3);
-  QuadSet<QT>::set(G.outT, G.tpos[o], q0, q1, q2, q3);
+  if (G.qslot && sizeof(QT) == 8) {  // two blocks of 32 pairs (SliceQuad)
+    const int o = G.qslot[e];
+    double2* q = reinterpret_cast<double2*>(G.out) + 2 * (long long)(o & ~31) + (o & 31);
+    q[0] = make_double2(q0, q1);
+    q[32] = make_double2(q2, q3);
+  } else {
+    QuadSet<QT>::set(G.out, G.qslot ? G.qslot[e] : e, q0, q1, q2, q3);
+  }
+  QuadSet<QT>::set(G.outT, G.tpos[e], q0, q1, q2, q3);
 }
 
 // ---------------------------------------------------------------------------
@@ -216,46 +223,53 @@ int cycle_init(ua_mesh* m) {
     AmgLevel& L = a->lev[l];
     Cycle::Lev& D = C.lev[l];
     D.sc = (double2*)dalloc(m, a, sizeof(double2) * (size_t)std::max(L.nn, 1), ok);
-    if (l > 0) {
-      D.ncol = upload(m, a, a->h_gcol[l], ok);
-    }
+    if (l > 0) D.ncol = upload(m, a, a->h_gcol[l], ok);
     if (l + 1 < nl) {
-      // Q: the A P pattern, on the finest level with its rows in slice order; Q': by coarse node,
+      // Q: the A P pattern, on the finest level in node slices; Q': by coarse node,
       // the fine nodes (positions) ascending
       const std::vector<int>&ap = a->h_apnp[l], &ac = a->h_apnc[l];
       const int nc = a->lev[l + 1].nn;
+      std::vector<int> qc;
       D.nq = (long long)ac.size();
-      std::vector<int> qp, qc, qr, tp(nc + 1, 0), tf(ac.size()), tpos(ac.size());
-      const std::vector<int>*pp = &ap, *pc = &ac;
+      std::vector<int> tp(nc + 1, 0), tf(ac.size()), tpos(ac.size());
       if (l == 0) {
-        qp.assign(L.nn + 1, 0);
-        qr.assign(L.nn, 0);
-        qc.resize(ac.size());
-        for (int k = 0; k < L.nn; ++k) {
-          const int g = SL.h_perm[k], b = ap[g], n = ap[g + 1] - b;
-          qr[g] = qp[k];
-          for (int t = 0; t < n; ++t) qc[qp[k] + t] = ac[b + t];
-          qp[k + 1] = qp[k] + n;
+        std::vector<long long> qo(kSellSlices * (size_t)SL.nsb + 1, 0);
+        std::vector<int> qs(ac.size());
+        for (int s = 0; s < nsys; ++s) {
+          const int n0 = L.node_off[s], n1 = L.node_off[s + 1], c0 = a->lev[1].node_off[s];
+          const size_t s0 = kSellSlices * (size_t)SL.h_sys_sb_off[s], s1 = kSellSlices * (size_t)SL.h_sys_sb_off[s + 1];
+          for (size_t i = s0; i < s1; ++i) {
+            const int k0 = n0 + 32 * (int)(i - s0), k1 = std::min(k0 + 32, n1);
+            int wd = 0;
+            for (int k = k0; k < k1; ++k) wd = std::max(wd, ap[SL.h_perm[k] + 1] - ap[SL.h_perm[k]]);
+            qo[i + 1] = qo[i] + 32LL * wd;
+            qc.resize(qo[i + 1], c0);
+            for (int k = k0; k < k1; ++k)
+              for (int e = ap[SL.h_perm[k]], t = 0; e < ap[SL.h_perm[k] + 1]; ++e, ++t) {
+                qs[e] = (int)(qo[i] + 32 * t + (k - k0));
+                qc[qs[e]] = ac[e];
+              }
+          }
         }
-        pp = &qp;
-        pc = &qc;
-        D.qptr = upload(m, a, qp, ok);
+        D.nq = qo.back();
+        if (D.nq > INT_MAX) ok = false;
+        D.qoff = upload(m, a, qo, ok);
         D.qcol = upload(m, a, qc, ok);
-        D.qrow = upload(m, a, qr, ok);
+        D.qslot = upload(m, a, qs, ok);
       } else {
-        D.qptr = L.apn_ptr;
         D.qcol = L.apn_col;
-        D.qrow = L.apn_ptr;
       }
-      for (int J : *pc) tp[J + 1]++;
+      for (int J : ac) tp[J + 1]++;
       for (int J = 0; J < nc; ++J) tp[J + 1] += tp[J];
       std::vector<int> nx(tp.begin(), tp.end() - 1);
-      for (int k = 0; k < L.nn; ++k)
-        for (int t = (*pp)[k]; t < (*pp)[k + 1]; ++t) {
-          const int u = nx[(*pc)[t]]++;
+      for (int k = 0; k < L.nn; ++k) {
+        const int g = l == 0 ? SL.h_perm[k] : k;
+        for (int e = ap[g]; e < ap[g + 1]; ++e) {
+          const int u = nx[ac[e]]++;
           tf[u] = k;
-          tpos[t] = u;
+          tpos[e] = u;
         }
+      }
       D.tptr = upload(m, a, tp, ok);
       D.tfine = upload(m, a, tf, ok);
       D.tpos = upload(m, a, tpos, ok);
@@ -322,8 +336,10 @@ int cycle_alloc_values(ua_mesh* m, bool fp32, bool lo) {
   Cycle& C = a->cyc;
   Sell& S = a->sell;
   bool ok = true;
-  auto need = [&](void** p, size_t bytes) {
-    if (!*p) *p = dalloc(m, a, std::max<size_t>(bytes, 32), ok);
+  auto need = [&](void** p, size_t bytes, bool zero = false) {
+    if (*p) return;
+    *p = dalloc(m, a, std::max<size_t>(bytes, 32), ok);
+    if (*p && zero && cudaMemsetAsync(*p, 0, std::max<size_t>(bytes, 32), m->stream) != cudaSuccess) ok = false;
   };
   const size_t nv = 4 * (size_t)S.slots;
   if (fp32) need((void**)&S.v32, sizeof(float) * nv);
@@ -334,8 +350,8 @@ int cycle_alloc_values(ua_mesh* m, bool fp32, bool lo) {
     // levels 1 .. nlev-2 hold an operator; node entries = dof entries / 4
     if (l > 0 && l + 1 < a->nlev) need(fp32 ? &D.a32 : &D.a64, (fp32 ? 16 : 32) * (size_t)(a->lev[l].nnz / 4));
     if (l + 1 < a->nlev) {
-      need(fp32 ? &D.qh : &D.qd, (fp32 ? 8 : 32) * (size_t)D.nq);
-      need(fp32 ? &D.th : &D.td, (fp32 ? 8 : 32) * (size_t)D.nq);
+      need(fp32 ? &D.qh : &D.qd, (fp32 ? 8 : 32) * (size_t)D.nq, l == 0);  // padding slots stay zero
+      need(fp32 ? &D.th : &D.td, (fp32 ? 8 : 32) * (size_t)a->lev[l].nap);
     }
   }
   return ok ? UA_OK : set_error(UA_ERR_OOM, "collapsed cycle: device allocation of the values failed");
@@ -383,7 +399,7 @@ static void fill_levels_t(ua_mesh* m, const int* sel, cudaStream_t st, long long
     AmgLevel& L = a->lev[l];
     Cycle::Lev& D = C.lev[l];
     add(CycSeg{0, l, L.nap, L.ap_node, L.apn_col, L.apn_ptr, L.nrow, D.sc, C.lev[l + 1].sc, L.sa_ap,
-               f ? L.sa_qh : L.sa_qd, L.ap_p, D.qrow, D.tpos, f ? D.qh : D.qd, f ? D.th : D.td});
+               f ? L.sa_qh : L.sa_qd, L.ap_p, D.qslot, D.tpos, f ? D.qh : D.qd, f ? D.th : D.td});
     if (l > 0)
       add(CycSeg{0, -1, L.ng, a->lev[l - 1].ac_node, D.ncol, L.gptr, L.nrow, D.sc, nullptr, L.A, nullptr, nullptr,
                  nullptr, nullptr, f ? D.a32 : D.a64, nullptr});
@@ -489,7 +505,7 @@ CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof) {
   for (int l = 0; l + 1 < a->nlev; ++l) {
     const AmgLevel& L = a->lev[l];
     const Cycle::Lev& D = C.lev[l];
-    A.lev[l] = CycLev{L.gptr, D.ncol, fp32 ? D.a32 : D.a64, D.qptr, D.qcol, fp32 ? D.qh : D.qd,
+    A.lev[l] = CycLev{L.gptr, D.ncol, fp32 ? D.a32 : D.a64, l ? L.apn_ptr : nullptr, D.qoff, D.qcol, fp32 ? D.qh : D.qd,
                       D.tptr, D.tfine, fp32 ? D.th : D.td, L.b, L.x2};
   }
   A.lev[a->nlev - 1].b = a->lev[a->nlev - 1].b;
@@ -613,6 +629,10 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
     cyc_stage<KT, LT, QT>(a.cyc, a.kv, a.lv, S, t, lo, hi, ar, lev, &fine, 4 * sizeof(KT), dense);
     const int n0 = S.n0[0], nn = S.nn[0], dep = S.depth;
     const bool stream = fine.cols == a.cyc.fine.cols;  // rows read from global memory
+    // restrict the updated residual after one more barrier, or b - alpha q from the two old vectors:
+    // the second gather costs more than the barrier once a CTA has kSplitSlices slices
+    const bool same = a.kv == a.lv;  // the cycle reads the method's operator
+    const bool split = S.nsl >= kSplitSlices * t.size;
     const V2* bL = (const V2*)a.cyc.lev[dep].b;
     V2 *r = (V2*)a.r, *rn = (V2*)a.r2;
     for (int i = lo + warp; i < hi; i += kCycWarps) {
@@ -632,6 +652,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
     double rz_old = 0;
     mark(CP_OTHER);
     while (rr0 != 0.0) {
+      const bool odd = its & 1;
       // z = cycle(r), the finest restriction done
       for (int l = 1; l < dep; ++l) {
         cyc_down<VT, QT>(lev[l], S, l, t, (const V2*)a.cyc.lev[l].b, (V2*)a.cyc.lev[l + 1].b);
@@ -645,13 +666,16 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
         zc = (const V2*)a.cyc.lev[l].z;
       }
       mark(CP_OTHER);
-      for_slices(lo, hi, n0, nn, [&](int i, int g, bool in) {
-        if (stream && lane == 0 && i + kCycWarps < hi) slice_prefetch<LT>(a.cyc.fine, a.lv, S.sl0 + i + kCycWarps);
+      for_slices(lo, hi, n0, nn, !same && odd, [&](int i, int g, bool in, int nx) {
+        if (stream && lane == 0 && nx >= lo && nx < hi) {
+          slice_prefetch<LT>(a.cyc.fine.sl_off, a.cyc.fine.cols, a.lv, S.sl0 + nx);
+          slice_prefetch<QT>(a.cyc.lev[0].qoff, a.cyc.lev[0].qcol, a.cyc.lev[0].qval, S.sl0 + nx);
+        }
         double v = 0;
         if (in) {
           const V2 bv = r[g];
           double z0, z1;
-          cyc_up0_node<LT, VT, QT>(fine, lev[0], S.sl0 + i, lane, g, r, zc, 1.0, z0, z1);
+          cyc_up0_node<LT, VT, QT>(fine, lev[0], S.sl0 + i, lane, r, zc, 1.0, z0, z1);
           V2 o;
           o.x = (VT)(2.0 * (double)bv.x + z0);
           o.y = (VT)(2.0 * (double)bv.y + z1);
@@ -667,8 +691,8 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
       const double beta = its ? rz / rz_old : 0.0;
       rz_old = rz;
       // p = z + beta p, q = A z + beta q, partials p.q
-      for_slices(lo, hi, n0, nn, [&](int i, int g, bool in) {
-        if (stream && lane == 0 && i + kCycWarps < hi) slice_prefetch<KT>(a.cyc.fine, a.kv, S.sl0 + i + kCycWarps);
+      for_slices(lo, hi, n0, nn, same || odd, [&](int i, int g, bool in, int nx) {
+        if (stream && lane == 0 && nx >= lo && nx < hi) slice_prefetch<KT>(a.cyc.fine.sl_off, a.cyc.fine.cols, a.kv, S.sl0 + nx);
         double v = 0;
         if (in) {
           V2 pn = z[g], po, qo;
@@ -677,7 +701,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
             qo = q[g];
           }
           double a0, a1;
-          slice_product<KT, VT>(fine, fine.kv, S.sl0 + i, lane, z, a0, a1);
+          slice_product<KT, VT>(fine.sl_off, fine.cols, fine.kv, S.sl0 + i, lane, z, a0, a1);
           if (its) {
             pn.x = (VT)((double)pn.x + beta * (double)po.x);
             pn.y = (VT)((double)pn.y + beta * (double)po.y);
@@ -721,7 +745,12 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
         v = lane_sum(v, 32);
         if (lane == 0) part_rr[S.sl0 + i] = v;
       }
-      cyc_down<VT, QT>(lev[0], S, 0, t, r, (V2*)a.cyc.lev[1].b, q, alpha);
+      if (split) {
+        UA_TEAM_SYNC(t);
+        cyc_down<VT, QT>(lev[0], S, 0, t, rn, (V2*)a.cyc.lev[1].b, nullptr, 0.0, 1.0, odd);
+      } else {
+        cyc_down<VT, QT>(lev[0], S, 0, t, r, (V2*)a.cyc.lev[1].b, q, alpha, 1.0, odd);
+      }
       ++its;
       UA_TEAM_SYNC(t);
       const double rr = team_sum(part_rr + S.sl0, S.nsl, red[2]);

@@ -1769,6 +1769,7 @@ struct SysState {
   double r = 0, rForce = 0, rWork = 0, gamma = 1, ResidualReduction = 1e10;
   double r0 = 0, rForce0 = 0, rWork0 = 0, r1 = 0, rForce1 = 0, rWork1 = 0;
   int kits = 0;
+  double keta = 0;  // the tolerance they were for
   // K and R in the work buffers are those of the current iterate (assembled ahead, at the
   // cost evaluation that found the iterate), so the next Newton system needs no assembly
   bool kfresh = false;
@@ -1906,6 +1907,23 @@ static int record_updates(ua_mesh* m, const std::vector<ua_newton_report*>& rep,
   return UA_OK;
 }
 
+// Iterations expected of the selected systems' linear solves, the weights of the resident solve's
+// schedule: those of the last step scaled with the digits asked for (a Newton step's tolerance is
+// known before its solve), at first the fifth root of the size (P1 meshes of 1,653 and 79,800 nodes
+// took 6 and 13).  Weighted with the last step's count alone, a third of the CTAs of 16 meshes waited
+// for the systems whose tolerance had tightened.
+static void expected_steps(const ua_mesh* m, const std::vector<int>& sel, const std::vector<SysState>& st,
+                           const std::vector<double>& eta, std::vector<int>& its) {
+  auto digits = [](double e) { return std::max(0.1, -std::log(std::max(e, 1e-30))); };
+  for (size_t s = 0; s < sel.size(); ++s) {
+    its[s] = 0;
+    if (!sel[s]) continue;
+    const double n = st[s].kits ? st[s].kits * digits(eta[s]) / digits(st[s].keta)
+                                : std::pow((double)(m->h_dof_off[s + 1] - m->h_dof_off[s]), 0.2);
+    its[s] = std::max(1, (int)std::lround(std::min(n, 1e6)));
+  }
+}
+
 // One Newton iteration (SSTREAM2dNR2.m:157-392) of every active system.
 // *any is false when no system was active.
 static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_report*>& rep,
@@ -1957,10 +1975,9 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
     double t1 = now_ms();
     t_asm += t1 - t0;
     // linear solve (:242-257); a resident solve is not waited for: its counts come with the costs
-    // (the iterations of the last step weigh the systems in the solve's schedule)
-    for (int s = 0; s < nsys; ++s) its[s] = sel[s] ? std::max(1, st[s].kits) : 0;
     std::vector<double> eta(nsys);
     for (int s = 0; s < nsys; ++s) eta[s] = forcing_term(p, st[s].rForce);
+    expected_steps(m, sel, st, eta, its);
     const std::vector<int> solved = sel;
     w->defer = true;
     rc = linear_solve(m, p, its, eta.data());
@@ -1994,7 +2011,11 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
     if (!first) cost0();
     if ((rc = finish_deferred(m, its))) return rc;
     t_sol += now_ms() - t1;
-    for (int s = 0; s < nsys; ++s) if (solved[s]) st[s].kits = its[s];
+    for (int s = 0; s < nsys; ++s)
+      if (solved[s]) {
+        st[s].kits = its[s];
+        st[s].keta = eta[s];
+      }
     for (int s = 0; s < nsys; ++s) {
       if (!sel[s]) continue;
       SysState& S = st[s];
