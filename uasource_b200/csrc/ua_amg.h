@@ -1,5 +1,6 @@
 // Aggregation AMG preconditioner of the uv tangent (internal interface).
 #pragma once
+#include <cmath>
 #include "ua_internal.h"
 
 namespace ua {
@@ -138,6 +139,30 @@ struct PcgSolve {
 // sel: systems to solve; steps: expected iterations (the schedule's weights)
 int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, const std::vector<int>& steps, int nsm,
                  long long* launches);
+// Weights of the hsw l1-Jacobi sweeps on the thickness block: the Chebyshev polynomial of degree hsw on
+// [kHSweepLow, 1] (l1 scaling bounds the spectrum by one) as Richardson steps; more than kHSweepMax
+// sweeps repeat the polynomial of that degree, plain sweeps first.  A sweep is a pass with a barrier, so
+// the fewest that cost no iterations: P1 141x71, eight plain sweeps 309 iterations and 23.2 ms a step,
+// five weighted ones 309 and 20.6 (three: 321, 19.8); P2 101x51, 346 and 41.7 against 364 and 39.6 (three:
+// 423, 40.9).
+constexpr int kHSweepMax = 16, kHSweepDefault = 5;
+constexpr double kHSweepLow = 0.3;
+struct HSweeps {
+  int n;
+  double om[kHSweepMax];
+  __host__ __device__ double weight(int q) const {
+    const int first = n <= kHSweepMax ? 0 : n % kHSweepMax;
+    return q < first ? 1.0 : om[(q - first) % kHSweepMax];
+  }
+};
+inline HSweeps h_sweeps(int n) {
+  HSweeps h{};
+  h.n = n;
+  const int d = n < kHSweepMax ? n : kHSweepMax;
+  for (int k = 0; k < d; ++k)
+    h.om[k] = 1.0 / (0.5 * (1.0 + kHSweepLow) + 0.5 * (1.0 - kHSweepLow) * cos(3.14159265358979323846 * (2 * k + 1) / (2.0 * d)));
+  return h;
+}
 struct GmSolve {
   const int* rowptr;      // 3-dof CSR
   const double* K;
@@ -147,7 +172,8 @@ struct GmSolve {
   double* dX;             // in: the particular solution on the constrained dofs; out: the solution
   const double* tol;      // [nsys] relative tolerances
   int *done, *its;
-  int mr, hsw, maxit, max_cycles;
+  int mr, maxit, max_cycles;
+  HSweeps hsw;
 };
 // restarted GMRES of the uvh system (ua_gmres.cu), restart up to gmres_resident_max_restart()
 int gmres_resident_max_restart();
