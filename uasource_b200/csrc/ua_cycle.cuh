@@ -74,9 +74,15 @@ struct TeamCtx {
 // Arrive and wait.  The wait is bounded (some seconds): a team that does not meet returns false in
 // every thread and the kernel ends with an error status.
 constexpr unsigned kTeamSpinLimit = 1u << 24;
-__device__ __forceinline__ bool team_sync(TeamCtx& t) {
+// f: run by one thread of another warp meanwhile.
+template <typename F>
+__device__ __forceinline__ bool team_sync(TeamCtx& t, F f) {
   __syncthreads();
-  if (t.size == 1) return true;
+  if (threadIdx.x == 32) f();
+  if (t.size == 1) {
+    __syncthreads();
+    return true;
+  }
   if (threadIdx.x == 0) {
     t.target += t.size;
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
@@ -93,6 +99,13 @@ __device__ __forceinline__ bool team_sync(TeamCtx& t) {
   }
   __syncthreads();
   return *t.ok != 0;
+}
+__device__ __forceinline__ bool team_sync(TeamCtx& t) {
+  if (t.size == 1) {
+    __syncthreads();
+    return true;
+  }
+  return team_sync(t, []() {});
 }
 
 // Sum of n partials by the whole CTA, the same bits in every thread of every CTA: thread t adds

@@ -13,7 +13,7 @@ namespace ua {
 
 constexpr int kGmMaxRestart = 48;  // the triangular factor and the rotations live in shared memory
 constexpr int kGmSlab = 64;        // slices whose dot products are combined at a time
-constexpr int kGmArena = 190 * 1024, kGmArenaSmall = 64 * 1024;
+constexpr int kGmArena = 180 * 1024, kGmArenaSmall = 64 * 1024;
 
 // Slices per partial sum: at most 2048 partials of a dot product per system (every CTA of the team
 // reads them all), a function of the system's size alone.
@@ -182,83 +182,175 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
   return v[0];
 }
 
+constexpr int kGmUpd = 512;  // node partials of a split update: 4 x 128 or 2 x 256
 struct GmShared {
   double R[kGmMaxRestart * (kGmMaxRestart + 1) / 2];  // packed columns of the triangular factor
   double cs[kGmMaxRestart], sn[kGmMaxRestart], g[kGmMaxRestart + 1], y[kGmMaxRestart];
   double h1[kGmMaxRestart + 1], h2[kGmMaxRestart + 1];
   double slab[8][kGmSlab];
+  double upd[3 * kGmUpd];
   double scal[4];
   int flag;
 };
 
 // Dot products of w with the basis vectors 0 .. nv-1 (nv = 0: with itself) over the slices of the
-// CTA's units; one partial per vector and unit.  Within a Gram-Schmidt pass a
-// thread reads the entries of w that it wrote (the slices of a slab go to the warps like those of
-// the update: kGmSlab is a multiple of the warps); after a product the CTA has to meet first.
-static_assert(kGmSlab % kCycWarps == 0, "");
+// CTA's units; one partial per vector and unit.  w may have been written by other warps: the CTA meets
+// first.  With one slice a unit the warps take pairs (slice, eight vectors), so that a CTA with four
+// slices keeps all sixteen busy.
+__device__ __forceinline__ double gm_dot8(const GmArgs& a, int g, bool in, int nv, int c, int lane) {
+  double v[8];
+  double2 wu = make_double2(0, 0);
+  double wh = 0;
+  if (in) {
+    wu = a.w.uv[g];
+    wh = a.w.h[g];
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    v[k] = 0;
+    if (in && (nv ? 8 * c + k < nv : k == 0)) {
+      const GmVec b = nv ? gm_basis(a, 8 * c + k) : a.w;
+      const double2 bu = b.uv[g];
+      v[k] = wu.x * bu.x + wu.y * bu.y + wh * b.h[g];
+    }
+  }
+  return warp_sum8(v, lane);
+}
 __device__ __forceinline__ void gm_dots(const GmArgs& a, GmShared& sh, const CycSys& S, int U, int u0, int u1, int nv,
                                         double* part) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n0 = S.n0[0], nn = S.nn[0];
   const int chunks = nv ? (nv + 7) >> 3 : 1, per = max(1, kGmSlab / U);
+  __syncthreads();
+  if (U == 1) {
+    const int ns = u1 - u0;
+    for (int q = warp; q < ns * chunks; q += kCycWarps) {
+      const int c = q / ns, i = u0 + (q - c * ns);
+      const double t = gm_dot8(a, n0 + 32 * i + lane, 32 * i + lane < nn, nv, c, lane);
+      if ((lane & 3) == 0 && (nv ? 8 * c + (lane >> 2) < nv : lane == 0)) part[(8 * c + (lane >> 2)) * a.part_ld + i] = t;
+    }
+    return;
+  }
   for (int ub = u0; ub < u1; ub += per) {
     const int ue = min(ub + per, u1), s0 = ub * U, s1 = min(ue * U, S.nsl);
     for (int c = 0; c < chunks; ++c) {
       for (int i = s0 + warp; i < s1; i += kCycWarps) {
-        const int g = n0 + 32 * i + lane;
-        const bool in = 32 * i + lane < nn;
-        double v[8];
-        double2 wu = make_double2(0, 0);
-        double wh = 0;
-        if (in) {
-          wu = a.w.uv[g];
-          wh = a.w.h[g];
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          v[k] = 0;
-          if (in && (nv ? 8 * c + k < nv : k == 0)) {
-            const GmVec b = nv ? gm_basis(a, 8 * c + k) : a.w;
-            const double2 bu = b.uv[g];
-            v[k] = wu.x * bu.x + wu.y * bu.y + wh * b.h[g];
-          }
-        }
-        const double t = warp_sum8(v, lane);
-        if ((lane & 3) == 0) {
-          if (U > 1) sh.slab[lane >> 2][i - s0] = t;
-          else if (nv ? 8 * c + (lane >> 2) < nv : lane == 0) part[(8 * c + (lane >> 2)) * a.part_ld + i] = t;
-        }
+        const double t = gm_dot8(a, n0 + 32 * i + lane, 32 * i + lane < nn, nv, c, lane);
+        if ((lane & 3) == 0) sh.slab[lane >> 2][i - s0] = t;
       }
-      if (U > 1) {
-        __syncthreads();
-        const int nu = ue - ub;
-        for (int k = threadIdx.x; k < 8 * nu; k += kCycThreads) {
-          const int q = k / nu, u = k - q * nu;
-          if (!(nv ? 8 * c + q < nv : q == 0)) continue;
-          double t = 0;
-          for (int i = u * U; i < min((u + 1) * U, s1 - s0); ++i) t += sh.slab[q][i];
-          part[(8 * c + q) * a.part_ld + ub + u] = t;
-        }
-        __syncthreads();
+      __syncthreads();
+      const int nu = ue - ub;
+      for (int k = threadIdx.x; k < 8 * nu; k += kCycThreads) {
+        const int q = k / nu, u = k - q * nu;
+        if (!(nv ? 8 * c + q < nv : q == 0)) continue;
+        double t = 0;
+        for (int i = u * U; i < min((u + 1) * U, s1 - s0); ++i) t += sh.slab[q][i];
+        part[(8 * c + q) * a.part_ld + ub + u] = t;
       }
+      __syncthreads();
     }
   }
 }
-// totals of nv dot products, a warp each
+// totals of nv dot products: a warp takes three at a time, four partials of each in flight per lane
 __device__ __forceinline__ void gm_totals(const GmArgs& a, const double* part, int units, int nv, double* out) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = warp; i < nv; i += kCycWarps) {
-    double t = 0;
-#pragma unroll 4
-    for (int k = lane; k < units; k += 32) t += __ldcg(part + i * a.part_ld + k);
-    t = lane_sum(t, 32);
-    if (lane == 0) out[i] = t;
+  for (int i0 = warp; i0 < nv; i0 += 3 * kCycWarps) {
+    double t[3] = {0, 0, 0};
+    for (int k0 = lane; k0 < units; k0 += 128) {
+      double v[3][4];
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          v[q][k] = i0 + q * kCycWarps < nv && k0 + 32 * k < units
+                        ? __ldcg(part + (i0 + q * kCycWarps) * a.part_ld + k0 + 32 * k) : 0.0;
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) t[q] += v[q][k];
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      if (i0 + q * kCycWarps < nv) {  // uniform over the warp
+        const double s = lane_sum(t[q], 32);
+        if (lane == 0) out[i0 + q * kCycWarps] = s;
+      }
   }
   __syncthreads();
 }
 
-#define UA_TEAM_SYNC(t)                                               \
+// sum over the vectors q = r, r + 4, ... <= j of h[q] b_q at node k (class r of four)
+__device__ __forceinline__ void gm_class_sum(const GmArgs& a, const double* h, int r, int j, int k, double (&o)[3]) {
+  o[0] = o[1] = o[2] = 0;
+#pragma unroll 5
+  for (int q = r; q <= j; q += 4) {
+    const GmVec b = gm_basis(a, q);
+    const double2 bu = b.uv[k];
+    o[0] = fma(h[q], bu.x, o[0]);
+    o[1] = fma(h[q], bu.y, o[1]);
+    o[2] = fma(h[q], b.h[k], o[2]);
+  }
+}
+// w -= sum_q h[q] b_q on the slices [lo, hi) and, if asked for, ws = D^-1/2 w.  The vectors are summed in
+// four classes q mod 4, added as (0 + 2) + (1 + 3).  A CTA with at most four (eight) slices gives a class
+// (two) to a warp, so that a warp waits for ten basis vectors instead of forty one after the other.
+__device__ __forceinline__ void gm_update(const GmArgs& a, GmShared& sh, const double* h, int j, int lo, int hi, int n0,
+                                          int nn, bool scaled) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ns = hi - lo;
+  auto write = [&](int k, double s0, double s1, double s2) {
+    double2 wu = a.w.uv[k];
+    wu.x -= s0;
+    wu.y -= s1;
+    a.w.uv[k] = wu;
+    a.w.h[k] -= s2;
+    if (scaled) {
+      const double2 d = a.scp[k];
+      a.ws[k] = make_double2(d.x * wu.x, d.y * wu.y);
+    }
+  };
+  const int G = ns <= 4 ? 4 : ns <= 8 ? 2 : 1;
+  if (G == 1) {
+    for (int i = lo + warp; i < hi; i += kCycWarps) {
+      const int k = n0 + 32 * i + lane;
+      if (32 * i + lane < nn) {
+        double c0[3], c1[3], c2[3], c3[3];
+        gm_class_sum(a, h, 0, j, k, c0);
+        gm_class_sum(a, h, 2, j, k, c2);
+        gm_class_sum(a, h, 1, j, k, c1);
+        gm_class_sum(a, h, 3, j, k, c3);
+        write(k, (c0[0] + c2[0]) + (c1[0] + c3[0]), (c0[1] + c2[1]) + (c1[1] + c3[1]),
+              (c0[2] + c2[2]) + (c1[2] + c3[2]));
+      }
+    }
+    return;
+  }
+  const int per = kCycWarps / G, i = lo + warp % per, r = warp / per, nl = 32 * per;  // slots per class
+  if (i < hi && 32 * i + lane < nn) {
+    double c[3];
+    gm_class_sum(a, h, r, j, n0 + 32 * i + lane, c);
+    if (G == 2) {
+      double d[3];
+      gm_class_sum(a, h, r + 2, j, n0 + 32 * i + lane, d);
+      for (int q = 0; q < 3; ++q) c[q] += d[q];
+    }
+    const int at = r * nl + 32 * (i - lo) + lane;
+    for (int q = 0; q < 3; ++q) sh.upd[q * kGmUpd + at] = c[q];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 32 * ns; e += kCycThreads)
+    if (32 * lo + e < nn) {
+      double s[3];
+      for (int q = 0; q < 3; ++q) {
+        const double* u = sh.upd + q * kGmUpd + e;
+        s[q] = G == 2 ? u[0] + u[nl] : (u[0] + u[2 * nl]) + (u[nl] + u[3 * nl]);
+      }
+      write(n0 + 32 * lo + e, s[0], s[1], s[2]);
+    }
+}
+
+#define UA_TEAM_SYNC(t) UA_TEAM_SYNC_WITH(t, []() {})
+#define UA_TEAM_SYNC_WITH(t, ...)                                     \
   do {                                                                \
-    if (!team_sync(t)) {                                              \
+    if (!team_sync(t, __VA_ARGS__)) {                                            \
       if (threadIdx.x == 0) *a.cyc.err = 1;                           \
       return;                                                         \
     }                                                                 \
@@ -323,7 +415,6 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
         a.w.h[k] = a.fs.h[k] - kx[2];
         a.ws[k] = make_double2(d.x * r.x, d.y * r.y);
       });
-      __syncthreads();
       gm_dots(a, sh, S, U, u0, u1, 0, part3);
       UA_TEAM_SYNC(t);
       gm_totals(a, part3, units, 1, sh.scal);
@@ -402,46 +493,31 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
           a.w.uv[k] = make_double2(kx[0], kx[1]);
           a.w.h[k] = kx[2];
         });
-        __syncthreads();
         gm_dots(a, sh, S, U, u0, u1, j + 1, part1);
         UA_TEAM_SYNC(t);
         for (int pass = 0; pass < 2; ++pass) {
           double* h = pass ? sh.h2 : sh.h1;
           gm_totals(a, pass ? part2 : part1, units, j + 1, h);
-          for (int i = lo + warp; i < hi; i += kCycWarps) {
-            const int k = n0 + 32 * i + lane;
-            if (32 * i + lane < nn) {
-              double2 wu = a.w.uv[k];
-              double wh = a.w.h[k];
-#pragma unroll 4
-              for (int q = 0; q <= j; ++q) {
-                const GmVec b = gm_basis(a, q);
-                const double2 bu = b.uv[k];
-                wu.x = fma(-h[q], bu.x, wu.x);
-                wu.y = fma(-h[q], bu.y, wu.y);
-                wh = fma(-h[q], b.h[k], wh);
-              }
-              a.w.uv[k] = wu;
-              a.w.h[k] = wh;
-              if (pass) {
-                const double2 d = a.scp[k];
-                a.ws[k] = make_double2(d.x * wu.x, d.y * wu.y);
-              }
-            }
-          }
+          gm_update(a, sh, h, j, lo, hi, n0, nn, pass != 0);
           gm_dots(a, sh, S, U, u0, u1, pass ? 0 : j + 1, pass ? part3 : part2);
-          UA_TEAM_SYNC(t);
+          // the previous rotations of the new column, while the team gathers
+          UA_TEAM_SYNC_WITH(t, [&]() {
+            if (!pass) return;
+            double* R = sh.R + j * (j + 1) / 2;
+            double up = sh.h1[0] + sh.h2[0];
+            for (int i = 0; i < j; ++i) {
+              const double nx = sh.h1[i + 1] + sh.h2[i + 1];
+              R[i] = sh.cs[i] * up + sh.sn[i] * nx;
+              up = -sh.sn[i] * up + sh.cs[i] * nx;
+            }
+            sh.scal[2] = up;
+          });
         }
         gm_totals(a, part3, units, 1, sh.scal);
         if (threadIdx.x == 0) {
           double* R = sh.R + j * (j + 1) / 2;
           const double hn = sqrt(fmax(sh.scal[0], 0.0));
-          double up = sh.h1[0] + sh.h2[0];
-          for (int i = 0; i < j; ++i) {  // previous rotations
-            const double nx = sh.h1[i + 1] + sh.h2[i + 1];
-            R[i] = sh.cs[i] * up + sh.sn[i] * nx;
-            up = -sh.sn[i] * up + sh.cs[i] * nx;
-          }
+          const double up = sh.scal[2];
           const double den = hypot(up, hn);
           sh.cs[j] = den > 0 ? up / den : 1.0;
           sh.sn[j] = den > 0 ? hn / den : 0.0;
