@@ -127,8 +127,9 @@ struct CycLev {
   void *b, *z;              // right-hand side and result, one pair per node (levels >= 1)
 };
 // one system of the handle: first node and node count on every level, slices, dense inverse
+// solo: first level that every CTA of a team works through for itself (depth: none)
 struct CycSys {
-  int depth, dn, doff, sl0, nsl;
+  int depth, solo, dn, doff, sl0, nsl;
   int n0[kCycMaxLev + 1], nn[kCycMaxLev + 1];
 };
 // node slices of the finest level; columns are slice positions
@@ -182,6 +183,7 @@ struct Cycle {
   double *gm_buf = nullptr, *gm_part = nullptr, *gm_v3 = nullptr, *gm_hinv = nullptr;
   int gm_mr = 0;
   void* d_r2 = nullptr;       // second residual buffer
+  std::vector<double> h_solo[2];   // per system: bytes of its solo levels
   std::vector<double> h_bytes[2];  // per system: bytes of the matrices a step reads (FP64, mixed)
   int* h_stage = nullptr;     // pinned staging of the schedule
   long long nslices = 0;

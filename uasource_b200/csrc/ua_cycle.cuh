@@ -221,11 +221,11 @@ __device__ __forceinline__ void stage_slices(Arena& ar, int lo, int hi, int qb, 
 // small levels first.  In a team with enough CTAs everything fits: a pass then waits for one
 // gather of the vector instead of three dependent loads.  [slo, shi): the CTA's slices of the finest
 // level (the passes of that level visit no others).  Every thread keeps the same pointers;
-// thread 0 publishes them.
+// thread 0 publishes them.  room: the arena holds everything but, perhaps, the solo levels.
 template <typename KT, typename LT, typename QT>
 __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, const void* lv, const CycSys& S,
                                           const TeamCtx& t, int slo, int shi, Arena& ar, LevS* lev, FineS* fine, int kslot,
-                                          const double*& dense) {
+                                          const double*& dense, bool room) {
   constexpr int qb = 4 * sizeof(QT), ab = 4 * sizeof(KT);
   int lo, hi;
   dense = A.dense + S.doff;
@@ -233,7 +233,22 @@ __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, cons
     copy8(p, (const char*)dense, 8LL * S.dn * S.dn);
     dense = (const double*)p;
   }
-  for (int l = S.depth - 1; l >= 0; --l) {
+  // the solo levels whole: ahead of the rest where the finest rows stay in global memory, else with
+  // what room is left
+  const int solo = t.size > 1 ? S.solo : S.depth;
+  auto stage_solo = [&]() {
+    for (int l = S.depth - 1; l >= solo; --l) {
+      const CycLev& G = A.lev[l];
+      LevS L{G.aptr, G.acol, (const char*)G.aval, G.qptr, G.qoff, G.qcol, (const char*)G.qval,
+             G.tptr, G.tfine, (const char*)G.tval};
+      stage_csr(ar, S.n0[l + 1], S.n0[l + 1] + S.nn[l + 1], qb, L.tptr, L.tfine, L.tval);
+      stage_csr(ar, S.n0[l], S.n0[l] + S.nn[l], qb, L.qptr, L.qcol, L.qval);
+      stage_csr(ar, S.n0[l], S.n0[l] + S.nn[l], ab, L.aptr, L.acol, L.aval);
+      if (threadIdx.x == 0) lev[l] = L;
+    }
+  };
+  if (!room) stage_solo();
+  for (int l = solo - 1; l >= 0; --l) {
     const CycLev& G = A.lev[l];
     LevS L{G.aptr, G.acol, (const char*)G.aval, G.qptr, G.qoff, G.qcol, (const char*)G.qval,
            G.tptr, G.tfine, (const char*)G.tval};
@@ -275,6 +290,7 @@ __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, cons
         }
     }
   }
+  if (room) stage_solo();
   if (threadIdx.x == 0) *fine = F;
   __syncthreads();
 }
@@ -457,6 +473,45 @@ __device__ __forceinline__ void cyc_dense(const CycSys& S, const double* M, cons
   __syncthreads();
 }
 
+// The levels from S.solo on by every CTA of the team for itself: from b (global, level S.solo) to z_c of
+// that level in shared memory, without a team barrier.  Levels of at most kSoloNodes nodes: their rows are
+// some tens of kilobytes, the passes a few hundred cycles between CTA barriers, where a team barrier and
+// the hand-over of a level through L2 cost 2.2 us each (P1 141x71, levels of 10011, 1128, 80 and 7 nodes:
+// 25.5 -> 23.0 us a PCG step).  Same sums in the same order as by the team.
+// buf: twice the nodes of those levels and of the coarsest one.
+constexpr int kSoloNodes = 128;
+constexpr int kSoloBuf = 4 * kSoloNodes + kAmgCoarseNodes;  // cycle_init leaves out levels that do not fit
+template <typename VT, typename KT, typename QT>
+__device__ __forceinline__ const typename Vec2<VT>::T* cyc_solo(const LevS* lev, const CycSys& S, const CycArgs& A,
+                                                                const double* dense, DenseSh& dsh,
+                                                                typename Vec2<VT>::T* zcs,
+                                                                typename Vec2<VT>::T* buf) {
+  using V2 = typename Vec2<VT>::T;
+  const TeamCtx one{0, 1, nullptr, 0u, nullptr};
+  const int s0 = S.solo, dep = S.depth;
+  const V2* b0 = (const V2*)A.lev[s0].b + S.n0[s0];
+  for (int i = threadIdx.x; i < S.nn[s0]; i += kCycThreads) buf[i] = b0[i];
+  __syncthreads();
+  V2* b = buf;
+  for (int l = s0; l < dep; ++l) {
+    V2* bc = b + S.nn[l];
+    cyc_down<VT, QT>(lev[l], S, l, one, b - S.n0[l], bc - S.n0[l + 1]);
+    b = bc;
+    __syncthreads();
+  }
+  cyc_dense<VT>(S, dense, b - S.n0[dep], dsh, zcs);
+  V2* z = b + S.nn[dep];
+  const V2* zc = zcs - S.n0[dep];
+  for (int l = dep - 1; l >= s0; --l) {
+    b -= S.nn[l];
+    cyc_up<VT, KT, QT>(lev[l], S, l, one, b - S.n0[l], z - S.n0[l], zc);
+    __syncthreads();
+    zc = z - S.n0[l];
+    z += S.nn[l];
+  }
+  return zc;
+}
+
 // CH slots k0 .. of a slice product of width k1: the columns and values load
 // together, then the gathered pairs.  Slots past the end repeat the last one with a zero vector
 // entry, so that nothing branches between the loads.
@@ -567,6 +622,7 @@ struct CycSchedule {
 void cycle_schedule(const std::vector<CycSys>& sys, const std::vector<int>& sel, const std::vector<int>& steps,
                     int nsm, CycSchedule& out);
 int upload_schedule(ua_mesh* m, const CycSchedule& s);
+void arena_size(const Cycle& C, const CycSchedule& sch, bool fp32, int most, int small, int& bytes, bool& room);
 CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof);
 // cooperative launch of a team kernel, one CTA per SM
 template <typename A>

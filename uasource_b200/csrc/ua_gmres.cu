@@ -90,6 +90,7 @@ struct GmArgs {
   const double* tol;        // [nsys]
   int *done, *its;
   int arena;
+  bool room;
 };
 
 __device__ __forceinline__ GmVec gm_basis(const GmArgs& a, int i) {
@@ -137,7 +138,7 @@ __device__ __forceinline__ double gm_hrow(const CycFine& F, const double* v3, in
   const int* cp = F.cols + off + lane;
   const double* vp = v3 + 9 * off + lane + (B ? 256 : 192);
   double acc = 0;
-  constexpr int CH = 5;
+  constexpr int CH = B ? 10 : 7;
   for (int k0 = 0; k0 < k1; k0 += CH) {
     int j[CH];
     double e0[CH], e1[CH];
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
   __shared__ LevS lev[kCycMaxLev];
   __shared__ FineS fine;
   __shared__ DenseSh dsh;
-  __shared__ double2 zcs[kAmgMaxDense / 2];
+  __shared__ double2 zcs[kAmgMaxDense / 2], sbuf[kSoloBuf];
   __shared__ GmShared sh;
   __shared__ int ok;
   const int4 c = a.cyc.cta[blockIdx.x];
@@ -382,11 +383,12 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
     Arena ar{arena_mem, a.arena, 0};
     const double* dense;
     const int n0 = S.n0[0], nn = S.nn[0], dep = S.depth, U = gm_unit(S.nsl), units = (S.nsl + U - 1) / U;
+    const int solo = t.size > 1 ? S.solo : dep;
     const double2* bL = (const double2*)a.cyc.lev[dep].b;
     int u0, u1;
     team_share(t, units, u0, u1);
     const int lo = u0 * U, hi = min(u1 * U, S.nsl);
-    cyc_stage<double, double, double>(a.cyc, a.lv, a.lv, S, t, lo, hi, ar, lev, &fine, 32, dense);
+    cyc_stage<double, double, double>(a.cyc, a.lv, a.lv, S, t, lo, hi, ar, lev, &fine, 32, dense, a.room);
     // vectors into slice order
     for (int i = lo + warp; i < hi; i += kCycWarps)
       if (32 * i + lane < nn) {
@@ -442,13 +444,14 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
           }
         cyc_down<double, double>(lev[0], S, 0, t, a.ws, (double2*)a.cyc.lev[1].b, nullptr, 0.0, inv);
         UA_TEAM_SYNC(t);
-        for (int l = 1; l < dep; ++l) {
+        for (int l = 1; l < solo; ++l) {
           cyc_down<double, double>(lev[l], S, l, t, (const double2*)a.cyc.lev[l].b, (double2*)a.cyc.lev[l + 1].b);
           UA_TEAM_SYNC(t);
         }
-        cyc_dense<double>(S, dense, bL, dsh, zcs);
         const double2* zc = zcs - S.n0[dep];
-        for (int l = dep - 1; l > 0; --l) {
+        if (solo < dep) zc = cyc_solo<double, double, double>(lev, S, a.cyc, dense, dsh, zcs, sbuf);
+        else cyc_dense<double>(S, dense, bL, dsh, zcs);
+        for (int l = solo - 1; l > 0; --l) {
           cyc_up<double, double, double>(lev[l], S, l, t, (const double2*)a.cyc.lev[l].b, (double2*)a.cyc.lev[l].z, zc);
           UA_TEAM_SYNC(t);
           zc = (const double2*)a.cyc.lev[l].z;
@@ -670,14 +673,7 @@ int gmres_resident(ua_mesh* m, const GmSolve& v, const std::vector<int>& sel, co
   A.tol = v.tol;
   A.done = v.done;
   A.its = v.its;
-  double need = 0;
-  for (const int4& ct : sch.cta)
-    for (int k = ct.x; k < ct.y; ++k) {
-      const CycSys& y = C.sys[sch.queue[k]];
-      need = std::max(need, C.h_bytes[0][sch.queue[k]] / ct.w + 8.0 * y.dn * y.dn);
-    }
-  need = 1.15 * need + 8192;
-  A.arena = need <= kGmArena ? std::max(16384, (int)need) & ~15 : kGmArenaSmall;
+  arena_size(C, sch, false, kGmArena, kGmArenaSmall, A.arena, A.room);
   UA_CUDA_TRY(cudaFuncSetAttribute(k_gmres_team, cudaFuncAttributeMaxDynamicSharedMemorySize, kGmArena));
   const int rc = launch_team(m, k_gmres_team, A, (int)sch.cta.size(), A.arena);
   ++*launches;

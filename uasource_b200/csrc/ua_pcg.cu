@@ -19,7 +19,7 @@ namespace ua {
 // set-up: values of the collapsed cycle for a new tangent
 // ---------------------------------------------------------------------------
 
-constexpr int kCycArena = 212 * 1024;       // with the kernel's static tables below 227 KB
+constexpr int kCycArena = 208 * 1024;       // with the kernel's static tables below 227 KB
 constexpr int kCycArenaSmall = 64 * 1024;
 constexpr int kSplitSlices = 12;
 
@@ -203,6 +203,22 @@ bool cycle_supported(const ua_mesh* m) {
   return coop != 0;
 }
 
+// Shared memory for a schedule's copies: what its CTAs' rows need, and their solo levels as far as the
+// maximum allows; rows that do not fit are left to L1 and L2.
+void arena_size(const Cycle& C, const CycSchedule& sch, bool fp32, int most, int small, int& bytes, bool& room) {
+  double need = 0, solo = 0;
+  for (const int4& ct : sch.cta)
+    for (int k = ct.x; k < ct.y; ++k) {
+      const int s = sch.queue[k];
+      const CycSys& y = C.sys[s];
+      need = std::max(need, (C.h_bytes[fp32][s] + (ct.w == 1 ? C.h_solo[fp32][s] : 0.0)) / ct.w + 8.0 * y.dn * y.dn);
+      if (ct.w > 1) solo = std::max(solo, C.h_solo[fp32][s] + 8192);
+    }
+  need = 1.15 * need + 8192;
+  room = need <= most;
+  bytes = room ? std::max(16384, (int)std::min((double)most, need + solo)) & ~15 : small;
+}
+
 // Lists and buffers of the collapsed cycle, once per handle (the node slices of the finest level
 // must be there).
 int cycle_init(ua_mesh* m) {
@@ -275,6 +291,7 @@ int cycle_init(ua_mesh* m) {
       D.tpos = upload(m, a, tpos, ok);
       for (int w = 0; w < 2; ++w) {  // bytes a step reads of this level (FP64, mixed form)
         C.h_bytes[w].resize(nsys, 0.0);
+        C.h_solo[w].resize(nsys, 0.0);
         for (int s = 0; s < nsys; ++s) {
           const int g0 = L.node_off[s], g1 = L.node_off[s + 1];
           if (g1 == g0) continue;
@@ -284,7 +301,7 @@ int cycle_init(ua_mesh* m) {
                  (w ? 28 : 36);
           else
             b += (double)(a->h_gptr[l][g1] - a->h_gptr[l][g0]) * (w ? 20 : 36);
-          C.h_bytes[w][s] += b + 8.0 * (g1 - g0);
+          (l > 0 && g1 - g0 <= kSoloNodes ? C.h_solo : C.h_bytes)[w][s] += b + 8.0 * (g1 - g0);
         }
       }
     }
@@ -293,7 +310,7 @@ int cycle_init(ua_mesh* m) {
   for (int s = 0; s < nsys; ++s) {
     CycSys& S = C.sys[s];
     std::memset(&S, 0, sizeof(S));
-    S.depth = a->depth[s];
+    S.depth = S.solo = a->depth[s];
     S.dn = a->h_dn[s];
     S.doff = a->h_doff[s];
     S.sl0 = kSellSlices * a->sell.h_sys_sb_off[s];
@@ -302,6 +319,10 @@ int cycle_init(ua_mesh* m) {
       S.nn[l] = a->lev[l].node_off[s + 1] - S.n0[l];
     }
     S.nsl = (S.nn[0] + 31) / 32;
+    for (int b = S.nn[S.depth]; S.solo > 1 && S.nn[S.solo - 1] <= kSoloNodes; --S.solo) {
+      b += 2 * S.nn[S.solo - 1];
+      if (b > kSoloBuf) break;
+    }
   }
   C.d_sys = upload(m, a, C.sys, ok);
   C.nslices = (long long)kSellSlices * a->sell.nsb;
@@ -579,6 +600,7 @@ struct PcgArgs {
   int *done, *its, *status;
   int maxit;
   int arena;                 // dynamic shared memory for copies of the matrices
+  bool room;                 // it holds every system's rows (solo levels apart)
 };
 
 // The whole PCG of the systems in the team's queue.  The passes of a step, a team barrier after
@@ -599,7 +621,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
   __shared__ FineS fine;
   __shared__ double red[3][32];
   __shared__ DenseSh dsh;
-  __shared__ V2 zcs[kAmgMaxDense / 2];
+  __shared__ V2 zcs[kAmgMaxDense / 2], sbuf[kSoloBuf];
   __shared__ int ok;
   const int4 c = a.cyc.cta[blockIdx.x];
   TeamCtx t{c.z, c.w, a.cyc.bar + 32 * a.cyc.team[blockIdx.x], 0u, &ok};
@@ -626,8 +648,8 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
     const double* dense;
     int lo, hi;
     team_share(t, S.nsl, lo, hi);
-    cyc_stage<KT, LT, QT>(a.cyc, a.kv, a.lv, S, t, lo, hi, ar, lev, &fine, 4 * sizeof(KT), dense);
-    const int n0 = S.n0[0], nn = S.nn[0], dep = S.depth;
+    cyc_stage<KT, LT, QT>(a.cyc, a.kv, a.lv, S, t, lo, hi, ar, lev, &fine, 4 * sizeof(KT), dense, a.room);
+    const int n0 = S.n0[0], nn = S.nn[0], dep = S.depth, solo = t.size > 1 ? S.solo : dep;
     const bool stream = fine.cols == a.cyc.fine.cols;  // rows read from global memory
     // restrict the updated residual after one more barrier, or b - alpha q from the two old vectors:
     // the second gather costs more than the barrier once a CTA has kSplitSlices slices
@@ -654,13 +676,14 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
     while (rr0 != 0.0) {
       const bool odd = its & 1;
       // z = cycle(r), the finest restriction done
-      for (int l = 1; l < dep; ++l) {
+      for (int l = 1; l < solo; ++l) {
         cyc_down<VT, QT>(lev[l], S, l, t, (const V2*)a.cyc.lev[l].b, (V2*)a.cyc.lev[l + 1].b);
         UA_TEAM_SYNC(t);
       }
-      cyc_dense<VT>(S, dense, bL, dsh, zcs);
       const V2* zc = zcs - S.n0[dep];
-      for (int l = dep - 1; l > 0; --l) {
+      if (solo < dep) zc = cyc_solo<VT, KT, QT>(lev, S, a.cyc, dense, dsh, zcs, sbuf);
+      else cyc_dense<VT>(S, dense, bL, dsh, zcs);
+      for (int l = solo - 1; l > 0; --l) {
         cyc_up<VT, KT, QT>(lev[l], S, l, t, (const V2*)a.cyc.lev[l].b, (V2*)a.cyc.lev[l].z, zc);
         UA_TEAM_SYNC(t);
         zc = (const V2*)a.cyc.lev[l].z;
@@ -801,14 +824,7 @@ int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, con
   A.r2 = C.d_r2;
   // shared memory for the copies: all of it where the largest share of a CTA fits, else what the
   // small levels take (the rest serves as L1 for the streamed rows)
-  double need = 0;
-  for (const int4& ct : sch.cta)
-    for (int k = ct.x; k < ct.y; ++k) {
-      const CycSys& y = C.sys[sch.queue[k]];
-      need = std::max(need, C.h_bytes[v.fp32][sch.queue[k]] / ct.w + 8.0 * y.dn * y.dn);
-    }
-  need = 1.15 * need + 8192;
-  A.arena = need <= kCycArena ? std::max(16384, (int)need) & ~15 : kCycArenaSmall;
+  arena_size(C, sch, v.fp32, kCycArena, kCycArenaSmall, A.arena, A.room);
   A.z = v.z;
   A.p = v.p;
   A.q = v.q;
