@@ -122,13 +122,13 @@ void cycle_fill_fine(ua_mesh* m, const int* colind0, const void* K0, bool fp32, 
 void cycle_fill_levels(ua_mesh* m, bool fp32, const int* sel, cudaStream_t st, long long* launches);
 struct PcgSolve {
   bool fp32, lo, prof;
-  const int *rb_start, *rb_sys;
-  int nrb;
   const int* sel;
-  const int *rowptr, *colind;
+  const int* colind;
   const void* K;
   const double* f;        // right-hand side (dofs)
-  double* dX;             // in: the particular solution on the constrained dofs; out: the solution
+  const int* dof_con;     // dof -> single-dof constraint or -1, with right-hand sides con_rhs at X + dX
+  const double *con_rhs, *X;
+  double *dX, *grhs;      // out: the solution; con_rhs - X
   void *r, *z, *p, *q;    // work, one pair per node in the value precision
   double* x;              // work, one FP64 pair per node
   const void* dw;

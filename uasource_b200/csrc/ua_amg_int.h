@@ -172,12 +172,11 @@ struct Cycle {
   // resident kernel: schedule (one int4 per CTA: queue begin, end, team rank, team size), queue,
   // team counters, per-slice partials, profile clocks
   int last_grid = 0;
-  int4* d_cta = nullptr;
-  int *d_queue = nullptr, *d_team = nullptr;
-  unsigned* d_bar = nullptr;
+  // one block uploaded per solve: error flag, per-CTA entries, teams, queue, barrier counters (zeros)
+  int* d_sched = nullptr;
+  int at_team = 0, at_queue = 0, at_bar = 0;
   double* d_part = nullptr;   // [3][slices]
   unsigned long long* d_prof = nullptr;
-  int* d_err = nullptr;
   int *d_ipos = nullptr, *d_pcol = nullptr;  // node -> slice position; slot columns as positions
   // uvh: basis and work vectors, partials, 3-dof tangent and inverse thickness l1 sums (slice order)
   double *gm_buf = nullptr, *gm_part = nullptr, *gm_v3 = nullptr, *gm_hinv = nullptr;

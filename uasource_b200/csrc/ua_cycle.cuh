@@ -174,13 +174,23 @@ struct Arena {
     return p;
   }
 };
-__device__ __forceinline__ void copy8(char* d, const char* s, long long bytes) {
-  for (long long i = threadIdx.x; i < bytes / 8; i += kCycThreads)
-    reinterpret_cast<uint2*>(d)[i] = reinterpret_cast<const uint2*>(s)[i];
+// Copies of global memory into the arena, asynchronous so that a stage waits once for all of them
+// (stage_wait); in the widest pieces the addresses allow.
+__device__ __forceinline__ void copy_in(void* d, const void* s, long long bytes) {
+  const unsigned sd = (unsigned)__cvta_generic_to_shared(d);
+  const char* p = (const char*)s;
+  const unsigned long long al = (unsigned long long)p | (unsigned long long)sd | (unsigned long long)bytes;
+  if (!(al & 15))
+    for (long long i = 16LL * threadIdx.x; i < bytes; i += 16 * kCycThreads)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sd + (unsigned)i), "l"(p + i) : "memory");
+  else if (!(al & 7))
+    for (long long i = 8LL * threadIdx.x; i < bytes; i += 8 * kCycThreads)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sd + (unsigned)i), "l"(p + i) : "memory");
+  else
+    for (long long i = 4LL * threadIdx.x; i < bytes; i += 4 * kCycThreads)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sd + (unsigned)i), "l"(p + i) : "memory");
 }
-__device__ __forceinline__ void copy4(int* d, const int* s, long long n) {
-  for (long long i = threadIdx.x; i < n; i += kCycThreads) d[i] = s[i];
-}
+__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // rows [lo, hi) of a node-CSR matrix with quads of qb bytes
 __device__ __forceinline__ void stage_csr(Arena& ar, int lo, int hi, int qb, const int*& ptr, const int*& col,
                                           const char*& val) {
@@ -191,9 +201,9 @@ __device__ __forceinline__ void stage_csr(Arena& ar, int lo, int hi, int qb, con
   char* pv = p;  // values first (16-byte aligned), then columns, then row pointers
   int* pc = reinterpret_cast<int*>(p + (((long long)(e1 - e0) * qb + 15) & ~15LL));
   int* pp = pc + (e1 - e0);
-  copy8(pv, val + (long long)e0 * qb, (long long)(e1 - e0) * qb);
-  copy4(pc, col + e0, e1 - e0);
-  copy4(pp, ptr + lo, hi - lo + 1);
+  copy_in(pv, val + (long long)e0 * qb, (long long)(e1 - e0) * qb);
+  copy_in(pc, col + e0, 4LL * (e1 - e0));
+  copy_in(pp, ptr + lo, 4LL * (hi - lo + 1));
   ptr = pp - lo;
   col = pc - e0;
   val = pv - (long long)e0 * qb;
@@ -209,9 +219,9 @@ __device__ __forceinline__ void stage_slices(Arena& ar, int lo, int hi, int qb, 
   long long* po = reinterpret_cast<long long*>(p);
   char* pv = p + ((8LL * (hi - lo + 1) + 15) & ~15LL);  // slots come in blocks of 32: 16-byte aligned
   int* pc = reinterpret_cast<int*>(pv + ne * qb);
-  for (int i = threadIdx.x; i <= hi - lo; i += kCycThreads) po[i] = off[lo + i];
-  copy8(pv, val + e0 * qb, ne * qb);
-  copy4(pc, col + e0, ne);
+  copy_in(po, off + lo, 8LL * (hi - lo + 1));
+  copy_in(pv, val + e0 * qb, ne * qb);
+  copy_in(pc, col + e0, 4 * ne);
   off = po - lo;
   col = pc - e0;
   val = pv - e0 * qb;
@@ -230,7 +240,7 @@ __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, cons
   int lo, hi;
   dense = A.dense + S.doff;
   if (char* p = ar.take(8LL * S.dn * S.dn)) {
-    copy8(p, (const char*)dense, 8LL * S.dn * S.dn);
+    copy_in(p, dense, 8LL * S.dn * S.dn);
     dense = (const double*)p;
   }
   // the solo levels whole: ahead of the rest where the finest rows stay in global memory, else with
@@ -272,26 +282,27 @@ __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, cons
     if (char* p = ar.take(ne * 4 + 8LL * (ns + 1))) {
       long long* po = reinterpret_cast<long long*>(p);
       int* pc = reinterpret_cast<int*>(po + ns + 1);
-      for (int i = threadIdx.x; i <= ns; i += kCycThreads) po[i] = F.sl_off[s0 + i];
-      copy4(pc, F.cols + e0, ne);
+      copy_in(po, F.sl_off + s0, 8LL * (ns + 1));
+      copy_in(pc, F.cols + e0, 4 * ne);
       F.sl_off = po - s0;
       F.cols = pc - e0;
       const int lb = 4 * sizeof(LT);
       if (char* q = ar.take(ne * lb)) {
-        copy8(q, F.lv + e0 * lb, ne * lb);
+        copy_in(q, F.lv + e0 * lb, ne * lb);
         const bool same = F.kv == F.lv;
         F.lv = q - e0 * lb;
         if (same) F.kv = F.lv;
       }
       if (kv != lv)
         if (char* q = ar.take(ne * kslot)) {
-          copy8(q, F.kv + e0 * kslot, ne * kslot);
+          copy_in(q, F.kv + e0 * kslot, ne * kslot);
           F.kv = q - e0 * kslot;
         }
     }
   }
   if (room) stage_solo();
   if (threadIdx.x == 0) *fine = F;
+  stage_wait();
   __syncthreads();
 }
 

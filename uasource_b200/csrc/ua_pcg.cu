@@ -219,6 +219,9 @@ void arena_size(const Cycle& C, const CycSchedule& sch, bool fp32, int most, int
   bytes = room ? std::max(16384, (int)std::min((double)most, need + solo)) & ~15 : small;
 }
 
+// the schedule's block for up to 1024 CTAs
+static size_t sched_ints(int nsys) { return 4 + 5 * 1024 + (size_t)nsys + 32 + 32 * 1024; }
+
 // Lists and buffers of the collapsed cycle, once per handle (the node slices of the finest level
 // must be there).
 int cycle_init(ua_mesh* m) {
@@ -327,13 +330,9 @@ int cycle_init(ua_mesh* m) {
   C.d_sys = upload(m, a, C.sys, ok);
   C.nslices = (long long)kSellSlices * a->sell.nsb;
   C.d_part = (double*)dalloc(m, a, sizeof(double) * 3 * (size_t)std::max(C.nslices, 1LL), ok);
-  C.d_cta = (int4*)dalloc(m, a, sizeof(int4) * 1024, ok);
-  C.d_team = (int*)dalloc(m, a, sizeof(int) * 1024, ok);
-  C.d_queue = (int*)dalloc(m, a, sizeof(int) * (size_t)nsys, ok);
-  C.d_bar = (unsigned*)dalloc(m, a, sizeof(unsigned) * 32 * 1024, ok);
+  C.d_sched = (int*)dalloc(m, a, sizeof(int) * sched_ints(nsys), ok);
   C.d_prof = (unsigned long long*)dalloc(m, a, sizeof(unsigned long long) * 2 * CP_COUNT, ok);
-  C.d_err = (int*)dalloc(m, a, sizeof(int), ok);
-  if (ok && cudaMallocHost(&C.h_stage, sizeof(int) * (5 * 1024 + (size_t)nsys)) != cudaSuccess) ok = false;
+  if (ok && cudaMallocHost(&C.h_stage, sizeof(int) * sched_ints(nsys)) != cudaSuccess) ok = false;
   if (!ok) {
     C.failed = true;
     return set_error(UA_ERR_OOM, "collapsed cycle: allocation failed");
@@ -508,14 +507,15 @@ int upload_schedule(ua_mesh* m, const CycSchedule& s) {
   Cycle& C = m->amg->cyc;
   const int nc = (int)s.cta.size(), nq = (int)s.queue.size();
   if (nc > 1024) return set_error(UA_ERR_INVALID, "resident solve: schedule of %d CTAs", nc);
-  std::memcpy(C.h_stage, s.cta.data(), sizeof(int4) * nc);
-  std::memcpy(C.h_stage + 4 * 1024, s.team.data(), sizeof(int) * nc);
-  std::memcpy(C.h_stage + 5 * 1024, s.queue.data(), sizeof(int) * nq);
-  UA_CUDA_TRY(cudaMemcpyAsync(C.d_cta, C.h_stage, sizeof(int4) * nc, cudaMemcpyHostToDevice, m->stream));
-  UA_CUDA_TRY(cudaMemcpyAsync(C.d_team, C.h_stage + 4 * 1024, sizeof(int) * nc, cudaMemcpyHostToDevice, m->stream));
-  UA_CUDA_TRY(cudaMemcpyAsync(C.d_queue, C.h_stage + 5 * 1024, sizeof(int) * nq, cudaMemcpyHostToDevice, m->stream));
-  UA_CUDA_TRY(cudaMemsetAsync(C.d_bar, 0, sizeof(unsigned) * 32 * (size_t)(s.team.back() + 1), m->stream));
-  UA_CUDA_TRY(cudaMemsetAsync(C.d_err, 0, sizeof(int), m->stream));
+  C.at_team = 4 + 4 * nc;
+  C.at_queue = C.at_team + nc;
+  C.at_bar = (C.at_queue + nq + 31) & ~31;
+  const int n = C.at_bar + 32 * (s.team.back() + 1);
+  std::memset(C.h_stage, 0, sizeof(int) * n);
+  std::memcpy(C.h_stage + 4, s.cta.data(), sizeof(int4) * nc);
+  std::memcpy(C.h_stage + C.at_team, s.team.data(), sizeof(int) * nc);
+  std::memcpy(C.h_stage + C.at_queue, s.queue.data(), sizeof(int) * nq);
+  UA_CUDA_TRY(cudaMemcpyAsync(C.d_sched, C.h_stage, sizeof(int) * n, cudaMemcpyHostToDevice, m->stream));
   return UA_OK;
 }
 
@@ -533,11 +533,11 @@ CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof) {
   A.fine = CycFine{a->sell.perm, a->sell.sl_off, C.d_pcol};
   A.sys = C.d_sys;
   A.dense = a->dense;
-  A.cta = C.d_cta;
-  A.team = C.d_team;
-  A.queue = C.d_queue;
-  A.bar = C.d_bar;
-  A.err = C.d_err;
+  A.cta = (const int4*)(C.d_sched + 4);
+  A.team = C.d_sched + C.at_team;
+  A.queue = C.d_sched + C.at_queue;
+  A.bar = (unsigned*)(C.d_sched + C.at_bar);
+  A.err = C.d_sched;
   A.prof = prof ? C.d_prof : nullptr;
   A.part = C.d_part;
   A.nslices = C.nslices;
@@ -548,34 +548,54 @@ CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof) {
 // device: PCG
 // ---------------------------------------------------------------------------
 
-// First residual in scaled form: r = D^-1/2 mask(f - K x0), LPR lanes per dof row.
-template <typename KT, typename VT, int LPR>
-__global__ void __launch_bounds__(256) k_cyc_r0(const int* rb_start, const int* rb_sys, const int* sel,
-                                                const int* node_off, const int* dof_off, const int* rowptr,
-                                                const int* colind, const KT* K, const double* x0, const double* f,
-                                                const double2* sc, const int* ipos, VT* r) {
-  const int blk = blockIdx.x, s = rb_sys[blk];
-  if (!sel[s]) return;
-  const int rs = rb_start[blk], re = rb_start[blk + 1];
-  const int no = node_off[s], nn = node_off[s + 1] - no, d0 = dof_off[s];
-  const int lane = threadIdx.x % LPR, grp = threadIdx.x / LPR, ngrp = blockDim.x / LPR;
-  for (int row0 = rs; row0 < re; row0 += ngrp) {
-    const int row = row0 + grp;
-    const bool valid = row < re;
-    double acc = 0;
-    if (valid)
-      for (int j = rowptr[row] + lane; j < rowptr[row + 1]; j += LPR) {
-        const double x = x0[colind[j]];
-        if (x != 0) acc += (double)K[j] * x;
-      }
-#pragma unroll
-    for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, LPR);
-    if (valid && lane == 0) {
-      const int i = row - d0, c = i >= nn ? 1 : 0, g = no + i - c * nn;
-      const double2 d = sc[g];
-      const double w = c ? d.y : d.x;
-      r[2 * (size_t)ipos[g] + c] = (VT)(w > 0 ? w * (f[row] - acc) : 0.0);
+// Start of a solve, four lanes per node: the particular solution on the constrained dofs (x0 = rhs - X
+// there, else zero) into dX and grhs, and the first residual in scaled form, r = D^-1/2 mask(f - K x0).
+// The neighbours' x0 are worked out anew from their constraints, so that zeroing dX, the particular
+// solution and the residual are one launch; a row's entries of K are read only beside a constrained dof
+// that moves.  Bound by the loads' latency: P1 141x71 7.4 us (three launches: 23 us), P2 401x201
+// 36 us (60 us).
+template <typename KT, typename VT>
+__global__ void __launch_bounds__(256) k_cyc_r0(int n, const int4* nrow, const int* node_off, const int* dof_off,
+                                                const int* colind, const KT* K, const int* dof_con,
+                                                const double* con_rhs, const double* X, const double* f,
+                                                const double2* sc, const int* ipos, VT* r, double* dX, double* grhs,
+                                                const int* sel) {
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, lane = threadIdx.x & 3;
+  if (g >= n) return;  // whole groups
+  const int4 q = nrow[g];
+  if (!sel[q.w]) return;
+  const int no = node_off[q.w], nn = node_off[q.w + 1] - no, i0 = dof_off[q.w] + (g - no), i1 = i0 + nn;
+  auto x0 = [&](int d) {
+    const int c = dof_con[d];
+    return c >= 0 ? con_rhs[c] - X[d] : 0.0;
+  };
+  double a0 = 0, a1 = 0;
+  for (int k = lane; k < q.z; k += 4) {
+    const int j = colind[q.x + k];
+    const double xu = x0(j), xv = x0(j + nn);
+    if (xu != 0) {
+      a0 += (double)K[q.x + k] * xu;
+      a1 += (double)K[q.y + k] * xu;
     }
+    if (xv != 0) {
+      a0 += (double)K[q.x + q.z + k] * xv;
+      a1 += (double)K[q.y + q.z + k] * xv;
+    }
+  }
+  const unsigned gmask = 0xfu << (threadIdx.x & 28);
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) {
+    a0 += __shfl_xor_sync(gmask, a0, o, 4);
+    a1 += __shfl_xor_sync(gmask, a1, o, 4);
+  }
+  if (lane < 2) {
+    const int i = lane ? i1 : i0, c = dof_con[i];
+    const double x = c >= 0 ? con_rhs[c] - X[i] : 0.0;
+    dX[i] = x;
+    if (c >= 0) grhs[c] = x;
+    const double2 d = sc[g];
+    const double w = lane ? d.y : d.x;
+    r[2 * (size_t)ipos[g] + lane] = (VT)(w > 0 ? w * (f[i] - (lane ? a1 : a0)) : 0.0);
   }
 }
 
@@ -838,15 +858,16 @@ int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, con
   A.its = v.its;
   A.status = v.status;
   A.maxit = v.maxit;
-  const int lpr_grid = v.nrb;
+  const AmgLevel& L0 = a->lev[0];
+  const int nb = std::max(1, (L0.nn + 63) / 64);
   if (v.fp32)
-    k_cyc_r0<float, float, 4><<<lpr_grid, 256, 0, m->stream>>>(
-        v.rb_start, v.rb_sys, v.sel, a->lev[0].d_node_off, a->lev[0].d_dof_off, v.rowptr, v.colind,
-        (const float*)v.K, v.dX, v.f, C.lev[0].sc, C.d_ipos, (float*)v.r);
+    k_cyc_r0<float, float><<<nb, 256, 0, m->stream>>>(L0.nn, L0.nrow, L0.d_node_off, L0.d_dof_off, v.colind,
+                                                      (const float*)v.K, v.dof_con, v.con_rhs, v.X, v.f, C.lev[0].sc,
+                                                      C.d_ipos, (float*)v.r, v.dX, v.grhs, v.sel);
   else
-    k_cyc_r0<double, double, 4><<<lpr_grid, 256, 0, m->stream>>>(
-        v.rb_start, v.rb_sys, v.sel, a->lev[0].d_node_off, a->lev[0].d_dof_off, v.rowptr, v.colind,
-        (const double*)v.K, v.dX, v.f, C.lev[0].sc, C.d_ipos, (double*)v.r);
+    k_cyc_r0<double, double><<<nb, 256, 0, m->stream>>>(L0.nn, L0.nrow, L0.d_node_off, L0.d_dof_off, v.colind,
+                                                        (const double*)v.K, v.dof_con, v.con_rhs, v.X, v.f,
+                                                        C.lev[0].sc, C.d_ipos, (double*)v.r, v.dX, v.grhs, v.sel);
   ++*launches;
   UA_CUDA_TRY(cudaGetLastError());
   const int nc = C.last_grid = (int)sch.cta.size();
@@ -858,14 +879,14 @@ int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, con
   return rc;
 }
 
-const int* resident_error_flag(const ua_mesh* m) { return m->amg->cyc.d_err; }
+const int* resident_error_flag(const ua_mesh* m) { return m->amg->cyc.d_sched; }
 
 // After the solve's stream has drained: whether every barrier was met, and the pass times (ms of
 // the whole grid) and counts of a profiled solve.
 int pcg_resident_status(ua_mesh* m, bool prof, double* ms, int* cnt) {
   Cycle& C = m->amg->cyc;
   int err = 0;
-  UA_CUDA_TRY(cudaMemcpy(&err, C.d_err, sizeof(int), cudaMemcpyDeviceToHost));
+  UA_CUDA_TRY(cudaMemcpy(&err, C.d_sched, sizeof(int), cudaMemcpyDeviceToHost));
   if (err) return set_error(UA_ERR_TIMEOUT, "resident solve: a team barrier was not met");
   if (prof) {
     unsigned long long h[2 * CP_COUNT];

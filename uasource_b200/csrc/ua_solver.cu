@@ -1443,10 +1443,10 @@ static int pcg_resident_solve(ua_mesh* m, const ua_params* p, bool fp32, const v
   v.fp32 = fp32;
   v.lo = fp32 && p->precond_bf16;
   v.prof = w->prof.on;
-  v.rb_start = w->rb_start; v.rb_sys = w->rb_sys; v.nrb = w->nrb;
   v.sel = w->sel;
-  v.rowptr = w->rowptr; v.colind = w->colind; v.K = K;
+  v.colind = w->colind; v.K = K;
   v.f = w->frhs; v.dX = w->dX;
+  v.dof_con = w->dof_con; v.con_rhs = w->con_rhs; v.X = w->X; v.grhs = w->grhs;
   v.r = w->kr; v.z = w->kz; v.p = w->kp; v.q = w->kq;
   v.x = (double*)w->kx0;
   v.dw = w->invd;
@@ -1540,12 +1540,12 @@ static int pcg_t(ua_mesh* m, const ua_params* p, const KT* K, int* its_out, cons
   } else {
     k_invdiag<KT, VT><<<(N + 255) / 256, 256, 0, m->stream>>>(N, K, w->diagpos, w->cmask, (VT*)w->invd), ++g_launches;
   }
+  if (res) return pcg_resident_solve(m, p, fp32, K, its_out);
   // particular solution on the constrained dofs
   k_zero_sel<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->dX), ++g_launches;
   if (w->nc)
     k_con_particular<<<(w->nc + 255) / 256, 256, 0, m->stream>>>(w->nc, w->con_dof, w->con_sys, w->sel, w->con_rhs,
                                                                  w->X, w->dX, w->grhs, con_pairs(w)), ++g_launches;
-  if (res) return pcg_resident_solve(m, p, fp32, K, its_out);
   VT *r = (VT*)w->kr, *z = (VT*)w->kz, *pp = (VT*)w->kp, *q = (VT*)w->kq;
   // with AMG the Jacobi-type kernels write the l1 pre-smoothed vector x0 and the V-cycle writes z (and r.z)
   const VT* invd = amg ? (const VT*)amg_invd0(m) : (const VT*)w->invd;
