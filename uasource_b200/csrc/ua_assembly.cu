@@ -428,9 +428,12 @@ enum { ND_X = 0, ND_Y, ND_H, ND_BL, ND_U, ND_V, ND_C, ND_A, ND_HB, ND_RHO, ND_M,
 enum { PR_UU = 0, PR_UUC, PR_VV, PR_VVC, PR_UV1, PR_UV2, PR_XV, PR_TX, PR_TY, PR_PX, PR_PY, PR_TN, PR_FN, kPairs };
 }  // namespace p2
 
-template <typename KT, bool GEN, int CTAS>
-__global__ void __launch_bounds__(CTAS == 2 ? 256 : 6 * p2::kMaxG, CTAS) uv_p2_kernel(DevMesh M, QuadTable Q, UvPhys P, UvIn in, UvOut out,
-                                                                 int G) {
+// One build for both launch shapes (128 registers): builds with other budgets round differently, and K and
+// R must not depend on the patches (a build of 168 for the one-CTA shape was 3% faster on P2 401x201, 763
+// against 790 us).
+template <typename KT, bool GEN>
+__global__ void __launch_bounds__(512) uv_p2_kernel(DevMesh M, QuadTable Q, UvPhys P, UvIn in,
+                                                                               UvOut out, int G) {
   using namespace p2;
   using p1::tanh_step;
   using I = ElemIdx<6>;
@@ -679,7 +682,7 @@ static cudaError_t launch_p2(const ua_mesh* m, const UvPhys& P, const UvIn& in, 
   const size_t base = uv_p2_smem_base(out.K != nullptr, sizeof(KT) == 4, E, m->dm.max_patch_hnodes);
   if (base + kP2Point > kLimit) return cudaErrorInvalidConfiguration;
   // elements of a group: what the shared memory of half an SM takes if that is 12 or more (two CTAs
-  // of 128 registers hide each other's staging and barriers), else of the whole one (one CTA of 168)
+  // hide each other's staging and barriers), else of the whole one
   int G = base < kHalf ? (int)((kHalf - base) / kP2Point) : 0;
   const bool two = G >= std::min(12, E);
   if (two) G = std::min(G, p2::kMaxG2);
@@ -687,8 +690,7 @@ static cudaError_t launch_p2(const ua_mesh* m, const UvPhys& P, const UvIn& in, 
   G = std::max(1, std::min(G, E));
   const size_t sm = base + (size_t)G * kP2Point;
   const bool gen = P.law != UA_SLIDING_WEERTMAN || P.melange;
-  auto kern = two ? (gen ? uv_p2_kernel<KT, true, 2> : uv_p2_kernel<KT, false, 2>)
-                  : (gen ? uv_p2_kernel<KT, true, 1> : uv_p2_kernel<KT, false, 1>);
+  auto kern = gen ? uv_p2_kernel<KT, true> : uv_p2_kernel<KT, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);

@@ -361,24 +361,25 @@ __global__ void __launch_bounds__(NOD == 3 ? 512 : 320) uvh_patch_kernel(DevMesh
 // Jacobian multiplied in, so that the rows need only the rule's tables); then a thread per (element, row
 // component, node) sums its 18 entries over the points in registers.  Groups of elements alternate
 // between the two phases.  Bound by the latency of both (few points per phase, one CTA an SM with the
-// tangent's 2.6 kB an element): P2 101x51 272 us with the tangent, 141 us without.
+// tangent's 2.6 kB an element): P2 101x51 285 us with the tangent, 103 us without.
 namespace p2h {
 constexpr int kIps = 16, kIpc = 8;
 enum { PR_UU = 0, PR_UUC, PR_VV, PR_VVC, PR_UV1, PR_UV2, PR_XV, PR_XH, PR_YH, PR_CH, PR_TX, PR_TY, PR_PX, PR_PY,
        PR_TN, PR_FN, PR_S, PR_HC, PR_HU, PR_HV, PR_HH, PR_TF, kPairs };
 constexpr size_t kPoint = (size_t)kIpc * kPairs * sizeof(double2);  // an element's points
-template <int CTAS> constexpr int kRows = CTAS == 2 ? 96 : 128;     // threads of a row component
 }  // namespace p2h
 
-template <bool GEN, int CTAS>
-__global__ void __launch_bounds__(3 * p2h::kRows<CTAS>, CTAS) uvh_p2_kernel(DevMesh M, QuadTable Q, UvhPhys P, UvhIn in,
-                                                                          UvOut out, int G) {
+// One build with the tangent (168 registers) and one without (128), whatever the launch shape: K and R must
+// not depend on the patches.
+template <bool GEN, bool KW>
+__global__ void __launch_bounds__(KW ? 384 : 512) uvh_p2_kernel(DevMesh M, QuadTable Q, UvhPhys P, UvhIn in,
+                                                                      UvOut out, int G, int rows) {
   using namespace p2h;
   extern __shared__ __align__(16) unsigned char smem[];
   const int p = blockIdx.x;
   const int s = M.patch_sys[p];
   if (in.active && !in.active[s]) return;
-  const bool kw = out.K != nullptr;
+  constexpr bool kw = KW;
   const int E = M.max_patch_elems, MH = M.max_patch_hnodes;
   double2* pts = reinterpret_cast<double2*>(smem);        // [G][kIpc][kPairs]
   double2* sD = pts + (size_t)G * kIpc * kPairs;          // reference derivatives [ip][6]
@@ -407,7 +408,8 @@ __global__ void __launch_bounds__(3 * p2h::kRows<CTAS>, CTAS) uvh_p2_kernel(DevM
   }
   __syncthreads();
   const int ngr = (ne + G - 1) / G, gs = (ne + ngr - 1) / ngr;  // groups of equal size
-  const int c = threadIdx.x / kRows<CTAS>, ri = threadIdx.x - c * kRows<CTAS>, el = ri / 6, a = ri - 6 * el;
+  // row component c (uniform over a warp where rows is a multiple of 32; else two meet in some warps)
+  const int c = threadIdx.x / rows, ri = threadIdx.x - c * rows, a = ri % 6, el = c < 3 ? ri / 6 : G;
   for (int gb = 0; gb < ne; gb += gs) {
     const int gn_ = min(gs, ne - gb);
     double ku[6] = {}, kv[6] = {}, kh[6] = {}, T = 0, F = 0;  // row c of node a against u, v, h
@@ -632,7 +634,7 @@ __global__ void __launch_bounds__(3 * p2h::kRows<CTAS>, CTAS) uvh_p2_kernel(DevM
     }
   }
   __syncthreads();
-  uvh_scatter<6, true, double>(M, out, p, s, uoff, voff, hoff, sK, sR, E, ne);
+  uvh_scatter<6, KW, double>(M, out, p, s, uoff, voff, hoff, sK, sR, E, ne);
 }
 
 static cudaError_t launch_p2h(const ua_mesh* m, const UvhPhys& P, const UvhIn& in, const UvOut& out) {
@@ -645,17 +647,17 @@ static cudaError_t launch_p2h(const ua_mesh* m, const UvhPhys& P, const UvhIn& i
   if (base + kPoint > kLimit) return cudaErrorInvalidConfiguration;
   // without the tangent two CTAs share an SM if each gets a group of at least eight elements
   const bool two = base + std::min(8, E) * kPoint <= kHalf;
-  const int rows = two ? kRows<2> : kRows<1>;
+  const int rows = two ? 84 : 128;
   const int G = std::max(1, std::min({(int)(((two ? kHalf : kLimit) - base) / kPoint), rows / 6, E}));
   const size_t sm = base + (size_t)G * kPoint;
   const bool gen = P.uv.law != UA_SLIDING_WEERTMAN || P.uv.melange;
-  auto kern = two ? (gen ? uvh_p2_kernel<true, 2> : uvh_p2_kernel<false, 2>)
-                  : (gen ? uvh_p2_kernel<true, 1> : uvh_p2_kernel<false, 1>);
+  auto kern = out.K ? (gen ? uvh_p2_kernel<true, true> : uvh_p2_kernel<false, true>)
+                    : (gen ? uvh_p2_kernel<true, false> : uvh_p2_kernel<false, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
-  kern<<<m->dm.npatch, 3 * rows, sm, m->stream>>>(m->dm, quad_table(6), P, in, out, G);
+  kern<<<m->dm.npatch, two ? 256 : 384, sm, m->stream>>>(m->dm, quad_table(6), P, in, out, G, rows);
   return cudaGetLastError();
 }
 
