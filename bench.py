@@ -460,17 +460,19 @@ def run_ours(args):
         "uv_p1_kernel<K off> (residual-only assembly)":
             (prof["asmR_ms"], prof["asmR_n"], (12 * ele_per_row + 48 + 8) * wr["asmR"],
              "per row: 12*Ne/rows connectivity + 48 nodal fields + 8 R"),
-        # node-sliced tangent copies: four values per column index, so 1 B of index per non-zero;
-        # one 4-byte node id per node (2 B per row); padding slots are not algorithmic bytes
-        "k_sell<float,float,SpMV> (PCG SpMV + p.q, node slices)":
-            (prof["spmv_ms"], prof["spmv_n"], 5 * wn["spmv"] + 11 * wr["spmv"],
-             "5 B/nnz (FP32 value + 1/4 column) + per row: 2 node id + 4 p + 4 q + 1 mask"),
-        "k_sell<bf16,float,residual> (finest-level residual of the pre-smoothed vector, BF16 node slices)":
-            (prof["amgR_ms"], prof["amgR_n"], 3 * wn["amgR"] + 15 * wr["amgR"],
-             "3 B/nnz (BF16 value + 1/4 column) + per row: 2 node id + 4 b + 4 x + 4 res + 1 mask"),
-        "k_sell<bf16,float,smoothing> (finest-level l1-Jacobi post-smoothing + r.z, BF16 node slices)":
-            (prof["amgP_ms"], prof["amgP_n"], 3 * wn["amgP"] + 19 * wr["amgP"],
-             "3 B/nnz (BF16 value + 1/4 column) + per row: 2 node id + 4 b + 4 xp + 4 invd + 4 z + 1 mask"),
+        # The finest-level passes of the resident PCG: times inside the kernel, one pass per system and
+        # step, team barriers included, weighted with the team's share of the GPU.  Node-sliced tangent
+        # copies: four values per column index, so 1 B of index per non-zero; the quads of the transfer
+        # Q and padding slots are not counted.
+        "k_pcg_team: p, q = A p and p.q (FP32 node slices)":
+            (prof["spmv_ms"], prof["spmv_n"], 5 * wn["spmv"] + 20 * wr["spmv"],
+             "5 B/nnz (FP32 value + 1/4 column) + per row: 4 z + 8 p + 8 q"),
+        "k_pcg_team: x, r update and finest restriction":
+            (prof["amgR_ms"], prof["amgR_n"], 36 * wr["amgR"],
+             "per row: 16 x + 8 r + 4 p + 4 q + 4 D (the transfer's quads not counted)"),
+        "k_pcg_team: finest up pass z = 2 r - A r + Q z_c and r.z (BF16 node slices)":
+            (prof["amgP_ms"], prof["amgP_n"], 3 * wn["amgP"] + 8 * wr["amgP"],
+             "3 B/nnz (BF16 value + 1/4 column) + per row: 4 r + 4 z (the transfer's quads not counted)"),
     }
     dom = max(cand, key=lambda c: cand[c][0])
     ms, n, alg_total, rule = cand[dom]
@@ -482,8 +484,7 @@ def run_ours(args):
     # `bench.py --batch 32 --legs mixed --steps 1 --warmup 1` (every system active), scaled to this
     # launch size
     traffic_ratio = {"uv_p1_kernel<K,": (133.05 + 48.05) / 145.44, "uv_p1_kernel<K off": None,
-                     "k_sell<float,float,SpMV": None, "k_sell<bf16,float,residual": None,
-                     "k_sell<bf16,float,smoothing": None}
+                     "k_pcg_team": None}
     tr = next((v for k, v in traffic_ratio.items() if dom.startswith(k)), None)
     # The assembly is bound by latency and FP64 issue, not HBM: its FP64 roofline beside the HBM one.
     # Executed FP64 operations per P1 element of the tangent+residual pass (2 DFMA + DADD + DMUL,
@@ -515,11 +516,11 @@ def run_ours(args):
             "classes_frac": {c: (v[2] / (v[0] / 1000) / 1e9 / hbm_peak if v[0] > 0 else None)
                              for c, v in cand.items()},
             # device time of the timed classes over the profiled solve's whole device time (the rest:
-            # coarse AMG levels, smoothed transfers, AMG set-up, vector updates and reductions)
+            # coarse AMG levels, AMG set-up, waiting teams)
             "timed_classes_share_of_device_time": total_k / max(float(prof_info.device_ms), 1e-12),
             # the profiled solve's device time by phase (event ranges on the library's stream):
             # tangent and residual assemblies, AMG numeric set-ups with the node-slice fills, the
-            # Krylov iterations (SpMV, V-cycles, vector updates, reductions, the per-chunk checks)
+            # Krylov iterations (the resident solves with their first residuals)
             "device_split": _device_split(prof, float(prof_info.device_ms))}
 
     cpu, vs_oracle = None, None
