@@ -5,6 +5,8 @@ summation orders, and stop at the same tolerance, so the converged velocities ag
 tolerances of the Newton solves (force tolerance 1e-20, i.e. a relative residual of 1e-10) and the
 iteration counts nearly.
 """
+import threading
+
 import numpy as np
 import pytest
 
@@ -139,3 +141,25 @@ def test_p2_assembly_does_not_depend_on_the_patches(ndof):
         out.append((Rv, K.data.copy()))
     for Rv, Kd in out[1:]:
         assert np.array_equal(Rv, out[0][0]) and np.array_equal(Kd, out[0][1])
+
+
+def test_solves_from_several_threads():
+    """Handles of different sizes, each with its own stream: resident launches of two solves overlap, and no
+    launch depends on what another thread set for its own."""
+    probs = [synth.ice_stream_shelf(141, 71, seed=1), synth.ice_stream_shelf(101, 51, seed=2),
+             synth.ice_stream_shelf(33, 17, nod=6, seed=3), synth.ice_stream_shelf(21, 11, seed=4)]
+    ref = [_uv(P)[0] for P in probs]
+    bad = []
+
+    def run(k):
+        try:
+            bad.extend((k, r) for r in range(8) if not np.array_equal(_uv(probs[k])[0], ref[k]))
+        except Exception as e:  # noqa: BLE001 - reported below
+            bad.append((k, repr(e)))
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(len(probs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad

@@ -251,10 +251,10 @@ cudaError_t adj_mass_matrix(const ua_mesh* m, double* Mval) {
 cudaError_t adj_dIdC(const ua_mesh* m, const UvPhys& P, const AdjIn& in, double* out) {
   const size_t sm = (size_t)m->nod * m->dm.max_patch_elems * sizeof(double);
   if (m->nod == 3) {
-    cudaFuncSetAttribute(k_dIdC_patch<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_dIdC_patch<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
     k_dIdC_patch<3><<<m->dm.npatch, 128, sm, m->stream>>>(m->dm, quad_table(3), P, in, out);
   } else {
-    cudaFuncSetAttribute(k_dIdC_patch<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(k_dIdC_patch<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
     k_dIdC_patch<6><<<m->dm.npatch, 128, sm, m->stream>>>(m->dm, quad_table(6), P, in, out);
   }
   return cudaGetLastError();

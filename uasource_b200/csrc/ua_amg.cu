@@ -1,15 +1,18 @@
 // Aggregation AMG preconditioner for the constrained uv tangent.
 //
 // Preconditions the inner PCG that replaces the reference's direct solve of
-// the Newton system (ABfgPreEliminate.m:110).  Node-based plain aggregation:
-// every level keeps Úa's dof layout [u; v] per system, a coarse node is an
-// aggregate of fine nodes and coarse dof (c, I) gathers the c-components of
-// its member nodes, so the prolongation P is piecewise constant per component
-// and the Galerkin operator P' A P is a pure summation.  Smoother: one
-// l1-Jacobi sweep (x += (b - A x) / sum_j |a_ij|) before and after the coarse
+// the Newton system (ABfgPreEliminate.m:110).  Every level keeps Úa's dof
+// layout [u; v] per system.  Default: smoothed aggregation, P = (I - w D^-1 A) P0
+// with P0 piecewise constant over the aggregates of fine nodes, on the first
+// transfer of a quadratic mesh the linear interpolation from the corner nodes;
+// the Galerkin operators P' A P are formed from every tangent.  Plain aggregation
+// (P0 itself, a pure summation) on request.  Smoother: one l1-Jacobi sweep
+// (x += kSmoothOmega (b - A x) / sum_j |a_ij|) before and after the coarse
 // correction, a symmetric V(1,1) cycle and so an SPD preconditioner for CG.
 // Coarsest level: a dense inverse per system (at most 2*kAmgCoarseNodes dofs)
-// applied as a matrix-vector product.
+// applied as a matrix-vector product.  The cycle itself runs in collapsed form
+// inside the resident solves (ua_cycle.cuh), or pass by pass (vcycle_t) where a
+// solve is launched.
 //
 // The hierarchy of a system depends only on that system's mesh and every
 // kernel works on per-system ranges in a fixed summation order, so a
@@ -1820,7 +1823,7 @@ int amg_numeric(ua_mesh* m, const int* rowptr0, const int* colind0, const void* 
     UA_CUDA_TRY(cudaMemcpyAsync(a->d_prefresh, hp, sizeof(int) * ns, cudaMemcpyHostToDevice, m->stream));
     psel = a->d_prefresh;
   }
-  const int sm = (int)(sizeof(double) * (size_t)a->maxdn * a->maxdn);
+  constexpr int sm = sizeof(double) * kAmgMaxDense * kAmgMaxDense;  // a constant: the attribute is the process's
   if (fp32)
     UA_CUDA_TRY(cudaFuncSetAttribute(k_amg_dense_inverse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   else

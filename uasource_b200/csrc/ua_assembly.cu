@@ -666,7 +666,7 @@ static cudaError_t launch_p1(const ua_mesh* m, const UvPhys& P, const UvIn& in, 
   size_t sm = uv_p1_smem(WITHK, sizeof(KT) == 4, m->dm.max_patch_elems, threads, m->dm.max_patch_hnodes);
   const bool gen = P.law != UA_SLIDING_WEERTMAN || P.melange;
   auto kern = gen ? p1_kernel<WITHK, KT, true>(rv) : p1_kernel<WITHK, KT, false>(rv);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
@@ -691,7 +691,7 @@ static cudaError_t launch_p2(const ua_mesh* m, const UvPhys& P, const UvIn& in, 
   const size_t sm = base + (size_t)G * kP2Point;
   const bool gen = P.law != UA_SLIDING_WEERTMAN || P.melange;
   auto kern = gen ? uv_p2_kernel<KT, true> : uv_p2_kernel<KT, false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;

@@ -5,6 +5,11 @@
 
 namespace ua {
 
+// The largest dynamic shared memory of a kernel without static shared memory.  A kernel's attribute is set
+// to this (or another constant) rather than to what a launch needs: the attribute is the process's, and a
+// thread with a smaller mesh would lower it between another thread's setting and launch.
+constexpr int kMaxDynSmem = 227 * 1024;
+
 // Inputs of the uv assembly.  Nodal fields are indexed by global node id;
 // velocities live in the dof vector X (system-major [u_s; v_s]) and the
 // assembly evaluates at X + gamma[s]*dX when dX is given (CalcCostFunctionNR.m:14-16).

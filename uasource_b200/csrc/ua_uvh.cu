@@ -653,7 +653,7 @@ static cudaError_t launch_p2h(const ua_mesh* m, const UvhPhys& P, const UvhIn& i
   const bool gen = P.uv.law != UA_SLIDING_WEERTMAN || P.uv.melange;
   auto kern = out.K ? (gen ? uvh_p2_kernel<true, true> : uvh_p2_kernel<false, true>)
                     : (gen ? uvh_p2_kernel<true, false> : uvh_p2_kernel<false, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
@@ -679,7 +679,7 @@ static cudaError_t launch_t(const ua_mesh* m, const UvhPhys& P, const UvhIn& in,
   if constexpr (WITHK) {
     if (P.uv.law == UA_SLIDING_WEERTMAN && !P.uv.melange) kern = uvh_patch_kernel<NOD, WITHK, KT, false>;
   }
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
   if (e != cudaSuccess) return e;
   int threads = ((E * NOD + 31) / 32) * 32;
   if (threads > (NOD == 3 ? 512 : 320)) return cudaErrorInvalidConfiguration;
