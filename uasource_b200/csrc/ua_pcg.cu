@@ -3,12 +3,12 @@
 //
 // What bounds the inner solve of a mesh up to some 100,000 nodes is not memory but the chain of
 // short passes: with one launch per pass a PCG step of the 141x71 mesh took 72 us in 19 launches
-// of about 3.8 us.  Here a step is 1 + 2 L passes for L levels above the dense one (24 us on that
-// mesh), a team barrier costs 1.25 us whatever the team's size, nothing is launched inside the
-// solve, the systems of a batch do not wait for one another and the host neither checks nor
-// over-runs the convergence.  With a launch per pass and with the resident kernel, one B200: uv P1
-// 141x71 FP64 25.8 and 12.9 ms, P2 101x51 mixed 41.6 and 21.6 ms, P2 401x201 FP64 180 and 125 ms,
-// 16 meshes of 2k-200k elements mixed 84 and 58 ms.
+// of about 3.8 us.  Here a step is 1 + 2 L passes for the L levels above the dense one and the solo
+// ones (20 us on that mesh), a team barrier costs 1.25 us whatever the team's size, nothing is
+// launched inside the solve, the systems of a batch do not wait for one another and the host neither
+// checks nor over-runs the convergence.  With a launch per pass and with the resident kernel as it
+// was first built, one B200: uv P1 141x71 FP64 25.8 and 12.9 ms, P2 101x51 mixed 41.6 and 21.6 ms, P2
+// 401x201 FP64 180 and 125 ms, 16 meshes of 2k-200k elements mixed 84 and 58 ms.
 #include <algorithm>
 #include <cstring>
 #include "ua_cycle.cuh"
@@ -443,6 +443,9 @@ void cycle_schedule(const std::vector<CycSys>& sys, const std::vector<int>& sel,
                     int nsm, CycSchedule& out) {
   constexpr double kLatency = 16.0, kNodesPerUs = 90.0;
   constexpr int kSlicesPerCta = 4;  // a team grows while each of its CTAs has at least this many slices
+  // up to so many slices one CTA with a slice a warp and no team barrier is as fast or faster (FP64, us a
+  // step, one CTA against a team: 8 slices 12.3 and 14.7, 12: 15.1 and 15.0, 16: 17.9 and 16.0)
+  constexpr int kOneCta = 12;
   std::vector<int> list;
   for (int s = 0; s < (int)sys.size(); ++s)
     if (sel[s]) list.push_back(s);
@@ -454,7 +457,7 @@ void cycle_schedule(const std::vector<CycSys>& sys, const std::vector<int>& sel,
   auto time = [&](int s, int T) {
     return std::max(1, steps[s]) * (kLatency + sys[s].nn[0] / (kNodesPerUs * T));
   };
-  auto cap = [&](int s) { return std::max(1, std::min(nsm, (sys[s].nsl + kSlicesPerCta - 1) / kSlicesPerCta)); };
+  auto cap = [&](int s) { return sys[s].nsl <= kOneCta ? 1 : std::max(1, std::min(nsm, (sys[s].nsl + kSlicesPerCta - 1) / kSlicesPerCta)); };
   if (2 * n <= nsm) {
     std::vector<int> T(n, 1);
     for (int left = nsm - n; left > 0; --left) {
