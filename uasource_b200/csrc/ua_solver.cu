@@ -118,6 +118,7 @@ struct Work {
   int* sel;        // [nsys]
   double* gamma;   // [nsys]
   unsigned char* cmask;  // [ndof]
+  int* arrived = nullptr;  // [nsys] blocks of a system that have finished a cost launch (k_cost leaves zeros)
   int* dof_con;    // [ndof]
   // constraints (mask form: one unit entry per row)
   int* con_dof = nullptr;
@@ -634,25 +635,27 @@ __global__ void k_pair_project_r0(int npair, const int* pair_rows, const int* co
 }
 
 // dl_c = (frhs - K dX)[dof_c]  (ABfgPreEliminate.m:138 with B a selection)
+constexpr int kMulL = 8;  // lanes per constraint: the row's entries are a chain of gathers (a thread per row: 7.8 us)
 template <typename KT>
-__global__ void k_con_multiplier(int nc, const int* con_dof, const int* con_sys, const int* sel, const int* rowptr,
-                                 const int* colind, const KT* K, const double* dX, const double* frhs,
-                                 double* dlam, ConPairs cp) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nc || !sel[con_sys[c]]) return;
+__global__ void __launch_bounds__(256) k_con_multiplier(int nc, const int* con_dof, const int* con_sys, const int* sel,
+                                                        const int* rowptr, const int* colind, const KT* K,
+                                                        const double* dX, const double* frhs, double* dlam,
+                                                        ConPairs cp) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) / kMulL, lane = threadIdx.x % kMulL;
+  if (c >= nc || !sel[con_sys[c]]) return;  // whole groups
+  const unsigned gmask = ((1u << kMulL) - 1u) << ((threadIdx.x & 31) & ~(kMulL - 1));
   auto row_res = [&](int d) {
     double acc = 0;
-    for (int j = rowptr[d]; j < rowptr[d + 1]; ++j) acc += (double)K[j] * dX[colind[j]];
+    for (int j = rowptr[d] + lane; j < rowptr[d + 1]; j += kMulL) acc += (double)K[j] * dX[colind[j]];
+#pragma unroll
+    for (int o = kMulL / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(gmask, acc, o, kMulL);
     return frhs[d] - acc;
   };
   const int d = con_dof[c];
-  if (con_is_pair(cp, c)) {  // y = b'(f - K x) (ABfgPreEliminate.m:138)
-    dlam[c] = cp.v1[c] * row_res(d) + cp.v2[c] * row_res(cp.dof2[c]);
-    return;
-  }
-  dlam[c] = row_res(d);
+  double y = row_res(d);
+  if (con_is_pair(cp, c)) y = cp.v1[c] * y + cp.v2[c] * row_res(cp.dof2[c]);  // y = b'(f - K x) (ABfgPreEliminate.m:138)
+  if (lane == 0) dlam[c] = y;
 }
-
 // frhs = -R - L' l  (SSTREAM2dNR2.m:235)
 __global__ void k_frhs(const int* rb_start, const int* rb_sys, const int* sel, const double* R, const int* dof_con,
                        const double* lam, double* frhs, const int* con_dof, ConPairs cp) {
@@ -664,91 +667,93 @@ __global__ void k_frhs(const int* rb_start, const int* rb_sys, const int* sel, c
   }
 }
 
-// Cost function rows (CalcCostFunctionNR.m:24-41): f = -R - L'(l + gamma dl);
-// partials sum f^2 and sum f.dX
-__global__ void __launch_bounds__(256) k_cost_rows(const int* rb_start, const int* rb_sys, int nrb, const int* sel,
-                                                   const double* R, const int* dof_con, const double* lam,
-                                                   const double* dlam, const double* gamma, const double* dX,
-                                                   double* part, const int* con_dof, ConPairs cp) {
+// Cost of every selected system: f = -R - L'(l + gamma dl) over its rows, with the constraint rows
+// g = c - L(X + gamma dX) taken by the block of their (first) dof; then rForce = (f'f + g'g)/Normalisation and
+// D2 = [f;g]'[dX;dl], or (write_norm) the normalisation f'f + 1000 eps.  One launch: the last of a system's
+// blocks to finish (counter `arrived`, left at zero) adds the partials in a fixed order.
+__global__ void __launch_bounds__(kRedThreads) k_cost(const int* rb_start, const int* rb_sys, const int* sys_rb_off,
+                                                      int nrb, const int* sel, const double* R, const int* dof_con,
+                                                      const double* lam, const double* dlam, const double* gamma,
+                                                      const double* X, const double* dX, const int* con_dof,
+                                                      const double* con_rhs, ConPairs cp, double* part, int* arrived,
+                                                      int nsys, double* sysv, int write_norm) {
   const int blk = blockIdx.x;
   const int s = rb_sys[blk];
+  if (!sel[s]) return;  // uniform over a system's blocks
   double v[2] = {0, 0};
-  if (sel[s]) {
-    const double gm = gamma ? gamma[s] : 0.0;
-    for (int i = rb_start[blk] + threadIdx.x; i < rb_start[blk + 1]; i += blockDim.x) {
-      const int c = dof_con ? dof_con[i] : -1;
-      double f = -R[i];
-      if (c >= 0) f -= con_coef(cp, con_dof, c, i) * (lam[c] + gm * dlam[c]);
-      v[0] += f * f;
-      if (dX) v[1] += f * dX[i];
+  const double gm = gamma ? gamma[s] : 0.0;
+  for (int i = rb_start[blk] + threadIdx.x; i < rb_start[blk + 1]; i += blockDim.x) {
+    const int c = dof_con ? dof_con[i] : -1;
+    double f = -R[i];
+    if (c >= 0) {
+      f -= con_coef(cp, con_dof, c, i) * (lam[c] + gm * dlam[c]);
+      if (con_dof[c] == i) {
+        double xv = X[i] + (gamma ? gm * dX[i] : 0.0);
+        if (con_is_pair(cp, c)) {  // g = c - L X on a two-entry row
+          const int d2 = cp.dof2[c];
+          xv = cp.v1[c] * xv + cp.v2[c] * (X[d2] + (gamma ? gm * dX[d2] : 0.0));
+        }
+        const double gv = con_rhs[c] - xv;
+        v[0] += gv * gv;
+        v[1] += gv * dlam[c];
+      }
     }
+    v[0] += f * f;
+    if (dX) v[1] += f * dX[i];
   }
   block_partials<2>(v, part, nrb, blk);
-}
-
-// Per-system cost: adds the constraint rows g = c - L(X + gamma dX), then
-// rForce = (f'f + g'g)/Normalisation and D2 = [f;g]'[dX;dl].
-__global__ void k_cost_reduce(const int* sys_rb_off, int nrb, const int* sel, const double* part, int nsys,
-                              double* sysv, const int* sys_con_off, const int* con_dof, const double* con_rhs,
-                              const double* X, const double* dX, const double* dlam, const double* gamma,
-                              int write_norm, ConPairs cp) {
-  const int s = blockIdx.x;
-  if (!sel[s]) return;
-  double o[2];
-  sys_sum<2>(part, nrb, sys_rb_off[s], sys_rb_off[s + 1], o);
-  // constraint rows, strided over the block, then a fixed-order tree sum
-  __shared__ double cg[2][kRedThreads];
-  double gg = 0, gd = 0;
-  if (sys_con_off) {
-    const double gm = gamma ? gamma[s] : 0.0;
-    for (int c = sys_con_off[s] + threadIdx.x; c < sys_con_off[s + 1]; c += blockDim.x) {
-      const int d = con_dof[c];
-      double xv = X[d] + (dX ? gm * dX[d] : 0.0);
-      if (con_is_pair(cp, c)) {  // g = c - L X on a two-entry row
-        const int d2 = cp.dof2[c];
-        xv = cp.v1[c] * xv + cp.v2[c] * (X[d2] + (dX ? gm * dX[d2] : 0.0));
-      }
-      const double gv = con_rhs[c] - xv;
-      gg += gv * gv;
-      if (dlam) gd += gv * dlam[c];
-    }
-  }
-  cg[0][threadIdx.x] = gg;
-  cg[1][threadIdx.x] = gd;
+  __threadfence();
+  __shared__ int last;
   __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) {
-      cg[0][threadIdx.x] += cg[0][threadIdx.x + st];
-      cg[1][threadIdx.x] += cg[1][threadIdx.x + st];
-    }
-    __syncthreads();
-  }
+  const int b0 = sys_rb_off[s], b1 = sys_rb_off[s + 1];
+  if (threadIdx.x == 0) last = atomicAdd(arrived + s, 1) == b1 - b0 - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double o[2];
+  sys_sum<2>(part, nrb, b0, b1, o);
   if (threadIdx.x != 0) return;
-  gg = cg[0][0];
-  gd = cg[1][0];
+  arrived[s] = 0;
   if (write_norm) {
     sysv[SV_NORM * nsys + s] = o[0] + 1000.0 * 2.220446049250313e-16;  // fext0'fext0+1000*eps
     return;
   }
-  sysv[SV_FF * nsys + s] = (o[0] + gg) / sysv[SV_NORM * nsys + s];
-  sysv[SV_FD * nsys + s] = o[1] + gd;
+  sysv[SV_FF * nsys + s] = o[0] / sysv[SV_NORM * nsys + s];
+  sysv[SV_FD * nsys + s] = o[1];
+}
+
+template <typename KT>
+static void con_multiplier(const Work* w, const KT* K, cudaStream_t st) {
+  k_con_multiplier<KT><<<(w->nc * kMulL + 255) / 256, 256, 0, st>>>(w->nc, w->con_dof, w->con_sys, w->sel, w->rowptr,
+                                                                   w->colind, K, w->dX, w->frhs, w->dlam, con_pairs(w)),
+      ++g_launches;
+}
+// norm: of the residual alone, without constraints
+static void launch_cost(ua_mesh* m, const double* gamma, bool norm) {
+  Work* w = m->work;
+  k_cost<<<w->nrb, kRedThreads, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sys_rb_off, w->nrb, w->sel, w->R,
+                                                norm ? nullptr : w->dof_con, w->lam, w->dlam, gamma, w->X,
+                                                !norm ? w->dX : nullptr, w->con_dof, w->con_rhs,
+                                                norm ? ConPairs{} : con_pairs(w), w->part, w->arrived, w->nsys, w->sysv,
+                                                norm),
+      ++g_launches;
 }
 
 // X += gamma dX, l += gamma dl for selected systems.
-__global__ void k_newton_update(const int* rb_start, const int* rb_sys, const int* sel, const double* gamma,
-                                double* X, const double* dX) {
+// (the blocks from nrb on take the multipliers)
+__global__ void __launch_bounds__(256) k_newton_update(const int* rb_start, const int* rb_sys, int nrb, const int* sel,
+                                                       const double* gamma, double* X, const double* dX, int nc,
+                                                       const int* con_sys, double* lam, const double* dlam) {
   const int blk = blockIdx.x;
+  if (blk >= nrb) {
+    const int c = (blk - nrb) * 256 + threadIdx.x;
+    if (c < nc && sel[con_sys[c]]) lam[c] += gamma[con_sys[c]] * dlam[c];
+    return;
+  }
   const int s = rb_sys[blk];
   if (!sel[s]) return;
   const double gm = gamma[s];
   for (int i = rb_start[blk] + threadIdx.x; i < rb_start[blk + 1]; i += blockDim.x) X[i] += gm * dX[i];
-}
-
-__global__ void k_lam_update(int nc, const int* con_sys, const int* sel, const double* gamma, double* lam,
-                             const double* dlam) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nc || !sel[con_sys[c]]) return;
-  lam[c] += gamma[con_sys[c]] * dlam[c];
 }
 
 // Constraint masks: cmask[dof] = 1 and dof_con[dof] = c for every constraint c.
@@ -858,6 +863,8 @@ static int ensure_work(ua_mesh* m, const ua_params* p) {
   }
   w->part = walloc<double>(m, 4 * (size_t)w->nrb);
   w->sysv = walloc<double>(m, SV_COUNT * (size_t)nsys);
+  w->arrived = walloc<int>(m, nsys);
+  if (w->arrived) UA_CUDA_TRY(cudaMemset(w->arrived, 0, sizeof(int) * nsys));
   w->done = walloc<int>(m, nsys);
   w->its = walloc<int>(m, nsys);
   w->status = walloc<int>(m, nsys);
@@ -866,7 +873,7 @@ static int ensure_work(ua_mesh* m, const ua_params* p) {
   w->cmask = walloc<unsigned char>(m, N);
   w->dof_con = walloc<int>(m, N);
   ok = ok && w->rowptr && w->colind && w->diagpos && w->scal && w->part && w->sysv && w->done && w->its &&
-       w->status && w->sel && w->gamma && w->cmask && w->dof_con && w->rb_start && w->rb_sys && w->sys_rb_off;
+       w->arrived && w->status && w->sel && w->gamma && w->cmask && w->dof_con && w->rb_start && w->rb_sys && w->sys_rb_off;
   if (!ok) { delete w; return set_error(UA_ERR_OOM, "device allocation of work buffers failed"); }
   w->nan_first = walloc<int>(m, 16);
   if (!w->nan_first) { delete w; return set_error(UA_ERR_OOM, "device allocation of work buffers failed"); }
@@ -1417,12 +1424,7 @@ static int cost_eval(ua_mesh* m, const ua_params* p, bool useDir, bool assembleR
     if (rc) return rc;
   }
   const double* gamma = useDir && !atX ? w->gamma : nullptr;
-  k_cost_rows<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->nrb, w->sel, w->R, w->dof_con, w->lam,
-                                             w->dlam, gamma, w->dX, w->part, w->con_dof, con_pairs(w)), ++g_launches;
-  k_cost_reduce<<<w->nsys, kRedThreads, 0, m->stream>>>(w->sys_rb_off, w->nrb, w->sel, w->part, w->nsys, w->sysv,
-                                                         w->sys_con_off, w->con_dof, w->con_rhs, w->X,
-                                                         useDir ? w->dX : nullptr, w->dlam, gamma, 0, con_pairs(w)),
-      ++g_launches;
+  launch_cost(m, gamma, false);
   UA_CUDA_TRY(cudaGetLastError());
   UA_CUDA_TRY(cudaMemcpyAsync(host ? host : w->h_sysv, w->sysv, SV_COUNT * w->nsys * sizeof(double),
                               cudaMemcpyDeviceToHost, m->stream));
@@ -1458,15 +1460,8 @@ static int pcg_resident_solve(ua_mesh* m, const ua_params* p, bool fp32, const v
   if (int rc = pcg_resident(m, v, sel, steps, w->nsm, &g_launches)) return rc;
   prof_end(m, kev);
   if (w->nc) {
-    if (fp32)
-      k_con_multiplier<float><<<(w->nc + 255) / 256, 256, 0, m->stream>>>(
-          w->nc, w->con_dof, w->con_sys, w->sel, w->rowptr, w->colind, (const float*)K, w->dX, w->frhs, w->dlam,
-          con_pairs(w));
-    else
-      k_con_multiplier<double><<<(w->nc + 255) / 256, 256, 0, m->stream>>>(
-          w->nc, w->con_dof, w->con_sys, w->sel, w->rowptr, w->colind, (const double*)K, w->dX, w->frhs, w->dlam,
-          con_pairs(w));
-    ++g_launches;
+    if (fp32) con_multiplier(w, (const float*)K, m->stream);
+    else con_multiplier(w, (const double*)K, m->stream);
   }
   UA_CUDA_TRY(cudaGetLastError());
   if (w->defer && !w->prof.on) return defer_result(m);
@@ -1716,9 +1711,7 @@ static int pcg_t(ua_mesh* m, const ua_params* p, const KT* K, int* its_out, cons
   }
   prof_end(m, kev);
   if (w->nc)
-    k_con_multiplier<KT><<<(w->nc + 255) / 256, 256, 0, m->stream>>>(w->nc, w->con_dof, w->con_sys, w->sel,
-                                                                     w->rowptr, w->colind, K, w->dX, w->frhs,
-                                                                     w->dlam, con_pairs(w)), ++g_launches;
+    con_multiplier(w, K, m->stream);
   UA_CUDA_TRY(cudaMemcpyAsync(w->h_int, w->its, w->nsys * sizeof(int), cudaMemcpyDeviceToHost, m->stream));
   UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
   for (int s = 0; s < w->nsys; ++s) its_out[s] = its_out[s] ? w->h_int[s] : 0;
@@ -1821,11 +1814,7 @@ static int newton_init(ua_mesh* m, const ua_params* p, const std::vector<int>& r
   }
   {
     if ((rc = assemble(m, p, false, false, w->X0, false))) return rc;
-    k_cost_rows<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->nrb, w->sel, w->R, nullptr, nullptr,
-                                               nullptr, nullptr, nullptr, w->part, nullptr, ConPairs{}), ++g_launches;
-    k_cost_reduce<<<nsys, kRedThreads, 0, m->stream>>>(w->sys_rb_off, w->nrb, w->sel, w->part, nsys, w->sysv,
-                                                       nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                                       nullptr, 1, con_pairs(w)), ++g_launches;
+    launch_cost(m, nullptr, true);
     UA_CUDA_TRY(cudaGetLastError());
   }
   // initial cost (:149-152) with zero direction
@@ -2097,10 +2086,9 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
     }
     if ((rc = set_sel(m, sel))) return rc;
     if ((rc = set_gamma(m, gam))) return rc;
-    k_newton_update<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->gamma, w->X, w->dX), ++g_launches;
-    if (w->nc)
-      k_lam_update<<<(w->nc + 255) / 256, 256, 0, m->stream>>>(w->nc, w->con_sys, w->sel, w->gamma, w->lam,
-                                                               w->dlam), ++g_launches;
+    k_newton_update<<<w->nrb + (w->nc + 255) / 256, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->nrb, w->sel, w->gamma, w->X,
+                                                                        w->dX, w->nc, w->con_sys, w->lam, w->dlam),
+        ++g_launches;
     UA_CUDA_TRY(cudaGetLastError());
     if ((rc = record_updates(m, rep, sel, gam))) return rc;
   }
@@ -2389,8 +2377,7 @@ static int bicgstab_t(ua_mesh* m, const ua_params* p, const KT* K, int* its_out,
     if (all || it >= p->krylov_maxit + chunk) break;
   }
   if (w->nc)
-    k_con_multiplier<KT><<<(w->nc + 255) / 256, 256, 0, m->stream>>>(w->nc, w->con_dof, w->con_sys, w->sel, w->rowptr,
-                                                                     w->colind, K, w->dX, w->frhs, w->dlam, con_pairs(w)), ++g_launches;
+    con_multiplier(w, K, m->stream);
   UA_CUDA_TRY(cudaMemcpyAsync(w->h_int, w->its, w->nsys * sizeof(int), cudaMemcpyDeviceToHost, m->stream));
   UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
   for (int s = 0; s < w->nsys; ++s) its_out[s] = its_out[s] ? w->h_int[s] : 0;
@@ -2637,9 +2624,7 @@ static int gmres_resident_solve(ua_mesh* m, const ua_params* p, const double* K,
   if (int rc = gmres_resident(m, v, sel, steps, w->nsm, &g_launches)) return rc;
   prof_end(m, kev);
   if (w->nc)
-    k_con_multiplier<double><<<(w->nc + 255) / 256, 256, 0, m->stream>>>(w->nc, w->con_dof, w->con_sys, w->sel,
-                                                                         w->rowptr, w->colind, K, w->dX, w->frhs,
-                                                                         w->dlam, con_pairs(w)), ++g_launches;
+    con_multiplier(w, K, m->stream);
   UA_CUDA_TRY(cudaGetLastError());
   if (w->defer && !w->prof.on) return defer_result(m);
   UA_CUDA_TRY(cudaMemcpyAsync(w->h_int, w->its, nsys * sizeof(int), cudaMemcpyDeviceToHost, m->stream));
@@ -2912,8 +2897,7 @@ static int gmres_t(ua_mesh* m, const ua_params* p, const KT* K, int* its_out, co
   for (int s = 0; s < nsys; ++s) hdone[s] = 1;
   UA_CUDA_TRY(cudaMemcpyAsync(w->done, hdone.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, st));
   if (w->nc)
-    k_con_multiplier<KT><<<(w->nc + 255) / 256, 256, 0, st>>>(w->nc, w->con_dof, w->con_sys, w->sel, w->rowptr,
-                                                              w->colind, K, w->dX, w->frhs, w->dlam, con_pairs(w)), ++g_launches;
+    con_multiplier(w, K, st);
   UA_CUDA_TRY(cudaGetLastError());
   UA_CUDA_TRY(cudaStreamSynchronize(st));
   for (int s = 0; s < nsys; ++s) its_out[s] = its_out[s] ? S[s].its : 0;
@@ -2986,11 +2970,7 @@ static int cost_eval_uvh(ua_mesh* m, const ua_params* p, bool assembleR = true, 
     int rc = assemble_uvh(m, p, false, true, false, false);
     if (rc) return rc;
   }
-  k_cost_rows<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->nrb, w->sel, w->R, w->dof_con, w->lam,
-                                             w->dlam, w->gamma, w->dX, w->part, w->con_dof, con_pairs(w)), ++g_launches;
-  k_cost_reduce<<<w->nsys, kRedThreads, 0, m->stream>>>(w->sys_rb_off, w->nrb, w->sel, w->part, w->nsys, w->sysv,
-                                                         w->sys_con_off, w->con_dof, w->con_rhs, w->X, w->dX, w->dlam,
-                                                         w->gamma, 0, con_pairs(w)), ++g_launches;
+  launch_cost(m, w->gamma, false);
   UA_CUDA_TRY(cudaGetLastError());
   UA_CUDA_TRY(cudaMemcpyAsync(host ? host : w->h_sysv, w->sysv, SV_COUNT * w->nsys * sizeof(double), cudaMemcpyDeviceToHost,
                               m->stream));
@@ -3032,10 +3012,7 @@ static int newton_run_uvh(ua_mesh* m, const ua_params* p, std::vector<ua_newton_
                                                                  w->X, con_pairs(w)), ++g_launches;
   // Fext0 at ZeroFields (:53-56); the normalisation of CalcCostFunctionNRuvh
   if ((rc = assemble_uvh(m, p, false, false, true, false))) return rc;
-  k_cost_rows<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->nrb, w->sel, w->R, nullptr, nullptr, nullptr,
-                                             nullptr, nullptr, w->part, nullptr, ConPairs{}), ++g_launches;
-  k_cost_reduce<<<nsys, kRedThreads, 0, m->stream>>>(w->sys_rb_off, w->nrb, w->sel, w->part, nsys, w->sysv, nullptr,
-                                                     nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 1, con_pairs(w)), ++g_launches;
+  launch_cost(m, nullptr, true);
   UA_CUDA_TRY(cudaGetLastError());
   for (int s = 0; s < nsys; ++s) { st[s] = UvhSys(); st[s].active = true; }
   while (true) {
@@ -3153,9 +3130,9 @@ static int newton_run_uvh(ua_mesh* m, const ua_params* p, std::vector<ua_newton_
     }
     if ((rc = set_sel(m, sel))) return rc;
     if ((rc = set_gamma(m, gam))) return rc;
-    k_newton_update<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->gamma, w->X, w->dX), ++g_launches;
-    if (w->nc)
-      k_lam_update<<<(w->nc + 255) / 256, 256, 0, m->stream>>>(w->nc, w->con_sys, w->sel, w->gamma, w->lam, w->dlam), ++g_launches;
+    k_newton_update<<<w->nrb + (w->nc + 255) / 256, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->nrb, w->sel, w->gamma, w->X,
+                                                                        w->dX, w->nc, w->con_sys, w->lam, w->dlam),
+        ++g_launches;
     UA_CUDA_TRY(cudaGetLastError());
     if ((rc = record_updates(m, rep, sel, gam))) return rc;
   }
