@@ -143,6 +143,14 @@ struct AsmTuning {
   int regs = 128;  // register budget of the P1 kernel: 128, 96 (128-thread CTAs) or 80
 };
 
+// Element rows of the P2 uvh assembly and the blocks of its element kernel (without, with the tangent),
+// on first use.
+struct UvhElemRows {
+  double *kel = nullptr, *rel = nullptr;
+  int4* blk[2] = {nullptr, nullptr};
+  int n[2] = {0, 0};
+};
+
 // Host-side mirror plus ownership of device buffers.
 struct DeviceBuffer {
   void* ptr = nullptr;
@@ -181,6 +189,7 @@ struct ua_mesh {
   std::vector<ua::HostSystem> sys;
   // host copies of symbolic data needed on the host
   std::vector<int> h_node_off, h_dof_off, h_knz_off, h_nnzn, h_elem_off;
+  ua::UvhElemRows uvh_rows;
   std::vector<int> h_nodeptr, h_nodecol;
   int nn_total = 0, ne_total = 0, ndof_total = 0;
   long long nnz_total = 0;

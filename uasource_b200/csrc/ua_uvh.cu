@@ -356,12 +356,13 @@ __global__ void __launch_bounds__(NOD == 3 ? 512 : 320) uvh_patch_kernel(DevMesh
 // ---------------------------------------------------------------------------
 //
 // A thread per (element, node) evaluates the physics of every point six times and keeps its 54 tangent
-// entries in shared memory (P2 101x51: 518 us with the tangent, 279 us without).  Here a thread per
+// entries in shared memory (P2 101x51: 506 us with the tangent, 279 us without).  Here a thread per
 // point evaluates it once and leaves 22 pairs of coefficients, in reference coordinates (the inverse
 // Jacobian multiplied in, so that the rows need only the rule's tables); then a thread per (element, row
-// component, node) sums its 18 entries over the points in registers.  Groups of elements alternate
-// between the two phases.  Bound by the latency of both (few points per phase, one CTA an SM with the
-// tangent's 2.6 kB an element): P2 101x51 285 us with the tangent, 103 us without.
+// component, node) sums its 18 entries over the points in registers.  The element rows go to global
+// memory, 2.9 kB an element, and a second kernel sums each patch's non-zeros over them: with the rows in
+// shared memory a patch held 50 elements and every element was evaluated in three patches (285 us and
+// 103 us; now 134 us and 62 us with the gather).  Bound by the latency of the two phases, few warps an SM.
 namespace p2h {
 constexpr int kIps = 16, kIpc = 8;
 enum { PR_UU = 0, PR_UUC, PR_VV, PR_VVC, PR_UV1, PR_UV2, PR_XV, PR_XH, PR_YH, PR_CH, PR_TX, PR_TY, PR_PX, PR_PY,
@@ -369,25 +370,23 @@ enum { PR_UU = 0, PR_UUC, PR_VV, PR_VVC, PR_UV1, PR_UV2, PR_XV, PR_XH, PR_YH, PR
 constexpr size_t kPoint = (size_t)kIpc * kPairs * sizeof(double2);  // an element's points
 }  // namespace p2h
 
-// One build with the tangent (168 registers) and one without (128), whatever the launch shape: K and R must
-// not depend on the patches.
+// blk: {system, first element, elements} of each block, at most G elements.  Rows of element e: tangent
+// kel[((6 e + a) 6 + b) 9 + 3 c + column component], residual parts rel[6 (6 e + a) + 2 c + {0, 1}].
 template <bool GEN, bool KW>
-__global__ void __launch_bounds__(KW ? 384 : 512) uvh_p2_kernel(DevMesh M, QuadTable Q, UvhPhys P, UvhIn in,
-                                                                      UvOut out, int G, int rows) {
+__global__ void __launch_bounds__(KW ? 384 : 256, KW ? 1 : 2) uvh_p2_elements(DevMesh M, QuadTable Q, UvhPhys P, UvhIn in,
+                                                                             const int4* blk, int G, int rows,
+                                                                             double* kel, double* rel) {
   using namespace p2h;
   extern __shared__ __align__(16) unsigned char smem[];
-  const int p = blockIdx.x;
-  const int s = M.patch_sys[p];
+  const int4 bk = blk[blockIdx.x];
+  const int s = bk.x, eb = bk.y, gn_ = bk.z;
   if (in.active && !in.active[s]) return;
   constexpr bool kw = KW;
-  const int E = M.max_patch_elems, MH = M.max_patch_hnodes;
+  const int MH = 6 * G;
   double2* pts = reinterpret_cast<double2*>(smem);        // [G][kIpc][kPairs]
   double2* sD = pts + (size_t)G * kIpc * kPairs;          // reference derivatives [ip][6]
   double* sN = reinterpret_cast<double*>(sD + kIps * 6);  // N [ip][6]
-  double* nd = sN + kIps * 6;                             // [F_COUNT][MH]
-  double* sR = nd + (size_t)F_COUNT * MH;                 // [36][E]
-  double* sK = sR + (size_t)36 * E;
-  const int e0 = M.patch_elem_ptr[p], ne = M.patch_elem_ptr[p + 1] - e0;
+  double* nd = sN + kIps * 6;                             // [F_COUNT][MH], node k of element el at 6 el + k
   const int no = M.sys_node_off[s], nn_s = M.sys_node_off[s + 1] - no;
   const int uoff = M.sys_dof_off[s] - no, voff = uoff + nn_s, hoff = voff + nn_s;
   const double gam = in.gamma ? in.gamma[s] : 0.0;
@@ -398,34 +397,25 @@ __global__ void __launch_bounds__(KW ? 384 : 512) uvh_p2_kernel(DevMesh M, QuadT
     sN[t] = Q.fun[t / 6][t % 6];
     sD[t] = make_double2(Q.der[t / 6][0][t % 6], Q.der[t / 6][1][t % 6]);
   }
-  const int hb0 = M.patch_hnode_ptr[p], nh = M.patch_hnode_ptr[p + 1] - hb0;
-  for (int t = threadIdx.x; t < nh; t += blockDim.x) {
-    int gn = __ldg(M.patch_hnodes + hb0 + t);
+  for (int t = threadIdx.x; t < 6 * gn_; t += blockDim.x) {
+    int gn = __ldg(M.conn + (size_t)(t % 6) * M.ne + eb + t / 6);
     bool okn = true;
     UA_CHECK_INDEX(M.dbg, gn, no, no + nn_s, BS_ELEM_NODE, okn);
     (void)okn;
     stage_node(M, P, in, S, gn, uoff, voff, hoff, gam, nd + t, MH);
   }
   __syncthreads();
-  const int ngr = (ne + G - 1) / G, gs = (ne + ngr - 1) / ngr;  // groups of equal size
   // row component c (uniform over a warp where rows is a multiple of 32; else two meet in some warps)
   const int c = threadIdx.x / rows, ri = threadIdx.x - c * rows, a = ri % 6, el = c < 3 ? ri / 6 : G;
-  for (int gb = 0; gb < ne; gb += gs) {
-    const int gn_ = min(gs, ne - gb);
+  {
     double ku[6] = {}, kv[6] = {}, kh[6] = {}, T = 0, F = 0;  // row c of node a against u, v, h
     for (int ip0 = 0; ip0 < kIps; ip0 += kIpc) {
       // (a) points
       for (int t = threadIdx.x; t < gn_ * kIpc; t += blockDim.x) {
         const int pe = t / kIpc, pi = t - pe * kIpc, ip = ip0 + pi;
-        const uint16_t* ln = M.patch_elnodes + (size_t)(e0 + gb + pe) * 6;
         int l[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          l[k] = __ldg(ln + k);
-          bool okn = true;
-          UA_CHECK_INDEX(M.dbg, l[k], 0, nh, BS_ELEM_NODE, okn);
-          (void)okn;
-        }
+        for (int k = 0; k < 6; ++k) l[k] = 6 * pe + k;
         const double* N = sN + ip * 6;
         const double2* dr = sD + ip * 6;
         auto itp = [&](int k) {
@@ -489,7 +479,7 @@ __global__ void __launch_bounds__(KW ? 384 : 512) uvh_p2_kernel(DevMesh M, QuadT
             int gn[6];
             double Nw[6];
 #pragma unroll
-            for (int k = 0; k < 6; ++k) { gn[k] = __ldg(M.patch_hnodes + hb0 + l[k]); Nw[k] = N[k]; }
+            for (int k = 0; k < 6; ++k) { gn[k] = __ldg(M.conn + (size_t)k * M.ne + eb + pe); Nw[k] = N[k]; }
             d = basal_drag_general(P.uv, Heint, deltaint, hint, Hint, rhoint, rhow, g, uint, vint, Cint, mint,
                                    drag_interp<6>(in.drag, gn, Nw));
           }
@@ -619,45 +609,129 @@ __global__ void __launch_bounds__(KW ? 384 : 512) uvh_p2_kernel(DevMesh M, QuadT
       __syncthreads();  // the points are rewritten
     }
     if (el < gn_) {
-      const int t = gb + el;
-      sR[(2 * c * 6 + a) * E + t] = T;
-      sR[((2 * c + 1) * 6 + a) * E + t] = F;
+      const size_t row = 6 * (size_t)(eb + el) + a;
+      rel[6 * row + 2 * c] = T;
+      rel[6 * row + 2 * c + 1] = F;
       if (kw) {
-        double* row = sK + (size_t)(a * 9 + 3 * c) * 6 * E + t;
 #pragma unroll
         for (int b = 0; b < 6; ++b) {
-          row[(0 * 6 + b) * E] = ku[b];
-          row[(1 * 6 + b) * E] = kv[b];
-          row[(2 * 6 + b) * E] = kh[b];
+          double* o = kel + (row * 6 + b) * 9 + 3 * c;
+          o[0] = ku[b];
+          o[1] = kv[b];
+          o[2] = kh[b];
         }
       }
     }
   }
-  __syncthreads();
-  uvh_scatter<6, KW, double>(M, out, p, s, uoff, voff, hoff, sK, sR, E, ne);
 }
 
-static cudaError_t launch_p2h(const ua_mesh* m, const UvhPhys& P, const UvhIn& in, const UvOut& out) {
+// The patches' non-zeros and residuals from the element rows, in increasing global element order.
+template <bool KW>
+__global__ void __launch_bounds__(256) uvh_p2_gather(DevMesh M, const int* active, UvOut out, const double* kel,
+                                                     const double* rel) {
+  const int p = blockIdx.x, s = M.patch_sys[p];
+  if (active && !active[s]) return;
+  const int no = M.sys_node_off[s], nn_s = M.sys_node_off[s + 1] - no;
+  const int uoff = M.sys_dof_off[s] - no, voff = uoff + nn_s, hoff = voff + nn_s;
+  const int e0 = M.patch_elem_ptr[p], ne = M.patch_elem_ptr[p + 1] - e0;
+  (void)ne;  // bounds-checked build
+  const int pn0 = M.patch_node_ptr[p], nr = M.patch_node_ptr[p + 1] - pn0;
+  if (KW) {
+    const int q1 = M.patch_q_ptr[p + 1];
+    const int nbase = M.nodeptr[no], nnzn = M.sys_nnzn[s], kbase = M.sys_knz_off[s];
+    double* Ko = reinterpret_cast<double*>(out.K);
+    for (int q = M.patch_q_ptr[p] + threadIdx.x; q < q1; q += blockDim.x) {
+      const uint32_t rk = __ldg(M.pq_rk + q);
+      const int r = rk >> 16, k = rk & 0xffff;
+      const int gnd = __ldg(M.patch_nodes + pn0 + r);
+      const int np0 = __ldg(M.nodeptr + gnd), deg = __ldg(M.nodeptr + gnd + 1) - np0, lp = np0 - nbase;
+      double v[9] = {};
+      const int cend = __ldg(M.pq_cptr + q + 1);
+      for (int c = __ldg(M.pq_cptr + q); c < cend; ++c) {
+        const uint16_t code = __ldg(M.contrib + c);
+        int ce = code >> 6;
+        const int a = (code >> 3) & 7, b = code & 7;
+        bool ok = true;
+        UA_CHECK_INDEX(M.dbg, ce, 0, ne, BS_CONTRIB_ELEM, ok);
+        if (!ok) continue;
+        const double* src = kel + ((size_t)36 * __ldg(M.patch_elems + e0 + ce) + 6 * a + b) * 9;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) v[i] += src[i];
+      }
+      size_t last = (size_t)kbase + 6 * (size_t)nnzn + 3 * (size_t)lp + 2 * (size_t)deg + k;  // largest index
+      bool okk = true;
+      UA_CHECK_INDEX(M.dbg, last, (size_t)kbase, (size_t)M.sys_knz_off[s + 1], BS_K_INDEX, okk);
+      (void)last;
+      if (!okk) continue;
+#pragma unroll
+      for (int cr = 0; cr < 3; ++cr) {
+        const size_t base = (size_t)kbase + (size_t)cr * 3 * nnzn + 3 * (size_t)lp;
+#pragma unroll
+        for (int cc = 0; cc < 3; ++cc) Ko[base + (size_t)cc * deg + k] = v[cr * 3 + cc];
+      }
+    }
+  }
+  for (int r = threadIdx.x; r < nr; r += blockDim.x) {
+    int gnd = __ldg(M.patch_nodes + pn0 + r);
+    bool okr = true;
+    UA_CHECK_INDEX(M.dbg, gnd, no, no + nn_s, BS_R_INDEX, okr);
+    if (!okr) continue;
+    const int q = __ldg(M.prow_diag + pn0 + r);
+    double acc[6] = {};
+    const int cend = __ldg(M.pq_cptr + q + 1);
+    for (int c = __ldg(M.pq_cptr + q); c < cend; ++c) {
+      const uint16_t code = __ldg(M.contrib + c);
+      int ce = code >> 6;
+      const int a = (code >> 3) & 7;
+      bool ok = true;
+      UA_CHECK_INDEX(M.dbg, ce, 0, ne, BS_CONTRIB_ELEM, ok);
+      if (!ok) continue;
+      const double* src = rel + ((size_t)6 * __ldg(M.patch_elems + e0 + ce) + a) * 6;
+#pragma unroll
+      for (int i = 0; i < 6; ++i) acc[i] += src[i];
+    }
+    out.R[uoff + gnd] = acc[0] - acc[1];
+    out.R[voff + gnd] = acc[2] - acc[3];
+    out.R[hoff + gnd] = acc[4] - acc[5];
+    if (out.Tint) { out.Tint[uoff + gnd] = acc[0]; out.Tint[voff + gnd] = acc[2]; out.Tint[hoff + gnd] = acc[4]; }
+    if (out.Fext) { out.Fext[uoff + gnd] = acc[1]; out.Fext[voff + gnd] = acc[3]; out.Fext[hoff + gnd] = acc[5]; }
+  }
+}
+
+// Groups of the element kernel: 21 elements on 384 threads with the tangent (one CTA an SM), 14 on 252
+// without (two).
+static cudaError_t launch_p2h(ua_mesh* m, const UvhPhys& P, const UvhIn& in, const UvOut& out) {
   using namespace p2h;
   if (quad_table(6).nip != kIps) return cudaErrorInvalidConfiguration;
-  constexpr size_t kLimit = 227 * 1024, kHalf = 113 * 1024;
-  const int E = m->dm.max_patch_elems;
-  const size_t base = (size_t)kIps * 18 * 8 + (size_t)F_COUNT * m->dm.max_patch_hnodes * 8 + (size_t)36 * E * 8 +
-                      (out.K ? (size_t)324 * E * 8 : 0);
-  if (base + kPoint > kLimit) return cudaErrorInvalidConfiguration;
-  // without the tangent two CTAs share an SM if each gets a group of at least eight elements
-  const bool two = base + std::min(8, E) * kPoint <= kHalf;
-  const int rows = two ? 84 : 128;
-  const int G = std::max(1, std::min({(int)(((two ? kHalf : kLimit) - base) / kPoint), rows / 6, E}));
-  const size_t sm = base + (size_t)G * kPoint;
+  const bool kw = out.K != nullptr;
+  const int G = kw ? 21 : 14, rows = kw ? 128 : 84, nsys = (int)m->sys.size();
+  UvhElemRows& B = m->uvh_rows;
+  if (!B.blk[kw]) {
+    std::vector<int4> v;
+    for (int s = 0; s < nsys; ++s)
+      for (int e = m->h_elem_off[s]; e < m->h_elem_off[s + 1]; e += G)
+        v.push_back(make_int4(s, e, std::min(G, m->h_elem_off[s + 1] - e), 0));
+    int4* d = (int4*)dev_alloc(m, sizeof(int4) * std::max<size_t>(v.size(), 1));
+    if (!d) return cudaErrorMemoryAllocation;
+    cudaError_t e = cudaMemcpy(d, v.data(), sizeof(int4) * v.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return e;
+    B.blk[kw] = d;
+    B.n[kw] = (int)v.size();
+  }
+  if (!B.rel && !(B.rel = (double*)dev_alloc(m, sizeof(double) * 36 * (size_t)m->dm.ne))) return cudaErrorMemoryAllocation;
+  if (kw && !B.kel && !(B.kel = (double*)dev_alloc(m, sizeof(double) * 324 * (size_t)m->dm.ne)))
+    return cudaErrorMemoryAllocation;
+  const size_t sm = (size_t)G * kPoint + (size_t)kIps * 18 * 8 + (size_t)F_COUNT * 6 * G * 8;
   const bool gen = P.uv.law != UA_SLIDING_WEERTMAN || P.uv.melange;
-  auto kern = out.K ? (gen ? uvh_p2_kernel<true, true> : uvh_p2_kernel<false, true>)
-                    : (gen ? uvh_p2_kernel<true, false> : uvh_p2_kernel<false, false>);
+  auto kern = kw ? (gen ? uvh_p2_elements<true, true> : uvh_p2_elements<false, true>)
+                 : (gen ? uvh_p2_elements<true, false> : uvh_p2_elements<false, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
-  kern<<<m->dm.npatch, two ? 256 : 384, sm, m->stream>>>(m->dm, quad_table(6), P, in, out, G, rows);
+  if (B.n[kw]) kern<<<B.n[kw], kw ? 384 : 256, sm, m->stream>>>(m->dm, quad_table(6), P, in, B.blk[kw], G, rows, B.kel, B.rel);
+  if (kw) uvh_p2_gather<true><<<m->dm.npatch, 256, 0, m->stream>>>(m->dm, in.active, out, B.kel, B.rel);
+  else uvh_p2_gather<false><<<m->dm.npatch, 256, 0, m->stream>>>(m->dm, in.active, out, B.kel, B.rel);
   return cudaGetLastError();
 }
 
@@ -687,7 +761,7 @@ static cudaError_t launch_t(const ua_mesh* m, const UvhPhys& P, const UvhIn& in,
   return cudaGetLastError();
 }
 
-cudaError_t launch_uvh_assembly(const ua_mesh* m, const UvhPhys& P, const UvhIn& in, const UvOut& out, bool withK) {
+cudaError_t launch_uvh_assembly(ua_mesh* m, const UvhPhys& P, const UvhIn& in, const UvOut& out, bool withK) {
   if (m->nod == 3) return withK ? launch_t<3, true, double>(m, P, in, out) : launch_t<3, false, double>(m, P, in, out);
   UvOut o = out;
   if (!withK) o.K = nullptr;
