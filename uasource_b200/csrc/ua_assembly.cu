@@ -407,49 +407,45 @@ size_t uv_p1_smem(bool withK, bool fp32, int E, int threads, int MH) {
 // with 2x2 matrices of the point: the ones in x and y (the Newton viscosity term is the rank-one
 // product of P_u = p1 Dx + q2 Dy and P_v = q1 Dy + q2 Dx) between the point's inverse Jacobian and
 // its transpose.  d_a and N_a are the same for every element, so what an element adds is 25
-// coefficients a point.  A patch's elements go in groups: (a) a thread per element and point
+// coefficients a point.  A CTA takes a group of elements: (a) a thread per element and point
 // interpolates, evaluates the physics once and leaves the coefficients in shared memory, kIpc points
 // at a time; (b) a thread per element and node a accumulates its rows of the three blocks and its
-// residual parts over those points in registers.  Then the patch's segmented sum (patch_scatter).
+// residual parts over those points in registers and writes them to global memory (78 values an element
+// and 24 residual parts).  A second kernel sums each patch's non-zeros over them.
 //
 // One thread per element held 78 + 24 accumulators and 78 nodal values, spilled most of them and ran
 // four warps per SM: 1.55 ms (tangent) and 0.52 ms (residual) for 160,000 elements in FP64, where
-// this split takes 0.76 and 0.34 ms (mixed, 10,000 elements: 0.36 and 0.15 before, 0.070 and 0.046
-// now).  At 128 registers two CTAs share an SM and hide each other's
-// staging and barriers (residual 0.34 ms against 0.52 with one CTA of 168 registers); the FP64
-// tangent needs the whole SM's shared memory and runs one.  The residual-only pass runs the same
-// code with the tangent's part switched off, so its R is the same bit for bit.  All of it in FP64;
-// the mixed form rounds the finished element entries.
+// this split took 0.76 and 0.34 ms with the rows in shared memory, a patch at a time, every element in
+// about two patches; with the rows through global memory 0.45 and 0.20 ms (mixed, 10,000 elements: 0.069 and 0.045, now 0.048 and 0.031).  At 128 registers two CTAs share an SM
+// and hide each other's staging and barriers.  The residual-only pass runs the same code with the
+// tangent's part switched off, so its R is the same bit for bit.  All of it in FP64; the mixed form rounds
+// the finished element entries.
 namespace p2 {
-constexpr int kMaxG = 64, kMaxG2 = 42, kIpc = 6, kIps = 16;
+constexpr int kMaxG = 42, kMinG = 8, kIpc = 6, kIps = 16;  // elements of a group
 // staged node fields
 enum { ND_X = 0, ND_Y, ND_H, ND_BL, ND_U, ND_V, ND_C, ND_A, ND_HB, ND_RHO, ND_M, ND_N, ND_COUNT };
 // pairs of coefficients of a point
 enum { PR_UU = 0, PR_UUC, PR_VV, PR_VVC, PR_UV1, PR_UV2, PR_XV, PR_TX, PR_TY, PR_PX, PR_PY, PR_TN, PR_FN, kPairs };
 }  // namespace p2
 
-// One build for both launch shapes (128 registers): builds with other budgets round differently, and K and
-// R must not depend on the patches (a build of 168 for the one-CTA shape was 3% faster on P2 401x201, 763
-// against 790 us).
+// blk: {system, first element, elements} of each block, at most G elements.  Rows of element e: tangent
+// kel[78 e + ..] (uu and vv upper triangles, then uv), residual parts rel[24 e + 6 part + a].
 template <typename KT, bool GEN>
-__global__ void __launch_bounds__(512) uv_p2_kernel(DevMesh M, QuadTable Q, UvPhys P, UvIn in,
-                                                                               UvOut out, int G) {
+__global__ void __launch_bounds__(256, 2) uv_p2_elements(DevMesh M, QuadTable Q, UvPhys P, UvIn in, const int4* blk, int G,
+                                                         KT* kel, double* rel) {
   using namespace p2;
   using p1::tanh_step;
   using I = ElemIdx<6>;
   extern __shared__ __align__(16) unsigned char smem[];
-  const int p = blockIdx.x;
-  const int s = M.patch_sys[p];
+  const int4 bk = blk[blockIdx.x];
+  const int s = bk.x, eb = bk.y, gn_ = bk.z;
   if (in.active && !in.active[s]) return;
-  const bool kw = out.K != nullptr;
-  const int E = M.max_patch_elems, MH = M.max_patch_hnodes;
+  const bool kw = kel != nullptr;
+  const int MH = 6 * G;
   double2* pts = reinterpret_cast<double2*>(smem);  // [G][kIpc][kPairs]
   double2* sD = pts + (size_t)G * kIpc * kPairs;              // reference derivatives [ip][6]
   double* sN = reinterpret_cast<double*>(sD + kIps * 6);      // N [ip][6], then the weights
-  double* nd = sN + kIps * 7;
-  double* sR = nd + (size_t)ND_COUNT * MH;
-  KT* sK = reinterpret_cast<KT*>(sR + (size_t)24 * E);
-  const int e0 = M.patch_elem_ptr[p], ne = M.patch_elem_ptr[p + 1] - e0;
+  double* nd = sN + kIps * 7;                                 // [ND_COUNT][MH], node k of element el at 6 el + k
   const int uoff = M.sys_dof_off[s] - M.sys_node_off[s];
   const int voff = uoff + (M.sys_node_off[s + 1] - M.sys_node_off[s]);
   const double gam = in.gamma ? in.gamma[s] : 0.0;
@@ -461,9 +457,8 @@ __global__ void __launch_bounds__(512) uv_p2_kernel(DevMesh M, QuadTable Q, UvPh
     sD[t] = make_double2(Q.der[t / 6][0][t % 6], Q.der[t / 6][1][t % 6]);
   }
   for (int t = threadIdx.x; t < kIps; t += blockDim.x) sN[kIps * 6 + t] = Q.w[t];
-  const int hb0 = M.patch_hnode_ptr[p], nh = M.patch_hnode_ptr[p + 1] - hb0;
-  for (int t = threadIdx.x; t < nh; t += blockDim.x) {
-    int gn = __ldg(M.patch_hnodes + hb0 + t);
+  for (int t = threadIdx.x; t < 6 * gn_; t += blockDim.x) {
+    int gn = __ldg(M.conn + (size_t)(t % 6) * M.ne + eb + t / 6);
     bool okn = true;
     UA_CHECK_INDEX(M.dbg, gn, M.sys_node_off[s], M.sys_node_off[s + 1], BS_ELEM_NODE, okn);
     (void)okn;
@@ -481,9 +476,7 @@ __global__ void __launch_bounds__(512) uv_p2_kernel(DevMesh M, QuadTable Q, UvPh
   }
   __syncthreads();
   const double rhow = S.rhow, g = S.g, ca = S.ca, sa = S.sa;
-  const int ngr = (ne + G - 1) / G, gs = (ne + ngr - 1) / ngr;  // groups of equal size
-  for (int gb = 0; gb < ne; gb += gs) {
-    const int gn_ = min(gs, ne - gb);
+  {
     // rows of this thread: element el of the group, node a
     const int el = threadIdx.x / 6, a = threadIdx.x - 6 * el;
     double kuu[6] = {}, kvv[6] = {}, kuv[6] = {}, Tx = 0, Fx = 0, Ty = 0, Fy = 0;
@@ -492,15 +485,9 @@ __global__ void __launch_bounds__(512) uv_p2_kernel(DevMesh M, QuadTable Q, UvPh
       // (a) points
       for (int t = threadIdx.x; t < gn_ * nip; t += blockDim.x) {
         const int pe = t / nip, pi = t - pe * nip, ip = ip0 + pi;
-        const uint16_t* ln = M.patch_elnodes + (size_t)(e0 + gb + pe) * 6;
         int l[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          l[k] = __ldg(ln + k);
-          bool okn = true;
-          UA_CHECK_INDEX(M.dbg, l[k], 0, nh, BS_ELEM_NODE, okn);
-          (void)okn;
-        }
+        for (int k = 0; k < 6; ++k) l[k] = 6 * pe + k;
         const double* N = sN + ip * 6;
         // derivVector.m:96-109, gradients by the chain rule
         double J11 = 0, J12 = 0, J21 = 0, J22 = 0, u1 = 0, u2 = 0, v1 = 0, v2 = 0, b1 = 0, b2 = 0;
@@ -546,7 +533,7 @@ __global__ void __launch_bounds__(512) uv_p2_kernel(DevMesh M, QuadTable Q, UvPh
           int gn[6];
           double Nw[6];
 #pragma unroll
-          for (int k = 0; k < 6; ++k) { gn[k] = __ldg(M.patch_hnodes + hb0 + l[k]); Nw[k] = N[k]; }
+          for (int k = 0; k < 6; ++k) { gn[k] = __ldg(M.conn + (size_t)k * M.ne + eb + pe); Nw[k] = N[k]; }
           d = basal_drag_general(P, Heint, 0.0, hint, Hint, rhoint, rhow, g, uint, vint, Cint, mint,
                                  drag_interp<6>(in.drag, gn, Nw));
         } else if (Heint > 0) {
@@ -621,34 +608,103 @@ __global__ void __launch_bounds__(512) uv_p2_kernel(DevMesh M, QuadTable Q, UvPh
       __syncthreads();  // the points are rewritten
     }
     if (el < gn_) {
-      const int t = gb + el;
-      sR[(0 * 6 + a) * E + t] = Tx;
-      sR[(1 * 6 + a) * E + t] = Fx;
-      sR[(2 * 6 + a) * E + t] = Ty;
-      sR[(3 * 6 + a) * E + t] = Fy;
+      double* r = rel + 24 * (size_t)(eb + el) + a;
+      r[0] = Tx;
+      r[6] = Fx;
+      r[12] = Ty;
+      r[18] = Fy;
       if (kw) {
+        KT* o = kel + (size_t)I::NKE * (eb + el);
 #pragma unroll
         for (int b = 0; b < 6; ++b) {
           if (b >= a) {  // the symmetric blocks keep their upper triangle
             const int y = I::sym(a, b);
-            sK[y * E + t] = (KT)kuu[b];
-            sK[(I::NS + y) * E + t] = (KT)kvv[b];
+            o[y] = (KT)kuu[b];
+            o[I::NS + y] = (KT)kvv[b];
           }
-          sK[(2 * I::NS + a * 6 + b) * E + t] = (KT)kuv[b];
+          o[2 * I::NS + a * 6 + b] = (KT)kuv[b];
         }
       }
     }
   }
-  __syncthreads();
-  patch_scatter<6, true, KT>(M, out, p, s, uoff, voff, sK, sR, E);
 }
 
-// shared memory of the P2 kernel without its points, and of one element's points
-static size_t uv_p2_smem_base(bool withK, bool fp32, int E, int MH) {
-  return (size_t)p2::kIps * 19 * 8 + (size_t)p2::ND_COUNT * MH * 8 + (size_t)24 * E * 8 +
-         (withK ? (size_t)ElemIdx<6>::NKE * E * (fp32 ? 4 : 8) : 0);
+// The patches' non-zeros and residuals from the element rows (the sums of patch_scatter).
+template <typename KT>
+__global__ void __launch_bounds__(256) uv_p2_gather(DevMesh M, const int* active, UvOut out, const KT* kel,
+                                                    const double* rel) {
+  using I = ElemIdx<6>;
+  const int p = blockIdx.x, s = M.patch_sys[p];
+  if (active && !active[s]) return;
+  const int uoff = M.sys_dof_off[s] - M.sys_node_off[s];
+  const int voff = uoff + (M.sys_node_off[s + 1] - M.sys_node_off[s]);
+  const int e0 = M.patch_elem_ptr[p], nep = M.patch_elem_ptr[p + 1] - e0;
+  (void)nep;  // bounds-checked build
+  const int pn0 = M.patch_node_ptr[p], nr = M.patch_node_ptr[p + 1] - pn0;
+  if (out.K) {
+    const int q1 = M.patch_q_ptr[p + 1], nbase = M.nodeptr[M.sys_node_off[s]], nnzn = M.sys_nnzn[s],
+              kbase = M.sys_knz_off[s];
+    for (int t = M.patch_q_ptr[p] + threadIdx.x; t < q1; t += blockDim.x) {
+      const uint32_t rk = __ldg(M.pq_rk + t);
+      const int r = rk >> 16, k = rk & 0xffff;
+      const int g = __ldg(M.patch_nodes + pn0 + r);
+      const int np0 = __ldg(M.nodeptr + g), deg = __ldg(M.nodeptr + g + 1) - np0, lp = np0 - nbase;
+      KT uu = 0, vv = 0, uv = 0, vu = 0;
+      const int c1 = __ldg(M.pq_cptr + t + 1);
+      for (int c = __ldg(M.pq_cptr + t); c < c1; ++c) {
+        const uint16_t code = __ldg(M.contrib + c);
+        int el = code >> 6;
+        const int a = (code >> 3) & 7, b = code & 7;
+        bool ok = true;
+        UA_CHECK_INDEX(M.dbg, el, 0, nep, BS_CONTRIB_ELEM, ok);
+        if (!ok) continue;
+        const KT* o = kel + (size_t)I::NKE * __ldg(M.patch_elems + e0 + el);
+        const int sy = I::sym(a, b);
+        uu += o[sy];
+        vv += o[I::NS + sy];
+        uv += o[2 * I::NS + a * 6 + b];
+        vu += o[2 * I::NS + b * 6 + a];
+      }
+      size_t b0 = (size_t)kbase + 2 * (size_t)lp;
+      size_t b1 = (size_t)kbase + 2 * (size_t)nnzn + 2 * (size_t)lp;
+      bool okk = true;
+      UA_CHECK_INDEX(M.dbg, b0, (size_t)kbase, (size_t)M.sys_knz_off[s + 1] - deg - k, BS_K_INDEX, okk);
+      UA_CHECK_INDEX(M.dbg, b1, (size_t)kbase, (size_t)M.sys_knz_off[s + 1] - deg - k, BS_K_INDEX, okk);
+      if (!okk) continue;
+      KT* Ko = reinterpret_cast<KT*>(out.K);
+      Ko[b0 + k] = uu;
+      Ko[b0 + deg + k] = uv;
+      Ko[b1 + k] = vu;
+      Ko[b1 + deg + k] = vv;
+    }
+  }
+  for (int r = threadIdx.x; r < nr; r += blockDim.x) {
+    int g = __ldg(M.patch_nodes + pn0 + r);
+    bool okr = true;
+    UA_CHECK_INDEX(M.dbg, g, M.sys_node_off[s], M.sys_node_off[s + 1], BS_R_INDEX, okr);
+    if (!okr) continue;
+    const int t = __ldg(M.prow_diag + pn0 + r);
+    double tx = 0, fx = 0, ty = 0, fy = 0;
+    const int c1 = __ldg(M.pq_cptr + t + 1);
+    for (int c = __ldg(M.pq_cptr + t); c < c1; ++c) {
+      const uint16_t code = __ldg(M.contrib + c);
+      int el = code >> 6;
+      const int a = (code >> 3) & 7;
+      bool ok = true;
+      UA_CHECK_INDEX(M.dbg, el, 0, nep, BS_CONTRIB_ELEM, ok);
+      if (!ok) continue;
+      const double* o = rel + 24 * (size_t)__ldg(M.patch_elems + e0 + el) + a;
+      tx += o[0];
+      fx += o[6];
+      ty += o[12];
+      fy += o[18];
+    }
+    out.R[uoff + g] = tx - fx;
+    out.R[voff + g] = ty - fy;
+    if (out.Tint) { out.Tint[uoff + g] = tx; out.Tint[voff + g] = ty; }
+    if (out.Fext) { out.Fext[uoff + g] = fx; out.Fext[voff + g] = fy; }
+  }
 }
-constexpr size_t kP2Point = (size_t)p2::kIpc * p2::kPairs * sizeof(double2);
 
 template <bool WITHK, typename KT, bool GEN>
 static auto p1_kernel(int rv) {
@@ -674,34 +730,44 @@ static cudaError_t launch_p1(const ua_mesh* m, const UvPhys& P, const UvIn& in, 
   return cudaGetLastError();
 }
 
+// Groups of up to kMaxG elements (two CTAs of 77 kB an SM), fewer on meshes that would leave SMs idle.
 template <typename KT>
-static cudaError_t launch_p2(const ua_mesh* m, const UvPhys& P, const UvIn& in, const UvOut& out) {
-  if (quad_table(6).nip != p2::kIps) return cudaErrorInvalidConfiguration;
-  constexpr size_t kLimit = 227 * 1024, kHalf = 113 * 1024;
-  const int E = m->dm.max_patch_elems;
-  const size_t base = uv_p2_smem_base(out.K != nullptr, sizeof(KT) == 4, E, m->dm.max_patch_hnodes);
-  if (base + kP2Point > kLimit) return cudaErrorInvalidConfiguration;
-  // elements of a group: what the shared memory of half an SM takes if that is 12 or more (two CTAs
-  // hide each other's staging and barriers), else of the whole one
-  int G = base < kHalf ? (int)((kHalf - base) / kP2Point) : 0;
-  const bool two = G >= std::min(12, E);
-  if (two) G = std::min(G, p2::kMaxG2);
-  else G = std::min((int)((kLimit - base) / kP2Point), p2::kMaxG);
-  G = std::max(1, std::min(G, E));
-  const size_t sm = base + (size_t)G * kP2Point;
+static cudaError_t launch_p2(ua_mesh* m, const UvPhys& P, const UvIn& in, const UvOut& out) {
+  using namespace p2;
+  if (quad_table(6).nip != kIps) return cudaErrorInvalidConfiguration;
+  const int nsys = (int)m->sys.size();
+  UvElemRows& B = m->uv_rows;
+  if (!B.blk) {
+    B.G = std::min(kMaxG, std::max(kMinG, (m->dm.ne + 295) / 296));
+    std::vector<int4> v;
+    for (int s = 0; s < nsys; ++s)
+      for (int e = m->h_elem_off[s]; e < m->h_elem_off[s + 1]; e += B.G)
+        v.push_back(make_int4(s, e, std::min(B.G, m->h_elem_off[s + 1] - e), 0));
+    int4* d = (int4*)dev_alloc(m, sizeof(int4) * std::max<size_t>(v.size(), 1));
+    if (!d) return cudaErrorMemoryAllocation;
+    cudaError_t e = cudaMemcpy(d, v.data(), sizeof(int4) * v.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return e;
+    B.blk = d;
+    B.n = (int)v.size();
+  }
+  void*& kel = sizeof(KT) == 4 ? B.kel32 : B.kel64;
+  if (!B.rel && !(B.rel = (double*)dev_alloc(m, sizeof(double) * 24 * (size_t)m->dm.ne))) return cudaErrorMemoryAllocation;
+  if (out.K && !kel && !(kel = dev_alloc(m, sizeof(KT) * ElemIdx<6>::NKE * (size_t)m->dm.ne))) return cudaErrorMemoryAllocation;
+  KT* k = out.K ? (KT*)kel : nullptr;
+  const size_t sm = (size_t)B.G * kIpc * kPairs * sizeof(double2) + (size_t)kIps * 19 * 8 + (size_t)ND_COUNT * 6 * B.G * 8;
   const bool gen = P.law != UA_SLIDING_WEERTMAN || P.melange;
-  auto kern = gen ? uv_p2_kernel<KT, true> : uv_p2_kernel<KT, false>;
+  auto kern = gen ? uv_p2_elements<KT, true> : uv_p2_elements<KT, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
-  const int threads = std::max(128, (6 * G + 31) & ~31);
-  kern<<<m->dm.npatch, threads, sm, m->stream>>>(m->dm, quad_table(6), P, in, out, G);
+  if (B.n) kern<<<B.n, 256, sm, m->stream>>>(m->dm, quad_table(6), P, in, B.blk, B.G, k, B.rel);
+  uv_p2_gather<KT><<<m->dm.npatch, 256, 0, m->stream>>>(m->dm, in.active, out, k, B.rel);
   return cudaGetLastError();
 }
 
 // threads: CTA size of the P1 kernel (128 or 256; 0 = 256); regs: its register budget (128, 96, 80)
-cudaError_t launch_uv_assembly(const ua_mesh* m, const UvPhys& P, const UvIn& in, const UvOut& out, bool withK,
+cudaError_t launch_uv_assembly(ua_mesh* m, const UvPhys& P, const UvIn& in, const UvOut& out, bool withK,
                                bool fp32K, int threads, int regs) {
   if (m->nod == 3) {  // residual-only: the tangent instantiation of the precision with out.K null
     UvOut o = out;

@@ -143,8 +143,14 @@ struct AsmTuning {
   int regs = 128;  // register budget of the P1 kernel: 128, 96 (128-thread CTAs) or 80
 };
 
-// Element rows of the P2 uvh assembly and the blocks of its element kernel (without, with the tangent),
-// on first use.
+// Element rows of the P2 assemblies and the blocks of their element kernels (uvh: without, with the
+// tangent), on first use.
+struct UvElemRows {  // P2 uv
+  void *kel32 = nullptr, *kel64 = nullptr;
+  double* rel = nullptr;
+  int4* blk = nullptr;
+  int n = 0, G = 0;
+};
 struct UvhElemRows {
   double *kel = nullptr, *rel = nullptr;
   int4* blk[2] = {nullptr, nullptr};
@@ -189,6 +195,7 @@ struct ua_mesh {
   std::vector<ua::HostSystem> sys;
   // host copies of symbolic data needed on the host
   std::vector<int> h_node_off, h_dof_off, h_knz_off, h_nnzn, h_elem_off;
+  ua::UvElemRows uv_rows;
   ua::UvhElemRows uvh_rows;
   std::vector<int> h_nodeptr, h_nodecol;
   int nn_total = 0, ne_total = 0, ndof_total = 0;

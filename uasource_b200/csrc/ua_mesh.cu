@@ -224,9 +224,6 @@ static int build_patch_plan(const ua_mesh* m, const std::vector<int>& conn, cons
   const std::vector<int>& nodeptr = m->h_nodeptr;
   const std::vector<int>& nodecol = m->h_nodecol;
   const int emax = max_patch_elements(nod, m->ndof);
-  // the P2 uv kernel also stages the nodes of the patch's elements: 160 elements fit with six nodes
-  // of their own each, a single node's fan (three nodes per element) fits up to emax
-  const int esoft = nod == 6 && m->ndof == 2 ? std::min(emax, 160) : emax;
   std::vector<int> mark(NE, -1), elocal(NE, -1);
   for (int s = 0; s < nsys; ++s) {
     int no = m->h_node_off[s], nn = m->sys[s].nn;
@@ -253,7 +250,7 @@ static int build_patch_plan(const ua_mesh* m, const std::vector<int>& conn, cons
         int g = key[idx].second;
         int add = 0;
         for (int t = n2e_ptr[g]; t < n2e_ptr[g + 1]; ++t) add += (mark[n2e[t]] != stamp);
-        if (!nodes.empty() && (int)elems.size() + add > esoft) break;
+        if (!nodes.empty() && (int)elems.size() + add > emax) break;
         if ((int)elems.size() + add > emax) return set_error(UA_ERR_BAD_MESH, "node %d touches too many elements", g);
         nodes.push_back(g);
         for (int t = n2e_ptr[g]; t < n2e_ptr[g + 1]; ++t)
