@@ -416,8 +416,9 @@ size_t uv_p1_smem(bool withK, bool fp32, int E, int threads, int MH) {
 // One thread per element held 78 + 24 accumulators and 78 nodal values, spilled most of them and ran
 // four warps per SM: 1.55 ms (tangent) and 0.52 ms (residual) for 160,000 elements in FP64, where
 // this split took 0.76 and 0.34 ms with the rows in shared memory, a patch at a time, every element in
-// about two patches; with the rows through global memory 0.45 and 0.20 ms (mixed, 10,000 elements: 0.069 and 0.045, now 0.048 and 0.031).  At 128 registers two CTAs share an SM
-// and hide each other's staging and barriers.  The residual-only pass runs the same code with the
+// about two patches; with the rows through global memory 0.45 and 0.20 ms (mixed, 10,000 elements:
+// 0.069 and 0.045, now 0.048 and 0.031).  At 128 registers two CTAs share an SM and hide each other's
+// staging and barriers.  The residual-only pass runs the same code with the
 // tangent's part switched off, so its R is the same bit for bit.  All of it in FP64; the mixed form rounds
 // the finished element entries.
 namespace p2 {
