@@ -1603,7 +1603,7 @@ static void csell_init(ua_mesh* m) {
     Sell& S = a->csell[l];
     if (L.nn < kCsellMinNodes) continue;
     std::vector<int> rowptr(L.ndof + 1);
-    if (cudaMemcpy(rowptr.data(), L.rowptr, sizeof(int) * rowptr.size(), cudaMemcpyDeviceToHost) != cudaSuccess) {
+    if (dev_read(m, rowptr.data(), L.rowptr, sizeof(int) * rowptr.size()) != cudaSuccess) {
       S.failed = true;
       return;
     }

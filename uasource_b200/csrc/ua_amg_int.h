@@ -249,7 +249,7 @@ template <class T>
 inline T* upload(ua_mesh* m, Amg* a, const std::vector<T>& v, bool& ok) {
   T* d = (T*)dev_alloc(m, std::max<size_t>(1, v.size()) * sizeof(T));
   if (!d) { ok = false; return nullptr; }
-  if (!v.empty() && cudaMemcpy(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) ok = false;
+  if (!v.empty() && dev_write(m, d, v.data(), v.size() * sizeof(T)) != cudaSuccess) ok = false;
   a->bytes += v.size() * sizeof(T);
   return d;
 }

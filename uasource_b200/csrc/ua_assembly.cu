@@ -746,7 +746,7 @@ static cudaError_t launch_p2(ua_mesh* m, const UvPhys& P, const UvIn& in, const 
         v.push_back(make_int4(s, e, std::min(B.G, m->h_elem_off[s + 1] - e), 0));
     int4* d = (int4*)dev_alloc(m, sizeof(int4) * std::max<size_t>(v.size(), 1));
     if (!d) return cudaErrorMemoryAllocation;
-    cudaError_t e = cudaMemcpy(d, v.data(), sizeof(int4) * v.size(), cudaMemcpyHostToDevice);
+    cudaError_t e = dev_write(m, d, v.data(), sizeof(int4) * v.size());
     if (e != cudaSuccess) return e;
     B.blk = d;
     B.n = (int)v.size();

@@ -228,6 +228,12 @@ int rebuild_patches(ua_mesh* m, PatchShape shape);
 AsmTuning tuned_assembly(int device, int nod, int ndof, bool* tuned = nullptr);
 void set_tuned_assembly(int device, int nod, int ndof, AsmTuning t);
 int set_error(int code, const char* fmt, ...);
+// Copies between the host and the device that are over on return, and a clear, all on the handle's stream.
+// That stream is created non-blocking, so nothing on the legacy stream is ordered before its kernels; and
+// cudaMemcpy from pageable memory may return when the data is staged, before it is on the device.
+cudaError_t dev_write(const ua_mesh* m, void* d, const void* h, size_t bytes);
+cudaError_t dev_read(const ua_mesh* m, void* h, const void* d, size_t bytes);
+cudaError_t dev_clear(const ua_mesh* m, void* d, size_t bytes);
 const QuadTable& quad_table(int nod);
 }  // namespace ua
 

@@ -48,6 +48,16 @@ void dev_free(ua_mesh* m, const void* p) {
     }
 }
 
+cudaError_t dev_write(const ua_mesh* m, void* d, const void* h, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, m->stream);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(m->stream);
+}
+cudaError_t dev_read(const ua_mesh* m, void* h, const void* d, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, m->stream);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(m->stream);
+}
+cudaError_t dev_clear(const ua_mesh* m, void* d, size_t bytes) { return cudaMemsetAsync(d, 0, bytes, m->stream); }
+
 void dev_free_all(ua_mesh* m) {
   for (auto& b : m->owned) cudaFree(b.ptr);
   m->owned.clear();
@@ -140,7 +150,7 @@ using namespace ua;
 static int upload(ua_mesh* m, const void* h, size_t bytes, void** d) {
   *d = dev_alloc(m, bytes);
   if (!*d) return set_error(UA_ERR_OOM, "device allocation of %zu bytes failed", bytes);
-  if (bytes) UA_CUDA_TRY(cudaMemcpy(*d, h, bytes, cudaMemcpyHostToDevice));
+  if (bytes) UA_CUDA_TRY(dev_write(m, *d, h, bytes));
   return UA_OK;
 }
 
@@ -554,8 +564,7 @@ extern "C" int ua_debug_bounds(const ua_mesh* m, int32_t* enabled, int32_t* site
   *enabled = 1;
   unsigned long long v = 0;
   UA_CUDA_TRY(cudaSetDevice(m->device));
-  UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
-  UA_CUDA_TRY(cudaMemcpy(&v, m->dm.dbg, sizeof(v), cudaMemcpyDeviceToHost));
+  UA_CUDA_TRY(dev_read(m, &v, m->dm.dbg, sizeof(v)));
   *site = (int32_t)(v >> 48);
   *index = (int64_t)(v & 0xffffffffffffULL);
 #else

@@ -889,11 +889,11 @@ const int* resident_error_flag(const ua_mesh* m) { return m->amg->cyc.d_sched; }
 int pcg_resident_status(ua_mesh* m, bool prof, double* ms, int* cnt) {
   Cycle& C = m->amg->cyc;
   int err = 0;
-  UA_CUDA_TRY(cudaMemcpy(&err, C.d_sched, sizeof(int), cudaMemcpyDeviceToHost));
+  UA_CUDA_TRY(dev_read(m, &err, C.d_sched, sizeof(int)));
   if (err) return set_error(UA_ERR_TIMEOUT, "resident solve: a team barrier was not met");
   if (prof) {
     unsigned long long h[2 * CP_COUNT];
-    UA_CUDA_TRY(cudaMemcpy(h, C.d_prof, sizeof(h), cudaMemcpyDeviceToHost));
+    UA_CUDA_TRY(dev_read(m, h, C.d_prof, sizeof(h)));
     for (int k = 0; k < CP_COUNT; ++k) {
       ms[k] += 1e-6 * (double)h[2 * k] / std::max(C.last_grid, 1);
       cnt[k] += (int)h[2 * k + 1];

@@ -212,12 +212,13 @@ static void prof_begin(ua_mesh* m, int kind, cudaEvent_t* ev) {
 }
 
 // Summed launch times, launch counts and work per timed kernel class.
-static void prof_collect(Work* w, double* kms, int* kn, double* knnz, double* krows) {
+static void prof_collect(const ua_mesh* m, double* kms, int* kn, double* knnz, double* krows) {
+  Work* w = m->work;
   const int nm = (int)w->prof.marks.size();
   std::vector<long long> act;
   if (w->prof.d_act && nm) {
     act.resize(2 * (size_t)std::min(nm, w->prof.act_cap));
-    cudaMemcpy(act.data(), w->prof.d_act, act.size() * sizeof(long long), cudaMemcpyDeviceToHost);
+    if (dev_read(m, act.data(), w->prof.d_act, act.size() * sizeof(long long)) != cudaSuccess) act.clear();
   }
   for (int i = 0; i < nm; ++i) {
     const auto& mk = w->prof.marks[i];
@@ -839,7 +840,7 @@ static int ensure_work(ua_mesh* m, const ua_params* p) {
   auto up = [&](const std::vector<int>& v) -> int* {
     int* d = walloc<int>(m, v.size());
     if (!d) { ok = false; return nullptr; }
-    cudaMemcpy(d, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice);
+    if (dev_write(m, d, v.data(), v.size() * sizeof(int)) != cudaSuccess) ok = false;
     return d;
   };
   w->rb_start = up(rb_start);
@@ -864,7 +865,7 @@ static int ensure_work(ua_mesh* m, const ua_params* p) {
   w->part = walloc<double>(m, 4 * (size_t)w->nrb);
   w->sysv = walloc<double>(m, SV_COUNT * (size_t)nsys);
   w->arrived = walloc<int>(m, nsys);
-  if (w->arrived) UA_CUDA_TRY(cudaMemset(w->arrived, 0, sizeof(int) * nsys));
+  if (w->arrived) UA_CUDA_TRY(dev_clear(m, w->arrived, sizeof(int) * nsys));
   w->done = walloc<int>(m, nsys);
   w->its = walloc<int>(m, nsys);
   w->status = walloc<int>(m, nsys);
@@ -3391,7 +3392,7 @@ static int newton_common(ua_mesh* m, const ua_params* p, ua_fields* F, const ua_
   cudaEventElapsedTime(&dev_ms, call_ev[0], call_ev[1]);
   double kms[PK_COUNT] = {}, knnz[PK_COUNT] = {}, krows[PK_COUNT] = {};
   int kn[PK_COUNT] = {};
-  prof_collect(w, kms, kn, knnz, krows);
+  prof_collect(m, kms, kn, knnz, krows);
   bool all_conv = true;
   for (int s = 0; s < nsys; ++s) {
     if (rep[s]) {
@@ -3417,14 +3418,14 @@ extern "C" int ua_uv_newton(ua_mesh* m, const ua_params* p, ua_fields* F, const 
   m->keep_last_tangent = false;
   if (rc != UA_OK && rc != UA_ERR_NOT_CONVERGED) return rc;
   Work* w = m->work;
-  if (R) UA_CUDA_TRY(cudaMemcpy(R, w->R, m->ndof_total * sizeof(double), cudaMemcpyDeviceToHost));
+  if (R) UA_CUDA_TRY(dev_read(m, R, w->R, m->ndof_total * sizeof(double)));
   if (Kvals) {
     if (p->precision == UA_PREC_MIXED) {
       std::vector<float> tmp(m->nnz_total);
-      UA_CUDA_TRY(cudaMemcpy(tmp.data(), w->Kf, tmp.size() * sizeof(float), cudaMemcpyDeviceToHost));
+      UA_CUDA_TRY(dev_read(m, tmp.data(), w->Kf, tmp.size() * sizeof(float)));
       for (size_t i = 0; i < tmp.size(); ++i) Kvals[i] = tmp[i];
     } else {
-      UA_CUDA_TRY(cudaMemcpy(Kvals, w->Kd, m->nnz_total * sizeof(double), cudaMemcpyDeviceToHost));
+      UA_CUDA_TRY(dev_read(m, Kvals, w->Kd, m->nnz_total * sizeof(double)));
     }
   }
   return rc;
@@ -3568,8 +3569,18 @@ extern "C" int ua_solve_kape_symmetric(int32_t n, const int64_t* Arowptr, const 
     rb_start.push_back(n);
     w->h_sys_rb_off = {0, w->nrb};
     std::vector<int> sel1 = {1}, coff = {0, (int)con_dof.size()}, csys(con_dof.size(), 0);
-    auto up_i = [&](const std::vector<int>& v) { int* d = walloc<int>(&tmp, v.size()); if (d) cudaMemcpy(d, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice); return d; };
-    auto up_d = [&](const double* v, size_t k) { double* d = walloc<double>(&tmp, k); if (d && k) cudaMemcpy(d, v, k * sizeof(double), cudaMemcpyHostToDevice); return d; };
+    cudaError_t cp = cudaSuccess;
+    auto copied = [&](cudaError_t e) { if (cp == cudaSuccess) cp = e; };
+    auto up_i = [&](const std::vector<int>& v) {
+      int* d = walloc<int>(&tmp, v.size());
+      if (d) copied(dev_write(&tmp, d, v.data(), v.size() * sizeof(int)));
+      return d;
+    };
+    auto up_d = [&](const double* v, size_t k) {
+      double* d = walloc<double>(&tmp, k);
+      if (d && k) copied(dev_write(&tmp, d, v, k * sizeof(double)));
+      return d;
+    };
     w->rb_start = up_i(rb_start); w->rb_sys = up_i(rb_sys); w->sys_rb_off = up_i(w->h_sys_rb_off);
     w->rowptr = up_i(rowptr); w->colind = up_i(col); w->diagpos = up_i(diagpos);
     w->Kd = up_d(Aval + Arowptr[0], nnz);
@@ -3596,8 +3607,12 @@ extern "C" int ua_solve_kape_symmetric(int32_t n, const int64_t* Arowptr, const 
       cleanup();
       return set_error(UA_ERR_OOM, "allocation failed");
     }
-    cudaMemcpy(w->cmask, cmask.data(), n, cudaMemcpyHostToDevice);
-    cudaMemset(w->X, 0, n * sizeof(double));
+    copied(dev_write(&tmp, w->cmask, cmask.data(), n));
+    copied(dev_clear(&tmp, w->X, n * sizeof(double)));
+    if (cp != cudaSuccess) {
+      cleanup();
+      return set_error(UA_ERR_CUDA, "ua_solve_kape_symmetric: upload failed: %s", cudaGetErrorString(cp));
+    }
     ua_params p;
     ua_params_default(&p);
     p.krylov_rtol = rtol > 0 ? rtol : 1e-12;
@@ -3608,12 +3623,13 @@ extern "C" int ua_solve_kape_symmetric(int32_t n, const int64_t* Arowptr, const 
     if (rc == UA_OK) {
       std::vector<double> dl(w->nc);
       int st = 0;
-      cudaMemcpy(x, w->dX, n * sizeof(double), cudaMemcpyDeviceToHost);
-      if (w->nc) cudaMemcpy(dl.data(), w->dlam, w->nc * sizeof(double), cudaMemcpyDeviceToHost);
-      cudaMemcpy(&st, w->status, sizeof(int), cudaMemcpyDeviceToHost);
+      copied(dev_read(&tmp, x, w->dX, n * sizeof(double)));
+      if (w->nc) copied(dev_read(&tmp, dl.data(), w->dlam, w->nc * sizeof(double)));
+      copied(dev_read(&tmp, &st, w->status, sizeof(int)));
       for (int c = 0; c < w->nc; ++c) y[c] = dl[c] / con_l[c];
       if (its) *its = kits[0];
-      if (st) rc = set_error(UA_ERR_KRYLOV, "PCG breakdown: A is not positive definite on the free dofs");
+      if (cp != cudaSuccess) rc = set_error(UA_ERR_CUDA, "ua_solve_kape_symmetric: %s", cudaGetErrorString(cp));
+      else if (st) rc = set_error(UA_ERR_KRYLOV, "PCG breakdown: A is not positive definite on the free dofs");
     }
   }
   cleanup();
@@ -4054,7 +4070,7 @@ static int uvh_common(ua_mesh* m, const ua_params* p, ua_fields* F, const ua_bcs
   cudaEventElapsedTime(&dev_ms, call_ev[0], call_ev[1]);
   double kms[PK_COUNT] = {}, knnz[PK_COUNT] = {}, krows[PK_COUNT] = {};
   int kn[PK_COUNT] = {};
-  prof_collect(w, kms, kn, knnz, krows);
+  prof_collect(m, kms, kn, knnz, krows);
   bool all_conv = true;
   const double t1 = now_ms();
   for (int s = 0; s < nsys; ++s) {
@@ -4291,7 +4307,7 @@ extern "C" int ua_serve_begin(ua_mesh* m, const ua_params* p, int32_t count, con
   const int nsys = w->nsys;
   std::vector<int> run(nsys, 0);
   std::vector<SysScal> sc(nsys);
-  UA_CUDA_TRY(cudaMemcpy(sc.data(), w->scal, nsys * sizeof(SysScal), cudaMemcpyDeviceToHost));
+  UA_CUDA_TRY(dev_read(m, sc.data(), w->scal, nsys * sizeof(SysScal)));
   int rc;
   for (int k = 0; k < count; ++k) {
     const int s = sys[k];
