@@ -416,8 +416,12 @@ int ua_uv_adjoint_dIdC(ua_mesh* m, const ua_params* p, const ua_fields* F, const
  * through the connectivity, the patch element lists, the contribution lists or the node-slice
  * columns checks the index against its range; the first violation is recorded (site: 1 patch
  * element id, 2 element node id, 3 contribution element, 4 tangent index, 5 residual row, 6 node-
- * slice column) and the access is skipped.  enabled = 0 in the release build. */
+ * slice column; in the resident solves 7 node-slice column, 8 column of a coarse operator or a
+ * transfer, 9 column of the uvh tangent; 10 element of a quadratic gather) and the access is
+ * skipped.  ua_debug_sites: the sites that the handle's kernels have checked so far (bit s: site s).
+ * enabled = 0 in the release build. */
 int ua_debug_bounds(const ua_mesh* m, int32_t* enabled, int32_t* site, int64_t* index);
+int ua_debug_sites(const ua_mesh* m, int32_t* enabled, uint64_t* sites);
 
 /* Free and total device memory (admission by free HBM). */
 int ua_mem_info(int32_t device, int64_t* free_bytes, int64_t* total_bytes);

@@ -150,6 +150,7 @@ struct CycArgs {
   unsigned long long* prof;
   double* part;        // [3][nslices]
   long long nslices;
+  unsigned long long* dbg;  // bounds-checked build
 };
 // Set-up data of the collapsed cycle: structure once per handle, values per tangent.
 struct Cycle {

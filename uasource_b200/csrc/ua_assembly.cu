@@ -459,8 +459,10 @@ __global__ void __launch_bounds__(256, 2) uv_p2_elements(DevMesh M, QuadTable Q,
   }
   for (int t = threadIdx.x; t < kIps; t += blockDim.x) sN[kIps * 6 + t] = Q.w[t];
   for (int t = threadIdx.x; t < 6 * gn_; t += blockDim.x) {
-    int gn = __ldg(M.conn + (size_t)(t % 6) * M.ne + eb + t / 6);
+    int e = eb + t / 6;
     bool okn = true;
+    UA_CHECK_INDEX(M.dbg, e, 0, M.ne, BS_PATCH_ELEM, okn);
+    int gn = __ldg(M.conn + (size_t)(t % 6) * M.ne + e);
     UA_CHECK_INDEX(M.dbg, gn, M.sys_node_off[s], M.sys_node_off[s + 1], BS_ELEM_NODE, okn);
     (void)okn;
     double u = __ldg(in.X + uoff + gn), v = __ldg(in.X + voff + gn);  // at X + gamma dX (CalcCostFunctionNR.m:14-16)
@@ -659,7 +661,10 @@ __global__ void __launch_bounds__(256) uv_p2_gather(DevMesh M, const int* active
         bool ok = true;
         UA_CHECK_INDEX(M.dbg, el, 0, nep, BS_CONTRIB_ELEM, ok);
         if (!ok) continue;
-        const KT* o = kel + (size_t)I::NKE * __ldg(M.patch_elems + e0 + el);
+        int e = __ldg(M.patch_elems + e0 + el);
+        UA_CHECK_INDEX(M.dbg, e, 0, M.ne, BS_GATHER_ELEM, ok);
+        if (!ok) continue;
+        const KT* o = kel + (size_t)I::NKE * e;
         const int sy = I::sym(a, b);
         uu += o[sy];
         vv += o[I::NS + sy];
@@ -694,7 +699,10 @@ __global__ void __launch_bounds__(256) uv_p2_gather(DevMesh M, const int* active
       bool ok = true;
       UA_CHECK_INDEX(M.dbg, el, 0, nep, BS_CONTRIB_ELEM, ok);
       if (!ok) continue;
-      const double* o = rel + 24 * (size_t)__ldg(M.patch_elems + e0 + el) + a;
+      int e = __ldg(M.patch_elems + e0 + el);
+      UA_CHECK_INDEX(M.dbg, e, 0, M.ne, BS_GATHER_ELEM, ok);
+      if (!ok) continue;
+      const double* o = rel + 24 * (size_t)e + a;
       tx += o[0];
       fx += o[6];
       ty += o[12];

@@ -69,6 +69,7 @@ struct TeamCtx {
   unsigned* bar;         // the team's arrival counter
   unsigned target;       // arrivals that end the next barrier
   int* ok;               // shared: the last barrier was met
+  unsigned long long* dbg;  // bounds-checked build
 };
 
 // Arrive and wait.  The wait is bounded (some seconds): a team that does not meet returns false in
@@ -311,7 +312,7 @@ __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, cons
 // zero vector pair.
 template <int W, int NV, int KC, bool TR, typename QT, typename G>
 __device__ __forceinline__ void row_chunk(const int* col, const char* val, int e, int ee, int lane, double sign, G get,
-                                          double (&a0)[NV], double (&a1)[NV]) {
+                                          ColRange range, double (&a0)[NV], double (&a1)[NV]) {
   using V2 = decltype(get(0));
   constexpr int qb = 4 * sizeof(QT), CH = NV * KC;
   int c[CH];
@@ -320,6 +321,7 @@ __device__ __forceinline__ void row_chunk(const int* col, const char* val, int e
   for (int k = 0; k < CH; ++k) {
     const int u = min(e + W * (k / NV) + (W / NV) * (k % NV) + lane, ee - 1);
     c[k] = col[u];
+    UA_CHECK_COL(range, c[k], BS_ROW_COL);
     m[k] = QuadRaw<QT>::load(val + (long long)u * qb);
   }
   V2 x[CH];
@@ -342,13 +344,13 @@ __device__ __forceinline__ void row_chunk(const int* col, const char* val, int e
 // transposed (restriction).  a0, a1: the virtual lanes' sums.
 template <int W, int NV, int KC, bool TR, typename QT, typename G>
 __device__ __forceinline__ void row_sums(const int* col, const char* val, int e, int ee, int lane, double sign, G get,
-                                         double (&a0)[NV], double (&a1)[NV]) {
+                                         ColRange range, double (&a0)[NV], double (&a1)[NV]) {
   while (e < ee) {
     if (KC == 1 || ee - e <= W) {
-      row_chunk<W, NV, 1, TR, QT>(col, val, e, ee, lane, sign, get, a0, a1);
+      row_chunk<W, NV, 1, TR, QT>(col, val, e, ee, lane, sign, get, range, a0, a1);
       e += W;
     } else {
-      row_chunk<W, NV, KC, TR, QT>(col, val, e, ee, lane, sign, get, a0, a1);
+      row_chunk<W, NV, KC, TR, QT>(col, val, e, ee, lane, sign, get, range, a0, a1);
       e += W * KC;
     }
   }
@@ -365,7 +367,7 @@ __device__ __forceinline__ double lanes_total(const double (&a)[NV]) {
 template <int NV, typename VT, typename QT>
 __device__ __forceinline__ void cyc_down_nv(const LevS& L, int c0, int lo, int hi, const typename Vec2<VT>::T* b,
                                             typename Vec2<VT>::T* bc, const typename Vec2<VT>::T* q2, double alpha,
-                                            double w, bool rev) {
+                                            double w, bool rev, ColRange range) {
   using V2 = typename Vec2<VT>::T;
   constexpr int lanes = kDownW / NV, nsub = kCycThreads / lanes, KC = sizeof(VT) == 4 ? (NV == 1 ? 4 : 2) : (NV == 1 ? 2 : 1);
   const int sub = threadIdx.x / lanes, lane = threadIdx.x & (lanes - 1);
@@ -382,7 +384,7 @@ __device__ __forceinline__ void cyc_down_nv(const LevS& L, int c0, int lo, int h
           x.y = (VT)((double)x.y - alpha * (double)y.y);
         }
         return x;
-      }, a0, a1);
+      }, range, a0, a1);
     const double s0 = lanes_total<kDownW, NV>(a0), s1 = lanes_total<kDownW, NV>(a1);
     if (valid && lane == 0) {
       V2 o;
@@ -399,16 +401,18 @@ __device__ __forceinline__ void cyc_down(const LevS& L, const CycSys& S, int l, 
                                          double w = 1.0, bool rev = false) {
   int lo, hi;
   team_share(t, S.nn[l + 1], lo, hi);
+  const ColRange range = UA_COL_RANGE(t.dbg, S.n0[l], S.nn[l]);
   if (hi - lo <= kCycThreads / kDownW)
-    cyc_down_nv<1, VT, QT>(L, S.n0[l + 1], lo, hi, b, bc, q2, alpha, w, rev);
+    cyc_down_nv<1, VT, QT>(L, S.n0[l + 1], lo, hi, b, bc, q2, alpha, w, rev, range);
   else
-    cyc_down_nv<4, VT, QT>(L, S.n0[l + 1], lo, hi, b, bc, q2, alpha, w, rev);
+    cyc_down_nv<4, VT, QT>(L, S.n0[l + 1], lo, hi, b, bc, q2, alpha, w, rev, range);
 }
 
 // z = 2 b - A b + Q z_c on level l >= 1 (zc: indexed by the coarse level's node numbers).
 template <int NV, typename VT, typename AT, typename QT>
 __device__ __forceinline__ void cyc_up_nv(const LevS& L, int n0, int lo, int hi, const typename Vec2<VT>::T* b,
-                                          typename Vec2<VT>::T* z, const typename Vec2<VT>::T* zc) {
+                                          typename Vec2<VT>::T* z, const typename Vec2<VT>::T* zc,
+                                          ColRange range, ColRange range_c) {
   using V2 = typename Vec2<VT>::T;
   constexpr int lanes = kUpW / NV, nsub = kCycThreads / lanes, KC = sizeof(VT) == 4 ? (NV == 1 ? 4 : 2) : (NV == 1 ? 2 : 1);
   const int sub = threadIdx.x / lanes, lane = threadIdx.x & (lanes - 1);
@@ -421,9 +425,9 @@ __device__ __forceinline__ void cyc_up_nv(const LevS& L, int n0, int lo, int hi,
     if (valid) {
       bv = b[g];
       row_sums<kUpW, NV, KC, false, AT>(L.acol, L.aval, L.aptr[g], L.aptr[g + 1], lane, -1.0,
-                                        [&](int c) { return b[c]; }, a0, a1);
+                                        [&](int c) { return b[c]; }, range, a0, a1);
       row_sums<kUpW, NV, KC, false, QT>(L.qcol, L.qval, L.qptr[g], L.qptr[g + 1], lane, 1.0,
-                                        [&](int c) { return zc[c]; }, a0, a1);
+                                        [&](int c) { return zc[c]; }, range_c, a0, a1);
     }
     const double s0 = lanes_total<kUpW, NV>(a0), s1 = lanes_total<kUpW, NV>(a1);
     if (valid && lane == 0) {
@@ -440,10 +444,11 @@ __device__ __forceinline__ void cyc_up(const LevS& L, const CycSys& S, int l, co
                                        const typename Vec2<VT>::T* zc) {
   int lo, hi;
   team_share(t, S.nn[l], lo, hi);
+  const ColRange range = UA_COL_RANGE(t.dbg, S.n0[l], S.nn[l]), range_c = UA_COL_RANGE(t.dbg, S.n0[l + 1], S.nn[l + 1]);
   if (hi - lo <= kCycThreads / kUpW)
-    cyc_up_nv<1, VT, AT, QT>(L, S.n0[l], lo, hi, b, z, zc);
+    cyc_up_nv<1, VT, AT, QT>(L, S.n0[l], lo, hi, b, z, zc, range, range_c);
   else
-    cyc_up_nv<4, VT, AT, QT>(L, S.n0[l], lo, hi, b, z, zc);
+    cyc_up_nv<4, VT, AT, QT>(L, S.n0[l], lo, hi, b, z, zc, range, range_c);
 }
 
 // The coarsest level of the system by every CTA of the team for itself (no team barrier follows):
@@ -498,7 +503,7 @@ __device__ __forceinline__ const typename Vec2<VT>::T* cyc_solo(const LevS* lev,
                                                                 typename Vec2<VT>::T* zcs,
                                                                 typename Vec2<VT>::T* buf) {
   using V2 = typename Vec2<VT>::T;
-  const TeamCtx one{0, 1, nullptr, 0u, nullptr};
+  const TeamCtx one{0, 1, nullptr, 0u, nullptr, A.dbg};
   const int s0 = S.solo, dep = S.depth;
   const V2* b0 = (const V2*)A.lev[s0].b + S.n0[s0];
   for (int i = threadIdx.x; i < S.nn[s0]; i += kCycThreads) buf[i] = b0[i];
@@ -528,7 +533,7 @@ __device__ __forceinline__ const typename Vec2<VT>::T* cyc_solo(const LevS* lev,
 // entry, so that nothing branches between the loads.
 template <int CH, typename KT, typename VT>
 __device__ __forceinline__ void slice_chunk(const int* cp, const char* vp, int lane, int k0, int k1,
-                                            const typename Vec2<VT>::T* v, double& a0, double& a1) {
+                                            const typename Vec2<VT>::T* v, ColRange range, double& a0, double& a1) {
   using V2 = typename Vec2<VT>::T;
   int j[CH];
   typename QuadRaw<KT>::T e[CH];
@@ -536,6 +541,7 @@ __device__ __forceinline__ void slice_chunk(const int* cp, const char* vp, int l
   for (int k = 0; k < CH; ++k) {
     const int kk = min(k0 + k, k1 - 1);
     j[k] = cp[32 * kk + lane];
+    UA_CHECK_COL(range, j[k], BS_SLICE_COL);
     e[k] = SliceQuad<KT>::load(vp + (long long)kk * (128 * sizeof(KT)), lane);
   }
   V2 x[CH];
@@ -561,7 +567,8 @@ __device__ __forceinline__ void slice_chunk(const int* cp, const char* vp, int l
 // unrolled loop takes the slots of its remainder one by one.
 template <typename KT, typename VT>
 __device__ __forceinline__ void slice_product(const long long* sl_off, const int* cols, const char* vals, int sl,
-                                              int lane, const typename Vec2<VT>::T* v, double& a0, double& a1) {
+                                              int lane, const typename Vec2<VT>::T* v, ColRange range, double& a0,
+                                              double& a1) {
   const long long off = sl_off[sl];
   const int k1 = (int)((sl_off[sl + 1] - off) >> 5);
   const int* cp = cols + off;
@@ -569,13 +576,13 @@ __device__ __forceinline__ void slice_product(const long long* sl_off, const int
   a0 = a1 = 0;
   for (int k0 = 0; k0 < k1;) {  // the width is the same for the whole warp
     if (sizeof(KT) < 8 && k1 - k0 > 5) {
-      slice_chunk<10, KT, VT>(cp, vp, lane, k0, k1, v, a0, a1);
+      slice_chunk<10, KT, VT>(cp, vp, lane, k0, k1, v, range, a0, a1);
       k0 += 10;
     } else if (k1 - k0 > 3) {
-      slice_chunk<5, KT, VT>(cp, vp, lane, k0, k1, v, a0, a1);
+      slice_chunk<5, KT, VT>(cp, vp, lane, k0, k1, v, range, a0, a1);
       k0 += 5;
     } else {
-      slice_chunk<3, KT, VT>(cp, vp, lane, k0, k1, v, a0, a1);
+      slice_chunk<3, KT, VT>(cp, vp, lane, k0, k1, v, range, a0, a1);
       k0 += 3;
     }
   }
@@ -615,12 +622,12 @@ __device__ __forceinline__ void for_slices(int lo, int hi, int n0, int nn, bool 
 
 // - w A^ b + Q z_c at the lane of slice sl, finest level (the caller adds 2 w b).
 template <typename LT, typename VT, typename QT>
-__device__ __forceinline__ void cyc_up0_node(const FineS& F, const LevS& L, int sl, int lane,
+__device__ __forceinline__ void cyc_up0_node(const FineS& F, const LevS& L, const CycSys& S, const TeamCtx& t, int sl, int lane,
                                              const typename Vec2<VT>::T* b, const typename Vec2<VT>::T* zc, double w,
                                              double& z0, double& z1) {
   double a0, a1, q0, q1;
-  slice_product<LT, VT>(F.sl_off, F.cols, F.lv, sl, lane, b, a0, a1);
-  slice_product<QT, VT>(L.qoff, L.qcol, L.qval, sl, lane, zc, q0, q1);
+  slice_product<LT, VT>(F.sl_off, F.cols, F.lv, sl, lane, b, UA_COL_RANGE(t.dbg, S.n0[0], S.nn[0]), a0, a1);
+  slice_product<QT, VT>(L.qoff, L.qcol, L.qval, sl, lane, zc, UA_COL_RANGE(t.dbg, S.n0[1], S.nn[1]), q0, q1);
   z0 = q0 - w * a0;
   z1 = q1 - w * a1;
 }

@@ -100,7 +100,7 @@ __device__ __forceinline__ GmVec gm_basis(const GmArgs& a, int i) {
 
 // (K v) at the lane of slice sl
 __device__ __forceinline__ void gm_product(const CycFine& F, const double* v3, int sl, int lane,
-                                           const GmVec& v, double (&r)[3]) {
+                                           const GmVec& v, ColRange range, double (&r)[3]) {
   const long long off = F.sl_off[sl];
   const int k1 = (int)((F.sl_off[sl + 1] - off) >> 5);
   const int* cp = F.cols + off + lane;
@@ -112,7 +112,8 @@ __device__ __forceinline__ void gm_product(const CycFine& F, const double* v3, i
     double xh[CH];
 #pragma unroll
     for (int k = 0; k < CH; ++k) {
-      const int j = __ldg(cp + 32 * min(k0 + k, k1 - 1));
+      int j = __ldg(cp + 32 * min(k0 + k, k1 - 1));
+      UA_CHECK_COL(range, j, BS_GM_COL);
       xu[k] = v.uv[j];
       xh[k] = v.h[j];
     }
@@ -132,7 +133,7 @@ __device__ __forceinline__ void gm_product(const CycFine& F, const double* v3, i
 // thickness row: B = 0: (K_hu v_u + K_hv v_v), B = 1: K_hh v_h
 template <int B>
 __device__ __forceinline__ double gm_hrow(const CycFine& F, const double* v3, int sl, int lane,
-                                          const double2* uv, const double* h) {
+                                          const double2* uv, const double* h, ColRange range) {
   const long long off = F.sl_off[sl];
   const int k1 = (int)((F.sl_off[sl + 1] - off) >> 5);
   const int* cp = F.cols + off + lane;
@@ -146,6 +147,7 @@ __device__ __forceinline__ double gm_hrow(const CycFine& F, const double* v3, in
     for (int k = 0; k < CH; ++k) {
       const int kk = min(k0 + k, k1 - 1);
       j[k] = __ldg(cp + 32 * kk);
+      UA_CHECK_COL(range, j[k], BS_GM_COL);
       e0[k] = __ldg(vp + 288 * kk);
       if (!B) e1[k] = __ldg(vp + 288 * kk + 32);
     }
@@ -372,7 +374,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
   __shared__ GmShared sh;
   __shared__ int ok;
   const int4 c = a.cyc.cta[blockIdx.x];
-  TeamCtx t{c.z, c.w, a.cyc.bar + 32 * a.cyc.team[blockIdx.x], 0u, &ok};
+  TeamCtx t{c.z, c.w, a.cyc.bar + 32 * a.cyc.team[blockIdx.x], 0u, &ok, a.cyc.dbg};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int qi = c.x; qi < c.y; ++qi) {
     const int s = a.cyc.queue[qi];
@@ -384,6 +386,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
     const double* dense;
     const int n0 = S.n0[0], nn = S.nn[0], dep = S.depth, U = gm_unit(S.nsl), units = (S.nsl + U - 1) / U;
     const int solo = t.size > 1 ? S.solo : dep;
+    const ColRange range = UA_COL_RANGE(t.dbg, n0, nn);
     const double2* bL = (const double2*)a.cyc.lev[dep].b;
     int u0, u1;
     team_share(t, units, u0, u1);
@@ -409,7 +412,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
       for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
         if (!in) return;
         double kx[3];
-        gm_product(a.cyc.fine, a.v3, S.sl0 + i, lane, a.x, kx);
+        gm_product(a.cyc.fine, a.v3, S.sl0 + i, lane, a.x, range, kx);
         const double2 f = a.fs.uv[k], d = a.scp[k];
         const double2 r = make_double2(f.x - kx[0], f.y - kx[1]);
         // constrained rows: f and the product are zero
@@ -459,7 +462,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
         for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
           if (!in) return;
           double z0, z1;
-          cyc_up0_node<double, double, double>(fine, lev[0], S.sl0 + i, lane, a.ws, zc, inv, z0, z1);
+          cyc_up0_node<double, double, double>(fine, lev[0], S, t, S.sl0 + i, lane, a.ws, zc, inv, z0, z1);
           const double2 d = a.scp[k], b = a.ws[k];
           a.z.uv[k] = make_double2(d.x * (2.0 * inv * b.x + z0), d.y * (2.0 * inv * b.y + z1));
         });
@@ -470,7 +473,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
         const double om0 = a.hsw.weight(0);
         for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
           if (!in) return;
-          const double b = vj.h[k] - gm_hrow<0>(a.cyc.fine, a.v3, S.sl0 + i, lane, a.z.uv, nullptr);
+          const double b = vj.h[k] - gm_hrow<0>(a.cyc.fine, a.v3, S.sl0 + i, lane, a.z.uv, nullptr, range);
           const double hi1 = a.hinv[k];
           a.bh[k] = hi1 > 0 ? b : 0.0;
           bufs[cur][k] = om0 * b * hi1;
@@ -482,7 +485,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
           double* zo = bufs[1 - cur];
           for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
             if (in)
-              zo[k] = zi[k] + om * (a.bh[k] - gm_hrow<1>(a.cyc.fine, a.v3, S.sl0 + i, lane, nullptr, zi)) * a.hinv[k];
+              zo[k] = zi[k] + om * (a.bh[k] - gm_hrow<1>(a.cyc.fine, a.v3, S.sl0 + i, lane, nullptr, zi, range)) * a.hinv[k];
           });
           UA_TEAM_SYNC(t);
           cur = 1 - cur;
@@ -492,7 +495,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
         for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
           if (!in) return;
           double kx[3];
-          gm_product(a.cyc.fine, a.v3, S.sl0 + i, lane, a.z, kx);
+          gm_product(a.cyc.fine, a.v3, S.sl0 + i, lane, a.z, range, kx);
           a.w.uv[k] = make_double2(kx[0], kx[1]);
           a.w.h[k] = kx[2];
         });

@@ -62,6 +62,8 @@ __host__ __device__ inline uint16_t pack_contrib(int el, int a, int b) {
 // release build compiles them out.
 #ifdef UA_BOUNDS_CHECK
 __device__ inline bool in_bounds(unsigned long long* dbg, long long i, long long lo, long long hi, int site) {
+  // the sites that were reached at all: a clean flag says nothing about a kernel that has no check
+  if (dbg && !((*(volatile unsigned long long*)(dbg + 1) >> site) & 1)) atomicOr(dbg + 1, 1ULL << site);
   if (i >= lo && i < hi) return true;
   if (dbg) atomicCAS(dbg, 0ULL, ((unsigned long long)(site & 0xffff) << 48) | ((unsigned long long)i & 0xffffffffffffULL));
   return false;
@@ -80,8 +82,31 @@ __device__ inline bool in_bounds(unsigned long long* dbg, long long i, long long
 #endif
 // check sites (bits 48-63 of the recorded flag)
 enum BoundsSite {
-  BS_PATCH_ELEM = 1, BS_ELEM_NODE = 2, BS_CONTRIB_ELEM = 3, BS_K_INDEX = 4, BS_R_INDEX = 5, BS_SELL_COL = 6
+  BS_PATCH_ELEM = 1, BS_ELEM_NODE = 2, BS_CONTRIB_ELEM = 3, BS_K_INDEX = 4, BS_R_INDEX = 5, BS_SELL_COL = 6,
+  // resident solves: columns of the node slices, of the coarse rows and transfers, of the uvh tangent
+  BS_SLICE_COL = 7, BS_ROW_COL = 8, BS_GM_COL = 9,
+  BS_GATHER_ELEM = 10  // elements of the P2 gathers
 };
+
+// The range of a gathered vector, beside the functions that read its index from a list (nothing in the
+// release build).
+#ifdef UA_BOUNDS_CHECK
+struct ColRange {
+  unsigned long long* dbg;
+  int lo, hi;
+};
+#define UA_COL_RANGE(dbg, lo, n) (ua::ColRange{(dbg), (lo), (lo) + (n)})
+#define UA_CHECK_COL(range, i, site)                                                                              \
+  do {                                                                                                            \
+    if (!ua::in_bounds((range).dbg, (long long)(i), (range).lo, (range).hi, (site))) (i) = (range).lo;           \
+  } while (0)
+#else
+struct ColRange {};
+#define UA_COL_RANGE(dbg, lo, n) (ua::ColRange{})
+#define UA_CHECK_COL(range, i, site) \
+  do {                               \
+  } while (0)
+#endif
 
 struct QuadTable {
   int nip;
@@ -123,7 +148,7 @@ struct DevMesh {
   const int* patch_hnodes;    // global node ids
   const uint16_t* patch_elnodes;  // [patch element][nod], aligned with patch_elems
   int max_patch_hnodes;
-  unsigned long long* dbg;    // first bounds violation (debug build; null otherwise)
+  unsigned long long* dbg;    // first bounds violation, sites reached (debug build; null otherwise)
 };
 
 // Patch shape: the nodes of a system of nn nodes are cut, in Morton order, into patches of

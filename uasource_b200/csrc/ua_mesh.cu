@@ -540,7 +540,7 @@ extern "C" int ua_mesh_create_batch(const ua_mesh_desc* descs, int32_t count, in
   if ((rc = install_patch_plan(m, plan))) goto fail;
 #ifdef UA_BOUNDS_CHECK
   {
-    const std::vector<unsigned long long> zero(1, 0ULL);
+    const std::vector<unsigned long long> zero(2, 0ULL);
     if ((rc = upload_vec(m, zero, (const unsigned long long**)&dm.dbg))) goto fail;
   }
 #else
@@ -553,6 +553,20 @@ fail:
   if (m->stream) cudaStreamDestroy(m->stream);
   delete m;
   return rc;
+}
+
+extern "C" int ua_debug_sites(const ua_mesh* m, int32_t* enabled, uint64_t* sites) {
+  if (!m || !enabled || !sites) return set_error(UA_ERR_INVALID, "ua_debug_sites: null argument");
+  *enabled = 0;
+  *sites = 0;
+#ifdef UA_BOUNDS_CHECK
+  *enabled = 1;
+  unsigned long long v = 0;
+  UA_CUDA_TRY(cudaSetDevice(m->device));
+  UA_CUDA_TRY(dev_read(m, &v, m->dm.dbg + 1, sizeof(v)));
+  *sites = v;
+#endif
+  return UA_OK;
 }
 
 // The first bounds violation a kernel of this handle recorded (bounds-checked build only).

@@ -544,6 +544,7 @@ CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof) {
   A.prof = prof ? C.d_prof : nullptr;
   A.part = C.d_part;
   A.nslices = C.nslices;
+  A.dbg = m->dm.dbg;
   return A;
 }
 
@@ -647,7 +648,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
   __shared__ V2 zcs[kAmgMaxDense / 2], sbuf[kSoloBuf];
   __shared__ int ok;
   const int4 c = a.cyc.cta[blockIdx.x];
-  TeamCtx t{c.z, c.w, a.cyc.bar + 32 * a.cyc.team[blockIdx.x], 0u, &ok};
+  TeamCtx t{c.z, c.w, a.cyc.bar + 32 * a.cyc.team[blockIdx.x], 0u, &ok, a.cyc.dbg};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   V2 *z = (V2*)a.z, *p = (V2*)a.p, *q = (V2*)a.q;
   const V2* dw = (const V2*)a.dw;
@@ -721,7 +722,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
         if (in) {
           const V2 bv = r[g];
           double z0, z1;
-          cyc_up0_node<LT, VT, QT>(fine, lev[0], S.sl0 + i, lane, r, zc, 1.0, z0, z1);
+          cyc_up0_node<LT, VT, QT>(fine, lev[0], S, t, S.sl0 + i, lane, r, zc, 1.0, z0, z1);
           V2 o;
           o.x = (VT)(2.0 * (double)bv.x + z0);
           o.y = (VT)(2.0 * (double)bv.y + z1);
@@ -747,7 +748,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
             qo = q[g];
           }
           double a0, a1;
-          slice_product<KT, VT>(fine.sl_off, fine.cols, fine.kv, S.sl0 + i, lane, z, a0, a1);
+          slice_product<KT, VT>(fine.sl_off, fine.cols, fine.kv, S.sl0 + i, lane, z, UA_COL_RANGE(t.dbg, n0, nn), a0, a1);
           if (its) {
             pn.x = (VT)((double)pn.x + beta * (double)po.x);
             pn.y = (VT)((double)pn.y + beta * (double)po.y);

@@ -398,8 +398,10 @@ __global__ void __launch_bounds__(KW ? 384 : 256, KW ? 1 : 2) uvh_p2_elements(De
     sD[t] = make_double2(Q.der[t / 6][0][t % 6], Q.der[t / 6][1][t % 6]);
   }
   for (int t = threadIdx.x; t < 6 * gn_; t += blockDim.x) {
-    int gn = __ldg(M.conn + (size_t)(t % 6) * M.ne + eb + t / 6);
+    int e = eb + t / 6;
     bool okn = true;
+    UA_CHECK_INDEX(M.dbg, e, 0, M.ne, BS_PATCH_ELEM, okn);
+    int gn = __ldg(M.conn + (size_t)(t % 6) * M.ne + e);
     UA_CHECK_INDEX(M.dbg, gn, no, no + nn_s, BS_ELEM_NODE, okn);
     (void)okn;
     stage_node(M, P, in, S, gn, uoff, voff, hoff, gam, nd + t, MH);
@@ -654,7 +656,10 @@ __global__ void __launch_bounds__(256) uvh_p2_gather(DevMesh M, const int* activ
         bool ok = true;
         UA_CHECK_INDEX(M.dbg, ce, 0, ne, BS_CONTRIB_ELEM, ok);
         if (!ok) continue;
-        const double* src = kel + ((size_t)36 * __ldg(M.patch_elems + e0 + ce) + 6 * a + b) * 9;
+        int e = __ldg(M.patch_elems + e0 + ce);
+        UA_CHECK_INDEX(M.dbg, e, 0, M.ne, BS_GATHER_ELEM, ok);
+        if (!ok) continue;
+        const double* src = kel + ((size_t)36 * e + 6 * a + b) * 9;
 #pragma unroll
         for (int i = 0; i < 9; ++i) v[i] += src[i];
       }
@@ -686,7 +691,10 @@ __global__ void __launch_bounds__(256) uvh_p2_gather(DevMesh M, const int* activ
       bool ok = true;
       UA_CHECK_INDEX(M.dbg, ce, 0, ne, BS_CONTRIB_ELEM, ok);
       if (!ok) continue;
-      const double* src = rel + ((size_t)6 * __ldg(M.patch_elems + e0 + ce) + a) * 6;
+      int e = __ldg(M.patch_elems + e0 + ce);
+      UA_CHECK_INDEX(M.dbg, e, 0, M.ne, BS_GATHER_ELEM, ok);
+      if (!ok) continue;
+      const double* src = rel + ((size_t)6 * e + a) * 6;
 #pragma unroll
       for (int i = 0; i < 6; ++i) acc[i] += src[i];
     }
