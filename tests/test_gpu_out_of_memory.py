@@ -1,0 +1,44 @@
+"""Calls that run out of device memory say so and leave the handle usable.
+
+Another allocation takes all but a set number of bytes of the device; the library's next cudaMalloc then
+fails with an error, nothing more.
+"""
+import contextlib
+
+import numpy as np
+import pytest
+
+import uasource_b200 as ua
+from uasource_b200 import lib as L
+from uasource_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@contextlib.contextmanager
+def _left(nbytes):
+    """Only nbytes of the device are free inside."""
+    torch = pytest.importorskip("torch")
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - int(nbytes), dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+
+
+def test_quadratic_assembly_without_room_for_its_element_rows():
+    P = synth.ice_stream_shelf(141, 101, nod=6, seed=2, transient=True)
+    mua = ua.CreateMUA(P.coordinates, P.connectivity, ndof=3)
+    F = ua.Fields.from_problem(P)
+    F.ub, F.vb = 100 * np.sin(P.coordinates[:, 0] / 2e4), 10 * np.cos(P.coordinates[:, 1] / 2e4)
+    R0, _ = ua.uvhAssembly(ua.CtrlVar(), mua, F, F.copy(), 0.1, Ronly=True)  # everything but the tangent
+    nnz, rows = mua.nnz(), P.connectivity.shape[0] * 36 * 9  # values of the tangent and of its element rows
+    with _left(8 * nnz + 4 * rows):  # the first fit, the second do not
+        with pytest.raises(L.UaError) as ei:
+            ua.uvhAssembly(ua.CtrlVar(), mua, F, F.copy(), 0.1)
+        assert ei.value.code == L.UA_ERR_OOM
+    R1, K = ua.uvhAssembly(ua.CtrlVar(), mua, F, F.copy(), 0.1)
+    assert np.array_equal(R0, R1) and np.isfinite(K.data).all() and K.nnz == nnz

@@ -1354,6 +1354,12 @@ static void* ring_slot(ua_mesh* m, size_t bytes) {
   return p;
 }
 
+// The quadratic assemblies allocate their element rows on first use.
+static int assembly_error(const char* what, cudaError_t e) {
+  if (e == cudaErrorMemoryAllocation) return set_error(UA_ERR_OOM, "%s assembly: device allocation failed", what);
+  return set_error(UA_ERR_CUDA, "%s assembly launch: %s", what, cudaGetErrorString(e));
+}
+
 static int set_sel(ua_mesh* m, const std::vector<int>& sel) {
   Work* w = m->work;
   int* h = (int*)ring_slot(m, w->nsys * sizeof(int));
@@ -1406,7 +1412,7 @@ static int assemble(ua_mesh* m, const ua_params* p, bool withK, bool useDir, con
   cudaError_t e = launch_uv_assembly(m, make_phys(p), in, out, withK, fp32, m->asm_threads, m->asm_regs);
   prof_end(m, ev);
   ++g_launches;
-  if (e != cudaSuccess) return set_error(UA_ERR_CUDA, "uv assembly launch: %s", cudaGetErrorString(e));
+  if (e != cudaSuccess) return assembly_error("uv", e);
   return UA_OK;
 }
 
@@ -2957,7 +2963,7 @@ static int assemble_uvh(ua_mesh* m, const ua_params* p, bool withK, bool useDir,
   cudaError_t e = launch_uvh_assembly(m, make_uvh_phys(p), in, out, withK);
   prof_end(m, ev);
   ++g_launches;
-  if (e != cudaSuccess) return set_error(UA_ERR_CUDA, "uvh assembly launch: %s", cudaGetErrorString(e));
+  if (e != cudaSuccess) return assembly_error("uvh", e);
   return UA_OK;
 }
 
