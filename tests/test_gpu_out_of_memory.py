@@ -42,3 +42,24 @@ def test_quadratic_assembly_without_room_for_its_element_rows():
         assert ei.value.code == L.UA_ERR_OOM
     R1, K = ua.uvhAssembly(ua.CtrlVar(), mua, F, F.copy(), 0.1)
     assert np.array_equal(R0, R1) and np.isfinite(K.data).all() and K.nnz == nnz
+
+
+def test_gmres_restart_without_room_for_its_basis():
+    P = synth.ice_stream_shelf(141, 101, seed=2, transient=True)
+    bcs = ua.BCs.from_problem(P)
+    m2, m3 = (ua.CreateMUA(P.coordinates, P.connectivity, ndof=d) for d in (2, 3))
+    F0 = ua.uv(ua.CtrlVar().set_force_tolerance(1e-20), m2, bcs, ua.Fields.from_problem(P))[0]
+
+    def step(restart):
+        ctrl = ua.CtrlVar(krylov_restart=restart).set_uvh_force_tolerance(1e-20)
+        F1, _, info = ua.uvh(ctrl, m3, F0, F0.copy(), bcs, 0.1)
+        assert info.converged
+        return np.concatenate([F1.ub, F1.vb, F1.h])
+
+    a = step(20)
+    with _left(4 << 20):  # the basis of 48 takes 19 MB, the work space of 20 gives back 18
+        with pytest.raises(L.UaError) as ei:
+            step(48)
+        assert ei.value.code == L.UA_ERR_OOM
+    assert np.array_equal(a, step(20))
+    assert np.linalg.norm(a - step(48)) <= 1e-9 * np.linalg.norm(a)

@@ -181,7 +181,7 @@ struct Cycle {
   int *d_ipos = nullptr, *d_pcol = nullptr;  // node -> slice position; slot columns as positions
   // uvh: basis and work vectors, partials, 3-dof tangent and inverse thickness l1 sums (slice order)
   double *gm_buf = nullptr, *gm_part = nullptr, *gm_v3 = nullptr, *gm_hinv = nullptr;
-  int gm_mr = 0;
+  int gm_mr = 0;  // restart that they are for (0: none)
   void* d_r2 = nullptr;       // second residual buffer
   std::vector<double> h_solo[2];   // per system: bytes of its solo levels
   std::vector<double> h_bytes[2];  // per system: bytes of the matrices a step reads (FP64, mixed)

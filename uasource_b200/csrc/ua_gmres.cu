@@ -7,6 +7,7 @@
 // thread of every CTA for itself, so the host takes no part until the solve ends.
 #include <algorithm>
 #include <cstring>
+#include "ua_alloc.h"
 #include "ua_cycle.cuh"
 
 namespace ua {
@@ -615,17 +616,13 @@ int gmres_resident(ua_mesh* m, const GmSolve& v, const std::vector<int>& sel, co
   }
   // partials of system s start at its own offset: one block of [vector][ld] per system
   const size_t np = (size_t)(2 * (v.mr + 1) + 1) * ld;
-  if (!C.gm_buf || C.gm_mr != v.mr) {
-    if (C.gm_buf) dev_free(m, C.gm_buf);
-    if (C.gm_part) dev_free(m, C.gm_part);
-    C.gm_buf = (double*)dev_alloc(m, sizeof(double) * (size_t)(3 * (v.mr + 1) + 18) * npad);
-    C.gm_part = (double*)dev_alloc(m, sizeof(double) * np * a->nsys);
-    if (!C.gm_v3) C.gm_v3 = (double*)dev_alloc(m, sizeof(double) * 9 * (size_t)std::max(S.slots, 1LL));
-    if (!C.gm_hinv) C.gm_hinv = (double*)dev_alloc(m, sizeof(double) * npad);
-    if (!C.gm_buf || !C.gm_part || !C.gm_v3 || !C.gm_hinv)
-      return set_error(UA_ERR_OOM, "device allocation of the GMRES basis failed");
-    C.gm_mr = v.mr;
-  }
+  if (!alloc_for(C.gm_mr, v.mr,
+                 {{(void**)&C.gm_buf, sizeof(double) * (size_t)(3 * (v.mr + 1) + 18) * npad},
+                  {(void**)&C.gm_part, sizeof(double) * np * a->nsys},
+                  {(void**)&C.gm_v3, sizeof(double) * 9 * (size_t)std::max(S.slots, 1LL)},
+                  {(void**)&C.gm_hinv, sizeof(double) * (size_t)npad}},
+                 [&](size_t n) { return dev_alloc(m, n); }, [&](void* p) { dev_free(m, p); }))
+    return set_error(UA_ERR_OOM, "device allocation of the GMRES basis failed");
   k_gm_fill<<<std::max(S.nsb, 1), 256, 0, m->stream>>>(CycFine{S.perm, S.sl_off, C.d_pcol}, S.sb_n0, S.sb_cnt,
                                                        S.sb_sys, m->dm.sys_node_off, m->dm.sys_dof_off, v.rowptr,
                                                        v.K, v.cmask, C.gm_v3, C.gm_hinv, v.sel), ++*launches;
