@@ -63,3 +63,37 @@ def test_gmres_restart_without_room_for_its_basis():
         assert ei.value.code == L.UA_ERR_OOM
     assert np.array_equal(a, step(20))
     assert np.linalg.norm(a - step(48)) <= 1e-9 * np.linalg.norm(a)
+
+
+def test_setup_lists_without_room_are_given_back():
+    P = synth.ice_stream_shelf(161, 121, seed=2)
+    bcs = ua.BCs.from_problem(P)
+
+    def solve(mua, **kw):
+        F, _, _, _, info = ua.uv(ua.CtrlVar(**kw).set_force_tolerance(1e-20), mua, bcs, ua.Fields.from_problem(P))
+        return np.concatenate([F.ub, F.vb]), info
+
+    def failure(mua):
+        try:
+            solve(mua)
+        except L.UaError as e:
+            return str(e)
+        return ""
+
+    solve(ua.CreateMUA(P.coordinates, P.connectivity))  # kernels are loaded
+    tried = []
+    for left in range(64, 0, -3):  # MB: down to where the lists are what does not fit
+        mua = ua.CreateMUA(P.coordinates, P.connectivity)
+        solve(mua, krylov_precond=L.UA_PC_JACOBI)
+        with _left(left << 20):
+            tried.append(failure(mua))
+            if "set-up lists" in tried[-1]:
+                held = mua.device_bytes()
+                for _ in range(3):
+                    assert "set-up lists" in failure(mua)
+                    assert mua.device_bytes() == held
+                break
+    else:
+        pytest.fail(f"no size at which the lists alone do not fit: {tried}")
+    x, info = solve(mua)
+    assert info.converged and np.array_equal(x, solve(mua)[0])

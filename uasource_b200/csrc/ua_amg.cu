@@ -1451,6 +1451,7 @@ __global__ void __launch_bounds__(32 * kSaPW, 4) k_sa_prolong(int nnb, const int
 static int sa_lists(ua_mesh* m, const int* rowptr0, const int* colind0) {
   Amg* a = m->amg;
   cudaStream_t st = m->stream;
+  const size_t mark = m->owned.size(), bytes = a->bytes;
   bool ok = true;
   auto grid = [](long long n, int t) { return (unsigned)std::max<long long>(1, (n + t - 1) / t); };
   unsigned long long* d_tot = (unsigned long long*)dalloc(m, a, sizeof(unsigned long long), ok);
@@ -1499,7 +1500,11 @@ static int sa_lists(ua_mesh* m, const int* rowptr0, const int* colind0) {
     if (rc == UA_ERR_OOM) ok = false;
     else if (rc) return rc;
   }
-  if (!ok) return set_error(UA_ERR_OOM, "AMG: device allocation of the set-up lists failed");
+  if (!ok) {  // the next set-up starts over
+    dev_free_since(m, mark);
+    a->bytes = bytes;
+    return set_error(UA_ERR_OOM, "AMG: device allocation of the set-up lists failed");
+  }
   UA_CUDA_TRY(cudaGetLastError());
   a->lists = true;
   return UA_OK;

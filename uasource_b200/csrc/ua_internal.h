@@ -247,6 +247,8 @@ namespace ua {
 void* dev_alloc(ua_mesh* m, size_t bytes);
 void dev_free(ua_mesh* m, const void* p);
 void dev_free_all(ua_mesh* m);
+// frees what was allocated after the handle owned `mark` buffers (a step that failed half way)
+void dev_free_since(ua_mesh* m, size_t mark);
 // rebuilds the patch plan of a handle with another shape (the results do not depend on it)
 int rebuild_patches(ua_mesh* m, PatchShape shape);
 // the process-wide tuning for (device, nod, ndof), set by ua_autotune; the default if none

@@ -58,6 +58,10 @@ cudaError_t dev_read(const ua_mesh* m, void* h, const void* d, size_t bytes) {
 }
 cudaError_t dev_clear(const ua_mesh* m, void* d, size_t bytes) { return cudaMemsetAsync(d, 0, bytes, m->stream); }
 
+void dev_free_since(ua_mesh* m, size_t mark) {
+  while (m->owned.size() > mark) dev_free(m, m->owned.back().ptr);
+}
+
 void dev_free_all(ua_mesh* m) {
   for (auto& b : m->owned) cudaFree(b.ptr);
   m->owned.clear();
