@@ -144,8 +144,9 @@ typedef struct ua_params {
     int32_t uvh_krylov;        /* UA_KRYLOV_*: inner solver of the unsymmetric uvh system */
     int32_t krylov_restart;    /* GMRES restart length m (uvh) */
     double krylov_eta_c, krylov_eta_max;  /* uv forcing term eta = clamp(c*sqrt(rForce), krylov_rtol, max) */
-    int32_t precond_bf16;      /* mixed precision: 1 = the AMG V-cycle's finest-level passes read a BF16
-                                  copy of the tangent (the PCG operator stays FP32) */
+    int32_t precond_bf16;      /* mixed precision: 1 = the AMG V-cycle's finest-level passes read BF16
+                                  copies of the tangent and of the transfer (the PCG operator and the coarse
+                                  levels stay FP32); 0 = they read the FP32 tangent and an FP32 transfer */
     int32_t amg_smoothed;      /* 1 = smoothed-aggregation prolongators (default), 0 = plain aggregation;
                                   fixed by a handle's first AMG solve */
     int32_t krylov_full_grid;  /* 0 = the AMG-preconditioned PCG launches only the row and node blocks of

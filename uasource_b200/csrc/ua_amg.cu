@@ -1556,7 +1556,7 @@ static int numeric_t(ua_mesh* m, const int* rowptr0, const int* colind0, const K
           UA_CUDA_TRY(cudaEventRecord(a->fork, st));
           UA_CUDA_TRY(cudaStreamWaitEvent(sd, a->fork, 0));
         }
-        cycle_fill_levels(m, sizeof(KT) == 4, sel, sd, launches);
+        cycle_fill_levels(m, sizeof(KT) == 4, cyc->lo, sel, sd, launches);
       }
       k_sa_Ac<KT><<<grid(C.ng * kSaAcL, 256), 256, 0, st>>>(C.ng, F.ac_node, C.gptr, C.nrow, Qv, APv, F.ac_lptr,
                                                             F.ac_l, (KT*)C.A, sel), ++*launches;

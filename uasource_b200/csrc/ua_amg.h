@@ -119,7 +119,7 @@ int cycle_alloc_values(ua_mesh* m, bool fp32, bool lo);
 // operators and every Q (after the last A P)
 void cycle_fill_fine(ua_mesh* m, const int* colind0, const void* K0, bool fp32, bool lo, const int* sel,
                      cudaStream_t st, long long* launches);
-void cycle_fill_levels(ua_mesh* m, bool fp32, const int* sel, cudaStream_t st, long long* launches);
+void cycle_fill_levels(ua_mesh* m, bool fp32, bool lo, const int* sel, cudaStream_t st, long long* launches);
 struct PcgSolve {
   bool fp32, lo, prof;
   const int* sel;

@@ -152,6 +152,12 @@ struct CycArgs {
   long long nslices;
   unsigned long long* dbg;  // bounds-checked build
 };
+// Value types of a form: FP64; the mixed form with the finest level in BF16; the mixed form all in FP32.
+// Q holds the smoothing of the operator beside it, so it has that operator's type: FP32 on the coarse levels
+// of the mixed form, BF16 on the finest only where the operator there is.  (BF16 everywhere was no faster:
+// 16 meshes mixed 44.3 ms against 44.1, P2 101x51 7.87 against 7.59.)
+enum CycForm { CF_FP64 = 0, CF_LO, CF_FP32, CF_COUNT };
+inline CycForm cyc_form(bool fp32, bool lo) { return !fp32 ? CF_FP64 : lo ? CF_LO : CF_FP32; }
 // Set-up data of the collapsed cycle: structure once per handle, values per tangent.
 struct Cycle {
   bool ready = false, failed = false;
@@ -167,7 +173,10 @@ struct Cycle {
     int *tptr = nullptr, *tfine = nullptr, *tpos = nullptr;    // Q' lists; tpos: A P entry -> entry of Q'
     double2* sc = nullptr;                                     // D^-1/2 per node (u, v)
     void *a32 = nullptr, *a64 = nullptr;                       // scaled operator quads (levels >= 1)
-    void *qh = nullptr, *qd = nullptr, *th = nullptr, *td = nullptr;  // Q and Q' quads (BF16, FP64)
+    // Q and Q' quads: BF16 on the finest level beside the BF16 operator, else FP32 or FP64 (CycForm)
+    void *qh = nullptr, *qf = nullptr, *qd = nullptr, *th = nullptr, *tf = nullptr, *td = nullptr;
+    void* q(int form, int l) const { return form == CF_FP64 ? qd : form == CF_LO && l == 0 ? qh : qf; }
+    void* t(int form, int l) const { return form == CF_FP64 ? td : form == CF_LO && l == 0 ? th : tf; }
   };
   std::vector<Lev> lev;
   // resident kernel: schedule (one int4 per CTA: queue begin, end, team rank, team size), queue,
@@ -183,8 +192,8 @@ struct Cycle {
   double *gm_buf = nullptr, *gm_part = nullptr, *gm_v3 = nullptr, *gm_hinv = nullptr;
   int gm_mr = 0;  // restart that they are for (0: none)
   void* d_r2 = nullptr;       // second residual buffer
-  std::vector<double> h_solo[2];   // per system: bytes of its solo levels
-  std::vector<double> h_bytes[2];  // per system: bytes of the matrices a step reads (FP64, mixed)
+  std::vector<double> h_solo[CF_COUNT];   // per system: bytes of its solo levels
+  std::vector<double> h_bytes[CF_COUNT];  // per system: bytes of the matrices a step reads
   int* h_stage = nullptr;     // pinned staging of the schedule
   long long nslices = 0;
   ~Cycle() {

@@ -233,11 +233,12 @@ __device__ __forceinline__ void stage_slices(Arena& ar, int lo, int hi, int qb, 
 // gather of the vector instead of three dependent loads.  [slo, shi): the CTA's slices of the finest
 // level (the passes of that level visit no others).  Every thread keeps the same pointers;
 // thread 0 publishes them.  room: the arena holds everything but, perhaps, the solo levels.
-template <typename KT, typename LT, typename QT>
+// QT, QC: Q of the finest level and of the coarse ones.
+template <typename KT, typename LT, typename QT, typename QC>
 __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, const void* lv, const CycSys& S,
                                           const TeamCtx& t, int slo, int shi, Arena& ar, LevS* lev, FineS* fine, int kslot,
                                           const double*& dense, bool room) {
-  constexpr int qb = 4 * sizeof(QT), ab = 4 * sizeof(KT);
+  constexpr int q0 = 4 * sizeof(QT), qb = 4 * sizeof(QC), ab = 4 * sizeof(KT);
   int lo, hi;
   dense = A.dense + S.doff;
   if (char* p = ar.take(8LL * S.dn * S.dn)) {
@@ -264,13 +265,13 @@ __device__ __forceinline__ void cyc_stage(const CycArgs& A, const void* kv, cons
     LevS L{G.aptr, G.acol, (const char*)G.aval, G.qptr, G.qoff, G.qcol, (const char*)G.qval,
            G.tptr, G.tfine, (const char*)G.tval};
     team_share(t, S.nn[l + 1], lo, hi);
-    stage_csr(ar, S.n0[l + 1] + lo, S.n0[l + 1] + hi, qb, L.tptr, L.tfine, L.tval);
+    stage_csr(ar, S.n0[l + 1] + lo, S.n0[l + 1] + hi, l ? qb : q0, L.tptr, L.tfine, L.tval);
     if (l > 0) {
       team_share(t, S.nn[l], lo, hi);
       stage_csr(ar, S.n0[l] + lo, S.n0[l] + hi, qb, L.qptr, L.qcol, L.qval);
       stage_csr(ar, S.n0[l] + lo, S.n0[l] + hi, ab, L.aptr, L.acol, L.aval);
     } else {
-      stage_slices(ar, S.sl0 + slo, S.sl0 + shi, qb, L.qoff, L.qcol, L.qval);
+      stage_slices(ar, S.sl0 + slo, S.sl0 + shi, q0, L.qoff, L.qcol, L.qval);
     }
     if (threadIdx.x == 0) lev[l] = L;
   }
@@ -640,8 +641,8 @@ struct CycSchedule {
 void cycle_schedule(const std::vector<CycSys>& sys, const std::vector<int>& sel, const std::vector<int>& steps,
                     int nsm, CycSchedule& out);
 int upload_schedule(ua_mesh* m, const CycSchedule& s);
-void arena_size(const Cycle& C, const CycSchedule& sch, bool fp32, int most, int small, int& bytes, bool& room);
-CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof);
+void arena_size(const Cycle& C, const CycSchedule& sch, CycForm form, int most, int small, int& bytes, bool& room);
+CycArgs cycle_args(const ua_mesh* m, CycForm form, bool prof);
 // cooperative launch of a team kernel, one CTA per SM
 template <typename A>
 inline int launch_team(ua_mesh* m, void (*k)(const A), const A& a, int nctas, int smem) {

@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
     int u0, u1;
     team_share(t, units, u0, u1);
     const int lo = u0 * U, hi = min(u1 * U, S.nsl);
-    cyc_stage<double, double, double>(a.cyc, a.lv, a.lv, S, t, lo, hi, ar, lev, &fine, 32, dense, a.room);
+    cyc_stage<double, double, double, double>(a.cyc, a.lv, a.lv, S, t, lo, hi, ar, lev, &fine, 32, dense, a.room);
     // vectors into slice order
     for (int i = lo + warp; i < hi; i += kCycWarps)
       if (32 * i + lane < nn) {
@@ -632,7 +632,7 @@ int gmres_resident(ua_mesh* m, const GmSolve& v, const std::vector<int>& sel, co
   if (sch.cta.empty()) return UA_OK;
   if (int rc = upload_schedule(m, sch)) return rc;
   GmArgs A{};
-  A.cyc = cycle_args(m, false, false);
+  A.cyc = cycle_args(m, CF_FP64, false);
   A.lv = S.v64;
   A.v3 = C.gm_v3;
   A.hinv = C.gm_hinv;
@@ -673,7 +673,7 @@ int gmres_resident(ua_mesh* m, const GmSolve& v, const std::vector<int>& sel, co
   A.tol = v.tol;
   A.done = v.done;
   A.its = v.its;
-  arena_size(C, sch, false, kGmArena, kGmArenaSmall, A.arena, A.room);
+  arena_size(C, sch, CF_FP64, kGmArena, kGmArenaSmall, A.arena, A.room);
   UA_CUDA_TRY(cudaFuncSetAttribute(k_gmres_team, cudaFuncAttributeMaxDynamicSharedMemorySize, kGmArena));
   const int rc = launch_team(m, k_gmres_team, A, (int)sch.cta.size(), A.arena);
   ++*launches;

@@ -149,7 +149,8 @@ struct CycSegs {
   int n;
   CycSeg s[2 * kCycMaxLev];
 };
-template <typename KT, typename PT, typename QT>
+// QT: Q of the finest level, QC: of the others
+template <typename KT, typename PT, typename QT, typename QC>
 __global__ void __launch_bounds__(256) k_cyc_levels(const CycSegs S, const int* depth, const int* sel) {
   int k = 0;
   while (k + 1 < S.n && blockIdx.x >= S.s[k + 1].b0) ++k;
@@ -181,10 +182,13 @@ __global__ void __launch_bounds__(256) k_cyc_levels(const CycSegs S, const int* 
     double2* q = reinterpret_cast<double2*>(G.out) + 2 * (long long)(o & ~31) + (o & 31);
     q[0] = make_double2(q0, q1);
     q[32] = make_double2(q2, q3);
+  } else if (G.qslot) {
+    QuadSet<QT>::set(G.out, G.qslot[e], q0, q1, q2, q3);
   } else {
-    QuadSet<QT>::set(G.out, G.qslot ? G.qslot[e] : e, q0, q1, q2, q3);
+    QuadSet<QC>::set(G.out, e, q0, q1, q2, q3);
   }
-  QuadSet<QT>::set(G.outT, G.tpos[e], q0, q1, q2, q3);
+  if (G.lev == 0) QuadSet<QT>::set(G.outT, G.tpos[e], q0, q1, q2, q3);
+  else QuadSet<QC>::set(G.outT, G.tpos[e], q0, q1, q2, q3);
 }
 
 // ---------------------------------------------------------------------------
@@ -205,14 +209,14 @@ bool cycle_supported(const ua_mesh* m) {
 
 // Shared memory for a schedule's copies: what its CTAs' rows need, and their solo levels as far as the
 // maximum allows; rows that do not fit are left to L1 and L2.
-void arena_size(const Cycle& C, const CycSchedule& sch, bool fp32, int most, int small, int& bytes, bool& room) {
+void arena_size(const Cycle& C, const CycSchedule& sch, CycForm form, int most, int small, int& bytes, bool& room) {
   double need = 0, solo = 0;
   for (const int4& ct : sch.cta)
     for (int k = ct.x; k < ct.y; ++k) {
       const int s = sch.queue[k];
       const CycSys& y = C.sys[s];
-      need = std::max(need, (C.h_bytes[fp32][s] + (ct.w == 1 ? C.h_solo[fp32][s] : 0.0)) / ct.w + 8.0 * y.dn * y.dn);
-      if (ct.w > 1) solo = std::max(solo, C.h_solo[fp32][s] + 8192);
+      need = std::max(need, (C.h_bytes[form][s] + (ct.w == 1 ? C.h_solo[form][s] : 0.0)) / ct.w + 8.0 * y.dn * y.dn);
+      if (ct.w > 1) solo = std::max(solo, C.h_solo[form][s] + 8192);
     }
   need = 1.15 * need + 8192;
   room = need <= most;
@@ -292,16 +296,17 @@ int cycle_init(ua_mesh* m) {
       D.tptr = upload(m, a, tp, ok);
       D.tfine = upload(m, a, tf, ok);
       D.tpos = upload(m, a, tpos, ok);
-      for (int w = 0; w < 2; ++w) {  // bytes a step reads of this level (FP64, mixed form)
+      for (int w = 0; w < CF_COUNT; ++w) {  // bytes a step reads of this level
+        const int qe = 4 + (w == CF_FP64 ? 32 : w == CF_LO && l == 0 ? 8 : 16);
         C.h_bytes[w].resize(nsys, 0.0);
         C.h_solo[w].resize(nsys, 0.0);
         for (int s = 0; s < nsys; ++s) {
           const int g0 = L.node_off[s], g1 = L.node_off[s + 1];
           if (g1 == g0) continue;
-          double b = 2.0 * (ap[g1] - ap[g0]) * (w ? 12 : 36);
+          double b = 2.0 * (ap[g1] - ap[g0]) * qe;
           if (l == 0)
             b += (double)(SL.h_sl_off[kSellSlices * SL.h_sys_sb_off[s + 1]] - SL.h_sl_off[kSellSlices * SL.h_sys_sb_off[s]]) *
-                 (w ? 28 : 36);
+                 (w == CF_FP64 ? 36 : w == CF_LO ? 28 : 20);
           else
             b += (double)(a->h_gptr[l][g1] - a->h_gptr[l][g0]) * (w ? 20 : 36);
           (l > 0 && g1 - g0 <= kSoloNodes ? C.h_solo : C.h_bytes)[w][s] += b + 8.0 * (g1 - g0);
@@ -370,8 +375,9 @@ int cycle_alloc_values(ua_mesh* m, bool fp32, bool lo) {
     // levels 1 .. nlev-2 hold an operator; node entries = dof entries / 4
     if (l > 0 && l + 1 < a->nlev) need(fp32 ? &D.a32 : &D.a64, (fp32 ? 16 : 32) * (size_t)(a->lev[l].nnz / 4));
     if (l + 1 < a->nlev) {
-      need(fp32 ? &D.qh : &D.qd, (fp32 ? 8 : 32) * (size_t)D.nq, l == 0);  // padding slots stay zero
-      need(fp32 ? &D.th : &D.td, (fp32 ? 8 : 32) * (size_t)a->lev[l].nap);
+      const bool half = lo && l == 0;
+      need(half ? &D.qh : fp32 ? &D.qf : &D.qd, (half ? 8 : fp32 ? 16 : 32) * (size_t)D.nq, l == 0);  // padding slots stay zero
+      need(half ? &D.th : fp32 ? &D.tf : &D.td, (half ? 8 : fp32 ? 16 : 32) * (size_t)a->lev[l].nap);
     }
   }
   return ok ? UA_OK : set_error(UA_ERR_OOM, "collapsed cycle: device allocation of the values failed");
@@ -400,10 +406,9 @@ void cycle_fill_fine(ua_mesh* m, const int* colind0, const void* K0, bool fp32, 
   else fill_fine_t<double>(m, colind0, (const double*)K0, lo, sel, st, launches);
 }
 
-template <typename KT>
-static void fill_levels_t(ua_mesh* m, const int* sel, cudaStream_t st, long long* launches) {
+template <typename KT, typename QT>
+static void fill_levels_t(ua_mesh* m, CycForm form, const int* sel, cudaStream_t st, long long* launches) {
   using PT = typename PQuadOf<KT>::T;
-  using QT = typename std::conditional<sizeof(KT) == 4, __nv_bfloat16, double>::type;
   constexpr bool f = sizeof(KT) == 4;
   Amg* a = m->amg;
   Cycle& C = a->cyc;
@@ -419,16 +424,17 @@ static void fill_levels_t(ua_mesh* m, const int* sel, cudaStream_t st, long long
     AmgLevel& L = a->lev[l];
     Cycle::Lev& D = C.lev[l];
     add(CycSeg{0, l, L.nap, L.ap_node, L.apn_col, L.apn_ptr, L.nrow, D.sc, C.lev[l + 1].sc, L.sa_ap,
-               f ? L.sa_qh : L.sa_qd, L.ap_p, D.qslot, D.tpos, f ? D.qh : D.qd, f ? D.th : D.td});
+               f ? L.sa_qh : L.sa_qd, L.ap_p, D.qslot, D.tpos, D.q(form, l), D.t(form, l)});
     if (l > 0)
       add(CycSeg{0, -1, L.ng, a->lev[l - 1].ac_node, D.ncol, L.gptr, L.nrow, D.sc, nullptr, L.A, nullptr, nullptr,
                  nullptr, nullptr, f ? D.a32 : D.a64, nullptr});
   }
-  if (nb) k_cyc_levels<KT, PT, QT><<<(unsigned)nb, 256, 0, st>>>(S, a->d_depth, sel), ++*launches;
+  if (nb) k_cyc_levels<KT, PT, QT, KT><<<(unsigned)nb, 256, 0, st>>>(S, a->d_depth, sel), ++*launches;
 }
-void cycle_fill_levels(ua_mesh* m, bool fp32, const int* sel, cudaStream_t st, long long* launches) {
-  if (fp32) fill_levels_t<float>(m, sel, st, launches);
-  else fill_levels_t<double>(m, sel, st, launches);
+void cycle_fill_levels(ua_mesh* m, bool fp32, bool lo, const int* sel, cudaStream_t st, long long* launches) {
+  if (!fp32) fill_levels_t<double, double>(m, CF_FP64, sel, st, launches);
+  else if (lo) fill_levels_t<float, __nv_bfloat16>(m, CF_LO, sel, st, launches);
+  else fill_levels_t<float, float>(m, CF_FP32, sel, st, launches);
 }
 
 // ---------------------------------------------------------------------------
@@ -522,15 +528,15 @@ int upload_schedule(ua_mesh* m, const CycSchedule& s) {
   return UA_OK;
 }
 
-CycArgs cycle_args(const ua_mesh* m, bool fp32, bool prof) {
+CycArgs cycle_args(const ua_mesh* m, CycForm form, bool prof) {
   const Amg* a = m->amg;
   const Cycle& C = a->cyc;
   CycArgs A{};
   for (int l = 0; l + 1 < a->nlev; ++l) {
     const AmgLevel& L = a->lev[l];
     const Cycle::Lev& D = C.lev[l];
-    A.lev[l] = CycLev{L.gptr, D.ncol, fp32 ? D.a32 : D.a64, l ? L.apn_ptr : nullptr, D.qoff, D.qcol, fp32 ? D.qh : D.qd,
-                      D.tptr, D.tfine, fp32 ? D.th : D.td, L.b, L.x2};
+    A.lev[l] = CycLev{L.gptr, D.ncol, form == CF_FP64 ? D.a64 : D.a32, l ? L.apn_ptr : nullptr, D.qoff, D.qcol,
+                      D.q(form, l), D.tptr, D.tfine, D.t(form, l), L.b, L.x2};
   }
   A.lev[a->nlev - 1].b = a->lev[a->nlev - 1].b;
   A.fine = CycFine{a->sell.perm, a->sell.sl_off, C.d_pcol};
@@ -636,8 +642,11 @@ struct PcgArgs {
 // partials crosses CTAs.
 // 512 threads of up to 128 registers, one CTA per SM: few warps, each with up to ten slots of its
 // slice in flight (1024 threads at 64 registers spilled 800 bytes a thread).
-template <typename KT, typename LT, typename VT, typename QT>
+// QT, QC: Q of the finest level and of the coarse ones.
+template <typename KT, typename LT, typename VT, typename QT, typename QC>
 __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
+  static_assert(sizeof(QT) >= sizeof(LT) && sizeof(QC) >= sizeof(KT),
+                "Q holds the smoothing of its level's operator and is no narrower than it");
   using V2 = typename Vec2<VT>::T;
   extern __shared__ __align__(16) char arena_mem[];
   __shared__ CycSys S;
@@ -672,7 +681,7 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
     const double* dense;
     int lo, hi;
     team_share(t, S.nsl, lo, hi);
-    cyc_stage<KT, LT, QT>(a.cyc, a.kv, a.lv, S, t, lo, hi, ar, lev, &fine, 4 * sizeof(KT), dense, a.room);
+    cyc_stage<KT, LT, QT, QC>(a.cyc, a.kv, a.lv, S, t, lo, hi, ar, lev, &fine, 4 * sizeof(KT), dense, a.room);
     const int n0 = S.n0[0], nn = S.nn[0], dep = S.depth, solo = t.size > 1 ? S.solo : dep;
     const bool stream = fine.cols == a.cyc.fine.cols;  // rows read from global memory
     // restrict the updated residual after one more barrier, or b - alpha q from the two old vectors:
@@ -701,14 +710,14 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
       const bool odd = its & 1;
       // z = cycle(r), the finest restriction done
       for (int l = 1; l < solo; ++l) {
-        cyc_down<VT, QT>(lev[l], S, l, t, (const V2*)a.cyc.lev[l].b, (V2*)a.cyc.lev[l + 1].b);
+        cyc_down<VT, QC>(lev[l], S, l, t, (const V2*)a.cyc.lev[l].b, (V2*)a.cyc.lev[l + 1].b);
         UA_TEAM_SYNC(t);
       }
       const V2* zc = zcs - S.n0[dep];
-      if (solo < dep) zc = cyc_solo<VT, KT, QT>(lev, S, a.cyc, dense, dsh, zcs, sbuf);
+      if (solo < dep) zc = cyc_solo<VT, KT, QC>(lev, S, a.cyc, dense, dsh, zcs, sbuf);
       else cyc_dense<VT>(S, dense, bL, dsh, zcs);
       for (int l = solo - 1; l > 0; --l) {
-        cyc_up<VT, KT, QT>(lev[l], S, l, t, (const V2*)a.cyc.lev[l].b, (V2*)a.cyc.lev[l].z, zc);
+        cyc_up<VT, KT, QC>(lev[l], S, l, t, (const V2*)a.cyc.lev[l].b, (V2*)a.cyc.lev[l].z, zc);
         UA_TEAM_SYNC(t);
         zc = (const V2*)a.cyc.lev[l].z;
       }
@@ -823,11 +832,11 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_pcg_team(const PcgArgs a) {
   }
 }
 
-template <typename KT, typename LT, typename VT, typename QT>
+template <typename KT, typename LT, typename VT, typename QT, typename QC>
 static int launch_pcg(ua_mesh* m, const PcgArgs& a, int nctas) {
-  UA_CUDA_TRY(cudaFuncSetAttribute(k_pcg_team<KT, LT, VT, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  UA_CUDA_TRY(cudaFuncSetAttribute(k_pcg_team<KT, LT, VT, QT, QC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    kCycArena));
-  return launch_team(m, k_pcg_team<KT, LT, VT, QT>, a, nctas, a.arena);
+  return launch_team(m, k_pcg_team<KT, LT, VT, QT, QC>, a, nctas, a.arena);
 }
 
 int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, const std::vector<int>& steps, int nsm,
@@ -841,14 +850,15 @@ int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, con
   if (v.prof) UA_CUDA_TRY(cudaMemsetAsync(C.d_prof, 0, sizeof(unsigned long long) * 2 * CP_COUNT, m->stream));
   const Sell& S = a->sell;
   PcgArgs A{};
-  A.cyc = cycle_args(m, v.fp32, v.prof);
+  const CycForm form = cyc_form(v.fp32, v.lo);
+  A.cyc = cycle_args(m, form, v.prof);
   A.kv = v.fp32 ? (const void*)S.v32 : (const void*)S.v64;
   A.lv = v.fp32 ? (v.lo ? (const void*)S.vlo : (const void*)S.v32) : (const void*)S.v64;
   A.r = v.r;
   A.r2 = C.d_r2;
   // shared memory for the copies: all of it where the largest share of a CTA fits, else what the
   // small levels take (the rest serves as L1 for the streamed rows)
-  arena_size(C, sch, v.fp32, kCycArena, kCycArenaSmall, A.arena, A.room);
+  arena_size(C, sch, form, kCycArena, kCycArenaSmall, A.arena, A.room);
   A.z = v.z;
   A.p = v.p;
   A.q = v.q;
@@ -876,9 +886,9 @@ int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, con
   UA_CUDA_TRY(cudaGetLastError());
   const int nc = C.last_grid = (int)sch.cta.size();
   int rc;
-  if (!v.fp32) rc = launch_pcg<double, double, double, double>(m, A, nc);
-  else if (v.lo) rc = launch_pcg<float, __nv_bfloat16, float, __nv_bfloat16>(m, A, nc);
-  else rc = launch_pcg<float, float, float, __nv_bfloat16>(m, A, nc);
+  if (!v.fp32) rc = launch_pcg<double, double, double, double, double>(m, A, nc);
+  else if (v.lo) rc = launch_pcg<float, __nv_bfloat16, float, __nv_bfloat16, float>(m, A, nc);
+  else rc = launch_pcg<float, float, float, float, float>(m, A, nc);
   ++*launches;
   return rc;
 }
