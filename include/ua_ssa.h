@@ -228,7 +228,9 @@ typedef struct ua_newton_report {
     int32_t cauchy_fallbacks;   /* times rLineminUa.m:96 would continue with the M-Cauchy step */
     int32_t retried;            /* uv.m:107-112 reset-and-retry happened */
     double r, rForce, rWork;    /* uvResidual (= r) */
-    double assembly_ms, solve_ms, total_ms;  /* host wall clock of the phases */
+    double assembly_ms, solve_ms;  /* of the Newton steps, on the handle's stream: tangent and right-hand side
+                                      (not those assembled ahead, with a cost), linear solve */
+    double total_ms;               /* host wall clock of the call */
     double device_ms;           /* CUDA-event time on the handle's stream, whole call */
     double kasmK_ms, kasmR_ms, kspmv_ms;     /* summed launch durations (profile=1) */
     int32_t kasmK_n, kasmR_n, kspmv_n;       /* launches timed */

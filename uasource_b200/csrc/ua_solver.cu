@@ -159,6 +159,7 @@ struct Work {
   int pcg_exec_maxit[32] = {};
   int pcg_exec_lpr[32] = {};
   int nsm = 148;  // SMs of the handle's device (grid of the list-driven kernels)
+  cudaEvent_t phase[3] = {};  // of a Newton step: its start, the end of its assembly, of its linear solve
 };
 
 // Two-entry constraint rows (ties, normal velocities): the second dof and the scaled coefficients
@@ -1388,6 +1389,24 @@ static int finish_deferred(ua_mesh* m, std::vector<int>& its) {
   for (int s = 0; s < w->nsys; ++s) its[s] = its[s] ? w->h_res[s] : 0;
   return UA_OK;
 }
+// The phases of a Newton step are timed on the stream: the host only enqueues them and waits once, for the
+// costs at its end.
+static int phase_mark(ua_mesh* m, int k) {
+  cudaEvent_t& e = m->work->phase[k];
+  if (!e) UA_CUDA_TRY(cudaEventCreate(&e));
+  UA_CUDA_TRY(cudaEventRecord(e, m->stream));
+  return UA_OK;
+}
+// adds the times of a step whose stream has drained since its last mark
+static int phase_times(ua_mesh* m, double& t_asm, double& t_sol) {
+  const cudaEvent_t* e = m->work->phase;
+  float a = 0, b = 0;
+  UA_CUDA_TRY(cudaEventElapsedTime(&a, e[0], e[1]));
+  UA_CUDA_TRY(cudaEventElapsedTime(&b, e[1], e[2]));
+  t_asm += a;
+  t_sol += b;
+  return UA_OK;
+}
 // Enqueues the counts of a resident solve for finish_deferred.
 static int defer_result(ua_mesh* m) {
   Work* w = m->work;
@@ -1945,7 +1964,7 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
     for (int s = 0; s < nsys; ++s) sel[s] = st[s].active ? 1 : 0;
     if ((rc = set_sel(m, sel))) return rc;
     // R and K (:197-213); the interval criterion 1 (default) always refreshes K
-    double t0 = now_ms();
+    if ((rc = phase_mark(m, 0))) return rc;
     bool refreshK = false;
     for (int s = 0; s < nsys; ++s)
       if (st[s].active && (((st[s].iteration - 1) % std::max(1, p->ModifiedNRuvIntervalCriterion)) == 0 ||
@@ -1968,8 +1987,7 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
       if ((rc = set_sel(m, sel))) return rc;
     }
     k_frhs<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->R, w->dof_con, w->lam, w->frhs, w->con_dof, con_pairs(w)), ++g_launches;
-    double t1 = now_ms();
-    t_asm += t1 - t0;
+    if ((rc = phase_mark(m, 1))) return rc;
     // linear solve (:242-257); a resident solve is not waited for: its counts come with the costs
     std::vector<double> eta(nsys);
     for (int s = 0; s < nsys; ++s) eta[s] = forcing_term(p, st[s].rForce);
@@ -1979,6 +1997,7 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
     rc = linear_solve(m, p, its, eta.data());
     w->defer = false;
     if (rc) return rc;
+    if ((rc = phase_mark(m, 2))) return rc;
     // gamma=0 (:260-283): R at X is the residual assembled with K above.  Only the first iteration
     // decides on it before gamma = 1 is evaluated; else the two costs come back together.
     bool first = false;
@@ -2006,7 +2025,7 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
     if ((rc = cost_eval(m, p, true, true, ahead))) return rc;
     if (!first) cost0();
     if ((rc = finish_deferred(m, its))) return rc;
-    t_sol += now_ms() - t1;
+    if ((rc = phase_times(m, t_asm, t_sol))) return rc;
     for (int s = 0; s < nsys; ++s)
       if (solved[s]) {
         st[s].kits = its[s];
@@ -3042,11 +3061,10 @@ static int newton_run_uvh(ua_mesh* m, const ua_params* p, std::vector<ua_newton_
     if (!any) break;
     for (int s = 0; s < nsys; ++s) sel[s] = st[s].active ? 1 : 0;
     if ((rc = set_sel(m, sel))) return rc;
-    double t0 = now_ms();
+    if ((rc = phase_mark(m, 0))) return rc;
     if ((rc = assemble_uvh(m, p, true, false, false, false))) return rc;  // :127
     k_frhs<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->R, w->dof_con, w->lam, w->frhs, w->con_dof, con_pairs(w)), ++g_launches;
-    double t1 = now_ms();
-    t_asm += t1 - t0;
+    if ((rc = phase_mark(m, 1))) return rc;
     for (int s = 0; s < nsys; ++s) its[s] = sel[s] ? std::max(1, st[s].kits) : 0;
     std::vector<double> eta(nsys);
     for (int s = 0; s < nsys; ++s) eta[s] = forcing_term_uvh(p, st[s].rForce == INFINITY ? 1.0 : st[s].rForce);
@@ -3058,6 +3076,7 @@ static int newton_run_uvh(ua_mesh* m, const ua_params* p, std::vector<ua_newton_
       w->defer = false;
       if (rc) return rc;
     }
+    if ((rc = phase_mark(m, 2))) return rc;
     // r0 = func(0), r1 = func(1) (:155-156); the two come back together, with the iteration counts
     for (int g1 = 0; g1 < 2; ++g1) {
       for (int s = 0; s < nsys; ++s) gam[s] = (double)g1;
@@ -3066,7 +3085,7 @@ static int newton_run_uvh(ua_mesh* m, const ua_params* p, std::vector<ua_newton_
       if ((rc = cost_eval_uvh(m, p, g1 != 0, g1 ? nullptr : w->h_sysv0, g1 != 0))) return rc;
     }
     if ((rc = finish_deferred(m, its))) return rc;
-    t_sol += now_ms() - t1;
+    if ((rc = phase_times(m, t_asm, t_sol))) return rc;
     for (int s = 0; s < nsys; ++s) {
       if (!sel[s]) continue;
       UvhSys& S = st[s];
@@ -3495,6 +3514,8 @@ extern "C" void ua_mesh_destroy(ua_mesh* m) {
     if (w->h_ring) cudaFreeHost(w->h_ring);
     if (w->h_nan) cudaFreeHost(w->h_nan);
     if (w->h_gamma) cudaFreeHost(w->h_gamma);
+    for (cudaEvent_t e : w->phase)
+      if (e) cudaEventDestroy(e);
     delete w;
   }
   amg_free(m->amg);
