@@ -157,8 +157,8 @@ typedef struct ua_params {
                                   (0 = by precision: every step in FP64, every fourth in the mixed form;
                                   1 = every step); the coarse operators P'KP always use the current
                                   tangent */
-    int32_t uvh_h_sweeps;      /* uvh block preconditioner: Chebyshev-weighted l1-Jacobi sweeps on the
-                                  thickness block K_hh (0 = default 5) */
+    int32_t uvh_h_sweeps;      /* uvh block preconditioner: l1-Jacobi sweeps on the thickness block K_hh
+                                  (0 = default 5) */
     int32_t krylov_sell;       /* 1 = the AMG-preconditioned uv PCG runs its SpMV and the V-cycle's
                                   finest-level passes on node-sliced (sliced ELL) copies of the tangent,
                                   both rows of a node per thread (default); 0 = CSR row kernels */

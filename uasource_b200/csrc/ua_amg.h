@@ -1,6 +1,5 @@
 // Aggregation AMG preconditioner of the uv tangent (internal interface).
 #pragma once
-#include <cmath>
 #include "ua_internal.h"
 
 namespace ua {
@@ -139,30 +138,14 @@ struct PcgSolve {
 // sel: systems to solve; steps: expected iterations (the schedule's weights)
 int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, const std::vector<int>& steps, int nsm,
                  long long* launches);
-// Weights of the hsw l1-Jacobi sweeps on the thickness block: the Chebyshev polynomial of degree hsw on
-// [kHSweepLow, 1] (l1 scaling bounds the spectrum by one) as Richardson steps; more than kHSweepMax
-// sweeps repeat the polynomial of that degree, plain sweeps first.  A sweep is a pass with a barrier, so
-// the fewest that cost no iterations: P1 141x71, eight plain sweeps 309 iterations and 23.2 ms a step,
-// five weighted ones 309 and 20.6 (three: 321, 19.8); P2 101x51, 346 and 41.7 against 364 and 39.6 (three:
-// 423, 40.9).
-constexpr int kHSweepMax = 16, kHSweepDefault = 5;
-constexpr double kHSweepLow = 0.3;
-struct HSweeps {
-  int n;
-  double om[kHSweepMax];
-  __host__ __device__ double weight(int q) const {
-    const int first = n <= kHSweepMax ? 0 : n % kHSweepMax;
-    return q < first ? 1.0 : om[(q - first) % kHSweepMax];
-  }
-};
-inline HSweeps h_sweeps(int n) {
-  HSweeps h{};
-  h.n = n;
-  const int d = n < kHSweepMax ? n : kHSweepMax;
-  for (int k = 0; k < d; ++k)
-    h.om[k] = 1.0 / (0.5 * (1.0 + kHSweepLow) + 0.5 * (1.0 - kHSweepLow) * cos(3.14159265358979323846 * (2 * k + 1) / (2.0 * d)));
-  return h;
-}
+// l1-Jacobi sweeps on the thickness block by default.  A sweep is a pass with a barrier; five take the time of
+// eight or less in steps that converge well, and their few more iterations do not move the step at which GMRES
+// stalls (milliseconds a step and iterations, five against eight: P1 141x71 0.1 a 19 and 303, 21 and 300; 0.3 a
+// 34 and 552, 37 and 529; P2 101x51 0.1 a 28 and 315, 29 and 280; 0.3 a 53 and 601, 53 and 518).  The sweeps are
+// not weighted: l1 scaling bounds the modulus of the spectrum, but the block is an advection, its eigenvalues
+// leave the real axis with the step, and Chebyshev weights, which are small on the axis alone, amplify there
+// (0.5 a: P1 61x43 533 -> 2514 iterations, P1 281x141 2746 -> no convergence).
+constexpr int kHSweepDefault = 5;
 struct GmSolve {
   const int* rowptr;      // 3-dof CSR
   const double* K;
@@ -173,7 +156,7 @@ struct GmSolve {
   const double* tol;      // [nsys] relative tolerances
   int *done, *its;
   int mr, maxit, max_cycles;
-  HSweeps hsw;
+  int hsw;                // sweeps on the thickness block
 };
 // restarted GMRES of the uvh system (ua_gmres.cu), restart up to gmres_resident_max_restart()
 int gmres_resident_max_restart();

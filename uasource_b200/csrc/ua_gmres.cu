@@ -87,7 +87,7 @@ struct GmArgs {
   double *part1, *part2, *part3;  // partials of the two Gram-Schmidt passes and of the norms, [vector][part_ld]
   long long npad, part_ld, part_sys;  // part_sys: doubles per system
   int mr, maxit, max_cycles;
-  HSweeps hsw;
+  int hsw;
   const double* tol;        // [nsys]
   int *done, *its;
   int arena;
@@ -470,23 +470,21 @@ __global__ void __launch_bounds__(kCycThreads, 1) k_gmres_team(const GmArgs a) {
         UA_TEAM_SYNC(t);
         // thickness rows; the sweeps ping-pong so that the last one writes z.h
         double* bufs[2] = {a.z.h, a.ht};
-        int cur = (a.hsw.n - 1) % 2 == 0 ? 0 : 1;
-        const double om0 = a.hsw.weight(0);
+        int cur = (a.hsw - 1) % 2 == 0 ? 0 : 1;
         for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
           if (!in) return;
           const double b = vj.h[k] - gm_hrow<0>(a.cyc.fine, a.v3, S.sl0 + i, lane, a.z.uv, nullptr, range);
           const double hi1 = a.hinv[k];
           a.bh[k] = hi1 > 0 ? b : 0.0;
-          bufs[cur][k] = om0 * b * hi1;
+          bufs[cur][k] = b * hi1;
         });
         UA_TEAM_SYNC(t);
-        for (int q = 1; q < a.hsw.n; ++q) {
-          const double om = a.hsw.weight(q);
+        for (int q = 1; q < a.hsw; ++q) {
           const double* zi = bufs[cur];
           double* zo = bufs[1 - cur];
           for_slices(lo, hi, n0, nn, false, [&](int i, int k, bool in, int) {
             if (in)
-              zo[k] = zi[k] + om * (a.bh[k] - gm_hrow<1>(a.cyc.fine, a.v3, S.sl0 + i, lane, nullptr, zi, range)) * a.hinv[k];
+              zo[k] = zi[k] + (a.bh[k] - gm_hrow<1>(a.cyc.fine, a.v3, S.sl0 + i, lane, nullptr, zi, range)) * a.hinv[k];
           });
           UA_TEAM_SYNC(t);
           cur = 1 - cur;

@@ -2548,13 +2548,13 @@ __global__ void __launch_bounds__(256) k_gm_resid(const int* rb_start, const int
 // z_h = invd_h (p_h - K_hu z_u - K_hv z_v), the velocity part z already set
 // (row (2, g) of a uvh tangent: blocks u, v, h of deg entries each).
 // Thickness rows of the block lower-triangular preconditioner: b_h = p_h - K_hu z_u (z_u
-// already in z), then the first weighted l1-Jacobi sweep zt_h = om b_h / l1_h.  A row of the uvh tangent
+// already in z), then the first l1-Jacobi sweep zt_h = b_h / l1_h.  A row of the uvh tangent
 // holds three blocks of deg columns (u, v, h).
 __global__ void __launch_bounds__(256) k_uvh_hrows(const int* rb_start, const int* rb_sys, const int* sel,
                                                    const int* done, const int* dof_off, const int* rowptr,
                                                    const int* colind, const double* K, const double* hl1,
                                                    const unsigned char* cmask, const double* p, const double* z,
-                                                   double* bh, double* zt, double om) {
+                                                   double* bh, double* zt) {
   const int blk = blockIdx.x;
   const int s = rb_sys[blk];
   if (!sel[s] || done[s]) return;
@@ -2567,7 +2567,7 @@ __global__ void __launch_bounds__(256) k_uvh_hrows(const int* rb_start, const in
     for (int q = q0; q < q0 + 2 * deg; ++q) acc += K[q] * z[colind[q]];
     const double b = p[row] - acc;
     bh[row] = b;
-    zt[row] = om * b / hl1[row];
+    zt[row] = b / hl1[row];
   }
 }
 
@@ -2588,12 +2588,12 @@ __global__ void __launch_bounds__(256) k_uvh_hl1(const int* rb_start, const int*
   }
 }
 
-// one weighted l1-Jacobi sweep on the thickness block: zout_h = zin_h + om (b_h - K_hh zin_h) / l1_h
+// one l1-Jacobi sweep on the thickness block: zout_h = zin_h + (b_h - K_hh zin_h) / l1_h
 __global__ void __launch_bounds__(256) k_uvh_hsweep(const int* rb_start, const int* rb_sys, const int* sel,
                                                     const int* done, const int* dof_off, const int* rowptr,
                                                     const int* colind, const double* K, const double* hl1,
                                                     const unsigned char* cmask, const double* bh,
-                                                    const double* zin, double* zout, double om) {
+                                                    const double* zin, double* zout) {
   const int blk = blockIdx.x;
   const int s = rb_sys[blk];
   if (!sel[s] || done[s]) return;
@@ -2604,7 +2604,7 @@ __global__ void __launch_bounds__(256) k_uvh_hsweep(const int* rb_start, const i
     const int q0 = rowptr[row], deg = (rowptr[row + 1] - q0) / 3;
     double acc = 0;
     for (int q = q0 + 2 * deg; q < q0 + 3 * deg; ++q) acc += K[q] * zin[colind[q]];
-    zout[row] = zin[row] + om * (bh[row] - acc) / hl1[row];
+    zout[row] = zin[row] + (bh[row] - acc) / hl1[row];
   }
 }
 
@@ -2642,7 +2642,7 @@ static int gmres_resident_solve(ua_mesh* m, const ua_params* p, const double* K,
   v.tol = w->sysv + SV_TOL2 * nsys;
   v.done = w->done; v.its = w->its;
   v.mr = mr;
-  v.hsw = h_sweeps(p->uvh_h_sweeps > 0 ? p->uvh_h_sweeps : kHSweepDefault);
+  v.hsw = p->uvh_h_sweeps > 0 ? p->uvh_h_sweeps : kHSweepDefault;
   v.maxit = p->krylov_maxit;
   v.max_cycles = std::max(1, p->krylov_maxit / mr + 1);
   cudaEvent_t kev[2];
@@ -2706,8 +2706,7 @@ static int gmres_t(ua_mesh* m, const ua_params* p, const KT* K, int* its_out, co
   const int lpr_uv = m->nod == 3 ? 1 : 2;
   // thickness block: l1-Jacobi sweeps on K_hh (the P2 consistent mass in K_hh is not diagonally
   // dominant, so a plain Jacobi step is a poor inverse and a plain Jacobi iteration diverges)
-  const HSweeps hs = h_sweeps(p->uvh_h_sweeps > 0 ? p->uvh_h_sweeps : kHSweepDefault);
-  const int hsw = hs.n;
+  const int hsw = p->uvh_h_sweeps > 0 ? p->uvh_h_sweeps : kHSweepDefault;
   if (m->ndof == 3)
     k_uvh_hl1<<<w->nrb, 256, 0, st>>>(w->rb_start, w->rb_sys, w->sel, m->dm.sys_dof_off, w->rowptr,
                                       (const double*)K, w->gm_hl1), ++g_launches;
@@ -2725,11 +2724,11 @@ static int gmres_t(ua_mesh* m, const ua_params* p, const KT* K, int* its_out, co
       int cur = (hsw - 1) % 2 == 0 ? 0 : 1;
       k_uvh_hrows<<<w->nrb, 256, 0, st>>>(w->rb_start, w->rb_sys, w->sel, w->done, m->dm.sys_dof_off, w->rowptr,
                                           w->colind, (const double*)K, w->gm_hl1, w->cmask, in, out, w->gm_hb,
-                                          bufs[cur], hs.weight(0)), ++g_launches;
+                                          bufs[cur]), ++g_launches;
       for (int k = 1; k < hsw; ++k) {
         k_uvh_hsweep<<<w->nrb, 256, 0, st>>>(w->rb_start, w->rb_sys, w->sel, w->done, m->dm.sys_dof_off,
                                              w->rowptr, w->colind, (const double*)K, w->gm_hl1, w->cmask, w->gm_hb,
-                                             bufs[cur], bufs[1 - cur], hs.weight(k)), ++g_launches;
+                                             bufs[cur], bufs[1 - cur]), ++g_launches;
         cur = 1 - cur;
       }
     }
