@@ -550,7 +550,7 @@ def run_ours(args):
                        "parallelism": f"replicas x{world}" + (", each rank its own seeded batch of this size "
                                                               "distribution" if world > 1 else ""),
                        "precision": "mixed",
-                       "krylov": "PCG, aggregation AMG V(1,1), adaptive forcing, CUDA-graph chunks",
+                       "krylov": "PCG, aggregation AMG V(1,1), adaptive forcing, one resident kernel a solve",
                        "newton_iterations_mean": float(np.mean(its)), "newton_iterations_max": int(max(its)),
                        "pcg_iterations_mean": float(np.mean(kits)), "converged": int(sum(i.converged for i in infos_mx))},
             "batch_latency_ms": {"p50": statistics.median(lat), "p99": lat[min(len(lat) - 1, int(0.99 * len(lat)))]},

@@ -159,9 +159,11 @@ typedef struct ua_params {
                                   tangent */
     int32_t uvh_h_sweeps;      /* uvh block preconditioner: l1-Jacobi sweeps on the thickness block K_hh
                                   (0 = default 5) */
-    int32_t krylov_sell;       /* 1 = the AMG-preconditioned uv PCG runs its SpMV and the V-cycle's
-                                  finest-level passes on node-sliced (sliced ELL) copies of the tangent,
-                                  both rows of a node per thread (default); 0 = CSR row kernels */
+    int32_t krylov_sell;       /* 1 (default) = AMG-preconditioned solves run in one resident kernel on the
+                                  node-sliced (sliced ELL) tangent and the collapsed V-cycle (uv PCG; uvh
+                                  GMRES with a restart of at most 48; smoothed hierarchies, one-entry
+                                  constraint rows), else the uv PCG pass by pass on node slices; 0 = pass by
+                                  pass on CSR rows */
     int32_t SlidingLaw;        /* UA_SLIDING_* (:171) */
     double Nzero;              /* lower value of the effective pressure (:445) */
     int32_t IncludeMelangeModelPhysics;  /* ocean and atmosphere drag on floating ice (BasalDrag.m:275-343);

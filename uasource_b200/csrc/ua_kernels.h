@@ -74,8 +74,6 @@ int adj_cg(const ua_mesh* m, const int* nodeptr, const int* nodecol, const doubl
 cudaError_t adj_scale(const ua_mesh* m, double s, double* x);
 constexpr int kAdjDotBlocks = 256;  // block partials of the adjoint's dot products
 
-size_t uvh_patch_smem(int nod, bool withK, bool fp32, int E);
-int uvh_fields_per_node();
 cudaError_t launch_uvh_assembly(ua_mesh* m, const UvhPhys& P, const UvhIn& in, const UvOut& out, bool withK);
 cudaError_t launch_uv_assembly(ua_mesh* m, const UvPhys& P, const UvIn& in, const UvOut& out, bool withK,
                                bool fp32K, int threads = 0, int regs = 0);

@@ -174,8 +174,9 @@ static size_t elem_smem_bytes(int nod, int ndof) {
   return (size_t)(9 * nod * nod + 6 * nod + 19 * nod) * sizeof(double);  // + staged nodal fields
 }
 
-// Largest element count per patch: shared memory of the assembly kernel and,
-// for the uvh kernel (one thread per element node), its block size.
+// Largest element count per patch: shared memory of the P1 assembly kernels and, for the uvh one (one
+// thread per element node), its block size.  P2 patches are those of the gathers, which sum over element
+// rows in global memory; their size is kept at what a kernel with the rows in shared memory took.
 static int max_patch_elements(int nod, int ndof) {
   const size_t budget = ndof == 2 ? 160 * 1024 : 200 * 1024;
   int e = (int)std::min<size_t>(1023, budget / elem_smem_bytes(nod, ndof));

@@ -123,7 +123,6 @@ struct Work {
   // constraints (mask form: one unit entry per row)
   int* con_dof = nullptr;
   int* con_sys = nullptr;
-  int* sys_con_off = nullptr;
   double* con_rhs = nullptr;
   double *lam = nullptr, *dlam = nullptr, *grhs = nullptr;
   // uvh: level-0 state and mass balance (nodal), BiCGStab vectors
@@ -148,7 +147,6 @@ struct Work {
   bool defer = false, deferred = false;
   int* nan_first = nullptr;  // device NaN scan result (9 ints) and its pinned host copy
   int* h_nan = nullptr;
-  double* h_gamma = nullptr;
   std::vector<int> h_sys_rb_off, h_sys_con_off;
   Prof prof;
   struct ServeState* serve = nullptr;
@@ -884,8 +882,7 @@ static int ensure_work(ua_mesh* m, const ua_params* p) {
       cudaMallocHost(&w->h_nan, 16 * sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&w->h_sysv0, SV_COUNT * sizeof(double) * nsys) != cudaSuccess ||
       cudaMallocHost(&w->h_res, sizeof(int) * (nsys + 1)) != cudaSuccess ||
-      cudaMallocHost(&w->h_ring, w->ring_cap = 65536 + 256 * (size_t)nsys) != cudaSuccess ||
-      cudaMallocHost(&w->h_gamma, sizeof(double) * nsys) != cudaSuccess) {
+      cudaMallocHost(&w->h_ring, w->ring_cap = 65536 + 256 * (size_t)nsys) != cudaSuccess) {
     delete w;
     return set_error(UA_ERR_OOM, "pinned host allocation failed");
   }
@@ -1283,7 +1280,6 @@ static int constraint_rows(const ua_mesh* m, const ua_bcs* bcs, int nB, std::vec
 
 static int build_constraints(ua_mesh* m, const ua_bcs* bcs, int nB) {
   Work* w = m->work;
-  const int nsys = m->dm.nsys;
   std::vector<int> con_dof, con_sys, sys_off, con_dof2;
   std::vector<double> rhs, con_v1, con_v2;
   if (int rc = constraint_rows(m, bcs, nB, con_dof, con_sys, rhs, sys_off, &con_dof2, &con_v1, &con_v2)) return rc;
@@ -1317,8 +1313,7 @@ static int build_constraints(ua_mesh* m, const ua_bcs* bcs, int nB) {
     w->lam = walloc<double>(m, cap);
     w->dlam = walloc<double>(m, cap);
     w->grhs = walloc<double>(m, cap);
-    if (!w->sys_con_off) w->sys_con_off = walloc<int>(m, nsys + 1);
-    if (!w->con_dof || !w->con_sys || !w->con_rhs || !w->lam || !w->dlam || !w->grhs || !w->sys_con_off)
+    if (!w->con_dof || !w->con_sys || !w->con_rhs || !w->lam || !w->dlam || !w->grhs)
       return set_error(UA_ERR_OOM, "constraint allocation failed");
   }
   w->nc = nc;
@@ -1328,8 +1323,6 @@ static int build_constraints(ua_mesh* m, const ua_bcs* bcs, int nB) {
     UA_CUDA_TRY(cudaMemcpyAsync(w->con_sys, con_sys.data(), nc * sizeof(int), cudaMemcpyHostToDevice, m->stream));
     UA_CUDA_TRY(cudaMemcpyAsync(w->con_rhs, rhs.data(), nc * sizeof(double), cudaMemcpyHostToDevice, m->stream));
   }
-  UA_CUDA_TRY(cudaMemcpyAsync(w->sys_con_off, sys_off.data(), (nsys + 1) * sizeof(int), cudaMemcpyHostToDevice,
-                              m->stream));
   // dof masks, on the device: cmask = 0 and dof_con = -1 everywhere, then one thread per
   // constraint (its dof is unique: repeated nodes were dropped above)
   UA_CUDA_TRY(cudaMemsetAsync(w->cmask, 0, m->ndof_total, m->stream));
@@ -3512,7 +3505,6 @@ extern "C" void ua_mesh_destroy(ua_mesh* m) {
     if (w->h_res) cudaFreeHost(w->h_res);
     if (w->h_ring) cudaFreeHost(w->h_ring);
     if (w->h_nan) cudaFreeHost(w->h_nan);
-    if (w->h_gamma) cudaFreeHost(w->h_gamma);
     for (cudaEvent_t e : w->phase)
       if (e) cudaEventDestroy(e);
     delete w;
@@ -3581,7 +3573,6 @@ extern "C" int ua_solve_kape_symmetric(int32_t n, const int64_t* Arowptr, const 
     if (w->h_sysv) cudaFreeHost(w->h_sysv);
     if (w->h_int) cudaFreeHost(w->h_int);
     if (w->h_nan) cudaFreeHost(w->h_nan);
-    if (w->h_gamma) cudaFreeHost(w->h_gamma);
     delete w;
     tmp.work = nullptr;
     dev_free_all(&tmp);
@@ -3594,7 +3585,7 @@ extern "C" int ua_solve_kape_symmetric(int32_t n, const int64_t* Arowptr, const 
     w->nrb = (int)rb_sys.size();
     rb_start.push_back(n);
     w->h_sys_rb_off = {0, w->nrb};
-    std::vector<int> sel1 = {1}, coff = {0, (int)con_dof.size()}, csys(con_dof.size(), 0);
+    std::vector<int> sel1 = {1}, csys(con_dof.size(), 0);
     cudaError_t cp = cudaSuccess;
     auto copied = [&](cudaError_t e) { if (cp == cudaSuccess) cp = e; };
     auto up_i = [&](const std::vector<int>& v) {
@@ -3622,14 +3613,13 @@ extern "C" int ua_solve_kape_symmetric(int32_t n, const int64_t* Arowptr, const 
     w->dof_con = up_i(dof_con);
     w->nc = (int)con_dof.size();
     if (w->nc) {
-      w->con_dof = up_i(con_dof); w->con_sys = up_i(csys); w->sys_con_off = up_i(coff);
+      w->con_dof = up_i(con_dof); w->con_sys = up_i(csys);
       w->con_rhs = up_d(con_rhs.data(), w->nc);
       w->dlam = walloc<double>(&tmp, w->nc); w->grhs = walloc<double>(&tmp, w->nc);
     }
     if (!w->Kd || !w->X || !w->dX || !w->kr || !w->kz || !w->kp || !w->kq || !w->invd || !w->part || !w->cmask ||
         cudaMallocHost(&w->h_sysv, SV_COUNT * sizeof(double)) != cudaSuccess ||
-        cudaMallocHost(&w->h_int, 8 * sizeof(int)) != cudaSuccess ||
-        cudaMallocHost(&w->h_gamma, sizeof(double)) != cudaSuccess) {
+        cudaMallocHost(&w->h_int, 8 * sizeof(int)) != cudaSuccess) {
       cleanup();
       return set_error(UA_ERR_OOM, "allocation failed");
     }
@@ -3708,8 +3698,8 @@ static std::atomic<void*> g_na_addr[kNaMaxDevices];
 // malformed (a column outside [0,n), a negative or decreasing row pointer,
 // or no non-zero at all), so no later kernel may index with it.
 __global__ void k_na_setup(int n, const int* rowptr, const int* col, int* diagpos, unsigned char* cmask,
-                           int* dof_con, double* X, int* rb_start, int* rb_sys, int nrb, int* sys_rb_off,
-                           int* sys_con_off, int nl, int* sel, int* flags) {
+                           int* dof_con, double* X, int* rb_start, int* rb_sys, int nrb, int* sys_rb_off, int* sel,
+                           int* flags) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
     int dp = -1;
@@ -3732,7 +3722,6 @@ __global__ void k_na_setup(int n, const int* rowptr, const int* col, int* diagpo
   if (i < nrb) rb_sys[i] = 0;
   if (i == 0) {
     sys_rb_off[0] = 0; sys_rb_off[1] = nrb;
-    sys_con_off[0] = 0; sys_con_off[1] = nl;
     sel[0] = 1;
     if (rowptr[n] <= rowptr[0]) atomicExch(&flags[3], 1);
   }
@@ -3835,12 +3824,11 @@ extern "C" int ua_solve_kape_symmetric_noalloc(int32_t n, const int32_t* Arowptr
   w.rb_start = small;                          // kNaMaxRb + 1
   w.rb_sys = small + kNaMaxRb + 1;             // kNaMaxRb
   w.sys_rb_off = small + 2 * kNaMaxRb + 1;     // 2
-  w.sys_con_off = small + 2 * kNaMaxRb + 3;    // 2
-  w.sel = small + 2 * kNaMaxRb + 5;
-  w.done = small + 2 * kNaMaxRb + 6;
-  w.its = small + 2 * kNaMaxRb + 7;
-  w.status = small + 2 * kNaMaxRb + 8;
-  int* flags = small + 2 * kNaMaxRb + 9;       // 4
+  w.sel = small + 2 * kNaMaxRb + 3;
+  w.done = small + 2 * kNaMaxRb + 4;
+  w.its = small + 2 * kNaMaxRb + 5;
+  w.status = small + 2 * kNaMaxRb + 6;
+  int* flags = small + 2 * kNaMaxRb + 7;       // 4
   w.part = dsmall; w.sysv = dsmall + 4 * kNaMaxRb;
   w.con_dof = con_i; w.con_sys = con_i + Cn;
   w.con_rhs = con_d; w.dlam = con_d + Cn; w.grhs = con_d + 2 * Cn;
@@ -3859,7 +3847,7 @@ extern "C" int ua_solve_kape_symmetric_noalloc(int32_t n, const int32_t* Arowptr
     return set_error(UA_ERR_CUDA, "no-alloc set-up failed");
   }
   k_na_setup<<<nb, 256, 0, st>>>(n, Arowptr, Acol, w.diagpos, cmask, w.dof_con, w.X, w.rb_start, w.rb_sys, nrb,
-                                 w.sys_rb_off, w.sys_con_off, nl, w.sel, flags);
+                                 w.sys_rb_off, w.sel, flags);
   if (nl)
     k_na_constraints<<<(nl + 255) / 256, 256, 0, st>>>(n, nl, Ldof, Lval, g, cmask, w.dof_con, w.con_dof, w.con_sys,
                                                       w.con_rhs, flags);

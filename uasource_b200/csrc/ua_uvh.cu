@@ -70,9 +70,14 @@ __device__ __forceinline__ void stage_node(const DevMesh& M, const UvhPhys& P, c
   f[F_B1 * ld] = GF * Bg + (1 - GF) * (Sg - rg * h1 / S.rhow);
 }
 
+// ---------------------------------------------------------------------------
+// linear elements
+// ---------------------------------------------------------------------------
+constexpr int NOD = 3, kThreads = 512;
+
 // The patch's non-zeros and residuals, summed over their element contributions in increasing global
 // element order.
-template <int NOD, bool WITHK, typename KT>
+template <bool WITHK, typename KT>
 __device__ __forceinline__ void uvh_scatter(const DevMesh& M, const UvOut& out, int p, int s, int uoff, int voff,
                                             int hoff, const KT* sK, const double* sR, int E, int ne) {
   const int pn0 = M.patch_node_ptr[p];
@@ -148,9 +153,9 @@ __device__ __forceinline__ void uvh_scatter(const DevMesh& M, const UvOut& out, 
 
 // GEN: any sliding law and the melange terms (Weertman chosen at run time); else Weertman only
 // (the general code stays out of that build)
-template <int NOD, bool WITHK, typename KT, bool GEN>
-__global__ void __launch_bounds__(NOD == 3 ? 512 : 320) uvh_patch_kernel(DevMesh M, QuadTable Q, UvhPhys P,
-                                                                          UvhIn in, UvOut out) {
+template <bool WITHK, typename KT, bool GEN>
+__global__ void __launch_bounds__(kThreads) uvh_patch_kernel(DevMesh M, QuadTable Q, UvhPhys P, UvhIn in,
+                                                             UvOut out) {
   constexpr int NB = 9 * NOD * NOD;   // tangent entries per element
   extern __shared__ __align__(16) unsigned char smem[];
   const int p = blockIdx.x;
@@ -191,32 +196,27 @@ __global__ void __launch_bounds__(NOD == 3 ? 512 : 320) uvh_patch_kernel(DevMesh
       for (int k = 0; k < 9 * NOD; ++k) sK[(size_t)(I * 9 * NOD + k) * E + el] = 0;
     }
     double Tx = 0, Fx = 0, Ty = 0, Fy = 0, Th = 0, Fh = 0;
-    // element area from the corner nodes (TriAreaFE.m / TriArea.m) -> l = sqrt(2*area) (:156)
-    const int c0 = 0, c1 = NOD == 3 ? 1 : 2, c2 = NOD == 3 ? 2 : 4;
-    const double area = 0.5 * fabs((fv(F_X, c0) - fv(F_X, c2)) * (fv(F_Y, c1) - fv(F_Y, c0)) -
-                                   (fv(F_X, c0) - fv(F_X, c1)) * (fv(F_Y, c2) - fv(F_Y, c0)));
+    // element area (TriAreaFE.m / TriArea.m) -> l = sqrt(2*area) (:156)
+    const double area = 0.5 * fabs((fv(F_X, 0) - fv(F_X, 2)) * (fv(F_Y, 1) - fv(F_Y, 0)) -
+                                   (fv(F_X, 0) - fv(F_X, 1)) * (fv(F_Y, 2) - fv(F_Y, 0)));
     const double lsupg = sqrt(2 * area);
-    double Dx[NOD], Dy[NOD], detJ = 0;
-    auto deriv = [&](int ip) {  // derivVector.m:96-109
-      double J11 = 0, J12 = 0, J21 = 0, J22 = 0;
+    // derivVector.m:96-109, constant over the element
+    double Dx[NOD], Dy[NOD], J11 = 0, J12 = 0, J21 = 0, J22 = 0;
 #pragma unroll
-      for (int a = 0; a < NOD; ++a) {
-        J11 += fv(F_X, a) * Q.der[ip][0][a];
-        J12 += fv(F_Y, a) * Q.der[ip][0][a];
-        J21 += fv(F_X, a) * Q.der[ip][1][a];
-        J22 += fv(F_Y, a) * Q.der[ip][1][a];
-      }
-      detJ = J11 * J22 - J12 * J21;
+    for (int a = 0; a < NOD; ++a) {
+      J11 += fv(F_X, a) * Q.der[0][0][a];
+      J12 += fv(F_Y, a) * Q.der[0][0][a];
+      J21 += fv(F_X, a) * Q.der[0][1][a];
+      J22 += fv(F_Y, a) * Q.der[0][1][a];
+    }
+    const double detJ = J11 * J22 - J12 * J21;
 #pragma unroll
-      for (int a = 0; a < NOD; ++a) {
-        Dx[a] = (J22 * Q.der[ip][0][a] - J12 * Q.der[ip][1][a]) / detJ;
-        Dy[a] = (-J21 * Q.der[ip][0][a] + J11 * Q.der[ip][1][a]) / detJ;
-      }
-    };
-    if (NOD == 3) deriv(0);
+    for (int a = 0; a < NOD; ++a) {
+      Dx[a] = (J22 * Q.der[0][0][a] - J12 * Q.der[0][1][a]) / detJ;
+      Dy[a] = (-J21 * Q.der[0][0][a] + J11 * Q.der[0][1][a]) / detJ;
+    }
 #pragma unroll 1
     for (int ip = 0; ip < Q.nip; ++ip) {
-      if (NOD != 3) deriv(ip);
       double N[NOD];
 #pragma unroll
       for (int a = 0; a < NOD; ++a) N[a] = Q.fun[ip][a];
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(NOD == 3 ? 512 : 320) uvh_patch_kernel(DevMesh
     sR[(5 * NOD + I) * E + el] = Fh;
   }
   __syncthreads();
-  uvh_scatter<NOD, WITHK, KT>(M, out, p, s, uoff, voff, hoff, sK, sR, E, ne);
+  uvh_scatter<WITHK, KT>(M, out, p, s, uoff, voff, hoff, sK, sR, E, ne);
 }
 
 // ---------------------------------------------------------------------------
@@ -743,34 +743,27 @@ static cudaError_t launch_p2h(ua_mesh* m, const UvhPhys& P, const UvhIn& in, con
   return cudaGetLastError();
 }
 
-size_t uvh_patch_smem(int nod, bool withK, bool fp32, int E) {
-  const int NB = 9 * nod * nod;
-  size_t k = withK ? (((size_t)NB * E * (fp32 ? 4 : 8) + 15) & ~(size_t)15) : 0;
-  return k + (size_t)6 * nod * E * 8 + (size_t)F_COUNT * E * nod * 8;
-}
-
-int uvh_fields_per_node() { return F_COUNT; }
-
-template <int NOD, bool WITHK, typename KT>
-static cudaError_t launch_t(const ua_mesh* m, const UvhPhys& P, const UvhIn& in, const UvOut& out) {
+template <bool WITHK, typename KT>
+static cudaError_t launch_p1h(const ua_mesh* m, const UvhPhys& P, const UvhIn& in, const UvOut& out) {
   const int E = m->dm.max_patch_elems;
-  size_t sm = uvh_patch_smem(NOD, WITHK, sizeof(KT) == 4, E);
+  const size_t k = WITHK ? (((size_t)9 * NOD * NOD * E * sizeof(KT) + 15) & ~(size_t)15) : 0;
+  const size_t sm = k + (size_t)6 * NOD * E * 8 + (size_t)F_COUNT * E * NOD * 8;
   // the residual-only pass keeps the general build: without the tangent its Weertman-only build
   // spills more registers than the general one
-  auto kern = uvh_patch_kernel<NOD, WITHK, KT, true>;
+  auto kern = uvh_patch_kernel<WITHK, KT, true>;
   if constexpr (WITHK) {
-    if (P.uv.law == UA_SLIDING_WEERTMAN && !P.uv.melange) kern = uvh_patch_kernel<NOD, WITHK, KT, false>;
+    if (P.uv.law == UA_SLIDING_WEERTMAN && !P.uv.melange) kern = uvh_patch_kernel<WITHK, KT, false>;
   }
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
   if (e != cudaSuccess) return e;
-  int threads = ((E * NOD + 31) / 32) * 32;
-  if (threads > (NOD == 3 ? 512 : 320)) return cudaErrorInvalidConfiguration;
+  const int threads = ((E * NOD + 31) / 32) * 32;
+  if (threads > kThreads) return cudaErrorInvalidConfiguration;
   kern<<<m->dm.npatch, threads, sm, m->stream>>>(m->dm, quad_table(NOD), P, in, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_uvh_assembly(ua_mesh* m, const UvhPhys& P, const UvhIn& in, const UvOut& out, bool withK) {
-  if (m->nod == 3) return withK ? launch_t<3, true, double>(m, P, in, out) : launch_t<3, false, double>(m, P, in, out);
+  if (m->nod == NOD) return withK ? launch_p1h<true, double>(m, P, in, out) : launch_p1h<false, double>(m, P, in, out);
   UvOut o = out;
   if (!withK) o.K = nullptr;
   return launch_p2h(m, P, in, o);
