@@ -157,8 +157,14 @@ struct Work {
   int pcg_exec_maxit[32] = {};
   int pcg_exec_lpr[32] = {};
   int nsm = 148;  // SMs of the handle's device (grid of the list-driven kernels)
-  cudaEvent_t phase[3] = {};  // of a Newton step: its start, the end of its assembly, of its linear solve
+  // times of a Newton step on the device (ns): start of its assembly, end of it, end of its linear solve;
+  // behind sysv, so that they come back with the costs
+  unsigned long long* stamp = nullptr;
+  size_t cost_bytes() const;
 };
+
+constexpr int kStamps = 3;
+size_t Work::cost_bytes() const { return sizeof(double) * (SV_COUNT * (size_t)nsys + kStamps); }
 
 // Two-entry constraint rows (ties, normal velocities): the second dof and the scaled coefficients
 // of every row; all null when every row has one unit entry (a dof selection).
@@ -191,6 +197,13 @@ __global__ void k_count_active(int nsys, const int* sel, const int* done, const 
   }
   if (threadIdx.x == 0) { out[0] = a[0]; out[1] = b[0]; }
 }
+
+// Phase times: kernels that a step launches anyway write the device's clock as they start (three event
+// records a step instead: P1 21x11 2.57 -> 2.71 ms).
+__device__ __forceinline__ void stamp_now(unsigned long long* t) {
+  if (t && blockIdx.x == 0 && threadIdx.x == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(*t));
+}
+__global__ void k_stamp(unsigned long long* t) { stamp_now(t); }
 
 static void prof_begin(ua_mesh* m, int kind, cudaEvent_t* ev) {
   Work* w = m->work;
@@ -658,7 +671,8 @@ __global__ void __launch_bounds__(256) k_con_multiplier(int nc, const int* con_d
 }
 // frhs = -R - L' l  (SSTREAM2dNR2.m:235)
 __global__ void k_frhs(const int* rb_start, const int* rb_sys, const int* sel, const double* R, const int* dof_con,
-                       const double* lam, double* frhs, const int* con_dof, ConPairs cp) {
+                       const double* lam, double* frhs, const int* con_dof, ConPairs cp, unsigned long long* stamp) {
+  stamp_now(stamp);
   const int blk = blockIdx.x;
   if (!sel[rb_sys[blk]]) return;
   for (int i = rb_start[blk] + threadIdx.x; i < rb_start[blk + 1]; i += blockDim.x) {
@@ -676,7 +690,9 @@ __global__ void __launch_bounds__(kRedThreads) k_cost(const int* rb_start, const
                                                       const double* lam, const double* dlam, const double* gamma,
                                                       const double* X, const double* dX, const int* con_dof,
                                                       const double* con_rhs, ConPairs cp, double* part, int* arrived,
-                                                      int nsys, double* sysv, int write_norm) {
+                                                      int nsys, double* sysv, int write_norm,
+                                                      unsigned long long* stamp) {
+  stamp_now(stamp);
   const int blk = blockIdx.x;
   const int s = rb_sys[blk];
   if (!sel[s]) return;  // uniform over a system's blocks
@@ -729,13 +745,13 @@ static void con_multiplier(const Work* w, const KT* K, cudaStream_t st) {
       ++g_launches;
 }
 // norm: of the residual alone, without constraints
-static void launch_cost(ua_mesh* m, const double* gamma, bool norm) {
+static void launch_cost(ua_mesh* m, const double* gamma, bool norm, unsigned long long* stamp = nullptr) {
   Work* w = m->work;
   k_cost<<<w->nrb, kRedThreads, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sys_rb_off, w->nrb, w->sel, w->R,
                                                 norm ? nullptr : w->dof_con, w->lam, w->dlam, gamma, w->X,
                                                 !norm ? w->dX : nullptr, w->con_dof, w->con_rhs,
                                                 norm ? ConPairs{} : con_pairs(w), w->part, w->arrived, w->nsys, w->sysv,
-                                                norm),
+                                                norm, stamp),
       ++g_launches;
 }
 
@@ -862,7 +878,8 @@ static int ensure_work(ua_mesh* m, const ua_params* p) {
     for (auto f : bv) { *f = walloc<double>(m, N); ok = ok && *f; }
   }
   w->part = walloc<double>(m, 4 * (size_t)w->nrb);
-  w->sysv = walloc<double>(m, SV_COUNT * (size_t)nsys);
+  w->sysv = walloc<double>(m, SV_COUNT * (size_t)nsys + kStamps);
+  w->stamp = w->sysv ? (unsigned long long*)(w->sysv + SV_COUNT * (size_t)nsys) : nullptr;
   w->arrived = walloc<int>(m, nsys);
   if (w->arrived) UA_CUDA_TRY(dev_clear(m, w->arrived, sizeof(int) * nsys));
   w->done = walloc<int>(m, nsys);
@@ -877,10 +894,10 @@ static int ensure_work(ua_mesh* m, const ua_params* p) {
   if (!ok) { delete w; return set_error(UA_ERR_OOM, "device allocation of work buffers failed"); }
   w->nan_first = walloc<int>(m, 16);
   if (!w->nan_first) { delete w; return set_error(UA_ERR_OOM, "device allocation of work buffers failed"); }
-  if (cudaMallocHost(&w->h_sysv, SV_COUNT * sizeof(double) * nsys) != cudaSuccess ||
+  if (cudaMallocHost(&w->h_sysv, w->cost_bytes()) != cudaSuccess ||
       cudaMallocHost(&w->h_int, 4 * sizeof(int) * (nsys + 1)) != cudaSuccess ||
       cudaMallocHost(&w->h_nan, 16 * sizeof(int)) != cudaSuccess ||
-      cudaMallocHost(&w->h_sysv0, SV_COUNT * sizeof(double) * nsys) != cudaSuccess ||
+      cudaMallocHost(&w->h_sysv0, w->cost_bytes()) != cudaSuccess ||
       cudaMallocHost(&w->h_res, sizeof(int) * (nsys + 1)) != cudaSuccess ||
       cudaMallocHost(&w->h_ring, w->ring_cap = 65536 + 256 * (size_t)nsys) != cudaSuccess) {
     delete w;
@@ -1382,23 +1399,11 @@ static int finish_deferred(ua_mesh* m, std::vector<int>& its) {
   for (int s = 0; s < w->nsys; ++s) its[s] = its[s] ? w->h_res[s] : 0;
   return UA_OK;
 }
-// The phases of a Newton step are timed on the stream: the host only enqueues them and waits once, for the
-// costs at its end.
-static int phase_mark(ua_mesh* m, int k) {
-  cudaEvent_t& e = m->work->phase[k];
-  if (!e) UA_CUDA_TRY(cudaEventCreate(&e));
-  UA_CUDA_TRY(cudaEventRecord(e, m->stream));
-  return UA_OK;
-}
-// adds the times of a step whose stream has drained since its last mark
-static int phase_times(ua_mesh* m, double& t_asm, double& t_sol) {
-  const cudaEvent_t* e = m->work->phase;
-  float a = 0, b = 0;
-  UA_CUDA_TRY(cudaEventElapsedTime(&a, e[0], e[1]));
-  UA_CUDA_TRY(cudaEventElapsedTime(&b, e[1], e[2]));
-  t_asm += a;
-  t_sol += b;
-  return UA_OK;
+// Adds the times of a step whose costs have come back: of its assembly, if it had one, and its linear solve.
+static void phase_times(const Work* w, bool assembled, double& t_asm, double& t_sol) {
+  const unsigned long long* t = (const unsigned long long*)(w->h_sysv + SV_COUNT * (size_t)w->nsys);
+  if (assembled) t_asm += 1e-6 * (double)(t[1] - t[0]);
+  t_sol += 1e-6 * (double)(t[2] - t[1]);
 }
 // Enqueues the counts of a resident solve for finish_deferred.
 static int defer_result(ua_mesh* m) {
@@ -1443,10 +1448,9 @@ static int cost_eval(ua_mesh* m, const ua_params* p, bool useDir, bool assembleR
     if (rc) return rc;
   }
   const double* gamma = useDir && !atX ? w->gamma : nullptr;
-  launch_cost(m, gamma, false);
+  launch_cost(m, gamma, false, atX ? w->stamp + 2 : nullptr);  // at X: the first launch after the linear solve
   UA_CUDA_TRY(cudaGetLastError());
-  UA_CUDA_TRY(cudaMemcpyAsync(host ? host : w->h_sysv, w->sysv, SV_COUNT * w->nsys * sizeof(double),
-                              cudaMemcpyDeviceToHost, m->stream));
+  UA_CUDA_TRY(cudaMemcpyAsync(host ? host : w->h_sysv, w->sysv, w->cost_bytes(), cudaMemcpyDeviceToHost, m->stream));
   if (wait) UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
   return UA_OK;
 }
@@ -1957,7 +1961,6 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
     for (int s = 0; s < nsys; ++s) sel[s] = st[s].active ? 1 : 0;
     if ((rc = set_sel(m, sel))) return rc;
     // R and K (:197-213); the interval criterion 1 (default) always refreshes K
-    if ((rc = phase_mark(m, 0))) return rc;
     bool refreshK = false;
     for (int s = 0; s < nsys; ++s)
       if (st[s].active && (((st[s].iteration - 1) % std::max(1, p->ModifiedNRuvIntervalCriterion)) == 0 ||
@@ -1972,6 +1975,7 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
       n_fresh += sel[s] && !asel[s];
       st[s].kfresh = false;
     }
+    if (n_asm > 0) k_stamp<<<1, 32, 0, m->stream>>>(w->stamp), ++g_launches;
     if (n_fresh == 0) {
       if ((rc = assemble(m, p, refreshK, false, w->X, false))) return rc;
     } else if (n_asm > 0) {  // only the systems whose K and R were not assembled ahead
@@ -1979,8 +1983,8 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
       if ((rc = assemble(m, p, refreshK, false, w->X, false))) return rc;
       if ((rc = set_sel(m, sel))) return rc;
     }
-    k_frhs<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->R, w->dof_con, w->lam, w->frhs, w->con_dof, con_pairs(w)), ++g_launches;
-    if ((rc = phase_mark(m, 1))) return rc;
+    k_frhs<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->R, w->dof_con, w->lam, w->frhs, w->con_dof, con_pairs(w),
+                                            w->stamp + 1), ++g_launches;
     // linear solve (:242-257); a resident solve is not waited for: its counts come with the costs
     std::vector<double> eta(nsys);
     for (int s = 0; s < nsys; ++s) eta[s] = forcing_term(p, st[s].rForce);
@@ -1990,7 +1994,6 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
     rc = linear_solve(m, p, its, eta.data());
     w->defer = false;
     if (rc) return rc;
-    if ((rc = phase_mark(m, 2))) return rc;
     // gamma=0 (:260-283): R at X is the residual assembled with K above.  Only the first iteration
     // decides on it before gamma = 1 is evaluated; else the two costs come back together.
     bool first = false;
@@ -2018,7 +2021,7 @@ static int newton_step(ua_mesh* m, const ua_params* p, std::vector<ua_newton_rep
     if ((rc = cost_eval(m, p, true, true, ahead))) return rc;
     if (!first) cost0();
     if ((rc = finish_deferred(m, its))) return rc;
-    if ((rc = phase_times(m, t_asm, t_sol))) return rc;
+    phase_times(w, n_asm > 0, t_asm, t_sol);
     for (int s = 0; s < nsys; ++s)
       if (solved[s]) {
         st[s].kits = its[s];
@@ -2990,8 +2993,7 @@ static int cost_eval_uvh(ua_mesh* m, const ua_params* p, bool assembleR = true, 
   }
   launch_cost(m, w->gamma, false);
   UA_CUDA_TRY(cudaGetLastError());
-  UA_CUDA_TRY(cudaMemcpyAsync(host ? host : w->h_sysv, w->sysv, SV_COUNT * w->nsys * sizeof(double), cudaMemcpyDeviceToHost,
-                              m->stream));
+  UA_CUDA_TRY(cudaMemcpyAsync(host ? host : w->h_sysv, w->sysv, w->cost_bytes(), cudaMemcpyDeviceToHost, m->stream));
   if (wait) UA_CUDA_TRY(cudaStreamSynchronize(m->stream));
   return UA_OK;
 }
@@ -3053,10 +3055,10 @@ static int newton_run_uvh(ua_mesh* m, const ua_params* p, std::vector<ua_newton_
     if (!any) break;
     for (int s = 0; s < nsys; ++s) sel[s] = st[s].active ? 1 : 0;
     if ((rc = set_sel(m, sel))) return rc;
-    if ((rc = phase_mark(m, 0))) return rc;
+    k_stamp<<<1, 32, 0, m->stream>>>(w->stamp), ++g_launches;
     if ((rc = assemble_uvh(m, p, true, false, false, false))) return rc;  // :127
-    k_frhs<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->R, w->dof_con, w->lam, w->frhs, w->con_dof, con_pairs(w)), ++g_launches;
-    if ((rc = phase_mark(m, 1))) return rc;
+    k_frhs<<<w->nrb, 256, 0, m->stream>>>(w->rb_start, w->rb_sys, w->sel, w->R, w->dof_con, w->lam, w->frhs, w->con_dof, con_pairs(w),
+                                            w->stamp + 1), ++g_launches;
     for (int s = 0; s < nsys; ++s) its[s] = sel[s] ? std::max(1, st[s].kits) : 0;
     std::vector<double> eta(nsys);
     for (int s = 0; s < nsys; ++s) eta[s] = forcing_term_uvh(p, st[s].rForce == INFINITY ? 1.0 : st[s].rForce);
@@ -3068,7 +3070,7 @@ static int newton_run_uvh(ua_mesh* m, const ua_params* p, std::vector<ua_newton_
       w->defer = false;
       if (rc) return rc;
     }
-    if ((rc = phase_mark(m, 2))) return rc;
+    k_stamp<<<1, 32, 0, m->stream>>>(w->stamp + 2), ++g_launches;
     // r0 = func(0), r1 = func(1) (:155-156); the two come back together, with the iteration counts
     for (int g1 = 0; g1 < 2; ++g1) {
       for (int s = 0; s < nsys; ++s) gam[s] = (double)g1;
@@ -3077,7 +3079,7 @@ static int newton_run_uvh(ua_mesh* m, const ua_params* p, std::vector<ua_newton_
       if ((rc = cost_eval_uvh(m, p, g1 != 0, g1 ? nullptr : w->h_sysv0, g1 != 0))) return rc;
     }
     if ((rc = finish_deferred(m, its))) return rc;
-    if ((rc = phase_times(m, t_asm, t_sol))) return rc;
+    phase_times(w, true, t_asm, t_sol);
     for (int s = 0; s < nsys; ++s) {
       if (!sel[s]) continue;
       UvhSys& S = st[s];
@@ -3505,8 +3507,6 @@ extern "C" void ua_mesh_destroy(ua_mesh* m) {
     if (w->h_res) cudaFreeHost(w->h_res);
     if (w->h_ring) cudaFreeHost(w->h_ring);
     if (w->h_nan) cudaFreeHost(w->h_nan);
-    for (cudaEvent_t e : w->phase)
-      if (e) cudaEventDestroy(e);
     delete w;
   }
   amg_free(m->amg);
