@@ -427,6 +427,9 @@ int ua_uv_adjoint_dIdC(ua_mesh* m, const ua_params* p, const ua_fields* F, const
  * enabled = 0 in the release build. */
 int ua_debug_bounds(const ua_mesh* m, int32_t* enabled, int32_t* site, int64_t* index);
 int ua_debug_sites(const ua_mesh* m, int32_t* enabled, uint64_t* sites);
+/* Debug build: the barrier of a resident solve's team of two CTAs, of which `ctas` (1 or 2) take part, with a
+ * wait of microseconds instead of seconds.  UA_OK, or UA_ERR_TIMEOUT as from a solve whose team did not meet. */
+int ua_debug_team_wait(const ua_mesh* m, int32_t ctas);
 
 /* Free and total device memory (admission by free HBM). */
 int ua_mem_info(int32_t device, int64_t* free_bytes, int64_t* total_bytes);

@@ -164,6 +164,7 @@ int gmres_resident(ua_mesh* m, const GmSolve& v, const std::vector<int>& sel, co
                    long long* launches);
 // device flag set by a resident solve whose team did not meet
 const int* resident_error_flag(const ua_mesh* m);
+int resident_error(int flag);  // UA_OK, or the error of a set flag
 // pass classes of a profiled resident solve: operator, finest restriction, finest up pass, rest
 int pcg_resident_status(ua_mesh* m, bool prof, double* ms, int* cnt);
 

@@ -76,7 +76,7 @@ struct TeamCtx {
 // every thread and the kernel ends with an error status.
 constexpr unsigned kTeamSpinLimit = 1u << 24;
 // f: run by one thread of another warp meanwhile.
-template <typename F>
+template <unsigned LIMIT = kTeamSpinLimit, typename F>
 __device__ __forceinline__ bool team_sync(TeamCtx& t, F f) {
   __syncthreads();
   if (threadIdx.x == 32) f();
@@ -88,7 +88,7 @@ __device__ __forceinline__ bool team_sync(TeamCtx& t, F f) {
     t.target += t.size;
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
     int ok = 0;
-    for (unsigned i = 0; i < kTeamSpinLimit; ++i) {
+    for (unsigned i = 0; i < LIMIT; ++i) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(t.bar) : "memory");
       if ((int)(v - t.target) >= 0) {

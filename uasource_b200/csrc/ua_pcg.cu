@@ -893,7 +893,20 @@ int pcg_resident(ua_mesh* m, const PcgSolve& v, const std::vector<int>& sel, con
   return rc;
 }
 
+#ifdef UA_BOUNDS_CHECK
+// Two CTAs' barrier, met by as many as are launched, with a wait of some microseconds.
+__global__ void k_team_probe(unsigned* bar, int* err) {
+  __shared__ int ok;
+  TeamCtx t{(int)blockIdx.x, 2, bar, 0u, &ok, nullptr};
+  if (!team_sync<4096>(t, []() {}) && threadIdx.x == 0) *err = 1;
+}
+#endif
+
 const int* resident_error_flag(const ua_mesh* m) { return m->amg->cyc.d_sched; }
+
+int resident_error(int flag) {
+  return flag ? set_error(UA_ERR_TIMEOUT, "resident solve: a team barrier was not met") : UA_OK;
+}
 
 // After the solve's stream has drained: whether every barrier was met, and the pass times (ms of
 // the whole grid) and counts of a profiled solve.
@@ -901,7 +914,7 @@ int pcg_resident_status(ua_mesh* m, bool prof, double* ms, int* cnt) {
   Cycle& C = m->amg->cyc;
   int err = 0;
   UA_CUDA_TRY(dev_read(m, &err, C.d_sched, sizeof(int)));
-  if (err) return set_error(UA_ERR_TIMEOUT, "resident solve: a team barrier was not met");
+  if (int rc = resident_error(err)) return rc;
   if (prof) {
     unsigned long long h[2 * CP_COUNT];
     UA_CUDA_TRY(dev_read(m, h, C.d_prof, sizeof(h)));
@@ -914,3 +927,25 @@ int pcg_resident_status(ua_mesh* m, bool prof, double* ms, int* cnt) {
 }
 
 }  // namespace ua
+
+extern "C" int ua_debug_team_wait(const ua_mesh* m, int32_t ctas) {
+  using namespace ua;
+  if (!m || ctas < 1 || ctas > 2) return set_error(UA_ERR_INVALID, "ua_debug_team_wait: bad argument");
+#ifdef UA_BOUNDS_CHECK
+  UA_CUDA_TRY(cudaSetDevice(m->device));
+  int* d = nullptr;  // flag, barrier counter
+  UA_CUDA_TRY(cudaMalloc(&d, 2 * sizeof(int)));
+  int flag = 0;
+  cudaError_t e = dev_clear(m, d, 2 * sizeof(int));
+  unsigned* bar = (unsigned*)d + 1;
+  void* args[] = {&bar, &d};
+  if (e == cudaSuccess)
+    e = cudaLaunchCooperativeKernel((const void*)k_team_probe, dim3(ctas), dim3(kCycThreads), args, 0, m->stream);
+  if (e == cudaSuccess) e = dev_read(m, &flag, d, sizeof(int));
+  cudaFree(d);
+  UA_CUDA_TRY(e);
+  return resident_error(flag);
+#else
+  return set_error(UA_ERR_INVALID, "ua_debug_team_wait: in the debug build only");
+#endif
+}

@@ -1395,7 +1395,7 @@ static int finish_deferred(ua_mesh* m, std::vector<int>& its) {
   Work* w = m->work;
   if (!w->deferred) return UA_OK;
   w->deferred = false;
-  if (w->h_res[w->nsys]) return set_error(UA_ERR_TIMEOUT, "resident solve: a team barrier was not met");
+  if (int rc = resident_error(w->h_res[w->nsys])) return rc;
   for (int s = 0; s < w->nsys; ++s) its[s] = its[s] ? w->h_res[s] : 0;
   return UA_OK;
 }

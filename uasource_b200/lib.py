@@ -191,6 +191,7 @@ SIGNATURES = {
     "ua_constraint_matrix": (C.c_int, [C.c_void_p, C.POINTER(ua_bcs), _ip, _ip, _dp, _dp]),
     "ua_serve_cancel": (C.c_int, [C.c_void_p, C.c_int32, _ip]),
     "ua_debug_bounds": (C.c_int, [C.c_void_p, _ip, _ip, _lp]),
+    "ua_debug_team_wait": (C.c_int, [C.c_void_p, C.c_int32]),
     "ua_debug_sites": (C.c_int, [C.c_void_p, _ip, C.POINTER(C.c_uint64)]),
     "ua_autotune": (C.c_int, [C.c_void_p, C.POINTER(ua_params), C.POINTER(ua_fields), C.c_int32, C.c_int32,
                               C.POINTER(ua_tune_report)]),
