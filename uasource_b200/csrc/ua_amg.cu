@@ -77,8 +77,8 @@ static int aggregate(int n, const std::vector<int>& ptr, const std::vector<int>&
 }
 
 // Linear interpolation of a six-node system from its corner nodes: per node its corners (ascending
-// corner ids) and weights, 1 at a corner and 1/2 at the two ends of a mid node's edge.  Corner ids
-// follow the node order.  Returns the number of corners, or 0 where the mesh does not allow it (a
+// corner ids, and their nodes) and weights, 1 at a corner and 1/2 at the two ends of a mid node's edge.  Corner
+// ids follow the node order.  Returns the number of corners, or 0 where the mesh does not allow it (a
 // node that is a corner of one element and a mid node of another, or in no element).
 //
 // A quadratic mesh is coarsened this way once, before the aggregation: the velocity tangent's
@@ -87,7 +87,7 @@ static int aggregate(int n, const std::vector<int>& ptr, const std::vector<int>&
 // quadratic graph gave 22) and the coarsening ratio is 4 instead of 16.  PCG iterations of one
 // Newton system (relative 1e-6): 101 x 51 vertices 108 -> 39, with the damped smoother below 80 -> 30.
 static int linear_corners(const HostSystem& hs, std::vector<int>& ptr, std::vector<int>& col,
-                          std::vector<double>& wgt) {
+                          std::vector<int>& node, std::vector<double>& wgt) {
   const int n = hs.nn, ne = hs.ne;
   std::vector<int> c0(n, -1), c1(n, -1);  // a mid node's edge ends; c0 = the node itself at a corner
   for (int e = 0; e < ne; ++e)
@@ -110,15 +110,19 @@ static int linear_corners(const HostSystem& hs, std::vector<int>& ptr, std::vect
   ptr.assign(1, 0);
   ptr.reserve(n + 1);
   col.clear();
+  node.clear();
   wgt.clear();
   for (int i = 0; i < n; ++i) {
     if (c1[i] < 0) {
       col.push_back(id[i]);
+      node.push_back(i);
       wgt.push_back(1.0);
     } else {
       if (id[c0[i]] < 0 || id[c1[i]] < 0) return 0;  // an edge end that is a mid node elsewhere
       col.push_back(id[c0[i]]);
       col.push_back(id[c1[i]]);
+      node.push_back(c0[i]);
+      node.push_back(c1[i]);
       wgt.push_back(0.5);
       wgt.push_back(0.5);
     }
@@ -174,16 +178,17 @@ static int amg_build(ua_mesh* m, bool smoothed) {
   std::vector<std::vector<int>> g_off{m->h_node_off}, g_ptr{m->h_nodeptr}, g_col{m->h_nodecol}, g_agg;
   // smoothed aggregation lists per transfer (index = fine level)
   std::vector<std::vector<int>> g_pnp, g_pnc, g_apnp, g_apnc, g_ptnp, g_ptnf, g_ptnk;
-  std::vector<double> pn_w;  // weights of the finest level's linear interpolation (else empty)
+  std::vector<double> pn_w;  // weights of the finest level's linear interpolation (else empty),
+  std::vector<int> pn_f;     // and the corner nodes they are for
   a->sa = smoothed;
   // quadratic meshes: the first transfer interpolates linearly from the corner nodes, for every
   // system of the handle or for none
-  std::vector<std::vector<int>> lin_ptr(nsys), lin_col(nsys);
+  std::vector<std::vector<int>> lin_ptr(nsys), lin_col(nsys), lin_f(nsys);
   std::vector<std::vector<double>> lin_w(nsys);
   std::vector<int> lin_n(nsys, 0);
   bool linear0 = smoothed && m->nod == 6;
   for (int s = 0; s < nsys && linear0; ++s)
-    linear0 = (lin_n[s] = linear_corners(m->sys[s], lin_ptr[s], lin_col[s], lin_w[s])) > 0;
+    linear0 = (lin_n[s] = linear_corners(m->sys[s], lin_ptr[s], lin_col[s], lin_f[s], lin_w[s])) > 0;
   std::vector<char> live(nsys, 1);
   auto fail = [&](const char* why) {
     delete a;
@@ -229,6 +234,7 @@ static int amg_build(ua_mesh* m, bool smoothed) {
           lpn = lin_ptr[s];
           lpc = lin_col[s];
           pn_w.insert(pn_w.end(), lin_w[s].begin(), lin_w[s].end());
+          for (int f : lin_f[s]) pn_f.push_back(no[s] + f);
         }
         for (int i = 0; i < n && !lin; ++i) {
           const size_t b0 = lpc.size();
@@ -416,7 +422,10 @@ static int amg_build(ua_mesh* m, bool smoothed) {
       AmgLevel& F = a->lev[l];
       const AmgLevel& C = a->lev[l + 1];
       F.sa_agg = upload(m, a, g_agg[l], ok);
-      if (l == 0 && linear0) F.pn_w = upload(m, a, pn_w, ok);
+      if (l == 0 && linear0) {
+        F.pn_w = upload(m, a, pn_w, ok);
+        F.pn_f = upload(m, a, pn_f, ok);
+      }
       F.pn_ptr = upload(m, a, g_pnp[l], ok);
       F.pn_col = upload(m, a, g_pnc[l], ok);
       F.apn_ptr = upload(m, a, g_apnp[l], ok);
@@ -1089,7 +1098,9 @@ __global__ void __launch_bounds__(1024) k_sa_scan(long long n, unsigned* v, unsi
 // Smoother diagonal and prolongator rows of fine node g, kSaGL lanes per node: the damped l1 diagonal
 // invd = kSmoothOmega / sum |a| over unmasked columns (0 on masked or empty rows) with its square root
 // sc and, in slice order, its inverse dw for the collapsed cycle; and P(g,:) = P0 - w/l1 A P0 on
-// unmasked rows and columns, or the linear interpolation pn_w.  The row's entries are staged in shared
+// unmasked rows and columns, or the linear interpolation pn_w from the unmasked ones of the corners pn_f: a
+// masked corner's error is zero, and where a mid node lies between two of them their columns alone would make
+// the coarse operator singular (a 2x2 mesh with its sides held: 40206 iterations instead of 29).  The row's entries are staged in shared
 // memory with their neighbours' aggregates; a lane owns an entry of P and takes the neighbours of its
 // aggregate in row order.  ST: the type of the sums (FP32 in the mixed-precision form, else FP64).
 // One pass over the row instead of an l1 kernel, a scattered P, a repacking and the scaling: latency on
@@ -1101,7 +1112,7 @@ template <typename KT, typename VT, typename QT>
 __global__ void __launch_bounds__(128) k_sa_P(int nf, const int4* nrow, const int* dof_off, const int* node_off,
                                               const int* colind, const KT* A, const unsigned char* mask,
                                               const int* agg, const int* pn_ptr, const int* pn_col,
-                                              const double* pn_w, QT* Q, VT* invd, double2* sc, VT* dw,
+                                              const double* pn_w, const int* pn_f, QT* Q, VT* invd, double2* sc, VT* dw,
                                               const int* ipos, const int* sel, const int* psel) {
   using ST = KT;
   __shared__ ST sv[128 / kSaGL][4][kSaStage];
@@ -1182,7 +1193,11 @@ __global__ void __launch_bounds__(128) k_sa_P(int nf, const int4* nrow, const in
   for (int t0 = 0; t0 < dP; t0 += kSaGL) {
     const int t = t0 + lane;
     if (pn_w) {  // the same weights for both components, no smoothing
-      if (t < dP) pq_set(Q + pr + t, m0 ? 0.0 : pn_w[pr + t], 0.0, 0.0, m1 ? 0.0 : pn_w[pr + t]);
+      if (t < dP) {
+        const int j0 = d0 + (pn_f[pr + t] - no), j1 = j0 + nn;
+        pq_set(Q + pr + t, m0 || (mask && mask[j0]) ? 0.0 : pn_w[pr + t], 0.0, 0.0,
+               m1 || (mask && mask[j1]) ? 0.0 : pn_w[pr + t]);
+      }
       continue;
     }
     const int J = t < dP ? pn_col[pr + t] : -1;
@@ -1536,7 +1551,7 @@ static int numeric_t(ua_mesh* m, const int* rowptr0, const int* colind0, const K
       KT* APv = (KT*)F.sa_ap;
       QT* Qv = (QT*)(sizeof(KT) == 4 ? F.sa_qh : F.sa_qd);
       k_sa_P<KT, VT, QT><<<grid((long long)F.nn * kSaGL, 128), 128, 0, st>>>(
-          F.nn, F.nrow, F.d_dof_off, F.d_node_off, ci, A, mk, F.sa_agg, F.pn_ptr, F.pn_col, F.pn_w, Qv, (VT*)F.invd,
+          F.nn, F.nrow, F.d_dof_off, F.d_node_off, ci, A, mk, F.sa_agg, F.pn_ptr, F.pn_col, F.pn_w, F.pn_f, Qv, (VT*)F.invd,
           cyc ? a->cyc.lev[l].sc : nullptr, cyc && l == 0 ? (VT*)cyc->dw : nullptr, a->cyc.d_ipos, sel, psel),
           ++*launches;
       if (cyc && l == 0) {  // the finest level's slice values need its diagonal only

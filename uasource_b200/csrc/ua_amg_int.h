@@ -53,7 +53,9 @@ struct AmgLevel {
   // smoothed aggregation, transfer from this level to the next (node-level lists, global ids):
   // pn: fine node -> coarse nodes of its neighbours' aggregates (the prolongator's node pattern);
   // apn: fine node -> coarse nodes of A P; ptn: coarse node -> (fine node, position in pn)
-  double* pn_w = nullptr;  // interpolation weights in pn order (the finest level of a quadratic mesh), else null
+  // interpolation weights in pn order and the corner nodes (the finest level of a quadratic mesh), else null
+  double* pn_w = nullptr;
+  int* pn_f = nullptr;
   int *sa_agg = nullptr, *pn_ptr = nullptr, *pn_col = nullptr, *apn_ptr = nullptr, *apn_col = nullptr;
   int *ptn_ptr = nullptr, *ptn_fine = nullptr, *ptn_k = nullptr;
   // lists of the set-up (sa_lists): per node {first entry of its u row, of its v row, degree, system};
