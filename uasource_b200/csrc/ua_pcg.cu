@@ -4,7 +4,7 @@
 // What bounds the inner solve of a mesh up to some 100,000 nodes is not memory but the chain of
 // short passes: with one launch per pass a PCG step of the 141x71 mesh took 72 us in 19 launches
 // of about 3.8 us.  Here a step is 1 + 2 L passes for the L levels above the dense one and the solo
-// ones (20 us on that mesh), a team barrier costs 1.25 us whatever the team's size, nothing is
+// ones (22 us on that mesh), a team barrier costs 1.25 us whatever the team's size, nothing is
 // launched inside the solve, the systems of a batch do not wait for one another and the host neither
 // checks nor over-runs the convergence.  With a launch per pass and with the resident kernel as it
 // was first built, one B200: uv P1 141x71 FP64 25.8 and 12.9 ms, P2 101x51 mixed 41.6 and 21.6 ms, P2
